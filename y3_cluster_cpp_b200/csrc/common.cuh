@@ -361,20 +361,7 @@ struct NfwUnit<float> {
 // centre, (1/pi) int_0^pi dth DSigma(d) (2 a^2 / d^2 - 1) with
 // d^2 = x^2 + x_mis^2 - 2 x x_mis cos th, a = x - x_mis cos th.  Returns the
 // sum over the GL nodes t0, t0 + dt, ... of [0, pi] (without the 1/pi), so
-// a warp can split the nodes.  The _cos form takes cos(theta) of the nodes.
-__device__ __forceinline__ double
-dsigma_single_partial_cos(const double* cth, const double* wth, int n, double x, double xm,
-                          int t0, int dt)
-{
-  double acc = 0.0;
-  for (int t = t0; t < n; t += dt) {
-    const double ct = cth[t];
-    const double d2 = x * x + xm * xm - 2.0 * x * xm * ct, a = x - xm * ct;
-    acc += wth[t] * NfwUnit<double>::dsigma(sqrt(d2)) * (2.0 * a * a / d2 - 1.0);
-  }
-  return acc;
-}
-
+// a warp can split the nodes.
 __device__ __forceinline__ double
 dsigma_single_partial(const double* th, const double* wth, int n, double x, double xm, int t0,
                       int dt)

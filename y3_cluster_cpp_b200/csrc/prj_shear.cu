@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "host_common.h"
+#include "nfw_table.cuh"
 #include "zkernel_table.h"
 
 namespace y3b {
@@ -122,9 +123,25 @@ struct PrjTables {
   const double *xr, *xz, *xi;    // xi_nl r, z, xi [n_xz][n_xr]
   int n_lx, n_lxm;
   const double *lx, *lxm, *ltab; // single-kernel table (n_lx = 0: quadrature)
-  int n_th;
-  const double *th, *wth;        // cos(theta) and weights of the GL nodes on [0, pi]
   double omega_m;
+};
+
+// The fixed-offset profile without a table: the 256-node GL rule over the
+// ring angle, and the 32, 64 and 128-node rules that give the same ring
+// average to FP64 rounding where the ring keeps clear of the offset centre.
+// At ring angle t the integrand has its nearest singularity (d = 0) at
+// t = i ln(x_mis / x), so an m-node rule on [0, pi] converges as
+// rho_E^-2m with rho_E = a + sqrt(a^2 - 1), a = exp(asinh(|ln(x_mis / x)| / pi)):
+// 1e-18 from the |ln| below on.  In 24-node theta grids over two decades
+// the rules average about 50 nodes a ring.
+constexpr int kRuleN0 = 32, kRuleN1 = 64, kRuleN2 = 128, kRuleN3 = 256;
+constexpr int kRuleTot = kRuleN0 + kRuleN1 + kRuleN2 + kRuleN3;
+constexpr double kRuleLn0 = 0.609, kRuleLn1 = 0.1587, kRuleLn2 = 0.0401;
+
+struct PrjQuad {
+  const double* rule;    // cos(t) [kRuleTot] | weights [kRuleTot] of the GL nodes on [0, pi]
+  const double* mass;    // 1 / r_s^2 [n_lnm] | profile amplitude without Omega_M [n_lnm]
+  const double* nfw;     // DeltaSigma polynomials
 };
 
 __device__ __forceinline__ double
@@ -134,19 +151,15 @@ hmf_dev(const PrjTables& T, double lnM, double z)
          (T.hmf_s * (lnM * kLog10e - kHmfPivot) + T.hmf_q);
 }
 
-// NFW_DSIGMA_MIS(R, R_mis, lnM), single kernel (nfw_dsigma_mis.hh:95-114):
-// r_s from rho_c, amplitude 2 r_s delta_c rho_c Omega_M 1e-12 [h Msun/pc^2].
+// NFW_DSIGMA_MIS(R, R_mis, lnM), single kernel (nfw_dsigma_mis.hh:95-114),
+// from its table: r_s from rho_c, amplitude 2 r_s delta_c rho_c Omega_M
+// 1e-12 [h Msun/pc^2].
 __device__ double
-dsigma_single(const PrjTables& T, double R, double Rmis, double lnM)
+dsigma_single_table(const PrjTables& T, double R, double Rmis, double lnM)
 {
   const double rs = nfw_rs(lnM, kConc, kRhoCrit);
-  const double x = R / rs, xm = Rmis / rs;
-  double unit;
-  if (T.n_lx) {
-    unit = exp(interp2d_clamp(T.lx, T.n_lx, T.lxm, T.n_lxm, T.ltab, log(x), log(xm)));
-  } else {  // mean tangential shear on the circle x around the offset centre
-    unit = dsigma_single_partial_cos(T.th, T.wth, T.n_th, x, xm, 0, 1) / kPiP;
-  }
+  const double unit = exp(
+    interp2d_clamp(T.lx, T.n_lx, T.lxm, T.n_lxm, T.ltab, log(R / rs), log(Rmis / rs)));
   return nfw_norm(lnM, kConc, kRhoCrit) * T.omega_m * unit;
 }
 
@@ -205,19 +218,88 @@ prj_psi_kernel(PrjTables T, int n_theta_tot, const int* tslice, const double* th
 }
 
 // The single-kernel profile DSigma_mis(R | theta D_A, M) of every (grid
-// point, theta node of its slice, mass node): one thread each, written to
-// V[g][(it - t0) n_lnm + iM] (max_pairs per grid point).
+// point, theta node of its slice, mass node), written to
+// V[g][(it - t0) n_lnm + iM] (max_pairs per grid point): from the table, one
+// thread per value.
 __global__ void __launch_bounds__(256)
-prj_profile_kernel(PrjTables T, int n_lnm, const double* lnm_x, const int* gp_slice,
-                   const double* gp_R, const int* t0, const double* theta, const double* DA,
-                   int max_pairs, double* V)
+prj_profile_table_kernel(PrjTables T, int n_lnm, const double* lnm_x, const int* gp_slice,
+                         const double* gp_R, const int* t0, const double* theta,
+                         const double* DA, int max_pairs, double* V)
 {
   const int g = blockIdx.y, sl = gp_slice[g];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int n_pairs = (t0[sl + 1] - t0[sl]) * n_lnm;
   if (k >= n_pairs) return;
   const int it = t0[sl] + k / n_lnm, iM = k % n_lnm;
-  V[(size_t)g * max_pairs + k] = dsigma_single(T, gp_R[g], theta[it] * DA[sl], lnm_x[iM]);
+  V[(size_t)g * max_pairs + k] =
+    dsigma_single_table(T, gp_R[g], theta[it] * DA[sl], lnm_x[iM]);
+}
+
+// One warp's ring average of NJ nodes a lane, for all masses: the mean
+// tangential shear on the circle of radius R around the offset centre,
+// (1/pi) int dt DSigma(d / r_s) (2 a^2 / d^2 - 1), d^2 = R^2 + Rm^2 -
+// 2 R Rm cos t, a = R - Rm cos t.  The geometry is shared by the masses,
+// which only scale d; eight masses accumulate side by side and are summed
+// over the lanes by halving exchanges (nine 64-bit shuffles for eight sums).
+template <int NJ>
+__device__ __forceinline__ void
+ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double Rm, int n_lnm,
+            double omega_m, int lane, double* __restrict__ out)
+{
+  double D2[NJ], A[NJ];
+  const double s2 = R * R + Rm * Rm, c2 = 2.0 * R * Rm;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const double ct = rule[lane + 32 * j], a = R - Rm * ct;
+    D2[j] = s2 - c2 * ct;
+    A[j] = rule[kRuleTot + lane + 32 * j] * (2.0 * a * a / D2[j] - 1.0) / kPiP;
+  }
+  for (int k0 = 0; k0 < n_lnm; k0 += 8) {
+    double acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const double q = __ldg(Q.mass + min(k0 + u, n_lnm - 1));
+      acc[u] = 0.0;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) acc[u] += A[j] * nfw_dsigma_w(Q.nfw, D2[j] * q);
+    }
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) {
+      const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+      for (int u = 0; u < h; ++u) {
+        const double send = up ? acc[u] : acc[u + h];
+        acc[u] = (up ? acc[u + h] : acc[u]) + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+      }
+    }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    const int k = k0 + (lane >> 2);
+    if ((lane & 3) == 0 && k < n_lnm) out[k] = Q.mass[n_lnm + k] * omega_m * acc[0];
+  }
+}
+
+// The same values by quadrature, one warp per (grid point, theta node): the
+// lanes take the ring's nodes, so the profile's table reads of a warp fall
+// on few, neighbouring segments.
+__global__ void __launch_bounds__(256)
+prj_profile_kernel(PrjQuad Q, double omega_m, int n_lnm, const int* gp_slice,
+                   const double* gp_R, const int* t0, const double* theta, const double* DA,
+                   int max_pairs, double* V)
+{
+  const int g = blockIdx.y, sl = gp_slice[g], lane = threadIdx.x & 31;
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= t0[sl + 1] - t0[sl]) return;
+  const double R = gp_R[g], Rm = theta[t0[sl] + i] * DA[sl], lr = fabs(log(Rm / R));
+  double* out = V + (size_t)g * max_pairs + (size_t)i * n_lnm;
+  if (lr >= kRuleLn0)
+    ring_masses<1>(Q, Q.rule, R, Rm, n_lnm, omega_m, lane, out);
+  else if (lr >= kRuleLn1)
+    ring_masses<2>(Q, Q.rule + kRuleN0, R, Rm, n_lnm, omega_m, lane, out);
+  else if (lr >= kRuleLn2)
+    ring_masses<4>(Q, Q.rule + kRuleN0 + kRuleN1, R, Rm, n_lnm, omega_m, lane, out);
+  else
+    ring_masses<8>(Q, Q.rule + kRuleN0 + kRuleN1 + kRuleN2, R, Rm, n_lnm, omega_m, lane, out);
 }
 
 // One block per grid point: the (theta, M) sums of both channels over the
@@ -260,8 +342,8 @@ prj_eval_kernel(int n_lnm, const int* gp_slice, const int* t0, const double* geo
 
 // Device buffers of one evaluation, kept by the handle and grown on demand.
 struct PrjBufs {
-  DevBuf<double> d_mh, d_hz, d_dn, d_bl, d_bz, d_bi, d_xr, d_xz, d_xi, d_lx, d_lxm, d_lt, d_th,
-    d_wth, d_lnx, d_lnw, d_theta, d_geom, d_bsel, d_zz, d_zc, d_chiz, d_thex, d_anchor, d_denom,
+  DevBuf<double> d_mh, d_hz, d_dn, d_bl, d_bz, d_bi, d_xr, d_xz, d_xi, d_lx, d_lxm, d_lt, d_quad,
+    d_lnx, d_lnw, d_theta, d_geom, d_bsel, d_zz, d_zc, d_chiz, d_thex, d_anchor, d_denom,
     d_wcl, d_AB, d_WZ, d_wrnd, d_psi, d_chio, d_zob, d_da, d_sci, d_gpR, d_out, d_V;
   DevBuf<int> d_t0, d_z0, d_ts, d_zs, d_gps;
 };
@@ -286,6 +368,55 @@ struct y3b_prj {
     if (stream) cudaStreamDestroy(stream);
   }
 };
+
+namespace y3b {
+namespace {
+
+// cos(t) [kRuleTot] | weights [kRuleTot] of the ring rules, formed once per
+// process.
+const std::vector<double>&
+ring_rules()
+{
+  static const std::vector<double> rules = [] {
+    std::vector<double> q, w, th, wth;
+    for (int m : {kRuleN0, kRuleN1, kRuleN2, kRuleN3}) {
+      h_gl(0.0, kPiP, m, th, wth);
+      for (double t : th) q.push_back(std::cos(t));
+      w.insert(w.end(), wth.begin(), wth.end());
+    }
+    q.insert(q.end(), w.begin(), w.end());
+    return q;
+  }();
+  return rules;
+}
+
+// The quadrature's constants on the device, once per handle: DeltaSigma
+// polynomials | ring rules | 1 / r_s^2 and the amplitude 2 r_s delta_c rho_c
+// 1e-12 of the mass nodes.
+int
+upload_quad(y3b_prj* h)
+{
+  const int n = h->cfg.n_lnm;
+  const double* nfw = nfw_table_host();
+  std::vector<double> q(nfw, nfw + kNfwSegs * kNfwCoef);
+  q.insert(q.end(), ring_rules().begin(), ring_rules().end());
+  const double delta_c =
+    (200.0 * kConc * kConc * kConc / 3.0) / (std::log(1.0 + kConc) - kConc / (1.0 + kConc));
+  std::vector<double> rs(n);
+  for (int i = 0; i < n; ++i) {
+    rs[i] = std::cbrt(3.0 * std::exp(h->lnm_x[i]) / (800.0 * kPiP * kRhoCrit)) / kConc;
+    q.push_back(1.0 / (rs[i] * rs[i]));
+  }
+  for (int i = 0; i < n; ++i) q.push_back(2.0 * rs[i] * delta_c * kRhoCrit * 1e-12);
+  y3b::DevBuf<double>& d = h->bufs.d_quad;
+  Y3B_TRY(d.upload(q.data(), q.size(), h->stream));
+  const int rc = cuda_status(cudaStreamSynchronize(h->stream), "upload of the ring rules");
+  if (rc) d.reset();
+  return rc;
+}
+
+}  // namespace
+}  // namespace y3b
 
 extern "C" int
 y3b_prj_create(const y3b_prj_config* cfg, y3b_prj** out)
@@ -573,16 +704,12 @@ y3b_prj_eval(y3b_prj* h, const y3b_prj_sample* S, double* out)
   Y3B_TRY(B.d_xz.upload(S->xi_z, S->n_xz, s));
   Y3B_TRY(B.d_xi.upload(S->xi_nl, (size_t)S->n_xr * S->n_xz, s));
   const bool table = !h->tab_lx.empty();
-  std::vector<double> thq, wthq;
   if (table) {
     Y3B_TRY(B.d_lx.upload(h->tab_lx.data(), h->tab_lx.size(), s));
     Y3B_TRY(B.d_lxm.upload(h->tab_lxm.data(), h->tab_lxm.size(), s));
     Y3B_TRY(B.d_lt.upload(h->tab_v.data(), h->tab_v.size(), s));
-  } else {
-    h_gl(0.0, kPiP, 256, thq, wthq);
-    for (double& x : thq) x = std::cos(x);  // the quadrature reads cos(theta) of its nodes
-    Y3B_TRY(B.d_th.upload(thq.data(), thq.size(), s));
-    Y3B_TRY(B.d_wth.upload(wthq.data(), wthq.size(), s));
+  } else if (!B.d_quad.get()) {
+    Y3B_TRY(upload_quad(h));
   }
   Y3B_TRY(B.d_lnx.upload(h->lnm_x.data(), n_lnm, s));
   Y3B_TRY(B.d_lnw.upload(h->lnm_w.data(), n_lnm, s));
@@ -618,8 +745,7 @@ y3b_prj_eval(y3b_prj* h, const y3b_prj_sample* S, double* out)
               S->cosmo.hmf_q, S->n_hl, S->n_hz, B.d_bl.get(), B.d_bz.get(), B.d_bi.get(), S->n_xr,
               S->n_xz, B.d_xr.get(), B.d_xz.get(), B.d_xi.get(),
               table ? (int)h->tab_lx.size() : 0, table ? (int)h->tab_lxm.size() : 0,
-              B.d_lx.get(), B.d_lxm.get(), B.d_lt.get(), table ? 0 : (int)thq.size(), B.d_th.get(),
-              B.d_wth.get(), om};
+              B.d_lx.get(), B.d_lxm.get(), B.d_lt.get(), om};
   if (nz_tot) {
     prj_z_kernel<<<nz_tot, 128, 0, s>>>(T, n_lnm, B.d_lnx.get(), B.d_lnw.get(), B.d_zs.get(),
                                         B.d_zz.get(), B.d_zc.get(), B.d_anchor.get(), B.d_denom.get(),
@@ -641,9 +767,17 @@ y3b_prj_eval(y3b_prj* h, const y3b_prj_sample* S, double* out)
   for (int k = 0; k < nsl; ++k) max_nt = std::max(max_nt, t0[k + 1] - t0[k]);
   const int max_pairs = std::max(max_nt * n_lnm, 1);
   Y3B_TRY(B.d_V.alloc((size_t)ngp * max_pairs));
-  prj_profile_kernel<<<dim3((max_pairs + 255) / 256, ngp), 256, 0, s>>>(
-    T, n_lnm, B.d_lnx.get(), B.d_gps.get(), B.d_gpR.get(), B.d_t0.get(), B.d_theta.get(), B.d_da.get(),
-    max_pairs, B.d_V.get());
+  if (table) {
+    prj_profile_table_kernel<<<dim3((max_pairs + 255) / 256, ngp), 256, 0, s>>>(
+      T, n_lnm, B.d_lnx.get(), B.d_gps.get(), B.d_gpR.get(), B.d_t0.get(), B.d_theta.get(),
+      B.d_da.get(), max_pairs, B.d_V.get());
+  } else {
+    const PrjQuad Q{B.d_quad.get() + kNfwSegs * kNfwCoef,
+                    B.d_quad.get() + kNfwSegs * kNfwCoef + 2 * kRuleTot, B.d_quad.get()};
+    prj_profile_kernel<<<dim3((max_nt + 7) / 8, ngp), 256, 0, s>>>(
+      Q, om, n_lnm, B.d_gps.get(), B.d_gpR.get(), B.d_t0.get(), B.d_theta.get(), B.d_da.get(),
+      max_pairs, B.d_V.get());
+  }
   count_launch();
   Y3B_CUDA(cudaGetLastError());
   prj_eval_kernel<<<ngp, 256, 0, s>>>(n_lnm, B.d_gps.get(), B.d_t0.get(), B.d_geom.get(),
