@@ -66,7 +66,8 @@ build()
       for (int j = 0; j < N; ++j) mono[j] += c * T[k][j];
     }
     long double scale = 1.0L;
-    for (int j = 0; j < N; ++j, scale /= half) out[(size_t)s * N + j] = (double)(mono[j] * scale);
+    for (int j = 0; j < N; ++j, scale /= half)
+      out[((size_t)(j / 2) * kNfwSegs + s) * 2 + j % 2] = (double)(mono[j] * scale);
   }
   return out;
 }

@@ -23,29 +23,28 @@ constexpr int kNfwE0 = -36, kNfwE1 = 22;                   // w in [2^kNfwE0, 2^
 constexpr int kNfwSegs = (kNfwE1 - kNfwE0) << kNfwBits;    // 1856
 constexpr int kNfwCoef = 8;                                // 64 bytes a segment, 116 KB
 
-// Coefficients [kNfwSegs][kNfwCoef], formed once per process.
+// Coefficient pairs [kNfwCoef / 2][kNfwSegs][2], formed once per process:
+// lanes whose w lie on neighbouring segments read neighbouring 16-byte words.
 const double* nfw_table_host();
 
-// The closed form outside the table's range, out of line: the rare path.
-static __device__ __noinline__ double
-nfw_dsigma_closed(double w)
-{
-  return NfwUnit<double>::dsigma(sqrt(w));
-}
-
-// DeltaSigma(sqrt(w)); tab in global memory (16-byte aligned).
+// DeltaSigma(sqrt(w)); tab in global memory (16-byte aligned).  A w outside
+// the range (NaN too) sets `outside`, and the caller evaluates the
+// closed form instead: no call in the inner loops, whose registers would be
+// spilled around it.
 __device__ __forceinline__ double
-nfw_dsigma_w(const double* __restrict__ tab, double w)
+nfw_dsigma_w(const double* __restrict__ tab, double w, bool& outside)
 {
   const int hi = __double2hiint(w);
-  const int seg = (hi >> (20 - kNfwBits)) - ((1023 + kNfwE0) << kNfwBits);
-  if ((unsigned)seg >= (unsigned)kNfwSegs) return nfw_dsigma_closed(w);
+  const int s = (hi >> (20 - kNfwBits)) - ((1023 + kNfwE0) << kNfwBits);
+  outside |= (unsigned)s >= (unsigned)kNfwSegs;
+  const int seg = min((unsigned)s, (unsigned)(kNfwSegs - 1));
   const double m = __hiloint2double((hi & 0xFFFFF) | 0x3FF00000, __double2loint(w));
   const int keep = ((1 << kNfwBits) - 1) << (20 - kNfwBits);
   const double t =
     m - __hiloint2double((hi & keep) | 0x3FF00000 | (1 << (19 - kNfwBits)), 0);
-  const double2* c = reinterpret_cast<const double2*>(tab + (size_t)seg * kNfwCoef);
-  const double2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2), c3 = __ldg(c + 3);
+  const double2* c = reinterpret_cast<const double2*>(tab) + seg;
+  const double2 c0 = __ldg(c), c1 = __ldg(c + kNfwSegs), c2 = __ldg(c + 2 * kNfwSegs),
+                c3 = __ldg(c + 3 * kNfwSegs);
   const double t2 = t * t;
   const double lo = fma(fma(c1.y, t, c1.x), t2, fma(c0.y, t, c0.x));
   const double up = fma(fma(c3.y, t, c3.x), t2, fma(c2.y, t, c2.x));

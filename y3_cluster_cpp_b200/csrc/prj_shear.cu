@@ -235,6 +235,25 @@ prj_profile_table_kernel(PrjTables T, int n_lnm, const double* lnm_x, const int*
     dsigma_single_table(T, gp_R[g], theta[it] * DA[sl], lnm_x[iM]);
 }
 
+// The ring averages with the closed-form profile, for rings that leave the
+// polynomials' range; out of line: the rare path.
+__device__ __noinline__ void
+ring_masses_closed(const PrjQuad& Q, const double* __restrict__ rule, int n, double R, double Rm,
+                   int n_lnm, double omega_m, int lane, double* __restrict__ out)
+{
+  for (int k = 0; k < n_lnm; ++k) {
+    const double q = Q.mass[k];
+    double acc = 0.0;
+    for (int t = lane; t < n; t += 32) {
+      const double ct = rule[t], D2 = R * R + Rm * Rm - 2.0 * R * Rm * ct, a = R - Rm * ct;
+      acc += rule[kRuleTot + t] * (2.0 * a * a / D2 - 1.0) / kPiP *
+             NfwUnit<double>::dsigma(sqrt(D2 * q));
+    }
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane == 0) out[k] = Q.mass[n_lnm + k] * omega_m * acc;
+  }
+}
+
 // One warp's ring average of NJ nodes a lane, for all masses: the mean
 // tangential shear on the circle of radius R around the offset centre,
 // (1/pi) int dt DSigma(d / r_s) (2 a^2 / d^2 - 1), d^2 = R^2 + Rm^2 -
@@ -247,6 +266,7 @@ ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double 
             double omega_m, int lane, double* __restrict__ out)
 {
   double D2[NJ], A[NJ];
+  bool outside = false;
   const double s2 = R * R + Rm * Rm, c2 = 2.0 * R * Rm;
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
@@ -261,7 +281,7 @@ ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double 
       const double q = __ldg(Q.mass + min(k0 + u, n_lnm - 1));
       acc[u] = 0.0;
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[u] += A[j] * nfw_dsigma_w(Q.nfw, D2[j] * q);
+      for (int j = 0; j < NJ; ++j) acc[u] += A[j] * nfw_dsigma_w(Q.nfw, D2[j] * q, outside);
     }
 #pragma unroll
     for (int h = 4; h >= 1; h >>= 1) {
@@ -277,12 +297,14 @@ ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double 
     const int k = k0 + (lane >> 2);
     if ((lane & 3) == 0 && k < n_lnm) out[k] = Q.mass[n_lnm + k] * omega_m * acc[0];
   }
+  if (__any_sync(0xffffffffu, outside))
+    ring_masses_closed(Q, rule, 32 * NJ, R, Rm, n_lnm, omega_m, lane, out);
 }
 
 // The same values by quadrature, one warp per (grid point, theta node): the
 // lanes take the ring's nodes, so the profile's table reads of a warp fall
 // on few, neighbouring segments.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 prj_profile_kernel(PrjQuad Q, double omega_m, int n_lnm, const int* gp_slice,
                    const double* gp_R, const int* t0, const double* theta, const double* DA,
                    int max_pairs, double* V)
