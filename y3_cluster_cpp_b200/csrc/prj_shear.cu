@@ -23,10 +23,12 @@
 // (fixed-offset) kernel: the reference's table when loaded, else its direct
 // quadrature.
 //
-// The grids (a few hundred nodes per slice) are built on the host in FP64 in
-// the reference's order; the z-line-of-sight sums, Psi, and the (theta, M)
-// dot products run on the device, one thread or block per independent sum,
-// each summed in a fixed order.
+// A call copies the sample's tables in one transfer and runs four kernels:
+// prj_slice_kernel (one block per slice: both grids, the line-of-sight sums),
+// prj_psi_kernel (one warp per theta node), prj_profile_kernel (one warp per
+// (grid point, theta node): the profile of every mass, contracted with the
+// slice's mass weights) and prj_sum_kernel (one block per grid point: the
+// theta sums).  Every sum has a fixed order.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -44,53 +46,6 @@ namespace {
 constexpr double kPiP = 3.14159265358979323846;
 constexpr double kConc = 4.0;  // NFW_DSIGMA_MIS(4, RHOC, SINGLE), sigma_prj_frozen_t.hh:71
 
-// ---- host-side interpolation with the reference's (GSL) semantics --------
-int
-h_cell(const double* xs, int n, double x)
-{
-  int lo = 0, hi = n - 1;
-  while (hi > lo + 1) {
-    int m = (lo + hi) / 2;
-    if (xs[m] > x)
-      hi = m;
-    else
-      lo = m;
-  }
-  return lo;
-}
-
-double
-h_lin_clamp(const double* xs, const double* ys, int n, double x)
-{
-  x = std::min(std::max(x, xs[0]), xs[n - 1]);
-  int i = h_cell(xs, n, x);
-  double dx = xs[i + 1] - xs[i];
-  return dx > 0.0 ? ys[i] + (x - xs[i]) / dx * (ys[i + 1] - ys[i]) : 0.0;
-}
-
-bool
-h_lin(const double* xs, const double* ys, int n, double x, double* out)
-{
-  if (!(x >= xs[0] && x <= xs[n - 1])) return false;
-  *out = h_lin_clamp(xs, ys, n, x);
-  return true;
-}
-
-double
-h_bilin_clamp(const double* xs, int nx, const double* ys, int ny, const double* zs, double x,
-              double y)
-{
-  x = std::min(std::max(x, xs[0]), xs[nx - 1]);
-  y = std::min(std::max(y, ys[0]), ys[ny - 1]);
-  int i = h_cell(xs, nx, x), j = h_cell(ys, ny, y);
-  double t = (x - xs[i]) / (xs[i + 1] - xs[i]);
-  double u = (y - ys[j]) / (ys[j + 1] - ys[j]);
-  const double* r0 = zs + (size_t)j * nx + i;
-  const double* r1 = r0 + nx;
-  return (1.0 - t) * (1.0 - u) * r0[0] + t * (1.0 - u) * r0[1] + (1.0 - t) * u * r1[0] +
-         t * u * r1[1];
-}
-
 // Gauss-Legendre nodes on [a, b] (p_operator_cuhre_t.hh:66-95).
 void
 h_gl(double a, double b, int n, std::vector<double>& x, std::vector<double>& w)
@@ -98,32 +53,32 @@ h_gl(double a, double b, int n, std::vector<double>& x, std::vector<double>& w)
   gl_nodes_host(a, b, n, x, w);
 }
 
-double
-omega_z_host(double z)  // OMEGA_Z_DES (omega_z_des.hh:15-33)
-{
-  static const double f1[6] = {0.0, 0.0, 0.0, -0.00262353, 0.01940118, 0.45133063};
-  static const double f2[6] = {1.33647377e+4, 1.35291046e+3, -1.26204891e+2,
-                               -2.83454918e+1, -2.26465905, 3.84958753e-1};
-  static const double f3[6] = {0, 0, -1.88101967, 4.8071839, -4.11424324, 1.18196785};
-  const double* c = z < 0.504 ? f1 : (z < 0.7 ? f2 : f3);
-  const double x = z < 0.504 ? z : (z < 0.7 ? z - 0.6 : z);
-  double out = 0.0;
-  for (int i = 0; i < 6; ++i) out = c[i] + x * out;
-  return out;
-}
-
 // ---- device side ----------------------------------------------------------
-struct PrjTables {
-  int n_hm, n_hz;
-  const double *mh, *hz, *dn;  // ln(m_h (Omega_M - Omega_nu)), z, dn/dlnM [n_hz][n_hm]
-  double hmf_s, hmf_q;
-  int n_bl, n_bz;
-  const double *bl, *bz, *bias;  // haloModel lnM, z, bias [n_bz][n_bl]
-  int n_xr, n_xz;
-  const double *xr, *xz, *xi;    // xi_nl r, z, xi [n_xz][n_xr]
+// Shapes, offsets and constants of one call.  The sample block holds, in
+// order, 8 scalars (Omega_M, Omega_nu, Omega_L, Omega_k, h0, hmf_s, hmf_q,
+// n(sci) > 1) and the tables; a slice's scratch its grids and sums.
+struct PrjDims {
+  int n_lnm, n_seg, n_zring, n_zouter, ngp, nsl, nR_max, nt_max, nz;  // n_seg: nodes a segment
+  double zt_low, zt_high, R_max;
+  int omega_z;
+  int n_hm, n_hz, nd, n_sci, n_bl, n_bz, n_xr, n_xz, n_blob, n_bzob;
+  long o_mh, o_hz, o_dn, o_dz, o_da, o_dc, o_sz, o_sv, o_bl, o_bz, o_bi, o_xr, o_xz, o_xi, o_bzob,
+    o_bs, o_blg;
+  long s_mh, s_xi, s_bd, s_th, s_geom, s_bsel, s_wcl_th, s_z, s_zc, s_chi, s_thex, s_ab, s_wz,
+    s_wrnd, s_wcl, s_scal, scratch;
+  // constants of the handle (device)
+  const double *lnm_x, *lnm_w, *anchor;        // [n_lnm]; anchor = w r_s
+  const double *gl_seg, *gl_ring, *gl_out;     // nodes | weights on [-1, 1]
+  const double *zk_z, *zk_s;                   // photo-z width
+  const double *sl_lob, *sl_zob, *radii;       // per slice; radii ascending, slices one after another
+  const double* gp_R;
+  const int *sl_lb, *r0, *gp_slice;            // r0 [nsl + 1]
+};
+
+// The single-kernel miscentring table (nfw_dsigma_mis.hh:62-72).
+struct PrjTable {
   int n_lx, n_lxm;
-  const double *lx, *lxm, *ltab; // single-kernel table (n_lx = 0: quadrature)
-  double omega_m;
+  const double *lx, *lxm, *ltab;
 };
 
 // The fixed-offset profile without a table: the 256-node GL rule over the
@@ -144,103 +99,291 @@ struct PrjQuad {
   const double* nfw;     // DeltaSigma polynomials
 };
 
-__device__ __forceinline__ double
-hmf_dev(const PrjTables& T, double lnM, double z)
-{
-  return interp2d_clamp(T.mh, T.n_hm, T.hz, T.n_hz, T.dn, lnM, z) *
-         (T.hmf_s * (lnM * kLog10e - kHmfPivot) + T.hmf_q);
-}
-
 // NFW_DSIGMA_MIS(R, R_mis, lnM), single kernel (nfw_dsigma_mis.hh:95-114),
 // from its table: r_s from rho_c, amplitude 2 r_s delta_c rho_c Omega_M
 // 1e-12 [h Msun/pc^2].
 __device__ double
-dsigma_single_table(const PrjTables& T, double R, double Rmis, double lnM)
+dsigma_single_table(const PrjTable& T, double R, double Rmis, double lnM)
 {
   const double rs = nfw_rs(lnM, kConc, kRhoCrit);
   const double unit = exp(
     interp2d_clamp(T.lx, T.n_lx, T.lxm, T.n_lxm, T.ltab, log(R / rs), log(Rmis / rs)));
-  return nfw_norm(lnM, kConc, kRhoCrit) * T.omega_m * unit;
+  return nfw_norm(lnM, kConc, kRhoCrit) * unit;
 }
 
-// Per (slice, z node): a_b(z) and the random-channel weights.  One block of
-// 128 threads per (slice, z); thread iM takes the mass nodes iM, iM + 128, ...
-__global__ void __launch_bounds__(128)
-prj_z_kernel(PrjTables T, int n_lnm, const double* lnm_x, const double* lnm_w,
-             const int* zslice, const double* zz, const double* zc, const double* anchor,
-             const double* denom, double* AB, double* WZ)
+// Per slice: the theta and z grids and the sums over the line of sight.
+// One block; the node counts are a few dozen to a few hundred, so the block
+// is bound by the latency of its phases (interpolations, the 40-step chi(z)
+// bisections), which run one node a thread.
+constexpr int kSliceThreads = 512;
+
+__global__ void __launch_bounds__(kSliceThreads)
+prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ scratch,
+                 int* __restrict__ nt_out, int* status)
 {
-  __shared__ double red[128];
-  const int u = blockIdx.x, sl = zslice[u];
-  const double z = zz[u], c = zc[u];
-  double num = 0.0;
-  for (int iM = threadIdx.x; iM < n_lnm; iM += blockDim.x) {
-    const double x = lnm_x[iM];
-    const double n = hmf_dev(T, x, z);
-    const double b = interp2d_clamp(T.bl, T.n_bl, T.bz, T.n_bz, T.bias, x, z);
-    num += anchor[(size_t)sl * n_lnm + iM] * n * b;
-    WZ[(size_t)u * n_lnm + iM] = c * n * lnm_w[iM];
+  const int sl = blockIdx.x, tid = threadIdx.x, nt_thr = blockDim.x;
+  const int lane = tid & 31, warp = tid >> 5, nw = nt_thr >> 5;
+  double* S = scratch + (size_t)sl * D.scratch;
+  const double om = B[0], h0 = B[4];
+  const double* dz = B + D.o_dz;
+  const double zob = D.sl_zob[sl];
+  __shared__ double sc[16], chis[5];
+  __shared__ int n_bd_s;
+  auto chi = [&](double z) { return interp1d_clamp(dz, B + D.o_dc, D.nd, z) * h0; };
+  constexpr double dz1 = 1.0e-3;
+  if (tid < 5) {
+    const double zq[5] = {zob, D.zt_low, D.zt_high, zob + dz1, zob - dz1};
+    chis[tid] = chi(zq[tid]);
   }
-  num = block_sum<128>(num, red);
-  if (threadIdx.x == 0) AB[u] = c * (num / denom[sl]);
-}
-
-// wrnd(slice, M) = sum over the slice's z nodes in order.
-__global__ void
-prj_wrnd_kernel(int n_slices, int n_lnm, const int* z0, const double* WZ, double* wrnd)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_slices * n_lnm) return;
-  const int sl = i / n_lnm, iM = i % n_lnm;
-  double acc = 0.0;
-  for (int u = z0[sl]; u < z0[sl + 1]; ++u) acc += WZ[(size_t)u * n_lnm + iM];
-  wrnd[i] = acc;
-}
-
-// Psi(theta) of every slice's theta node, z nodes in order.
-__global__ void
-prj_psi_kernel(PrjTables T, int n_theta_tot, const int* tslice, const double* theta,
-               const int* z0, const double* chi_z, const double* th_excl, const double* AB,
-               const double* chi_o, const double* zob, double* psi)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_theta_tot) return;
-  const int sl = tslice[i];
-  const double th = theta[i], ct = cos(th), co = chi_o[sl], zo = zob[sl];
-  double acc = 0.0;
-  for (int u = z0[sl]; u < z0[sl + 1]; ++u) {
-    if (th <= th_excl[u]) continue;
-    const double cz = chi_z[u];
-    const double dchi = sqrt(fmax(cz * cz + co * co - 2.0 * cz * co * ct, 0.0));
-    acc += AB[u] * interp2d_clamp(T.xr, T.n_xr, T.xz, T.n_xz, T.xi, dchi, zo);
+  // HMF mass axis ln(m_h (Omega_M - Omega_nu)) and xi_NL(r, z_obs)
+  for (int i = tid; i < D.n_hm; i += nt_thr) S[D.s_mh + i] = log(B[D.o_mh + i] * (om - B[1]));
+  {
+    const double* xz = B + D.o_xz;
+    const double y = fmin(fmax(zob, xz[0]), xz[D.n_xz - 1]);
+    const int j = bsearch_cell(xz, D.n_xz, y);
+    const double u = (y - xz[j]) / (xz[j + 1] - xz[j]);
+    const double* r0 = B + D.o_xi + (size_t)j * D.n_xr;
+    const double* r1 = r0 + D.n_xr;
+    for (int i = tid; i < D.n_xr; i += nt_thr) S[D.s_xi + i] = (1.0 - u) * r0[i] + u * r1[i];
   }
-  psi[i] = acc;
+  __syncthreads();
+  if (tid == 0) {
+    const double chi_o = chis[0], D_A = chi_o / (1.0 + zob);
+    const double Rl = pow(D.sl_lob[sl] / 100.0, 0.2), R_excl = Rl * (1.0 + zob);
+    // theta breakpoints (sp_detail::build_theta_grid, sigma_prj_t.hh:95-180):
+    // the radii ascend, so the sorted list is a merge of theta_R with the
+    // five others; those outside (0, theta_max] are left out and neighbours
+    // closer than 1e-6 kept once.
+    const int ra = D.r0[sl], nR = D.r0[sl + 1] - ra;
+    const double th_lam = Rl * (1.0 + zob) / chi_o, th_ex = R_excl / chi_o;
+    int top = nR - 1;
+    while (top > 0 && isnan(D.radii[ra + top])) --top;
+    const double t_min = D.radii[ra] / D_A, t_max = D.radii[ra + top] / D_A;
+    const double th_max = fmax(D.R_max / D_A, 3.0 * t_max);
+    const double lower = fmax(1.0e-8, 0.1 * fmin(th_ex, fmin(t_min, th_lam)));
+    double sp[5] = {lower, th_ex, th_lam, 2.0 * th_lam, th_max};
+    for (int a = 1; a < 5; ++a)
+      for (int b = a; b > 0 && sp[b] < sp[b - 1]; --b) {
+        const double v = sp[b];
+        sp[b] = sp[b - 1];
+        sp[b - 1] = v;
+      }
+    double* bd = S + D.s_bd;
+    int n = 0;
+    double back = 0.0, last = 0.0;  // last kept, last of the sorted list
+    auto put = [&](double x) {
+      if (n == 0 || x > back * (1.0 + 1.0e-6)) {
+        bd[n++] = x;
+        back = x;
+      }
+      last = x;
+    };
+    int is = 0, ir = 0;
+    while (is < 5 || ir < nR) {
+      const double tr = ir < nR ? D.radii[ra + ir] / D_A : 0.0;
+      double x;
+      if (ir >= nR || (is < 5 && sp[is] <= tr)) {
+        x = sp[is++];
+      } else {
+        x = tr;
+        ++ir;
+      }
+      if (!(isfinite(x) && x > 0.0 && x <= th_max)) continue;
+      if (n == 0 && x > lower) put(lower);
+      put(x);
+    }
+    if (n == 0) put(lower);
+    if (last < th_max) put(th_max);
+    n_bd_s = n;
+    // b_sel asymptotes linear in z_obs (sigma_prj_frozen_t.hh:200-217)
+    const double* bz = B + D.o_bzob;
+    const int nzb = D.n_bzob, nlb = D.n_blob, lb = D.sl_lb[sl];
+    int j = 0;
+    while (j + 1 < nzb && bz[j + 1] < zob) ++j;
+    const int j0 = j + 1 < nzb ? j : max(nzb - 2, 0), j1 = j + 1 < nzb ? j + 1 : nzb - 1;
+    const double za = bz[j0], zb = bz[j1];
+    const double f = zb > za ? fmin(fmax((zob - za) / (zb - za), 0.0), 1.0) : 0.0;
+    const double* bs = B + D.o_bs;
+    const double* bl = B + D.o_blg;
+    sc[0] = (1.0 - f) * bs[j0 * nlb + lb] + f * bs[j1 * nlb + lb];
+    sc[1] = (1.0 - f) * bl[j0 * nlb + lb] + f * bl[j1 * nlb + lb];
+    sc[2] = 2.5 / th_lam;
+    sc[3] = 0.5 * th_lam;
+    // line-of-sight ranges (sigma_prj_frozen_t.hh:380-455)
+    const double dchi_dz = (chis[3] - chis[4]) / (2.0 * dz1);
+    const double dz_ex = R_excl / dchi_dz;
+    sc[4] = fmax(zob - dz_ex, D.zt_low);
+    sc[5] = fmin(zob + dz_ex, D.zt_high);
+    sc[6] = R_excl;
+    sc[7] = chi_o - chis[1];
+    sc[8] = chis[2] - chi_o;
+    S[D.s_scal] = chi_o;
+    S[D.s_scal + 1] = D_A;
+    S[D.s_scal + 2] =
+      B[7] != 0.0 ? interp1d_clamp(B + D.o_sz, B + D.o_sv, D.n_sci, zob) : 0.0;
+  }
+  __syncthreads();
+  const double chi_o = chis[0], R_excl = sc[6];
+  const int n_th = (n_bd_s - 1) * D.n_seg;
+  const int n_f = R_excl < sc[7] ? D.n_zouter : 0, n_r = sc[5] > sc[4] ? D.n_zring : 0;
+  const int n_b = R_excl < sc[8] ? D.n_zouter : 0, nz = n_f + n_r + n_b;
+  for (int i = tid; i < D.nz + n_th; i += nt_thr) {
+    if (i >= D.nz) {  // theta node
+      const int t = i - D.nz, s = t / D.n_seg, q = t - s * D.n_seg;
+      const double a = log(S[D.s_bd + s]), b = log(S[D.s_bd + s + 1]), hl = 0.5 * (b - a);
+      const double th = exp(0.5 * (a + b) + hl * D.gl_seg[q]);
+      S[D.s_th + t] = th;
+      S[D.s_geom + t] = hl * D.gl_seg[D.n_seg + q] * th * 2.0 * kPiP * sin(th);
+      S[D.s_bsel + t] = sc[0] + (sc[1] - sc[0]) * (1.0 / (1.0 + exp(-sc[2] * (th - sc[3]))));
+      continue;
+    }
+    // z node: front wing (farthest first), ring, back wing
+    double z, wz;
+    if (i >= nz) {
+      S[D.s_zc + i] = 0.0;
+      continue;
+    }
+    if (i >= n_f && i < n_f + n_r) {
+      const int q = i - n_f;
+      const double hl = 0.5 * (sc[5] - sc[4]);
+      z = 0.5 * (sc[4] + sc[5]) + hl * D.gl_ring[q];
+      wz = hl * D.gl_ring[D.n_zring + q];
+    } else {
+      const bool fg = i < n_f;
+      const int q = fg ? n_f - 1 - i : i - n_f - n_r;
+      const double a = log(R_excl), b = log(fg ? sc[7] : sc[8]), hl = 0.5 * (b - a);
+      const double dis = exp(0.5 * (a + b) + hl * D.gl_out[q]);
+      const double target = fg ? chi_o - dis : chi_o + dis;
+      double lo = 0.001, hi = 2.0;  // sigma_prj_frozen_t.hh:458-468
+      for (int it = 0; it < 40; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        if (chi(mid) < target)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      z = 0.5 * (lo + hi);
+      wz = hl * D.gl_out[D.n_zouter + q] * dis / ((chi(z + dz1) - chi(z - dz1)) / (2.0 * dz1));
+    }
+    const double chz = chi(z);
+    double dv;
+    if (!dv_do_dz(dz, B + D.o_da, D.nd, om, B[2], B[3], h0, z, &dv)) {
+      set_err(status, kDevDomain);
+      dv = 0.0;
+    }
+    const double up = (z - zob) / interp1d_clamp(D.zk_z, D.zk_s, kZKernelNodes, z);
+    const double wph = fabs(up) < 1.0 ? 1.0 - up * up : 0.0;
+    S[D.s_z + i] = z;
+    S[D.s_zc + i] = dv * (D.omega_z ? omega_z_des(z) : 1.0) * wz * wph;
+    S[D.s_chi + i] = chz;
+    // sp_detail::theta_excl_at_z (sigma_prj_t.hh:185-194)
+    const double ce =
+      (chz * chz + chi_o * chi_o - R_excl * R_excl) / (2.0 * chz * chi_o + 1.0e-30);
+    S[D.s_thex + i] = ce >= 1.0 - 1.0e-12 ? 0.0 : acos(fmax(ce, -1.0));
+  }
+  if (tid == 0) nt_out[sl] = n_th;
+  __syncthreads();
+  // n and b at every z node of non-zero weight and, in the last item, at
+  // z_obs: one warp a node, lanes over the masses.
+  for (int i = warp; i <= D.nz; i += nw) {
+    const bool anchor = i == D.nz;
+    const double c = anchor ? 1.0 : S[D.s_zc + i], z = anchor ? zob : (c != 0.0 ? S[D.s_z + i] : 0.0);
+    double num = 0.0;
+    for (int k = lane; k < D.n_lnm; k += 32) {
+      if (c == 0.0) {  // the reference skips these nodes entirely
+        S[D.s_wz + (size_t)i * D.n_lnm + k] = 0.0;
+        continue;
+      }
+      const double x = D.lnm_x[k];
+      const double n = interp2d_clamp(S + D.s_mh, D.n_hm, B + D.o_hz, D.n_hz, B + D.o_dn, x, z) *
+                       (B[5] * (x * kLog10e - kHmfPivot) + B[6]);
+      const double b =
+        interp2d_clamp(B + D.o_bl, D.n_bl, B + D.o_bz, D.n_bz, B + D.o_bi, x, z);
+      num += D.anchor[k] * n * b;
+      if (anchor)
+        S[D.s_wcl + k] = D.lnm_w[k] * n * b;
+      else
+        S[D.s_wz + (size_t)i * D.n_lnm + k] = c * n * D.lnm_w[k];
+    }
+    for (int off = 16; off > 0; off >>= 1) num += __shfl_xor_sync(0xffffffffu, num, off);
+    if (lane == 0) {
+      if (anchor)
+        sc[9] = num + 1.0e-300;
+      else
+        S[D.s_ab + i] = num;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < D.nz; i += nt_thr) {
+    const double c = S[D.s_zc + i];
+    S[D.s_ab + i] = c != 0.0 ? c * (S[D.s_ab + i] / sc[9]) : 0.0;
+  }
+  for (int k = tid; k < D.n_lnm; k += nt_thr) {
+    double acc = 0.0;
+    for (int i = 0; i < D.nz; ++i) acc += S[D.s_wz + (size_t)i * D.n_lnm + k];
+    S[D.s_wrnd + k] = acc;
+  }
 }
 
-// The single-kernel profile DSigma_mis(R | theta D_A, M) of every (grid
-// point, theta node of its slice, mass node), written to
-// V[g][(it - t0) n_lnm + iM] (max_pairs per grid point): from the table, one
-// thread per value.
+// The clustered channel's weight g_theta b_sel Psi of every theta node: one
+// warp a node, lanes over the z nodes.
 __global__ void __launch_bounds__(256)
-prj_profile_table_kernel(PrjTables T, int n_lnm, const double* lnm_x, const int* gp_slice,
-                         const double* gp_R, const int* t0, const double* theta,
-                         const double* DA, int max_pairs, double* V)
+prj_psi_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ scratch,
+               const int* __restrict__ nt)
 {
-  const int g = blockIdx.y, sl = gp_slice[g];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n_pairs = (t0[sl + 1] - t0[sl]) * n_lnm;
-  if (k >= n_pairs) return;
-  const int it = t0[sl] + k / n_lnm, iM = k % n_lnm;
-  V[(size_t)g * max_pairs + k] =
-    dsigma_single_table(T, gp_R[g], theta[it] * DA[sl], lnm_x[iM]);
+  const int sl = blockIdx.y, lane = threadIdx.x & 31;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (t >= nt[sl]) return;
+  double* S = scratch + (size_t)sl * D.scratch;
+  const double th = S[D.s_th + t], ct = cos(th), co = S[D.s_scal];
+  const double* xr = B + D.o_xr;
+  const double* row = S + D.s_xi;
+  double acc = 0.0;
+  for (int u = lane; u < D.nz; u += 32) {
+    if (S[D.s_zc + u] == 0.0 || th <= S[D.s_thex + u]) continue;
+    const double cz = S[D.s_chi + u];
+    const double dchi = sqrt(fmax(cz * cz + co * co - 2.0 * cz * co * ct, 0.0));
+    const double r = fmin(fmax(dchi, xr[0]), xr[D.n_xr - 1]);
+    const int i = bsearch_cell(xr, D.n_xr, r);
+    const double f = (r - xr[i]) / (xr[i + 1] - xr[i]);
+    acc += S[D.s_ab + u] * ((1.0 - f) * row[i] + f * row[i + 1]);
+  }
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if (lane == 0) S[D.s_wcl_th + t] = S[D.s_geom + t] * S[D.s_bsel + t] * acc;
+}
+
+// The mass contractions sum_M wrnd(M) DSigma_mis and sum_M w_M n b DSigma_mis
+// of every (grid point, theta node): P[g][t] = (rnd, cl).  From the table,
+// one warp a node, lanes over the masses.
+__global__ void __launch_bounds__(256)
+prj_profile_table_kernel(PrjDims D, PrjTable T, const double* __restrict__ scratch,
+                         const int* __restrict__ nt, double2* __restrict__ P)
+{
+  const int g = blockIdx.y, sl = D.gp_slice[g], lane = threadIdx.x & 31;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (t >= nt[sl]) return;
+  const double* S = scratch + (size_t)sl * D.scratch;
+  const double R = D.gp_R[g], Rm = S[D.s_th + t] * S[D.s_scal + 1];
+  double ar = 0.0, ac = 0.0;
+  for (int k = lane; k < D.n_lnm; k += 32) {
+    const double v = dsigma_single_table(T, R, Rm, D.lnm_x[k]);
+    ar += S[D.s_wrnd + k] * v;
+    ac += S[D.s_wcl + k] * v;
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    ar += __shfl_xor_sync(0xffffffffu, ar, off);
+    ac += __shfl_xor_sync(0xffffffffu, ac, off);
+  }
+  if (lane == 0) P[(size_t)g * D.nt_max + t] = make_double2(ar, ac);
 }
 
 // The ring averages with the closed-form profile, for rings that leave the
 // polynomials' range; out of line: the rare path.
-__device__ __noinline__ void
+__device__ __noinline__ double2
 ring_masses_closed(const PrjQuad& Q, const double* __restrict__ rule, int n, double R, double Rm,
-                   int n_lnm, double omega_m, int lane, double* __restrict__ out)
+                   int n_lnm, const double* __restrict__ w, const double* __restrict__ wc, int lane)
 {
+  double ar = 0.0, ac = 0.0;
   for (int k = 0; k < n_lnm; ++k) {
     const double q = Q.mass[k];
     double acc = 0.0;
@@ -250,22 +393,25 @@ ring_masses_closed(const PrjQuad& Q, const double* __restrict__ rule, int n, dou
              NfwUnit<double>::dsigma(sqrt(D2 * q));
     }
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0) out[k] = Q.mass[n_lnm + k] * omega_m * acc;
+    ar += w[k] * Q.mass[n_lnm + k] * acc;
+    ac += wc[k] * Q.mass[n_lnm + k] * acc;
   }
+  return make_double2(ar, ac);
 }
 
-// One warp's ring average of NJ nodes a lane, for all masses: the mean
+// One warp's ring average of NJ nodes a lane, for all masses, contracted with
+// the mass weights w and wc: the mean
 // tangential shear on the circle of radius R around the offset centre,
 // (1/pi) int dt DSigma(d / r_s) (2 a^2 / d^2 - 1), d^2 = R^2 + Rm^2 -
 // 2 R Rm cos t, a = R - Rm cos t.  The geometry is shared by the masses,
 // which only scale d; eight masses accumulate side by side and are summed
 // over the lanes by halving exchanges (nine 64-bit shuffles for eight sums).
 template <int NJ>
-__device__ __forceinline__ void
+__device__ __forceinline__ double2
 ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double Rm, int n_lnm,
-            double omega_m, int lane, double* __restrict__ out)
+            const double* __restrict__ w, const double* __restrict__ wc, int lane)
 {
-  double D2[NJ], A[NJ];
+  double D2[NJ], A[NJ], ar = 0.0, ac = 0.0;
   bool outside = false;
   const double s2 = R * R + Rm * Rm, c2 = 2.0 * R * Rm;
 #pragma unroll
@@ -295,61 +441,68 @@ ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double 
     acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
     acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
     const int k = k0 + (lane >> 2);
-    if ((lane & 3) == 0 && k < n_lnm) out[k] = Q.mass[n_lnm + k] * omega_m * acc[0];
+    if ((lane & 3) == 0 && k < n_lnm) {
+      const double v = Q.mass[n_lnm + k] * acc[0];
+      ar += w[k] * v;
+      ac += wc[k] * v;
+    }
   }
   if (__any_sync(0xffffffffu, outside))
-    ring_masses_closed(Q, rule, 32 * NJ, R, Rm, n_lnm, omega_m, lane, out);
-}
-
-// The same values by quadrature, one warp per (grid point, theta node): the
-// lanes take the ring's nodes, so the profile's table reads of a warp fall
-// on few, neighbouring segments.
-__global__ void __launch_bounds__(256, 3)
-prj_profile_kernel(PrjQuad Q, double omega_m, int n_lnm, const int* gp_slice,
-                   const double* gp_R, const int* t0, const double* theta, const double* DA,
-                   int max_pairs, double* V)
-{
-  const int g = blockIdx.y, sl = gp_slice[g], lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= t0[sl + 1] - t0[sl]) return;
-  const double R = gp_R[g], Rm = theta[t0[sl] + i] * DA[sl], lr = fabs(log(Rm / R));
-  double* out = V + (size_t)g * max_pairs + (size_t)i * n_lnm;
-  if (lr >= kRuleLn0)
-    ring_masses<1>(Q, Q.rule, R, Rm, n_lnm, omega_m, lane, out);
-  else if (lr >= kRuleLn1)
-    ring_masses<2>(Q, Q.rule + kRuleN0, R, Rm, n_lnm, omega_m, lane, out);
-  else if (lr >= kRuleLn2)
-    ring_masses<4>(Q, Q.rule + kRuleN0 + kRuleN1, R, Rm, n_lnm, omega_m, lane, out);
-  else
-    ring_masses<8>(Q, Q.rule + kRuleN0 + kRuleN1 + kRuleN2, R, Rm, n_lnm, omega_m, lane, out);
-}
-
-// One block per grid point: the (theta, M) sums of both channels over the
-// profile values of prj_profile_kernel.
-__global__ void __launch_bounds__(256)
-prj_eval_kernel(int n_lnm, const int* gp_slice, const int* t0, const double* geom,
-                const double* bsel, const double* psi, const double* wrnd, const double* wcl,
-                const double* sci, int max_pairs, const double* V, double* out)
-{
-  __shared__ double red[256];
-  const int g = blockIdx.x, sl = gp_slice[g];
-  const double* Vg = V + (size_t)g * max_pairs;
-  double rnd = 0.0, cl = 0.0;
-  for (int it = t0[sl] + threadIdx.x; it < t0[sl + 1]; it += blockDim.x) {
-    const double* v_it = Vg + (size_t)(it - t0[sl]) * n_lnm;
-    double ar = 0.0, ac = 0.0;
-    for (int iM = 0; iM < n_lnm; ++iM) {
-      const double v = v_it[iM];
-      ar += wrnd[(size_t)sl * n_lnm + iM] * v;
-      ac += wcl[(size_t)sl * n_lnm + iM] * v;
-    }
-    rnd += geom[it] * ar;
-    cl += geom[it] * bsel[it] * psi[it] * ac;
+    return ring_masses_closed(Q, rule, 32 * NJ, R, Rm, n_lnm, w, wc, lane);
+  for (int off = 16; off >= 4; off >>= 1) {
+    ar += __shfl_xor_sync(0xffffffffu, ar, off);
+    ac += __shfl_xor_sync(0xffffffffu, ac, off);
   }
-  rnd = block_sum<256>(rnd, red);
-  cl = block_sum<256>(cl, red);
+  return make_double2(ar, ac);
+}
+
+// The same contractions by quadrature, one warp per (grid point, theta
+// node): the lanes take the ring's nodes, so the profile's table reads of a
+// warp fall on few, neighbouring segments.  12 slices x 10 radii x ~130
+// theta x 24 masses: 98 us, bound by those reads (L1).
+__global__ void __launch_bounds__(256, 3)
+prj_profile_kernel(PrjDims D, PrjQuad Q, const double* __restrict__ scratch,
+                   const int* __restrict__ nt, double2* __restrict__ P)
+{
+  const int g = blockIdx.y, sl = D.gp_slice[g], lane = threadIdx.x & 31;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (t >= nt[sl]) return;
+  const double* S = scratch + (size_t)sl * D.scratch;
+  const double R = D.gp_R[g], Rm = S[D.s_th + t] * S[D.s_scal + 1], lr = fabs(log(Rm / R));
+  const double *w = S + D.s_wrnd, *wc = S + D.s_wcl;
+  double2 v;
+  if (lr >= kRuleLn0)
+    v = ring_masses<1>(Q, Q.rule, R, Rm, D.n_lnm, w, wc, lane);
+  else if (lr >= kRuleLn1)
+    v = ring_masses<2>(Q, Q.rule + kRuleN0, R, Rm, D.n_lnm, w, wc, lane);
+  else if (lr >= kRuleLn2)
+    v = ring_masses<4>(Q, Q.rule + kRuleN0 + kRuleN1, R, Rm, D.n_lnm, w, wc, lane);
+  else
+    v = ring_masses<8>(Q, Q.rule + kRuleN0 + kRuleN1 + kRuleN2, R, Rm, D.n_lnm, w, wc, lane);
+  if (lane == 0) P[(size_t)g * D.nt_max + t] = v;
+}
+
+// The theta sums of one grid point; block 0 also copies the status word
+// behind the results.
+__global__ void __launch_bounds__(128)
+prj_sum_kernel(PrjDims D, const double* __restrict__ B, const double* __restrict__ scratch,
+               const int* __restrict__ nt, const double2* __restrict__ P,
+               const int* __restrict__ status, double* __restrict__ out)
+{
+  __shared__ double red[128];
+  const int g = blockIdx.x, sl = D.gp_slice[g];
+  const double* S = scratch + (size_t)sl * D.scratch;
+  const double2* Pg = P + (size_t)g * D.nt_max;
+  double rnd = 0.0, cl = 0.0;
+  for (int t = threadIdx.x; t < nt[sl]; t += blockDim.x) {
+    const double2 v = Pg[t];
+    rnd += S[D.s_geom + t] * v.x;
+    cl += S[D.s_wcl_th + t] * v.y;
+  }
+  rnd = block_sum<128>(rnd, red) * B[0];  // the amplitude's Omega_M
+  cl = block_sum<128>(cl, red) * B[0];
   if (threadIdx.x == 0) {
-    const double tot = rnd + cl, s = sci[sl];
+    const double tot = rnd + cl, s = S[D.s_scal + 2];
     double* o = out + (size_t)g * 9;
     o[0] = tot;
     o[1] = rnd;
@@ -357,17 +510,32 @@ prj_eval_kernel(int n_lnm, const int* gp_slice, const int* t0, const double* geo
     o[3] = o[6] = tot * s;
     o[4] = o[7] = rnd * s;
     o[5] = o[8] = cl * s;
+    if (g == 0) *reinterpret_cast<int*>(out + (size_t)D.ngp * 9) = *status;
   }
 }
 
 }  // namespace
 
-// Device buffers of one evaluation, kept by the handle and grown on demand.
+// Device and pinned buffers of the handle, grown on demand.
 struct PrjBufs {
-  DevBuf<double> d_mh, d_hz, d_dn, d_bl, d_bz, d_bi, d_xr, d_xz, d_xi, d_lx, d_lxm, d_lt, d_quad,
-    d_lnx, d_lnw, d_theta, d_geom, d_bsel, d_zz, d_zc, d_chiz, d_thex, d_anchor, d_denom,
-    d_wcl, d_AB, d_WZ, d_wrnd, d_psi, d_chio, d_zob, d_da, d_sci, d_gpR, d_out, d_V;
-  DevBuf<int> d_t0, d_z0, d_ts, d_zs, d_gps;
+  DevBuf<double> d_const, d_quad, d_tab, d_blk, d_scratch, d_P, d_out;
+  DevBuf<int> d_int, d_nt;
+  double* h_stage = nullptr;
+  size_t stage_cap = 0;
+  ~PrjBufs()
+  {
+    if (h_stage) cudaFreeHost(h_stage);
+  }
+  int stage(size_t n)  // pinned doubles
+  {
+    if (n <= stage_cap) return Y3B_OK;
+    if (h_stage) cudaFreeHost(h_stage);
+    h_stage = nullptr;
+    stage_cap = 0;
+    Y3B_CUDA(cudaHostAlloc((void**)&h_stage, n * sizeof(double), cudaHostAllocDefault));
+    stage_cap = n;
+    return Y3B_OK;
+  }
 };
 
 }  // namespace y3b
@@ -382,7 +550,7 @@ struct y3b_prj {
   std::vector<double> sl_zob;
   std::vector<std::vector<double>> sl_Rs;    // distinct radii, first-appearance order
   std::vector<double> lnm_x, lnm_w;
-  std::vector<double> tab_lx, tab_lxm, tab_v;
+  int tab_lx = 0, tab_lxm = 0;               // shape of the miscentring table in bufs.d_tab
   y3b::PrjBufs bufs;
   cudaStream_t stream = nullptr;
   ~y3b_prj()
@@ -435,6 +603,137 @@ upload_quad(y3b_prj* h)
   const int rc = cuda_status(cudaStreamSynchronize(h->stream), "upload of the ring rules");
   if (rc) d.reset();
   return rc;
+}
+
+// The handle's constants: mass nodes, weights and anchors w r_s (NFW_DSIGMA_MIS::
+// r_s, nfw_dsigma_mis.hh:82-88), unit GL rules, the photo-z width table, the
+// slices' centres and ascending radii, the grid points.
+int
+upload_const(y3b_prj* h)
+{
+  const y3b_prj_config& c = h->cfg;
+  std::vector<double> q, x, w;
+  auto put = [&](const std::vector<double>& v) { q.insert(q.end(), v.begin(), v.end()); };
+  put(h->lnm_x);
+  put(h->lnm_w);
+  for (int i = 0; i < c.n_lnm; ++i)
+    q.push_back(h->lnm_w[i] *
+                (std::cbrt(3.0 * std::exp(h->lnm_x[i]) / (800.0 * kPiP * kRhoCrit)) / kConc));
+  for (int n : {c.n_per_seg, c.n_zring, c.n_zouter}) {
+    h_gl(-1.0, 1.0, n, x, w);
+    put(x);
+    put(w);
+  }
+  q.insert(q.end(), kZKernelZ, kZKernelZ + kZKernelNodes);
+  q.insert(q.end(), kZKernelSigma, kZKernelSigma + kZKernelNodes);
+  for (int lb : h->sl_lb) q.push_back(h->lob[lb]);
+  put(h->sl_zob);
+  std::vector<int> ints(h->sl_lb);
+  int off = 0;
+  for (const auto& Rs : h->sl_Rs) {
+    std::vector<double> s(Rs);
+    std::sort(s.begin(), s.end(),  // a NaN last: it never becomes a breakpoint
+              [](double a, double b) { return std::isnan(b) ? !std::isnan(a) : a < b; });
+    put(s);
+    ints.push_back(off);
+    off += (int)s.size();
+  }
+  ints.push_back(off);
+  put(h->gp_R);
+  ints.insert(ints.end(), h->gp_slice.begin(), h->gp_slice.end());
+  Y3B_TRY(h->bufs.d_const.upload(q.data(), q.size(), h->stream));
+  Y3B_TRY(h->bufs.d_int.upload(ints.data(), ints.size(), h->stream));
+  return cuda_status(cudaStreamSynchronize(h->stream), "upload of the handle's constants");
+}
+
+// Shapes and offsets of one call.
+PrjDims
+layout(const y3b_prj* h, const y3b_prj_sample& S)
+{
+  const y3b_prj_config& c = h->cfg;
+  PrjDims D{};
+  D.n_lnm = c.n_lnm;
+  D.n_seg = c.n_per_seg;
+  D.n_zring = c.n_zring;
+  D.n_zouter = c.n_zouter;
+  D.ngp = c.n_gp;
+  D.nsl = (int)h->sl_lb.size();
+  size_t n_radii = 0;
+  for (const auto& Rs : h->sl_Rs) {
+    D.nR_max = std::max(D.nR_max, (int)Rs.size());
+    n_radii += Rs.size();
+  }
+  D.nt_max = (D.nR_max + 6) * c.n_per_seg;  // five more breakpoints, and the two ends
+  D.nz = c.n_zring + 2 * c.n_zouter;
+  D.zt_low = c.zt_low;
+  D.zt_high = c.zt_high;
+  D.R_max = c.R_max_cMpch;
+  D.omega_z = c.include_omega_z;
+  D.n_hm = S.t.n_hm;
+  D.n_hz = S.t.n_hz;
+  D.nd = S.t.n_dist;
+  D.n_sci = S.t.n_sci;
+  D.n_bl = S.n_hl;
+  D.n_bz = S.n_hz;
+  D.n_xr = S.n_xr;
+  D.n_xz = S.n_xz;
+  D.n_blob = S.n_blob;
+  D.n_bzob = S.n_bzob;
+  long o = 8;
+  auto blk = [&](long& at, long n) { at = o, o += n; };
+  blk(D.o_mh, D.n_hm);
+  blk(D.o_hz, D.n_hz);
+  blk(D.o_dn, (long)D.n_hz * D.n_hm);
+  blk(D.o_dz, D.nd);
+  blk(D.o_da, D.nd);
+  blk(D.o_dc, D.nd);
+  blk(D.o_sz, std::max(D.n_sci, 0));
+  blk(D.o_sv, std::max(D.n_sci, 0));
+  blk(D.o_bl, D.n_bl);
+  blk(D.o_bz, D.n_bz);
+  blk(D.o_bi, (long)D.n_bl * D.n_bz);
+  blk(D.o_xr, D.n_xr);
+  blk(D.o_xz, D.n_xz);
+  blk(D.o_xi, (long)D.n_xr * D.n_xz);
+  blk(D.o_bzob, D.n_bzob);
+  blk(D.o_bs, (long)D.n_bzob * D.n_blob);
+  blk(D.o_blg, (long)D.n_bzob * D.n_blob);
+  o = 0;
+  blk(D.s_mh, D.n_hm);
+  blk(D.s_xi, D.n_xr);
+  blk(D.s_bd, D.nR_max + 7);
+  blk(D.s_th, D.nt_max);
+  blk(D.s_geom, D.nt_max);
+  blk(D.s_bsel, D.nt_max);
+  blk(D.s_wcl_th, D.nt_max);
+  for (long* at : {&D.s_z, &D.s_zc, &D.s_chi, &D.s_thex, &D.s_ab}) blk(*at, D.nz);
+  blk(D.s_wz, (long)D.nz * D.n_lnm);
+  blk(D.s_wrnd, D.n_lnm);
+  blk(D.s_wcl, D.n_lnm);
+  blk(D.s_scal, 4);
+  D.scratch = o;
+  const double* q = h->bufs.d_const.get();
+  auto take = [&](size_t n) {
+    const double* at = q;
+    q += n;
+    return at;
+  };
+  D.lnm_x = take(c.n_lnm);
+  D.lnm_w = take(c.n_lnm);
+  D.anchor = take(c.n_lnm);
+  D.gl_seg = take(2 * (size_t)c.n_per_seg);
+  D.gl_ring = take(2 * (size_t)c.n_zring);
+  D.gl_out = take(2 * (size_t)c.n_zouter);
+  D.zk_z = take(kZKernelNodes);
+  D.zk_s = take(kZKernelNodes);
+  D.sl_lob = take(D.nsl);
+  D.sl_zob = take(D.nsl);
+  D.radii = take(n_radii);
+  D.gp_R = take(c.n_gp);
+  D.sl_lb = h->bufs.d_int.get();
+  D.r0 = D.sl_lb + D.nsl;
+  D.gp_slice = D.r0 + D.nsl + 1;
+  return D;
 }
 
 }  // namespace
@@ -494,6 +793,7 @@ y3b_prj_create(const y3b_prj_config* cfg, y3b_prj** out)
   h_gl(cfg->lnm_low, cfg->lnm_high, cfg->n_lnm, h->lnm_x, h->lnm_w);
   int rc = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking),
                        "cudaStreamCreate");
+  if (!rc) rc = upload_const(h);
   if (rc) {
     delete h;
     return rc;
@@ -516,9 +816,7 @@ y3b_prj_set_mis_table(y3b_prj* h, int n_lx, const double* logx, int n_lxm,
   clear_error();
   if (!h) return Y3B_ERR_INVALID;
   if (n_lx == 0) {
-    h->tab_lx.clear();
-    h->tab_lxm.clear();
-    h->tab_v.clear();
+    h->tab_lx = h->tab_lxm = 0;
     return Y3B_OK;
   }
   if (n_lx < 2 || n_lxm < 2 || !logx || !logxmis || !log_tab) {
@@ -530,9 +828,14 @@ y3b_prj_set_mis_table(y3b_prj* h, int n_lx, const double* logx, int n_lxm,
       set_error("y3b_prj_set_mis_table: non-finite table entry");
       return Y3B_ERR_DOMAIN;
     }
-  h->tab_lx.assign(logx, logx + n_lx);
-  h->tab_lxm.assign(logxmis, logxmis + n_lxm);
-  h->tab_v.assign(log_tab, log_tab + (size_t)n_lx * n_lxm);
+  h->tab_lx = h->tab_lxm = 0;
+  std::vector<double> tab(logx, logx + n_lx);
+  tab.insert(tab.end(), logxmis, logxmis + n_lxm);
+  tab.insert(tab.end(), log_tab, log_tab + (size_t)n_lx * n_lxm);
+  Y3B_TRY(h->bufs.d_tab.upload(tab.data(), tab.size(), h->stream));
+  Y3B_CUDA(cudaStreamSynchronize(h->stream));
+  h->tab_lx = n_lx;
+  h->tab_lxm = n_lxm;
   return Y3B_OK;
 }
 
@@ -548,267 +851,89 @@ y3b_prj_eval(y3b_prj* h, const y3b_prj_sample* S, double* out)
     set_error("y3b_prj_eval: incomplete sample (tables of at least two nodes each)");
     return Y3B_ERR_INVALID;
   }
-  const y3b_prj_config& c = h->cfg;
   const y3b_tables& t = S->t;
-  const double h0 = S->cosmo.h0, om = S->cosmo.om;
-  const int n_lnm = c.n_lnm, nsl = (int)h->sl_lb.size();
-  const double* dz = t.dist_z;
-  auto chi = [&](double z) { return h_lin_clamp(dz, S->dist_dc, t.n_dist, z) * h0; };
-  // HMF on the host for the slices' z_obs: ln(m_h (Omega_M - Omega_nu)) axis.
-  std::vector<double> mh(t.n_hm);
-  for (int i = 0; i < t.n_hm; ++i) mh[i] = std::log(t.hmf_m_h[i] * (om - S->cosmo.onu));
-  auto hmf = [&](double lnM, double z) {
-    return h_bilin_clamp(mh.data(), t.n_hm, t.hmf_z, t.n_hz, t.dndlnmh, lnM, z) *
-           (S->cosmo.hmf_s * (lnM * 0.4342944819 - 13.8124426028) + S->cosmo.hmf_q);
-  };
-  auto hmb = [&](double lnM, double z) {
-    return h_bilin_clamp(S->halo_lnM, S->n_hl, S->halo_z, S->n_hz, S->bias, lnM, z);
-  };
-  auto r_s = [&](double lnM) {  // NFW_DSIGMA_MIS::r_s (nfw_dsigma_mis.hh:82-88)
-    return std::cbrt(3.0 * std::exp(lnM) / (800.0 * kPiP * kRhoCrit)) / kConc;
-  };
-  auto invert_chi = [&](double target) {  // sigma_prj_frozen_t.hh:458-468
-    double lo = 0.001, hi = 2.0;
-    for (int it = 0; it < 40; ++it) {
-      const double mid = 0.5 * (lo + hi);
-      if (chi(mid) < target)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    return 0.5 * (lo + hi);
-  };
-  // Host-built per-slice grids and factors.
-  std::vector<int> t0(1, 0), z0(1, 0), tslice, zslice;
-  std::vector<double> theta, geom, bsel, zz, zc, chiz, thex;
-  std::vector<double> sl_chi(nsl), sl_da(nsl), sl_sci(nsl), denom(nsl);
-  std::vector<double> anchor((size_t)nsl * n_lnm), wcl((size_t)nsl * n_lnm);
-  for (int k = 0; k < nsl; ++k) {
-    const double lobc = h->lob[h->sl_lb[k]], zob = h->sl_zob[k];
-    const double chi_o = chi(zob), D_A_o = chi_o / (1.0 + zob);
-    const double Rl = std::pow(lobc / 100.0, 0.2), R_excl = Rl * (1.0 + zob);
-    sl_chi[k] = chi_o;
-    sl_da[k] = D_A_o;
-    sl_sci[k] = t.n_sci > 1 ? h_lin_clamp(t.sci_z, t.sci_val, t.n_sci, zob) : 0.0;
-    // theta grid (sp_detail::build_theta_grid, sigma_prj_t.hh:95-180)
-    const auto& Rs = h->sl_Rs[k];
-    const double th_lam = Rl * (1.0 + zob) / chi_o, th_ex = R_excl / chi_o;
-    double trmin = th_lam, trmax = th_lam;
-    if (!Rs.empty()) {
-      trmin = trmax = Rs[0] / D_A_o;
-      for (double R : Rs) {
-        trmin = std::min(trmin, R / D_A_o);
-        trmax = std::max(trmax, R / D_A_o);
-      }
-    }
-    const double th_max = std::max(c.R_max_cMpch / D_A_o, 3.0 * trmax);
-    const double lower = std::max(1.0e-8, 0.1 * std::min({th_ex, trmin, th_lam}));
-    std::vector<double> bp{lower, th_ex};
-    for (double R : Rs) bp.push_back(R / D_A_o);
-    bp.push_back(th_lam);
-    bp.push_back(2.0 * th_lam);
-    bp.push_back(th_max);
-    std::vector<double> bc;
-    for (double x : bp)
-      if (std::isfinite(x) && x > 0.0 && x <= th_max) bc.push_back(x);
-    std::sort(bc.begin(), bc.end());
-    if (bc.empty() || bc.front() > lower) bc.insert(bc.begin(), lower);
-    if (bc.back() < th_max) bc.push_back(th_max);
-    std::vector<double> bd{bc.front()};
-    for (size_t i = 1; i < bc.size(); ++i)
-      if (bc[i] > bd.back() * (1.0 + 1.0e-6)) bd.push_back(bc[i]);
-    // b_sel asymptotes linear in z_obs (sigma_prj_frozen_t.hh:200-217)
-    const int nzb = S->n_bzob, nlb = S->n_blob;
-    int j = 0;
-    while (j + 1 < nzb && S->bsel_zob[j + 1] < zob) ++j;
-    const int j0 = j + 1 < nzb ? j : std::max(nzb - 2, 0), j1 = j + 1 < nzb ? j + 1 : nzb - 1;
-    const double za = S->bsel_zob[j0], zb = S->bsel_zob[j1];
-    const double f = std::clamp(zb > za ? (zob - za) / (zb - za) : 0.0, 0.0, 1.0);
-    const int lb = h->sl_lb[k];
-    if (lb >= nlb) {
-      set_error("y3b_prj_eval: b_sel_marginalised has %d richness bins, bin %d requested", nlb,
-                lb);
+  for (int lb : h->sl_lb)
+    if (lb >= S->n_blob) {
+      set_error("y3b_prj_eval: b_sel_marginalised has %d richness bins, bin %d requested",
+                S->n_blob, lb);
       return Y3B_ERR_INVALID;
     }
-    const double Bs = (1.0 - f) * S->b_small[j0 * nlb + lb] + f * S->b_small[j1 * nlb + lb];
-    const double Bl = (1.0 - f) * S->b_large[j0 * nlb + lb] + f * S->b_large[j1 * nlb + lb];
-    const double k_sig = 2.5 / th_lam, th0 = 0.5 * th_lam;
-    std::vector<double> ux, uw;
-    for (size_t s = 0; s + 1 < bd.size(); ++s) {
-      h_gl(std::log(bd[s]), std::log(bd[s + 1]), c.n_per_seg, ux, uw);
-      for (int q = 0; q < c.n_per_seg; ++q) {
-        const double th = std::exp(ux[q]), w = uw[q] * th;
-        theta.push_back(th);
-        geom.push_back(w * 2.0 * kPiP * std::sin(th));
-        bsel.push_back(Bs + (Bl - Bs) * (1.0 / (1.0 + std::exp(-k_sig * (th - th0)))));
-        tslice.push_back(k);
-      }
-    }
-    t0.push_back((int)theta.size());
-    // n, b at z_obs, the a_b(z) anchor and the cl-channel mass weights
-    double den = 0.0;
-    for (int iM = 0; iM < n_lnm; ++iM) {
-      const double x = h->lnm_x[iM], no = hmf(x, zob), bo = hmb(x, zob);
-      const double a = h->lnm_w[iM] * r_s(x);
-      anchor[(size_t)k * n_lnm + iM] = a;
-      den += a * no * bo;
-      wcl[(size_t)k * n_lnm + iM] = h->lnm_w[iM] * no * bo;
-    }
-    denom[k] = den + 1.0e-300;
-    // line-of-sight z grid (sigma_prj_frozen_t.hh:380-455)
-    const double dz1 = 1.0e-3;
-    const double chi_fg = chi(c.zt_low), chi_bg = chi(c.zt_high);
-    const double dchi_dz = (chi(zob + dz1) - chi(zob - dz1)) / (2.0 * dz1);
-    const double dz_ex = R_excl / dchi_dz;
-    const double zr_lo = std::max(zob - dz_ex, c.zt_low), zr_hi = std::min(zob + dz_ex, c.zt_high);
-    std::vector<double> zs, wzs, zr, wr;
-    std::vector<double> zf, wf, zb2, wb2;
-    if (zr_hi > zr_lo) h_gl(zr_lo, zr_hi, c.n_zring, zr, wr);
-    auto outer = [&](double dis_max, double sign, std::vector<double>& zo_, std::vector<double>& wo_) {
-      if (!(R_excl < dis_max)) return;
-      h_gl(std::log(R_excl), std::log(dis_max), c.n_zouter, ux, uw);
-      zo_.resize(c.n_zouter);
-      wo_.resize(c.n_zouter);
-      for (int i = 0; i < c.n_zouter; ++i) {
-        const double dis = std::exp(ux[i]);
-        const double zi = invert_chi(chi_o + sign * dis);
-        const double ddz = (chi(zi + dz1) - chi(zi - dz1)) / (2.0 * dz1);
-        zo_[i] = zi;
-        wo_[i] = uw[i] * dis / ddz;
-      }
-    };
-    outer(chi_o - chi_fg, -1.0, zf, wf);
-    outer(chi_bg - chi_o, 1.0, zb2, wb2);
-    for (size_t i = zf.size(); i--;) {
-      zs.push_back(zf[i]);
-      wzs.push_back(wf[i]);
-    }
-    zs.insert(zs.end(), zr.begin(), zr.end());
-    wzs.insert(wzs.end(), wr.begin(), wr.end());
-    zs.insert(zs.end(), zb2.begin(), zb2.end());
-    wzs.insert(wzs.end(), wb2.begin(), wb2.end());
-    for (size_t i = 0; i < zs.size(); ++i) {
-      const double z = zs[i], chz = chi(z);
-      double da;
-      if (!h_lin(dz, t.dist_da, t.n_dist, z, &da)) {
-        set_error("argument out of range in Interp1D (z = %g outside distances/z)", z);
-        return Y3B_ERR_DOMAIN;
-      }
-      const double ez = std::sqrt(om * (1 + z) * (1 + z) * (1 + z) +
-                                  S->cosmo.ok * (1 + z) * (1 + z) + S->cosmo.ol);
-      const double dv = 2997.92 * (1.0 + z) * (1.0 + z) * da * h0 * da * h0 / ez;
-      const double omz = c.include_omega_z ? omega_z_host(z) : 1.0;
-      const double sgz = h_lin_clamp(kZKernelZ, kZKernelSigma, kZKernelNodes, z);
-      const double up = (z - zob) / sgz;
-      const double wph = std::abs(up) < 1.0 ? 1.0 - up * up : 0.0;
-      const double cz = dv * omz * wzs[i] * wph;
-      if (cz == 0.0) continue;  // the reference skips these nodes entirely
-      zz.push_back(z);
-      zc.push_back(cz);
-      chiz.push_back(chz);
-      // sp_detail::theta_excl_at_z (sigma_prj_t.hh:185-194)
-      double ce = (chz * chz + chi_o * chi_o - R_excl * R_excl) / (2.0 * chz * chi_o + 1.0e-30);
-      thex.push_back(ce >= 1.0 - 1.0e-12 ? 0.0 : std::acos(std::max(ce, -1.0)));
-      zslice.push_back(k);
-    }
-    z0.push_back((int)zz.size());
-  }
-  // Device buffers.
+  const PrjDims D = layout(h, *S);
   cudaStream_t s = h->stream;
-  y3b::PrjBufs& B = h->bufs;  // kept by the handle: no device allocation after the first call
-  Y3B_TRY(B.d_mh.upload(mh.data(), mh.size(), s));
-  Y3B_TRY(B.d_hz.upload(t.hmf_z, t.n_hz, s));
-  Y3B_TRY(B.d_dn.upload(t.dndlnmh, (size_t)t.n_hz * t.n_hm, s));
-  Y3B_TRY(B.d_bl.upload(S->halo_lnM, S->n_hl, s));
-  Y3B_TRY(B.d_bz.upload(S->halo_z, S->n_hz, s));
-  Y3B_TRY(B.d_bi.upload(S->bias, (size_t)S->n_hl * S->n_hz, s));
-  Y3B_TRY(B.d_xr.upload(S->xi_r, S->n_xr, s));
-  Y3B_TRY(B.d_xz.upload(S->xi_z, S->n_xz, s));
-  Y3B_TRY(B.d_xi.upload(S->xi_nl, (size_t)S->n_xr * S->n_xz, s));
-  const bool table = !h->tab_lx.empty();
-  if (table) {
-    Y3B_TRY(B.d_lx.upload(h->tab_lx.data(), h->tab_lx.size(), s));
-    Y3B_TRY(B.d_lxm.upload(h->tab_lxm.data(), h->tab_lxm.size(), s));
-    Y3B_TRY(B.d_lt.upload(h->tab_v.data(), h->tab_v.size(), s));
-  } else if (!B.d_quad.get()) {
-    Y3B_TRY(upload_quad(h));
+  PrjBufs& B = h->bufs;  // kept by the handle: no allocation after the first call
+  const bool table = h->tab_lx > 0;
+  if (!table && !B.d_quad.get()) Y3B_TRY(upload_quad(h));
+  // The sample's block, with the status word (zero) behind it.
+  const size_t blk = (size_t)D.o_blg + (size_t)D.n_bzob * D.n_blob, n_out = (size_t)D.ngp * 9 + 1;
+  Y3B_TRY(B.stage(blk + 1 + n_out));
+  Y3B_TRY(B.d_blk.alloc(blk + 1));
+  Y3B_TRY(B.d_scratch.alloc((size_t)D.nsl * D.scratch));
+  Y3B_TRY(B.d_nt.alloc(D.nsl));
+  Y3B_TRY(B.d_P.alloc(2 * (size_t)D.ngp * D.nt_max));
+  Y3B_TRY(B.d_out.alloc(n_out));
+  double* b = B.h_stage;
+  const double sc[8] = {S->cosmo.om, S->cosmo.onu, S->cosmo.ol, S->cosmo.ok, S->cosmo.h0,
+                        S->cosmo.hmf_s, S->cosmo.hmf_q, t.n_sci > 1 ? 1.0 : 0.0};
+  std::memcpy(b, sc, sizeof sc);
+  auto put = [&](long at, const double* v, size_t n) {
+    if (n) std::memcpy(b + at, v, n * sizeof(double));
+  };
+  put(D.o_mh, t.hmf_m_h, D.n_hm);
+  put(D.o_hz, t.hmf_z, D.n_hz);
+  put(D.o_dn, t.dndlnmh, (size_t)D.n_hz * D.n_hm);
+  put(D.o_dz, t.dist_z, D.nd);
+  put(D.o_da, t.dist_da, D.nd);
+  put(D.o_dc, S->dist_dc, D.nd);
+  if (t.n_sci > 1) {
+    put(D.o_sz, t.sci_z, D.n_sci);
+    put(D.o_sv, t.sci_val, D.n_sci);
   }
-  Y3B_TRY(B.d_lnx.upload(h->lnm_x.data(), n_lnm, s));
-  Y3B_TRY(B.d_lnw.upload(h->lnm_w.data(), n_lnm, s));
-  Y3B_TRY(B.d_theta.upload(theta.data(), theta.size(), s));
-  Y3B_TRY(B.d_geom.upload(geom.data(), geom.size(), s));
-  Y3B_TRY(B.d_bsel.upload(bsel.data(), bsel.size(), s));
-  Y3B_TRY(B.d_ts.upload(tslice.data(), tslice.size(), s));
-  Y3B_TRY(B.d_t0.upload(t0.data(), t0.size(), s));
-  Y3B_TRY(B.d_z0.upload(z0.data(), z0.size(), s));
-  const int nz_tot = (int)zz.size(), nth_tot = (int)theta.size(), ngp = c.n_gp;
-  if (nz_tot) {
-    Y3B_TRY(B.d_zz.upload(zz.data(), nz_tot, s));
-    Y3B_TRY(B.d_zc.upload(zc.data(), nz_tot, s));
-    Y3B_TRY(B.d_chiz.upload(chiz.data(), nz_tot, s));
-    Y3B_TRY(B.d_thex.upload(thex.data(), nz_tot, s));
-    Y3B_TRY(B.d_zs.upload(zslice.data(), nz_tot, s));
-  }
-  Y3B_TRY(B.d_anchor.upload(anchor.data(), anchor.size(), s));
-  Y3B_TRY(B.d_denom.upload(denom.data(), nsl, s));
-  Y3B_TRY(B.d_wcl.upload(wcl.data(), wcl.size(), s));
-  Y3B_TRY(B.d_chio.upload(sl_chi.data(), nsl, s));
-  Y3B_TRY(B.d_zob.upload(h->sl_zob.data(), nsl, s));
-  Y3B_TRY(B.d_da.upload(sl_da.data(), nsl, s));
-  Y3B_TRY(B.d_sci.upload(sl_sci.data(), nsl, s));
-  Y3B_TRY(B.d_gps.upload(h->gp_slice.data(), ngp, s));
-  Y3B_TRY(B.d_gpR.upload(h->gp_R.data(), ngp, s));
-  Y3B_TRY(B.d_AB.alloc(std::max(nz_tot, 1)));
-  Y3B_TRY(B.d_WZ.alloc((size_t)std::max(nz_tot, 1) * n_lnm));
-  Y3B_TRY(B.d_wrnd.alloc((size_t)nsl * n_lnm));
-  Y3B_TRY(B.d_psi.alloc(std::max(nth_tot, 1)));
-  Y3B_TRY(B.d_out.alloc((size_t)ngp * 9));
-  PrjTables T{t.n_hm, t.n_hz, B.d_mh.get(), B.d_hz.get(), B.d_dn.get(), S->cosmo.hmf_s,
-              S->cosmo.hmf_q, S->n_hl, S->n_hz, B.d_bl.get(), B.d_bz.get(), B.d_bi.get(), S->n_xr,
-              S->n_xz, B.d_xr.get(), B.d_xz.get(), B.d_xi.get(),
-              table ? (int)h->tab_lx.size() : 0, table ? (int)h->tab_lxm.size() : 0,
-              B.d_lx.get(), B.d_lxm.get(), B.d_lt.get(), om};
-  if (nz_tot) {
-    prj_z_kernel<<<nz_tot, 128, 0, s>>>(T, n_lnm, B.d_lnx.get(), B.d_lnw.get(), B.d_zs.get(),
-                                        B.d_zz.get(), B.d_zc.get(), B.d_anchor.get(), B.d_denom.get(),
-                                        B.d_AB.get(), B.d_WZ.get());
-    count_launch();
-    Y3B_CUDA(cudaGetLastError());
-  }
-  prj_wrnd_kernel<<<(nsl * n_lnm + 127) / 128, 128, 0, s>>>(nsl, n_lnm, B.d_z0.get(), B.d_WZ.get(),
-                                                             B.d_wrnd.get());
+  put(D.o_bl, S->halo_lnM, D.n_bl);
+  put(D.o_bz, S->halo_z, D.n_bz);
+  put(D.o_bi, S->bias, (size_t)D.n_bl * D.n_bz);
+  put(D.o_xr, S->xi_r, D.n_xr);
+  put(D.o_xz, S->xi_z, D.n_xz);
+  put(D.o_xi, S->xi_nl, (size_t)D.n_xr * D.n_xz);
+  put(D.o_bzob, S->bsel_zob, D.n_bzob);
+  put(D.o_bs, S->b_small, (size_t)D.n_bzob * D.n_blob);
+  put(D.o_blg, S->b_large, (size_t)D.n_bzob * D.n_blob);
+  b[blk] = 0.0;
+  Y3B_CUDA(cudaMemcpyAsync(B.d_blk.get(), b, (blk + 1) * sizeof(double), cudaMemcpyHostToDevice, s));
+  int* status = reinterpret_cast<int*>(B.d_blk.get() + blk);
+  double2* P = reinterpret_cast<double2*>(B.d_P.get());
+  const dim3 per_theta((D.nt_max + 7) / 8, D.nsl), per_gp((D.nt_max + 7) / 8, D.ngp);
+  prj_slice_kernel<<<D.nsl, kSliceThreads, 0, s>>>(D, B.d_blk.get(), B.d_scratch.get(),
+                                                   B.d_nt.get(), status);
   count_launch();
   Y3B_CUDA(cudaGetLastError());
-  prj_psi_kernel<<<(nth_tot + 127) / 128, 128, 0, s>>>(T, nth_tot, B.d_ts.get(), B.d_theta.get(),
-                                                       B.d_z0.get(), B.d_chiz.get(), B.d_thex.get(),
-                                                       B.d_AB.get(), B.d_chio.get(), B.d_zob.get(),
-                                                       B.d_psi.get());
+  prj_psi_kernel<<<per_theta, 256, 0, s>>>(D, B.d_blk.get(), B.d_scratch.get(), B.d_nt.get());
   count_launch();
   Y3B_CUDA(cudaGetLastError());
-  int max_nt = 0;
-  for (int k = 0; k < nsl; ++k) max_nt = std::max(max_nt, t0[k + 1] - t0[k]);
-  const int max_pairs = std::max(max_nt * n_lnm, 1);
-  Y3B_TRY(B.d_V.alloc((size_t)ngp * max_pairs));
   if (table) {
-    prj_profile_table_kernel<<<dim3((max_pairs + 255) / 256, ngp), 256, 0, s>>>(
-      T, n_lnm, B.d_lnx.get(), B.d_gps.get(), B.d_gpR.get(), B.d_t0.get(), B.d_theta.get(),
-      B.d_da.get(), max_pairs, B.d_V.get());
+    const double* tb = B.d_tab.get();
+    const PrjTable T{h->tab_lx, h->tab_lxm, tb, tb + h->tab_lx, tb + h->tab_lx + h->tab_lxm};
+    prj_profile_table_kernel<<<per_gp, 256, 0, s>>>(D, T, B.d_scratch.get(), B.d_nt.get(), P);
   } else {
-    const PrjQuad Q{B.d_quad.get() + kNfwSegs * kNfwCoef,
-                    B.d_quad.get() + kNfwSegs * kNfwCoef + 2 * kRuleTot, B.d_quad.get()};
-    prj_profile_kernel<<<dim3((max_nt + 7) / 8, ngp), 256, 0, s>>>(
-      Q, om, n_lnm, B.d_gps.get(), B.d_gpR.get(), B.d_t0.get(), B.d_theta.get(), B.d_da.get(),
-      max_pairs, B.d_V.get());
+    const double* qd = B.d_quad.get();
+    const PrjQuad Q{qd + kNfwSegs * kNfwCoef, qd + kNfwSegs * kNfwCoef + 2 * kRuleTot, qd};
+    prj_profile_kernel<<<per_gp, 256, 0, s>>>(D, Q, B.d_scratch.get(), B.d_nt.get(), P);
   }
   count_launch();
   Y3B_CUDA(cudaGetLastError());
-  prj_eval_kernel<<<ngp, 256, 0, s>>>(n_lnm, B.d_gps.get(), B.d_t0.get(), B.d_geom.get(),
-                                      B.d_bsel.get(), B.d_psi.get(), B.d_wrnd.get(), B.d_wcl.get(),
-                                      B.d_sci.get(), max_pairs, B.d_V.get(), B.d_out.get());
+  prj_sum_kernel<<<D.ngp, 128, 0, s>>>(D, B.d_blk.get(), B.d_scratch.get(), B.d_nt.get(), P,
+                                       status, B.d_out.get());
   count_launch();
   Y3B_CUDA(cudaGetLastError());
-  Y3B_CUDA(cudaMemcpyAsync(out, B.d_out.get(), (size_t)ngp * 9 * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
+  double* ho = B.h_stage + blk + 1;
+  Y3B_CUDA(cudaMemcpyAsync(ho, B.d_out.get(), n_out * sizeof(double), cudaMemcpyDeviceToHost, s));
   Y3B_CUDA(cudaStreamSynchronize(s));
+  int st;
+  std::memcpy(&st, ho + n_out - 1, sizeof st);
+  if (st == kDevDomain) {
+    set_error("argument out of range in Interp1D (a line-of-sight z node outside distances/z)");
+    return Y3B_ERR_DOMAIN;
+  }
+  if (st != kDevOk) return device_status_rc(st);
+  std::memcpy(out, ho, (n_out - 1) * sizeof(double));
   return Y3B_OK;
 }
