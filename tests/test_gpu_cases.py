@@ -34,3 +34,11 @@ def _compare(case, tol, seed=3):
 def test_projection_shear_by_quadrature(gpu, n_lnm, radii, n_per_seg):
     _compare(dict(kind="prj", radii=radii, n_lnm=n_lnm, n_per_seg=n_per_seg, n_zring=7,
                   n_zouter=9), 1e-9)
+
+
+# 33 masses: a partial last group of eight; the distinct (R_mis, R) pairs are
+# shared by the z_obs bins; radii from 0.1 to 30 cover both quadrature forms.
+@pytest.mark.parametrize("mor,n_lnm,radii", [("hod", 2, 1), ("lognormal", 33, 4), ("hod", 96, 15)])
+def test_module_chain(gpu, mor, n_lnm, radii):
+    _compare(dict(kind="module", mor=mor, tab_m=40, tab_z=24, n_q=17, n_lnm=n_lnm, n_z=19,
+                  radii=radii), 1e-9)

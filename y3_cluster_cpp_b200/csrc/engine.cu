@@ -1194,22 +1194,12 @@ shear_phi_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_
 // nodes, so the mixed form reads both profiles with the same weights.
 constexpr int kMisNx = 2048;
 
+// The miscentred rows come from launch_mis_pairs, the centred one from here.
 __global__ void __launch_bounds__(128)
-mis_table_kernel(ShearDev sh, MisQuad quad, int n_pairs, double u0, double du, double* tab)
+cen_table_kernel(double u0, double du, double* row)
 {
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= (long long)(n_pairs + 1) * kMisNx) return;
-  const int pair = (int)(w / kMisNx), j = (int)(w % kMisNx);
-  if (pair == n_pairs) {  // the centred profile (warp-uniform branch)
-    if (lane == 0) tab[w] = NfwUnit<double>::dsigma(exp(u0 + j * du));
-    return;
-  }
-  const int i = pair / sh.n_R, iR = pair % sh.n_R;
-  const double ratio = sh.tau_mis * pow(sh.lob[i] / 100.0, 0.2) / sh.R[iR];
-  const double x = exp(u0 + j * du);
-  const double v = warp_sum(mis_partial<double>(quad, x, ratio * x, true, lane));
-  if (lane == 0) tab[w] = v;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < kMisNx) row[j] = NfwUnit<double>::dsigma(exp(u0 + j * du));
 }
 
 // Phi_i(R, k) of the mixed form from the table, one thread per (point, k):
@@ -1889,11 +1879,23 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
     e->mis_du = (std::log(x_hi * 1.5) - e->mis_u0) / (kMisNx - 1);
     const int n_pairs = e->nI_max * sh.n_R;
     if ((rc = e->mis_tab.alloc((size_t)(n_pairs + 1) * kMisNx))) return fail(rc);
-    const long long threads = (long long)(n_pairs + 1) * kMisNx * 32;
-    mis_table_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, e->stream>>>(
-      sh, e->quad.view(), n_pairs, e->mis_u0, e->mis_du, e->mis_tab.get());
+    std::vector<double> ratio(n_pairs);  // x_mis / x of each (i, R)
+    for (int i = 0; i < e->nI_max; ++i)
+      for (int r = 0; r < sh.n_R; ++r)
+        ratio[i * sh.n_R + r] = sh.tau_mis * std::pow(sh.lob[i] / 100.0, 0.2) / sh.R[r];
+    DevBuf<double> d_ratio;
+    if ((rc = d_ratio.upload(ratio.data(), ratio.size(), e->stream)) ||
+        (rc = e->quad.ensure_nfw(e->stream)))
+      return fail(rc);
+    const MisPairs a{n_pairs, kMisNx,    nullptr,   d_ratio.get(),   nullptr, 1.0, 1.0,
+                     1.0,     e->mis_u0, e->mis_du, e->mis_tab.get()};
+    if ((rc = launch_mis_pairs(e->quad.view(), e->quad.nfw.get(), a, e->stream))) return fail(rc);
+    cen_table_kernel<<<(kMisNx + 127) / 128, 128, 0, e->stream>>>(
+      e->mis_u0, e->mis_du, e->mis_tab.get() + (size_t)n_pairs * kMisNx);
     count_launch();
-    if ((rc = cuda_status(cudaGetLastError(), "mis_table_kernel"))) return fail(rc);
+    if ((rc = cuda_status(cudaGetLastError(), "cen_table_kernel")) ||
+        (rc = cuda_status(cudaStreamSynchronize(e->stream), "sync")))
+      return fail(rc);
   }
   // Device memory against the HBM budget.
   const size_t N = cfg->max_points;

@@ -16,10 +16,12 @@
 
 #include "common.cuh"
 #include "host_common.h"
+#include "nfw_table.cuh"
 
 namespace y3b {
 
 int gl_nodes_device(double a, double b, int n, double* xs, double* ws, cudaStream_t s);
+int cos_device(const double* x, int n, double* out, cudaStream_t s);
 
 // Miscentred profile quadrature nodes in s: two GL panels split at the
 // ring-crossing kink s_k = x / x_mis (R / R_mis, mass independent).
@@ -28,6 +30,7 @@ struct MisQuad {
   double s_max;
   const double* th;              // GL nodes on [0, pi] [n_theta]
   const double* wth;
+  const double* cth;             // cos(th) [n_theta]
   const double* t1;              // GL nodes on [-1,1] [n1]
   const double* w1;
   const double* t2;              // [n_s - n1]
@@ -63,7 +66,7 @@ mis_partial(const MisQuad& q, T x, T xmis, bool want_delta, int lane)
     const T r = xmis * (T)s;
     T inner = 0;
     for (int t = lane; t < q.n_theta; t += 32) {
-      T ct = (T)cos(q.th[t]);
+      T ct = (T)q.cth[t];
       T d2 = x * x + r * r - (T)2 * x * r * ct;
       T d = sqrt(d2);
       T v;
@@ -89,11 +92,37 @@ warp_sum(T v)
   return v;
 }
 
+// Arguments of launch_mis_pairs: DeltaSigma_mis of n_pairs (R, R_mis) pairs
+// at nx scale radii each, out[pair][k].
+//   r_s nodes (lnM given): r_s of lnM[k] at concentration conc and density
+//   rho; out carries the amplitude 2 r_s delta_c rho 1e-12 amp.
+//   x nodes (lnM null): x = R / r_s = exp(u0 + k du), R = 1, unit profile.
+struct MisPairs {
+  int n_pairs, nx;
+  const double* R;      // [n_pairs] (ignored with x nodes)
+  const double* rmis;   // [n_pairs]; with x nodes x_mis / x
+  const double* lnM;    // [nx]
+  double conc, rho, amp;
+  double u0, du;
+  double* out;
+};
+
+int launch_mis_pairs(const MisQuad& q, const double* nfw, const MisPairs& a, cudaStream_t s);
+
 // Device GL tables for the miscentring quadrature, cached per (n_theta, n_s).
 struct MisQuadCache {
   int n_theta = -1, n_s = -1;
   double s_max = 0.0;
-  DevBuf<double> th, wth, t1, w1, t2, w2, t0, w0;
+  DevBuf<double> th, wth, cth, t1, w1, t2, w2, t0, w0;
+  DevBuf<double> nfw;  // DeltaSigma polynomials (ensure_nfw)
+  int ensure_nfw(cudaStream_t s)
+  {
+    if (nfw.get()) return Y3B_OK;
+    Y3B_TRY(nfw.upload(nfw_table_host(), (size_t)kNfwSegs * kNfwCoef, s));
+    const int rc = cuda_status(cudaStreamSynchronize(s), "upload of the DeltaSigma polynomials");
+    if (rc) nfw.reset();
+    return rc;
+  }
   int ensure(int nt, int ns, double smax, cudaStream_t s)
   {
     if (nt == n_theta && ns == n_s && smax == s_max) return Y3B_OK;
@@ -104,6 +133,7 @@ struct MisQuadCache {
     int n1 = ns / 2;
     Y3B_TRY(th.alloc(nt));
     Y3B_TRY(wth.alloc(nt));
+    Y3B_TRY(cth.alloc(nt));
     Y3B_TRY(t1.alloc(n1));
     Y3B_TRY(w1.alloc(n1));
     Y3B_TRY(t2.alloc(ns - n1));
@@ -111,6 +141,7 @@ struct MisQuadCache {
     Y3B_TRY(t0.alloc(ns));
     Y3B_TRY(w0.alloc(ns));
     Y3B_TRY(gl_nodes_device(0.0, kPi, nt, th.get(), wth.get(), s));
+    Y3B_TRY(cos_device(th.get(), nt, cth.get(), s));
     Y3B_TRY(gl_nodes_device(-1.0, 1.0, n1, t1.get(), w1.get(), s));
     Y3B_TRY(gl_nodes_device(-1.0, 1.0, ns - n1, t2.get(), w2.get(), s));
     Y3B_TRY(gl_nodes_device(-1.0, 1.0, ns, t0.get(), w0.get(), s));
@@ -128,6 +159,7 @@ struct MisQuadCache {
     q.s_max = s_max;
     q.th = th.get();
     q.wth = wth.get();
+    q.cth = cth.get();
     q.t1 = t1.get();
     q.w1 = w1.get();
     q.t2 = t2.get();
