@@ -224,6 +224,16 @@ pdf_lob(double x, double mu, double sigma, double tau, double fprj)
   return (1.0 - fprj) * g + fprj * tau * emg_tail(x, mu, sigma, tau);
 }
 
+// EMG parameters at a richness from the eight coefficients c at its z.
+__device__ __forceinline__ void
+plob_from_coef(const double* c, double ltr, double* mu, double* sigma, double* tau, double* fprj)
+{
+  *mu = c[2] + c[3] * ltr;
+  *sigma = c[5] * pow(ltr, c[4]);
+  *tau = c[1] / pow(ltr, c[0]);
+  *fprj = fmin(1.0, c[7] / pow(1.0 + exp(-ltr), c[6]));
+}
+
 // The eight EMG coefficients are linear splines in z with constant
 // extrapolation (prj_params.py:122-130); coef is [8][n].
 __device__ __forceinline__ void
@@ -233,10 +243,7 @@ plob_params(int n, const double* zs, const double* coef, double ltr, double z,
   double c[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) c[k] = interp1d_clamp(zs, coef + k * n, n, z);
-  *mu = c[2] + c[3] * ltr;
-  *sigma = c[5] * pow(ltr, c[4]);
-  *tau = c[1] / pow(ltr, c[0]);
-  *fprj = fmin(1.0, c[7] / pow(1.0 + exp(-ltr), c[6]));
+  plob_from_coef(c, ltr, mu, sigma, tau, fprj);
 }
 
 // ---------------------------------------------------------------------------

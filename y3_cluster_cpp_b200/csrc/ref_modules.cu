@@ -11,8 +11,11 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <utility>
 #include <vector>
+
+#include <cuda.h>
 
 #include "common.cuh"
 #include "host_common.h"
@@ -99,7 +102,14 @@ hod_density(double ltr, double M, double ms, double lcentral, const double* hod)
   return density;
 }
 
-__global__ void __launch_bounds__(128)
+// CHAIN: the distinct richness bins are consecutive edges, pair p = edges
+// (p, p + 1), at most kChainEdges edges (the wall grids of the configs): the
+// CDF differences and sums then stay in registers; other layouts index
+// per-thread arrays in local memory.
+constexpr int kChainEdges = 9;
+
+template <bool CHAIN>
+__global__ void __launch_bounds__(128, 6)
 sel_function_kernel(SelFuncArgs a)
 {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -133,10 +143,17 @@ sel_function_kernel(SelFuncArgs a)
   }
   const bool degenerate = !(hi > lo);
   const double half = 0.5 * (hi - lo), mid = 0.5 * (hi + lo);
+  // The eight EMG coefficients depend on z alone: one lane each.
+  const double cl =
+    interp1d_clamp(a.plob_z, a.plob_coef + (lane & 7) * a.n_plob, a.n_plob, z);
+  double c[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) c[k] = __shfl_sync(0xffffffffu, cl, k);
 
-  double acc[kMaxPairs];
-  for (int p = 0; p < a.n_pairs; ++p) acc[p] = 0.0;
-  for (int t = lane; t < a.n_q; t += 32) {
+  double acc[CHAIN ? kChainEdges - 1 : kMaxPairs];
+#pragma unroll
+  for (int p = 0; p < (CHAIN ? kChainEdges - 1 : kMaxPairs); ++p) acc[p] = 0.0;
+  for (int t = lane; t < a.n_q && !degenerate; t += 32) {
     double ltr = mid + half * a.gl_t[t];
     double W = half * a.gl_w[t];
     double P;
@@ -147,26 +164,160 @@ sel_function_kernel(SelFuncArgs a)
       P = exp(-0.5 * d * d) / (kSqrt2Pi * a.mor[3] * ltr * D);
     }
     double mu, sg, tau, fp;
-    plob_params(a.n_plob, a.plob_z, a.plob_coef, ltr, z, &mu, &sg, &tau, &fp);
-    double cdf[kMaxEdges];
-    for (int e = 0; e < a.n_edges; ++e) cdf[e] = cdf_lob(a.edges[e], mu, sg, tau, fp);
-    for (int p = 0; p < a.n_pairs; ++p)
-      acc[p] += W * (cdf[a.pair_hi[p]] - cdf[a.pair_lo[p]]) * P;
+    plob_from_coef(c, ltr, &mu, &sg, &tau, &fp);
+    if constexpr (CHAIN) {
+      const double WP = W * P;
+      double prev = cdf_lob(a.edges[0], mu, sg, tau, fp);
+#pragma unroll
+      for (int e = 1; e < kChainEdges; ++e) {
+        if (e < a.n_edges) {
+          const double v = cdf_lob(a.edges[e], mu, sg, tau, fp);
+          acc[e - 1] += WP * (v - prev);
+          prev = v;
+        }
+      }
+    } else {
+      double cdf[kMaxEdges];
+      for (int e = 0; e < a.n_edges; ++e) cdf[e] = cdf_lob(a.edges[e], mu, sg, tau, fp);
+      for (int p = 0; p < a.n_pairs; ++p)
+        acc[p] += W * (cdf[a.pair_hi[p]] - cdf[a.pair_lo[p]]) * P;
+    }
   }
-  for (int p = 0; p < a.n_pairs; ++p) {
+#pragma unroll
+  for (int p = 0; p < (CHAIN ? kChainEdges - 1 : kMaxPairs); ++p) {
+    if (p >= a.n_pairs) break;
     double v = acc[p];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     acc[p] = v;
   }
-  if (lane == 0) {
-    for (int k = 0; k < a.n_bins; ++k) {
-      double Si = degenerate ? 0.0 : acc[a.bin_pair[k]];
-      double Kj = phi_cdf((a.zob_max[k] - z) / a.sigma_z[k]) -
-                  phi_cdf((a.zob_min[k] - z) / a.sigma_z[k]);
-      a.S_out[((size_t)k * a.n_z + j) * a.n_lnm + m] = Si * Kj;
-    }
+  // One bin a lane.
+  for (int k = lane; k < a.n_bins; k += 32) {
+    double Si = 0.0;
+#pragma unroll
+    for (int p = 0; p < (CHAIN ? kChainEdges - 1 : kMaxPairs); ++p)
+      if (p < a.n_pairs && p == a.bin_pair[k]) Si = acc[p];
+    if (degenerate) Si = 0.0;
+    const double Kj = phi_cdf((a.zob_max[k] - z) / a.sigma_z[k]) -
+                      phi_cdf((a.zob_min[k] - z) / a.sigma_z[k]);
+    a.S_out[((size_t)k * a.n_z + j) * a.n_lnm + m] = Si * Kj;
   }
+}
+
+// Chained bins (see above)?
+static bool
+chained(const std::vector<int>& lo, const std::vector<int>& hi, size_t n_edges)
+{
+  if (n_edges > (size_t)kChainEdges || lo.size() + 1 != n_edges) return false;
+  for (size_t p = 0; p < lo.size(); ++p)
+    if (lo[p] != (int)p || hi[p] != (int)p + 1) return false;
+  return true;
+}
+
+static int
+launch_sel_function(const SelFuncArgs& a, bool chain, cudaStream_t s)
+{
+  const long long warps = (long long)a.n_lnm * a.n_z;
+  const int blocks = (int)((warps * 32 + 127) / 128);
+  if (chain)
+    sel_function_kernel<true><<<blocks, 128, 0, s>>>(a);
+  else
+    sel_function_kernel<false><<<blocks, 128, 0, s>>>(a);
+  count_launch();
+  return cuda_status(cudaGetLastError(), "sel_function_kernel");
+}
+
+}  // namespace y3b
+
+namespace y3b {
+
+constexpr int kNoAllocMaxQ = 1024;      // N_q
+constexpr int kNoAllocMaxBins = 256;    // bins
+constexpr int kNoAllocMaxPlob = 256;    // projection-table z nodes
+constexpr size_t kNoAllocScratchDoubles =
+  2 * kNoAllocMaxQ + kMaxEdges + 3 * kNoAllocMaxBins + 9 * kNoAllocMaxPlob +
+  (2 * kMaxPairs + kNoAllocMaxBins);    // last term holds the int tables
+static __device__ __align__(256) double g_selfunc_scratch[kNoAllocScratchDoubles];
+
+// Device workspace of y3b_sel_function (inputs, GL rule, results): 2 MiB hold
+// a 12-bin table of 192 x 64 cells and more.  Allocating and freeing 1.2 MB a
+// call took 0.6 ms, at times tens of ms; one call at a time uses the array
+// (g_selfunc_mu), an overlapping or larger one allocates its own.
+constexpr size_t kSelFuncWork = 262144;  // doubles
+static __device__ __align__(256) double g_selfunc_work[kSelFuncWork];
+static std::mutex g_selfunc_mu;
+
+// Device address of g_selfunc_scratch, looked up once per device context
+// (host code may not use the symbol itself: it names a host-side stand-in).
+// The address belongs to the context the module image was loaded into: a
+// caller that resets the device gets a new context, in which the array lives
+// elsewhere, so the cache is keyed by the context's unique id and the lookup
+// is repeated for a new one.
+static std::mutex g_scratch_mu;
+static void* g_scratch_addr[128];
+static void* g_work_addr[128];
+static unsigned long long g_scratch_ctx[128];
+
+// Unique id of the calling thread's current context (0 if it cannot be
+// read, in which case the address is looked up on every call).  The driver
+// entry points are fetched through the runtime: the library links no
+// driver-API import.
+static unsigned long long
+current_context_id()
+{
+  using GetCurrentFn = CUresult (*)(CUcontext*);
+  using GetIdFn = CUresult (*)(CUcontext, unsigned long long*);
+  static GetCurrentFn get_current = nullptr;
+  static GetIdFn get_id = nullptr;
+  static bool resolved = false;
+  if (!resolved) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_current = reinterpret_cast<GetCurrentFn>(f);
+    f = nullptr;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_id = reinterpret_cast<GetIdFn>(f);
+    resolved = true;
+  }
+  CUcontext ctx = nullptr;
+  unsigned long long id = 0;
+  if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx ||
+      get_id(ctx, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
+static int
+scratch_address(double** out, double** work = nullptr)
+{
+  int dev = 0;
+  Y3B_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 128) {
+    set_error("y3b_sel_function_noalloc: device index %d out of range", dev);
+    return Y3B_ERR_INVALID;
+  }
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  const unsigned long long ctx = current_context_id();
+  if (!g_scratch_addr[dev] || ctx == 0 || ctx != g_scratch_ctx[dev]) {
+    void* p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, g_selfunc_scratch);
+    if (e != cudaSuccess || !p) {
+      set_error("cudaGetSymbolAddress(g_selfunc_scratch): %s", cudaGetErrorString(e));
+      return Y3B_ERR_CUDA;
+    }
+    void* w = nullptr;
+    Y3B_CUDA(cudaGetSymbolAddress(&w, g_selfunc_work));
+    g_work_addr[dev] = w;
+    g_scratch_addr[dev] = p;
+    // The lookup made the device's context current if it was not yet.
+    g_scratch_ctx[dev] = ctx ? ctx : current_context_id();
+  }
+  *out = static_cast<double*>(g_scratch_addr[dev]);
+  if (work) *work = static_cast<double*>(g_work_addr[dev]);
+  return Y3B_OK;
 }
 
 }  // namespace y3b
@@ -220,24 +371,37 @@ y3b_sel_function(const y3b_selfunc_config* cfg, const y3b_mor* mor,
     return Y3B_ERR_UNSUPPORTED;
   }
   cudaStream_t s = 0;
-  DevBuf<double> d_edges, d_zmin, d_zmax, d_sz, d_pz, d_pc, d_glt, d_glw, d_lnm, d_z, d_S;
-  DevBuf<int> d_plo, d_phi, d_bp;
-  Y3B_TRY(d_edges.upload(edges.data(), edges.size(), s));
-  Y3B_TRY(d_zmin.upload(cfg->zob_min, nb, s));
-  Y3B_TRY(d_zmax.upload(cfg->zob_max, nb, s));
-  Y3B_TRY(d_sz.upload(cfg->sigma_z, nb, s));
-  Y3B_TRY(d_pz.upload(plob->z, plob->n, s));
-  Y3B_TRY(d_pc.upload(plob->coef, 8 * (size_t)plob->n, s));
-  Y3B_TRY(d_plo.upload(plo.data(), plo.size(), s));
-  Y3B_TRY(d_phi.upload(phi_.data(), phi_.size(), s));
-  Y3B_TRY(d_bp.upload(bin_pair.data(), nb, s));
-  Y3B_TRY(d_glt.alloc(cfg->n_q));
-  Y3B_TRY(d_glw.alloc(cfg->n_q));
-  Y3B_TRY(d_lnm.alloc(cfg->n_lnm));
-  Y3B_TRY(d_z.alloc(cfg->n_z));
-  size_t nS = (size_t)nb * cfg->n_z * cfg->n_lnm;
-  Y3B_TRY(d_S.alloc(nS));
-  Y3B_TRY(gl_nodes_device(-1.0, 1.0, cfg->n_q, d_glt.get(), d_glw.get(), s));
+  // The inputs (copied at once) | GL rule | lnM | z | S.
+  const size_t ne = edges.size(), np = plob->n, nS = (size_t)nb * cfg->n_z * cfg->n_lnm;
+  std::vector<double> in(edges);
+  in.insert(in.end(), cfg->zob_min, cfg->zob_min + nb);
+  in.insert(in.end(), cfg->zob_max, cfg->zob_max + nb);
+  in.insert(in.end(), cfg->sigma_z, cfg->sigma_z + nb);
+  in.insert(in.end(), plob->z, plob->z + np);
+  in.insert(in.end(), plob->coef, plob->coef + 8 * np);
+  std::vector<int> ints(plo);
+  ints.insert(ints.end(), phi_.begin(), phi_.end());
+  ints.insert(ints.end(), bin_pair.begin(), bin_pair.end());
+  const size_t n_in = in.size();
+  in.resize(n_in + (ints.size() + 1) / 2);
+  std::memcpy(in.data() + n_in, ints.data(), ints.size() * sizeof(int));
+  const size_t need = in.size() + 2 * (size_t)cfg->n_q + cfg->n_lnm + cfg->n_z + nS;
+  std::unique_lock<std::mutex> lock(g_selfunc_mu, std::defer_lock);
+  DevBuf<double> own;
+  double *dev = nullptr, *unused = nullptr;
+  if (need <= kSelFuncWork && lock.try_lock()) {
+    Y3B_TRY(scratch_address(&unused, &dev));
+  } else {
+    Y3B_TRY(own.alloc(need));
+    dev = own.get();
+  }
+  Y3B_CUDA(cudaMemcpyAsync(dev, in.data(), in.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+  double* d_glt = dev + in.size();
+  double* d_glw = d_glt + cfg->n_q;
+  double* d_lnm = d_glw + cfg->n_q;
+  double* d_z = d_lnm + cfg->n_lnm;
+  double* d_S = d_z + cfg->n_z;
+  Y3B_TRY(gl_nodes_device(-1.0, 1.0, cfg->n_q, d_glt, d_glw, s));
 
   SelFuncArgs a;
   a.n_lnm = cfg->n_lnm;
@@ -253,28 +417,24 @@ y3b_sel_function(const y3b_selfunc_config* cfg, const y3b_mor* mor,
   a.mor_kind = mor->kind;
   for (int i = 0; i < 8; ++i) a.mor[i] = mor->p[i];
   a.n_plob = plob->n;
-  a.plob_z = d_pz.get();
-  a.plob_coef = d_pc.get();
-  a.edges = d_edges.get();
-  a.pair_lo = d_plo.get();
-  a.pair_hi = d_phi.get();
-  a.bin_pair = d_bp.get();
-  a.zob_min = d_zmin.get();
-  a.zob_max = d_zmax.get();
-  a.sigma_z = d_sz.get();
-  a.gl_t = d_glt.get();
-  a.gl_w = d_glw.get();
-  a.lnm_out = d_lnm.get();
-  a.z_out = d_z.get();
-  a.S_out = d_S.get();
-  long long warps = (long long)cfg->n_lnm * cfg->n_z;
-  int blocks = (int)((warps * 32 + 127) / 128);
-  sel_function_kernel<<<blocks, 128, 0, s>>>(a);
-  count_launch();
-  Y3B_CUDA(cudaGetLastError());
-  Y3B_CUDA(cudaMemcpyAsync(lnm_out, d_lnm.get(), cfg->n_lnm * sizeof(double), cudaMemcpyDeviceToHost, s));
-  Y3B_CUDA(cudaMemcpyAsync(z_out, d_z.get(), cfg->n_z * sizeof(double), cudaMemcpyDeviceToHost, s));
-  Y3B_CUDA(cudaMemcpyAsync(S_out, d_S.get(), nS * sizeof(double), cudaMemcpyDeviceToHost, s));
+  a.edges = dev;
+  a.zob_min = a.edges + ne;
+  a.zob_max = a.zob_min + nb;
+  a.sigma_z = a.zob_max + nb;
+  a.plob_z = a.sigma_z + nb;
+  a.plob_coef = a.plob_z + np;
+  a.pair_lo = reinterpret_cast<const int*>(dev + n_in);
+  a.pair_hi = a.pair_lo + plo.size();
+  a.bin_pair = a.pair_hi + phi_.size();
+  a.gl_t = d_glt;
+  a.gl_w = d_glw;
+  a.lnm_out = d_lnm;
+  a.z_out = d_z;
+  a.S_out = d_S;
+  Y3B_TRY(launch_sel_function(a, chained(plo, phi_, edges.size()), s));
+  Y3B_CUDA(cudaMemcpyAsync(lnm_out, d_lnm, cfg->n_lnm * sizeof(double), cudaMemcpyDeviceToHost, s));
+  Y3B_CUDA(cudaMemcpyAsync(z_out, d_z, cfg->n_z * sizeof(double), cudaMemcpyDeviceToHost, s));
+  Y3B_CUDA(cudaMemcpyAsync(S_out, d_S, nS * sizeof(double), cudaMemcpyDeviceToHost, s));
   Y3B_CUDA(cudaStreamSynchronize(s));
   return Y3B_OK;
 }
@@ -294,17 +454,22 @@ struct SelGLTablesDev {
   const double* sv;
 };
 
-__global__ void
-hmf_axis_kernel(const double* m_h, int n, double om_minus_onu, double* out)
+// One CTA per bin b: W_b[k] = sum_q zfac[q] hmf(k, q) sel_b(k, q)
+// (n_operator_sel_gl_t.hh:115-124), one warp per lnM node with the lanes over
+// q, then the plain lnM moments n0, n1, m2 with fixed-order tree sums
+// (129-141).  Everything that depends on q alone (z factor, HMF and selection
+// z cells) is formed once, one q a thread; a thread that summed a node's 64 q
+// by itself, both bilinear searches per term, took 190 us at 96 x 64.  A
+// selection cell of -1 marks a z outside its box (sel_function_t.hh:228-242).
+constexpr int kBuildThreads = 1024;
+
+__host__ __device__ inline size_t
+build_smem_bytes(int n_z)
 {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = log(m_h[i] * om_minus_onu);
+  return ((size_t)3 * n_z + kBuildThreads) * sizeof(double) + (size_t)2 * n_z * sizeof(int);
 }
 
-// One CTA per bin b; thread k evaluates W_b[k] = sum_q zfac[q] hmf(k,q)
-// sel_b(k,q) (n_operator_sel_gl_t.hh:115-124); the block then forms the
-// plain lnM moments n0, n1, m2 with fixed-order tree sums (129-141).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBuildThreads)
 selgl_build_kernel(int n_lnm, int n_z, const double* lnm_x, const double* lnm_w,
                    const double* z_x, const double* z_w, double lnm_lo, double lnm_hi,
                    y3b_cosmo c, SelGLTablesDev t, int include_sci, int n_sel_lnm,
@@ -314,8 +479,14 @@ selgl_build_kernel(int n_lnm, int n_z, const double* lnm_x, const double* lnm_w,
 {
   extern __shared__ double sh[];
   double* zfac = sh;             // [n_z]
-  double* red = sh + n_z;        // [blockDim.x]
-  const int b = blockIdx.x;
+  double* hu = zfac + n_z;       // [n_z] weight in the HMF z cell
+  double* su = hu + n_z;         // [n_z] weight in the selection z cell
+  double* red = su + n_z;        // [blockDim.x]
+  int* hy = reinterpret_cast<int*>(red + kBuildThreads);  // [n_z] HMF z cell
+  int* sy = hy + n_z;                                     // [n_z] selection z cell, or -1
+  const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double slo = sel_lnm[0], shi = sel_lnm[n_sel_lnm - 1];
+  const double zlo = sel_z[0], zhi = sel_z[n_sel_z - 1];
   for (int q = threadIdx.x; q < n_z; q += blockDim.x) {
     double z = z_x[q], dv;
     if (!dv_do_dz(t.dz, t.da, t.n_dist, c.om, c.ol, c.ok, c.h0, z, &dv)) {
@@ -324,28 +495,53 @@ selgl_build_kernel(int n_lnm, int n_z, const double* lnm_x, const double* lnm_w,
     }
     double sci = (include_sci && t.n_sci > 0) ? interp1d_clamp(t.sz, t.sv, t.n_sci, z) : 1.0;
     zfac[q] = z_w[q] * dv * omega_z_des(z) * sci;
+    const double zh = fmin(fmax(z, t.hz[0]), t.hz[t.n_hz - 1]);
+    const int yh = bsearch_cell(t.hz, t.n_hz, zh);
+    hy[q] = yh;
+    hu[q] = (zh - t.hz[yh]) / (t.hz[yh + 1] - t.hz[yh]);
+    const int ys = z < zlo || z > zhi ? -1 : bsearch_cell(sel_z, n_sel_z, z);
+    sy[q] = ys;
+    su[q] = ys < 0 ? 0.0 : (z - sel_z[ys]) / (sel_z[ys + 1] - sel_z[ys]);
   }
   __syncthreads();
-  // Table box of the selection function (sel_function_t.hh:228-242).
-  const double slo = sel_lnm[0], shi = sel_lnm[n_sel_lnm - 1];
-  const double zlo = sel_z[0], zhi = sel_z[n_sel_z - 1];
   const double* plane = S_stack + (size_t)b * n_sel_z * n_sel_lnm;
-  double n0 = 0.0, n1 = 0.0;
-  for (int k = threadIdx.x; k < n_lnm; k += blockDim.x) {
-    double lnM = lnm_x[k];
+  for (int k = warp; k < n_lnm; k += kBuildThreads / 32) {
+    const double lnM = lnm_x[k];
+    const double xh = fmin(fmax(lnM, t.hax[0]), t.hax[t.n_hm - 1]);
+    const int ih = bsearch_cell(t.hax, t.n_hm, xh);
+    const double th = (xh - t.hax[ih]) / (t.hax[ih + 1] - t.hax[ih]);
+    const double hs = c.hmf_s * (lnM * kLog10e - kHmfPivot) + c.hmf_q;
+    const bool in = !(lnM < slo || lnM > shi);
+    const double xs = fmin(fmax(lnM, slo), shi);
+    const int is = bsearch_cell(sel_lnm, n_sel_lnm, xs);
+    const double ts = (xs - sel_lnm[is]) / (sel_lnm[is + 1] - sel_lnm[is]);
     double acc = 0.0;
-    for (int q = 0; q < n_z; ++q) {
-      double z = z_x[q];
-      double h = interp2d_clamp(t.hax, t.n_hm, t.hz, t.n_hz, t.dn, lnM, z) *
-                 (c.hmf_s * (lnM * kLog10e - kHmfPivot) + c.hmf_q);
-      double s = (lnM < slo || lnM > shi || z < zlo || z > zhi)
-                   ? 0.0
-                   : interp2d_clamp(sel_lnm, n_sel_lnm, sel_z, n_sel_z, plane, lnM, z);
+    for (int q = lane; q < n_z; q += 32) {
+      const double u = hu[q];
+      const double* h0 = t.dn + (size_t)hy[q] * t.n_hm + ih;
+      const double* h1 = h0 + t.n_hm;
+      const double h = ((1.0 - th) * (1.0 - u) * h0[0] + th * (1.0 - u) * h0[1] +
+                        (1.0 - th) * u * h1[0] + th * u * h1[1]) *
+                       hs;
+      double s = 0.0;
+      if (in && sy[q] >= 0) {
+        const double v = su[q];
+        const double* s0 = plane + (size_t)sy[q] * n_sel_lnm + is;
+        const double* s1 = s0 + n_sel_lnm;
+        s = (1.0 - ts) * (1.0 - v) * s0[0] + ts * (1.0 - v) * s0[1] + (1.0 - ts) * v * s1[0] +
+            ts * v * s1[1];
+      }
       acc += zfac[q] * h * s;
     }
-    W[(size_t)b * n_lnm + k] = acc;
-    n0 += lnm_w[k] * acc;
-    n1 += lnm_w[k] * acc * lnM;
+    acc = warp_sum(acc);
+    if (lane == 0) W[(size_t)b * n_lnm + k] = acc;
+  }
+  __syncthreads();
+  double n0 = 0.0, n1 = 0.0;
+  for (int k = threadIdx.x; k < n_lnm; k += blockDim.x) {
+    const double w = lnm_w[k] * W[(size_t)b * n_lnm + k];
+    n0 += w;
+    n1 += w * lnm_x[k];
   }
   n0 = block_sum<1024>(n0, red);
   n1 = block_sum<1024>(n1, red);
@@ -466,15 +662,14 @@ struct y3b_selgl {
   y3b_selgl_config cfg;
   cudaStream_t stream = nullptr;
   y3b::DevBuf<double> lnm_x, lnm_w, z_x, z_w;
-  y3b::DevBuf<double> W, norm, eff, mu2;
-  y3b::DevBuf<double> hax, hz, dn, dz, da, sz, sv, sel_lnm, sel_z, S;
-  y3b::DevBuf<int> status;
+  y3b::DevBuf<double> W, mom;   // mom: norm | lnm_eff | mu2 [n_bins each] | status word
+  y3b::DevBuf<double> tab, S;   // the sample's tables in one block; S_stack
   y3b::MisQuadCache quad;
   y3b::DevBuf<double> sh_in, sh_mis, sh_out;   // shear_by_pairs
   y3b::DevBuf<int> sh_int;
   y3b::DevBuf<double> tab_lx, tab_lxm, tab_v;  // miscentred-profile table (optional)
   int tab_nlx = 0, tab_nlxm = 0;
-  std::vector<double> h_norm, h_eff, h_mu2, h_lnm_x, h_lnm_w;
+  std::vector<double> h_norm, h_eff, h_mu2, h_lnm_x, h_lnm_w, h_tab;
   int n_bins = 0;
   bool built = false;
   double omega_m = 0.0;
@@ -507,7 +702,6 @@ y3b_selgl_create(const y3b_selgl_config* cfg, y3b_selgl** out)
   if (rc == Y3B_OK) rc = h->lnm_w.alloc(cfg->n_lnm);
   if (rc == Y3B_OK) rc = h->z_x.alloc(cfg->n_z);
   if (rc == Y3B_OK) rc = h->z_w.alloc(cfg->n_z);
-  if (rc == Y3B_OK) rc = h->status.alloc(1);
   if (rc == Y3B_OK)
     rc = y3b::gl_nodes_device(cfg->lnm_low, cfg->lnm_high, cfg->n_lnm, h->lnm_x.get(),
                               h->lnm_w.get(), h->stream);
@@ -570,54 +764,52 @@ y3b_selgl_build(y3b_selgl* h, const y3b_cosmo* c, const y3b_tables* t,
     return Y3B_ERR_INVALID;
   }
   cudaStream_t s = h->stream;
-  const int nb = sel->n_bins;
+  const int nb = sel->n_bins, n_sci = include_sci ? t->n_sci : 0;
   Y3B_TRY(h->W.alloc((size_t)nb * h->cfg.n_lnm));
-  Y3B_TRY(h->norm.alloc(nb));
-  Y3B_TRY(h->eff.alloc(nb));
-  Y3B_TRY(h->mu2.alloc(nb));
-  Y3B_TRY(h->hz.upload(t->hmf_z, t->n_hz, s));
-  Y3B_TRY(h->dn.upload(t->dndlnmh, (size_t)t->n_hz * t->n_hm, s));
-  Y3B_TRY(h->dz.upload(t->dist_z, t->n_dist, s));
-  Y3B_TRY(h->da.upload(t->dist_da, t->n_dist, s));
-  if (include_sci) {
-    Y3B_TRY(h->sz.upload(t->sci_z, t->n_sci, s));
-    Y3B_TRY(h->sv.upload(t->sci_val, t->n_sci, s));
-  }
-  Y3B_TRY(h->sel_lnm.upload(sel->lnm, sel->n_lnm, s));
-  Y3B_TRY(h->sel_z.upload(sel->z, sel->n_z, s));
+  Y3B_TRY(h->mom.alloc(3 * (size_t)nb + 1));
+  // One block: HMF mass axis ln(m_h (Omega_M - Omega_nu)) (hmf_t.hh:15-25) |
+  // z | dn/dlnM | distances | Sigma_crit^-1 | selection axes.
+  std::vector<double>& v = h->h_tab;
+  v.clear();
+  auto put = [&](const double* p, size_t n) {
+    const size_t at = v.size();
+    if (n) v.insert(v.end(), p, p + n);
+    return at;
+  };
+  const size_t o_ax = put(t->hmf_m_h, t->n_hm), o_hz = put(t->hmf_z, t->n_hz);
+  for (int i = 0; i < t->n_hm; ++i) v[o_ax + i] = std::log(v[o_ax + i] * (c->om - c->onu));
+  const size_t o_dn = put(t->dndlnmh, (size_t)t->n_hz * t->n_hm);
+  const size_t o_dz = put(t->dist_z, t->n_dist), o_da = put(t->dist_da, t->n_dist);
+  const size_t o_sz = put(t->sci_z, n_sci), o_sv = put(t->sci_val, n_sci);
+  const size_t o_sl = put(sel->lnm, sel->n_lnm), o_sel_z = put(sel->z, sel->n_z);
+  Y3B_TRY(h->tab.upload(v.data(), v.size(), s));
   Y3B_TRY(h->S.upload(sel->S_stack, (size_t)nb * sel->n_z * sel->n_lnm, s));
-  // HMF mass axis ln(m_h (Omega_M - Omega_nu)) (hmf_t.hh:15-25).
-  DevBuf<double> mh;
-  Y3B_TRY(mh.upload(t->hmf_m_h, t->n_hm, s));
-  Y3B_TRY(h->hax.alloc(t->n_hm));
-  hmf_axis_kernel<<<(t->n_hm + 127) / 128, 128, 0, s>>>(mh.get(), t->n_hm, c->om - c->onu,
-                                                        h->hax.get());
-  count_launch();
-  Y3B_CUDA(cudaGetLastError());
-  Y3B_CUDA(cudaMemsetAsync(h->status.get(), 0, sizeof(int), s));
-  SelGLTablesDev td{t->n_hm, t->n_hz, t->n_dist, include_sci ? t->n_sci : 0,
-                    h->hax.get(), h->hz.get(), h->dn.get(), h->dz.get(), h->da.get(),
-                    include_sci ? h->sz.get() : nullptr, include_sci ? h->sv.get() : nullptr};
-  int threads = 32;
-  while (threads < h->cfg.n_lnm && threads < 256) threads <<= 1;
-  size_t shm = (h->cfg.n_z + threads) * sizeof(double);
-  selgl_build_kernel<<<nb, threads, shm, s>>>(
+  double* mom = h->mom.get();
+  int* status = reinterpret_cast<int*>(mom + 3 * (size_t)nb);
+  Y3B_CUDA(cudaMemsetAsync(status, 0, sizeof(double), s));
+  const double* d = h->tab.get();
+  SelGLTablesDev td{t->n_hm, t->n_hz, t->n_dist, n_sci, d + o_ax, d + o_hz, d + o_dn, d + o_dz,
+                    d + o_da, include_sci ? d + o_sz : nullptr,
+                    include_sci ? d + o_sv : nullptr};
+  const size_t shm = build_smem_bytes(h->cfg.n_z);
+  if (shm > 48 * 1024)
+    Y3B_CUDA(cudaFuncSetAttribute(selgl_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)shm));
+  selgl_build_kernel<<<nb, kBuildThreads, shm, s>>>(
     h->cfg.n_lnm, h->cfg.n_z, h->lnm_x.get(), h->lnm_w.get(), h->z_x.get(), h->z_w.get(),
-    h->cfg.lnm_low, h->cfg.lnm_high, *c, td, include_sci, sel->n_lnm, h->sel_lnm.get(),
-    sel->n_z, h->sel_z.get(), h->S.get(), h->W.get(), h->norm.get(), h->eff.get(), h->mu2.get(),
-    h->status.get());
+    h->cfg.lnm_low, h->cfg.lnm_high, *c, td, include_sci, sel->n_lnm, d + o_sl, sel->n_z,
+    d + o_sel_z, h->S.get(), h->W.get(), mom, mom + nb, mom + 2 * (size_t)nb, status);
   count_launch();
   Y3B_CUDA(cudaGetLastError());
-  h->h_norm.resize(nb);
-  h->h_eff.resize(nb);
-  h->h_mu2.resize(nb);
-  Y3B_CUDA(cudaMemcpyAsync(h->h_norm.data(), h->norm.get(), nb * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
-  Y3B_CUDA(cudaMemcpyAsync(h->h_eff.data(), h->eff.get(), nb * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
-  Y3B_CUDA(cudaMemcpyAsync(h->h_mu2.data(), h->mu2.get(), nb * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
-  int st = read_device_status(h->status.get(), s);
+  std::vector<double> hm(3 * (size_t)nb + 1);
+  Y3B_CUDA(cudaMemcpyAsync(hm.data(), mom, hm.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+  Y3B_CUDA(cudaStreamSynchronize(s));
+  h->h_norm.assign(hm.begin(), hm.begin() + nb);
+  h->h_eff.assign(hm.begin() + nb, hm.begin() + 2 * (size_t)nb);
+  h->h_mu2.assign(hm.begin() + 2 * (size_t)nb, hm.end() - 1);
+  int code;
+  std::memcpy(&code, &hm.back(), sizeof code);
+  const int st = device_status_rc(code);
   h->n_bins = nb;
   h->omega_m = c->om;
   h->built = (st == Y3B_OK);
@@ -977,90 +1169,6 @@ y3b_nfw_mis(int which, int n, const double* r, const double* rmis, const double*
 // bin pairing, the per-bin photo-z edges and widths, the projection table)
 // lives in one file-scope __device__ array of fixed size that every call
 // shares.
-#include <cuda.h>
-
-#include <mutex>
-
-namespace y3b {
-
-constexpr int kNoAllocMaxQ = 1024;      // N_q
-constexpr int kNoAllocMaxBins = 256;    // bins
-constexpr int kNoAllocMaxPlob = 256;    // projection-table z nodes
-constexpr size_t kNoAllocScratchDoubles =
-  2 * kNoAllocMaxQ + kMaxEdges + 3 * kNoAllocMaxBins + 9 * kNoAllocMaxPlob +
-  (2 * kMaxPairs + kNoAllocMaxBins);    // last term holds the int tables
-static __device__ __align__(256) double g_selfunc_scratch[kNoAllocScratchDoubles];
-
-// Device address of g_selfunc_scratch, looked up once per device context
-// (host code may not use the symbol itself: it names a host-side stand-in).
-// The address belongs to the context the module image was loaded into: a
-// caller that resets the device gets a new context, in which the array lives
-// elsewhere, so the cache is keyed by the context's unique id and the lookup
-// is repeated for a new one.
-static std::mutex g_scratch_mu;
-static void* g_scratch_addr[128];
-static unsigned long long g_scratch_ctx[128];
-
-// Unique id of the calling thread's current context (0 if it cannot be
-// read, in which case the address is looked up on every call).  The driver
-// entry points are fetched through the runtime: the library links no
-// driver-API import.
-static unsigned long long
-current_context_id()
-{
-  using GetCurrentFn = CUresult (*)(CUcontext*);
-  using GetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-  static GetCurrentFn get_current = nullptr;
-  static GetIdFn get_id = nullptr;
-  static bool resolved = false;
-  if (!resolved) {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<GetCurrentFn>(f);
-    f = nullptr;
-    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<GetIdFn>(f);
-    resolved = true;
-  }
-  CUcontext ctx = nullptr;
-  unsigned long long id = 0;
-  if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx ||
-      get_id(ctx, &id) != CUDA_SUCCESS)
-    return 0;
-  return id;
-}
-
-static int
-scratch_address(double** out)
-{
-  int dev = 0;
-  Y3B_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 128) {
-    set_error("y3b_sel_function_noalloc: device index %d out of range", dev);
-    return Y3B_ERR_INVALID;
-  }
-  std::lock_guard<std::mutex> lock(g_scratch_mu);
-  const unsigned long long ctx = current_context_id();
-  if (!g_scratch_addr[dev] || ctx == 0 || ctx != g_scratch_ctx[dev]) {
-    void* p = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&p, g_selfunc_scratch);
-    if (e != cudaSuccess || !p) {
-      set_error("cudaGetSymbolAddress(g_selfunc_scratch): %s", cudaGetErrorString(e));
-      return Y3B_ERR_CUDA;
-    }
-    g_scratch_addr[dev] = p;
-    // The lookup made the device's context current if it was not yet.
-    g_scratch_ctx[dev] = ctx ? ctx : current_context_id();
-  }
-  *out = static_cast<double*>(g_scratch_addr[dev]);
-  return Y3B_OK;
-}
-
-}  // namespace y3b
-
 extern "C" int
 y3b_sel_function_noalloc(const y3b_selfunc_config* cfg, const y3b_mor* mor,
                          const y3b_plob* plob, double* lnm_dev, double* z_dev, double* S_dev,
@@ -1175,9 +1283,5 @@ y3b_sel_function_noalloc(const y3b_selfunc_config* cfg, const y3b_mor* mor,
   a.lnm_out = lnm_dev;
   a.z_out = z_dev;
   a.S_out = S_dev;
-  long long warps = (long long)cfg->n_lnm * cfg->n_z;
-  int blocks = (int)((warps * 32 + 127) / 128);
-  sel_function_kernel<<<blocks, 128, 0, s>>>(a);
-  count_launch();
-  return cuda_status(cudaGetLastError(), "sel_function_kernel (noalloc)");
+  return launch_sel_function(a, chained(plo, phi_, edges.size()), s);
 }
