@@ -42,3 +42,50 @@ def test_projection_shear_by_quadrature(gpu, n_lnm, radii, n_per_seg):
 def test_module_chain(gpu, mor, n_lnm, radii):
     _compare(dict(kind="module", mor=mor, tab_m=40, tab_z=24, n_q=17, n_lnm=n_lnm, n_z=19,
                   radii=radii), 1e-9)
+
+
+# The FP64 form on one node set: node counts of one tile and a remainder,
+# both table ends of the radii, and no shear.
+@pytest.mark.parametrize("n,n_m,n_z,n_t,radii", [(1, 33, 16, 40, 15), (3, 64, 32, 64, 1),
+                                                 (5, 65, 48, 97, 2), (2, 130, 16, 33, 0)])
+def test_fp64_engine(gpu, n, n_m, n_z, n_t, radii):
+    _compare(dict(kind="engine", api="device", precision="fp64", n=n, radii=radii, hmf_fp32=False,
+                  loglike=False, mixed_density=False, n_m=n_m, n_z=n_z, n_t=n_t, n_o=32, n_zo=9),
+             1e-11)
+
+
+def test_fp64_shear_outside_the_profile_table(gpu):
+    """Omega_m = 60 lies beyond the profile table (0.01 to 1, widened by 1.5
+    in x): such a point takes the direct quadrature, next to others that do
+    not.  With Sigma_crit^-1 = 1 the shear is the weighted sum of
+    y3b_nfw_mis profiles over the mass weights; both sides sum ~33 FP64 terms
+    of profiles good to ~1e-14."""
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+    from y3_cluster_cpp_b200 import synthetic
+
+    pts = [synthetic.fiducial(1) for _ in range(3)]
+    for p in pts:
+        p.tables["sci_val"] = np.ones_like(p.tables["sci_val"])
+    pts[1].om = 60.0
+    g = synthetic.grid(1, n_m=33, n_z=16, n_t=40, n_o=16, n_zo=8)
+    so = synthetic.shear_opts(n_theta=16, n_s=32, n_R=4)
+    t = pts[0].tables
+    eng = E.Engine([g], len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]),
+                   synthetic.plob_baseline(), max_points=3, n_sci=len(t["sci_z"]), shear=so)
+    out = eng.eval(pts, E.FP64, grid_of=lambda p: 0, weights=True)
+    lnM, wm = (v.cpu().numpy() for v in cases._gl(g["lnm_lo"], g["lnm_hi"], 33))
+    conc = so["c0"] * (np.exp(lnM) / so["c_pivot"]) ** so["c_slope"]
+    for p in range(3):
+        want = np.zeros((12, 4))
+        for k in range(33):
+            rho = cases.RHO_CRIT * pts[p].om
+            cen = E.nfw_mis("dsigma_single", so["R"], 1e-9, lnM[k], conc[k], rho, 16, 32, 20.0)
+            for i in range(4):
+                rmis = so["tau_mis"] * (so["lob_centers"][i] / 100) ** 0.2
+                mis = E.nfw_mis("dsigma", so["R"], rmis, lnM[k], conc[k], rho, 16, 32, 20.0)
+                phi = (1 - so["f_mis"]) * cen + so["f_mis"] * mis
+                for b in range(i, 12, 4):
+                    want[b] += wm[k] * out["W"][p, b, k] * phi
+        np.testing.assert_allclose(out["shear"][p], want, rtol=1e-11)
+    eng.close()

@@ -201,6 +201,7 @@ constexpr int kPrepThreads = 128;
 constexpr int kYfHdr = 8;        // floats of yf_kernel's FP32 header
 constexpr int kYfRowFields = 8;  // fields of yf_kernel's per-row block
 
+constexpr int kStatusWords = 2;  // device words reset by every evaluation
 constexpr int kEvalChunks = 8;  // chunks of a large host-buffer evaluation
 
 // Per-point prep, one CTA per point.  The point's packed tables (without the
@@ -1149,49 +1150,51 @@ direct_wreduce_kernel(const GridDev* grids, const PointDev* pts, const double* s
 // ---------------------------------------------------------------------------
 // Stacked miscentred profile Phi_i(R, k) = norm_k [(1 - f) DSigma(R / r_s)
 // + f DSigma_mis(R / r_s, tau R_lambda(lam_i) / r_s)], c(M) = c0 (M/Mp)^s,
-// rho = Omega_m rho_crit.  One warp per (point, i, R, k).
-template <typename T>
+// rho = Omega_m rho_crit, by direct quadrature: the FP64 form's points whose
+// x = R / r_s leaves the engine's profile table (Omega_m outside 0.01 to 1),
+// listed by shear_tab64_kernel.  One warp per (point, i, R, k).
 __global__ void __launch_bounds__(128)
-shear_phi_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_stride,
-                 ShearDev sh, MisQuad quad, double* Phi, int nI_max, int grid_mask)
+shear_phi_kernel(const GridDev* grids, const PointDev* pts, const int* list, const int* n_list,
+                 int w_stride, ShearDev sh, MisQuad quad, double* Phi, int nI_max)
 {
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long per_point = (long long)nI_max * sh.n_R * w_stride;
-  if (w >= per_point * n_points) return;
-  const int p = (int)(w / per_point);
-  long long r = w % per_point;
-  const int k = (int)(r % w_stride);
-  r /= w_stride;
-  const int iR = (int)(r % sh.n_R);
-  const int i = (int)(r / sh.n_R);
-  const PointDev pt = pts[p];
-  if (!grid_in_mask(grid_mask, pt.grid)) return;
-  const GridDev& G = grids[pt.grid];
-  if (i >= G.nI || k >= G.n_m) return;
-  const double lnM = G.xm[k];
-  const double c = sh.c0 * pow(exp(lnM) / sh.c_pivot, sh.c_slope);
-  const double rho = kRhoCrit * pt.om;
-  const double rs = nfw_rs(lnM, c, rho);
-  const double rmis = sh.tau_mis * pow(sh.lob[i] / 100.0, 0.2);
-  const double R = sh.R[iR];
-  T mis = mis_partial<T>(quad, (T)(R / rs), (T)(rmis / rs), true, lane);
-  mis = warp_sum(mis);
-  if (lane == 0) {
-    const double cen = (double)NfwUnit<T>::dsigma((T)(R / rs));
-    Phi[(((size_t)p * nI_max + i) * sh.n_R + iR) * w_stride + k] =
-      nfw_norm(lnM, c, rho) * ((1.0 - sh.f_mis) * cen + sh.f_mis * (double)mis);
+  const long long n = per_point * *n_list, step = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n;
+       w += step) {
+    const int p = list[w / per_point];
+    long long r = w % per_point;
+    const int k = (int)(r % w_stride);
+    r /= w_stride;
+    const int iR = (int)(r % sh.n_R);
+    const int i = (int)(r / sh.n_R);
+    const PointDev pt = pts[p];
+    const GridDev& G = grids[pt.grid];
+    if (i >= G.nI || k >= G.n_m) continue;
+    const double lnM = G.xm[k];
+    const double c = sh.c0 * pow(exp(lnM) / sh.c_pivot, sh.c_slope);
+    const double rho = kRhoCrit * pt.om;
+    const double rs = nfw_rs(lnM, c, rho);
+    const double rmis = sh.tau_mis * pow(sh.lob[i] / 100.0, 0.2);
+    const double R = sh.R[iR];
+    const double mis = warp_sum(mis_partial<double>(quad, R / rs, rmis / rs, true, lane));
+    if (lane == 0)
+      Phi[(((size_t)p * nI_max + i) * sh.n_R + iR) * w_stride + k] =
+        nfw_norm(lnM, c, rho) *
+        ((1.0 - sh.f_mis) * NfwUnit<double>::dsigma(R / rs) + sh.f_mis * mis);
   }
 }
 
-// Miscentred profile table for the mixed form.  For a richness bin i and a
+// Miscentred profile table.  For a richness bin i and a
 // radius R the ratio x_mis / x = r_mis,i / R does not depend on the point or
 // the mass, so DeltaSigma_mis(x, x_mis) is a smooth function of u = ln x
 // alone: tabulated once per engine in FP64 at kMisNx nodes per (i, R) pair
-// (the same direct quadrature as the FP64 form), read with 4-point Lagrange
-// interpolation in u (relative error ~1e-8 at this spacing).  One more row
-// after the (i, R) pairs holds the centred DeltaSigma_NFW(x) on the same
-// nodes, so the mixed form reads both profiles with the same weights.
+// (the direct quadrature).  The mixed form reads it with 4-point Lagrange
+// interpolation in u (relative error ~1e-8 at this spacing), the FP64 form
+// with 6 points: DeltaSigma is analytic for |Im u| < pi, so at the spacing
+// du ~ 0.006 their error is about (5/2 3/2 1/2)^2 (du / pi)^6 ~ 1e-16.  One
+// more row after the (i, R) pairs holds the centred DeltaSigma_NFW(x) on the
+// same nodes, so both profiles are read with the same weights.
 constexpr int kMisNx = 2048;
 
 // The miscentred rows come from launch_mis_pairs, the centred one from here.
@@ -1249,6 +1252,61 @@ shear_tab_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_
     }
   }
   if (bad) set_err(status, kDevDomain);
+}
+
+// Phi_i(R, k) of the FP64 form from the table, one thread per (point, k,
+// R): 64 x 128 closed-form evaluations a value by direct quadrature took 16.6
+// ms for 12 points at 64 masses.  r_s is a power of the mass, so a point
+// stays inside the table when its first and last masses do; the others are
+// appended to `list` (thread k = 0, R = 0) and redone by shear_phi_kernel.
+// Table nodes kept clear of the ends by a node more than the weights need.
+__global__ void __launch_bounds__(128)
+shear_tab64_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_stride,
+                   ShearDev sh, const double* tab, double u0, double inv_du, double* Phi,
+                   int nI_max, int grid_mask, int* list, int* n_list)
+{
+  const int iR = blockIdx.y;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)n_points * w_stride) return;
+  const int p = (int)(t / w_stride), k = (int)(t % w_stride);
+  const PointDev pt = pts[p];
+  if (!grid_in_mask(grid_mask, pt.grid)) return;
+  const GridDev& G = grids[pt.grid];
+  if (k >= G.n_m) return;
+  const double rho = kRhoCrit * pt.om;
+  auto conc = [&](double lnM) { return sh.c0 * pow(exp(lnM) / sh.c_pivot, sh.c_slope); };
+  if (k == 0 && iR == 0) {
+    bool in = true;
+    for (int e = 0; e < 2; ++e) {
+      const double lnM = G.xm[e ? G.n_m - 1 : 0], l = log(nfw_rs(lnM, conc(lnM), rho));
+      for (int r = 0; r < sh.n_R; ++r) {
+        const double tt = (sh.lnR[r] - l - u0) * inv_du;
+        in &= tt >= 3.0 && tt <= kMisNx - 5.0;
+      }
+    }
+    if (!in) list[atomicAdd(n_list, 1)] = p;
+  }
+  const double lnM = G.xm[k], c = conc(lnM);
+  const double norm = nfw_norm(lnM, c, rho);
+  const double tt = (sh.lnR[iR] - log(nfw_rs(lnM, c, rho)) - u0) * inv_du;
+  const int j = (int)fmin(fmax(floor(tt), 2.0), kMisNx - 4.0);
+  // Lagrange weights of the nodes j - 2 .. j + 3 at f = tt - j.
+  const double f = tt - j;
+  const double a = f + 2.0, b = f + 1.0, d = f - 1.0, e = f - 2.0, g = f - 3.0;
+  const double l[6] = {-b * f * d * e * g / 120.0, a * f * d * e * g / 24.0,
+                       -a * b * d * e * g / 12.0,  a * b * f * e * g / 12.0,
+                       -a * b * f * d * g / 24.0,  a * b * f * d * e / 120.0};
+  auto read = [&](const double* row) {
+    const double* y = row + j - 2;
+    double v = 0.0;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v += l[m] * __ldg(y + m);
+    return v;
+  };
+  const double cen = (1.0 - sh.f_mis) * read(tab + (size_t)nI_max * sh.n_R * kMisNx);
+  for (int i = 0; i < G.nI; ++i)
+    Phi[(((size_t)p * nI_max + i) * sh.n_R + iR) * w_stride + k] =
+      norm * (cen + sh.f_mis * read(tab + ((size_t)i * sh.n_R + iR) * kMisNx));
 }
 
 // N_b = sum_k w_k W_b(k); N_b(R) = sum_k w_k W^g_b(k) Phi_i(R, k).  CTA per
@@ -1340,12 +1398,13 @@ struct y3b_engine {
   y3b::TableLayout lay;
   y3b::ShearDev shear;
   y3b::MisQuadCache quad;
-  y3b::DevBuf<double> mis_tab;          // [nI_max * n_R + 1][kMisNx], mixed form
+  y3b::DevBuf<double> mis_tab;          // [nI_max * n_R + 1][kMisNx]
   double mis_u0 = 0.0, mis_du = 1.0;
   cudaStream_t stream = nullptr;
   y3b::DevBuf<y3b::PointDev> pts;
   y3b::DevBuf<double> tables, s64, W, Wg, Phi, counts, shear_out;
   y3b::DevBuf<float> s32;
+  // status: code of the device-side checks | points listed for shear_phi_kernel
   y3b::DevBuf<int> status, order, tile_start;
   y3b::DevBuf<int> stage_ct;  // [2] lam_t stages issued / dense, last contraction
   y3b::DevBuf<int> tile_list;
@@ -1920,7 +1979,7 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
       (rc = e->s64.alloc(N * e->s64_stride)) || (rc = e->s32.alloc(N * e->s32_stride)) ||
       (rc = e->W.alloc(N * e->nB_max * (size_t)e->w_stride)) ||
       (rc = e->Wg.alloc(N * e->nB_max * (size_t)e->w_stride)) ||
-      (rc = e->counts.alloc(N * e->nB_max)) || (rc = e->status.alloc(1)) ||
+      (rc = e->counts.alloc(N * e->nB_max)) || (rc = e->status.alloc(kStatusWords)) ||
       (rc = e->stage_ct.alloc(2)) ||
       (rc = e->order.alloc(N)) || (rc = e->tile_start.alloc(N + 1)) ||
       (rc = e->tile_list.alloc(N * (size_t)e->tile_cap_pp)) ||
@@ -2021,7 +2080,7 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
     set_error("an engine with FP32 dndlnmh tables (hmf_fp32) evaluates the mixed form only");
     return Y3B_ERR_INVALID;
   }
-  Y3B_CUDA(cudaMemsetAsync(e->status.get(), 0, sizeof(int), s));
+  Y3B_CUDA(cudaMemsetAsync(e->status.get(), 0, kStatusWords * sizeof(int), s));
   // The stage counters cover one evaluation call: zeroed by its first chunk.
   if (w_off == 0 && prec == Y3B_MIXED)
     Y3B_CUDA(cudaMemsetAsync(e->stage_ct.get(), 0, 2 * sizeof(int), s));
@@ -2086,16 +2145,22 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
   const bool shear = e->cfg.with_shear && d_shear;
   if (shear) {
     StageTimer t(e, s, 2);
-    long long warps = (long long)n * e->nI_max * e->shear.n_R * e->w_stride;
-    long long blocks = (warps * 32 + 127) / 128;
-    if (prec == Y3B_FP64)
-      shear_phi_kernel<double><<<(unsigned)blocks, 128, 0, s>>>(
-        e->d_grids.get(), d_pts, n, e->w_stride, e->shear, e->quad.view(), Phi,
-        e->nI_max, grid_mask);
-    else
-      shear_tab_kernel<<<(unsigned)(((long long)n * e->w_stride + 127) / 128), 128, 0, s>>>(
+    const unsigned blocks = (unsigned)(((long long)n * e->w_stride + 127) / 128);
+    if (prec == Y3B_FP64) {
+      int *list = e->order.get(), *n_list = e->status.get() + 1;  // order: the mixed form's planner
+      shear_tab64_kernel<<<dim3(blocks, e->shear.n_R), 128, 0, s>>>(
+        e->d_grids.get(), d_pts, n, e->w_stride, e->shear, e->mis_tab.get(), e->mis_u0,
+        1.0 / e->mis_du, Phi, e->nI_max, grid_mask, list, n_list);
+      count_launch();
+      Y3B_CUDA(cudaGetLastError());
+      shear_phi_kernel<<<4 * e->n_ctas, 128, 0, s>>>(e->d_grids.get(), d_pts, list, n_list,
+                                                     e->w_stride, e->shear, e->quad.view(), Phi,
+                                                     e->nI_max);
+    } else {
+      shear_tab_kernel<<<blocks, 128, 0, s>>>(
         e->d_grids.get(), d_pts, n, e->w_stride, e->shear, e->mis_tab.get(), e->mis_u0,
         1.0 / e->mis_du, Phi, e->nI_max, grid_mask, e->status.get());
+    }
     count_launch();
     Y3B_CUDA(cudaGetLastError());
   }
