@@ -44,10 +44,13 @@ def test_module_chain(gpu, mor, n_lnm, radii):
                   radii=radii), 1e-9)
 
 
-# The FP64 form on one node set: node counts of one tile and a remainder,
-# both table ends of the radii, and no shear.
+# The FP64 form: lnM tiles of 64 rows, groups of 32 z_t columns and stages of
+# 16 lam_t nodes, whole and with remainders; more points than one workspace
+# round (128); both table ends of the radii, and no shear.
 @pytest.mark.parametrize("n,n_m,n_z,n_t,radii", [(1, 33, 16, 40, 15), (3, 64, 32, 64, 1),
-                                                 (5, 65, 48, 97, 2), (2, 130, 16, 33, 0)])
+                                                 (5, 65, 48, 97, 2), (2, 130, 16, 33, 0),
+                                                 (3, 256, 128, 256, 0), (1, 2, 16, 2, 0),
+                                                 (150, 40, 16, 48, 0)])
 def test_fp64_engine(gpu, n, n_m, n_z, n_t, radii):
     _compare(dict(kind="engine", api="device", precision="fp64", n=n, radii=radii, hmf_fp32=False,
                   loglike=False, mixed_density=False, n_m=n_m, n_z=n_z, n_t=n_t, n_o=32, n_zo=9),

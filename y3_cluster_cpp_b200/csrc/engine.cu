@@ -27,6 +27,7 @@
 #include "host_common.h"
 #include "likelihood.cuh"
 #include "mis_quad.cuh"
+#include "mor_norm.cuh"
 
 namespace y3b {
 
@@ -56,6 +57,15 @@ uk_kernel(int nI, int n_z, int n_t, int n_t_pad, const double* wl, const double*
   if (idx >= nI * n_z * n_t_pad) return;
   const int t = idx % n_t_pad, iq = idx / n_t_pad;
   UK[idx] = t < n_t ? (float)(wl[t] * Ki[(size_t)iq * n_t + t]) : 0.f;
+}
+
+__global__ void
+uk64_kernel(int nI, int n_z, int n_t, const double* wl, const double* Ki, double* UK)
+{
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= nI * n_z * n_t) return;
+  const int q = idx % n_z, t = (idx / n_z) % n_t, i = idx / (n_z * n_t);
+  UK[idx] = wl[t] * Ki[((size_t)i * n_z + q) * n_t + t];
 }
 
 struct SzBins {
@@ -115,30 +125,9 @@ struct PrepArgs {
   size_t f_stride;
   int* win_tile;    // mixed form: [n][win_stride] lam_t stage window per local tile
   int win_stride;
+  int f64_rounds;   // FP64 form: the matrix product has a workspace
+  int *list, *n_list;  // FP64 form: points left to the direct sum
 };
-
-// MOR normalisation D = Phi(b) - Phi(a) in FP64, a = (l_lo - mu)/s,
-// b = (l_hi - mu)/s.  The lam_t domain is many sigma wide, so at most one
-// tail is open: D = 1 exactly when both are below half an FP64 ulp
-// (a < -8.5, b > 8.5); with one tail closed D = Phi(b) or Phi(-a), a single
-// erfc on the side that does not cancel.  Kept out of line: the rare path.
-__device__ __noinline__ double
-mor_norm_slow(double a, double b)
-{
-  constexpr double kInvSqrt2 = 0.70710678118654752440;
-  if (a < -8.5)  // low tail closed: D = Phi(b)
-    return b < 0.0 ? 0.5 * erfc(-b * kInvSqrt2) : 1.0 - 0.5 * erfc(b * kInvSqrt2);
-  if (b > 8.5)  // high tail closed: D = Phi(-a)
-    return a > 0.0 ? 0.5 * erfc(a * kInvSqrt2) : 1.0 - 0.5 * erfc(-a * kInvSqrt2);
-  return phi_diff(a, b);
-}
-
-__device__ __forceinline__ double
-mor_norm(double a, double b)
-{
-  if (a < -8.5 && b > 8.5) return 1.0;
-  return mor_norm_slow(a, b);
-}
 
 // v 2^e for an integer-valued e: two power-of-two factors, each a normal
 // FP32 value, so the product is exact wherever it is a normal or subnormal
@@ -149,26 +138,6 @@ mul_pow2(float v, double e)
   const int ei = (int)fmin(fmax(e, -252.0), 254.0);
   const int e1 = ei >> 1, e2 = ei - e1;
   return (v * __int_as_float((e1 + 127) << 23)) * __int_as_float((e2 + 127) << 23);
-}
-
-// ln D for the same D, finite where D itself underflows FP64 (mu more than
-// ~38 sigma outside the lam_t domain).  With Q(x) = erfc(x / sqrt 2) / 2 =
-// erfcx(x / sqrt 2) exp(-x^2 / 2) / 2: for 0 < a < b, D = Q(a) - Q(b) and
-// ln D = ln Q(a) + log1p(-Q(b) / Q(a)); for a < b < 0, D = Q(-b) - Q(-a)
-// likewise; otherwise mu lies inside the domain and D is not small.
-__device__ __noinline__ double
-ln_mor_norm(double a, double b)
-{
-  constexpr double kInvSqrt2 = 0.70710678118654752440;
-  if (a > 0.0) {
-    const double ra = erfcx(a * kInvSqrt2), rb = erfcx(b * kInvSqrt2);
-    return log(0.5 * ra) - 0.5 * a * a + log1p(-(rb / ra) * exp(-0.5 * (b - a) * (b + a)));
-  }
-  if (b < 0.0) {
-    const double ra = erfcx(-a * kInvSqrt2), rb = erfcx(-b * kInvSqrt2);
-    return log(0.5 * rb) - 0.5 * b * b + log1p(-(ra / rb) * exp(-0.5 * (a - b) * (a + b)));
-  }
-  return log(mor_norm(a, b));
 }
 
 // ln D in FP32, the same cases as ln_mor_norm; with both tails open (mu
@@ -201,7 +170,7 @@ constexpr int kPrepThreads = 128;
 constexpr int kYfHdr = 8;        // floats of yf_kernel's FP32 header
 constexpr int kYfRowFields = 8;  // fields of yf_kernel's per-row block
 
-constexpr int kStatusWords = 2;  // device words reset by every evaluation
+constexpr int kStatusWords = 3;  // device words reset by every evaluation
 constexpr int kEvalChunks = 8;  // chunks of a large host-buffer evaluation
 
 // Per-point prep, one CTA per point.  The point's packed tables (without the
@@ -209,7 +178,9 @@ constexpr int kEvalChunks = 8;  // chunks of a large host-buffer evaluation
 // with bulk (TMA) copies completing on an mbarrier; then, per point:
 //   both forms: cz_q = v_q dV(z_q) Omega(z_q), czs_q = cz_q Sci(z_q),
 //         alpha_k, beta_q (s64);
-//   FP64 form: P0 = n(M_k,z_q) / (sqrt(2 pi) s D_kq);
+//   FP64 form: the HMF cells and weights, the matrix product's header and
+//         windows; P0 = n(M_k,z_q) / (sqrt(2 pi) s D_kq) for the points it
+//         does not admit, which are listed for the direct sum;
 //   mixed form: a_k, b_q, delta_t, c1, c2, C_j(q), C^g_j(q) for the
 //         contraction, the lam_t windows, and yf_kernel's inputs (row
 //         blocks, z rows, the log2 D table).
@@ -454,6 +425,65 @@ prep_kernel(PrepArgs a)
   if (!a.mixed) {
     double* __restrict__ P0 = s64 + Gp->o_P0;
     const double xl0 = Gp->xl[0], xl1 = Gp->xl[Gp->n_t - 1];
+    // Matrix-product form (fp64_form.cu): centres on multiples of 2^-20 (the
+    // differences from them are exact), the exponents of its factors G and
+    // H and of the edge factor exp(v^2 / 2 s^2) together below kF64MaxExp
+    // (F = S / (G H) then stays in range too where the product matters), and
+    // the lam_t window of each 64-row tile: outside mu -+ sqrt(e^2 + (8.7 s)^2),
+    // e the distance of mu to the domain, the renormalised density is below
+    // 4e-17 of its peak.
+    constexpr double kSnap = 1048576.0, kWin64 = 8.7;
+    const double a0 = rint(A0 * kSnap) / kSnap, b0 = rint(B0 * kSnap) / kSnap, l0 = a0 + b0;
+    const double am = 0.5 * ((red[3] - red[2]) - (red[5] - red[4])) + 1e-6;
+    const double bm = 0.5 * (red[5] - red[4]) + 1e-6;
+    const double dm = fmax(fabs(xl0 - l0), fabs(xl1 - l0));
+    const double vm = fmax(fmax(xl0 - red[2], red[3] - xl1), 0.0);
+    const double ex = (bm * (dm + am + 0.5 * bm) + 0.5 * vm * vm) * inv_s * inv_s;
+    const bool product = a.f64_rounds && ex <= kF64MaxExp;
+    double* hdr = s64 + Gp->o_f64;
+    if (tid == 0) {
+      hdr[0] = product ? 1.0 : 0.0;
+      hdr[1] = a0;
+      hdr[2] = b0;
+      if (!product) a.list[atomicAdd(a.n_list, 1)] = p;
+    }
+    if (product) {
+      for (int k = tid; k < n_m; k += blockDim.x) {
+        s64[Gp->o_kx + k] = k_x[k];
+        s64[Gp->o_kt + k] = k_t[k];
+        s64[Gp->o_kf + k] = k_f[k];
+      }
+      for (int q = tid; q < n_z; q += blockDim.x) {
+        s64[Gp->o_qy + q] = q_y[q];
+        s64[Gp->o_qu + q] = q_u[q];
+      }
+      int* win = reinterpret_cast<int*>(hdr + 4);
+      const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+      const int ns = (Gp->n_t + kF64Chunk - 1) / kF64Chunk;
+      for (int m = warp; m * kF64Rows < n_m; m += nw) {
+        double lo = 1e300, hi = -1e300;
+        for (int k = m * kF64Rows + lane; k < min(n_m, (m + 1) * kF64Rows); k += 32) {
+          lo = fmin(lo, k_alpha[k]);
+          hi = fmax(hi, k_alpha[k]);
+        }
+        for (int off = 16; off > 0; off >>= 1) {
+          lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+          hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+        }
+        if (lane) continue;
+        lo += red[4];
+        hi += red[5];
+        const double e_lo = fmin(fmax(lo, ll_lo), ll_hi) - lo, w2 = kWin64 * sig * kWin64 * sig;
+        const double e_hi = fmin(fmax(hi, ll_lo), ll_hi) - hi;
+        const double x_lo = lo - sqrt(e_lo * e_lo + w2), x_hi = hi + sqrt(e_hi * e_hi + w2);
+        const double* xl = Gp->xl;
+        int s0 = 0, s1 = ns;  // stages with a node inside [x_lo, x_hi]
+        while (s0 < ns - 1 && xl[min(Gp->n_t, (s0 + 1) * kF64Chunk) - 1] < x_lo) ++s0;
+        while (s1 > s0 + 1 && xl[(s1 - 1) * kF64Chunk] > x_hi) --s1;
+        win[m] = s0 | (s1 << 16);
+      }
+      return;
+    }
     for (int idx = tid; idx < n_z * n_m; idx += blockDim.x) {
       const int q = idx / n_m, k = idx - q * n_m;
       const double t = k_t[k], u = q_u[q];
@@ -1072,19 +1102,30 @@ yf_kernel(PrepArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// FP64 plain form.  CTA = (z node q, point); thread k sums over lam_t with one
-// FP64 exp per node: V_i(q, k) = P0_kq sum_t u_t K_i(t, q) exp(-(l_t - mu)^2/2s^2)
-// (with the edge factor exp(-v^2 / 2 s^2) moved into P0 for mu outside the
-// nodes' span).
+// FP64 plain form, for the points that the matrix product (fp64_form.cu) does
+// not admit, listed by the prep kernel.  CTA = (listed point, z node q) in
+// turn; thread k sums over lam_t with one FP64 exp per node:
+// V_i(q, k) = P0_kq sum_t u_t K_i(t, q) exp(-(l_t - mu)^2/2s^2) (with the edge
+// factor exp(-v^2 / 2 s^2) moved into P0 for mu outside the nodes' span).
+__device__ void direct_main(const PointDev& pt, const GridDev& G, double* s64, int q, double* dsh);
+
 __global__ void __launch_bounds__(256)
-direct_main_kernel(const GridDev* grids, const PointDev* pts, double* s64all, int grid_mask)
+direct_main_kernel(const GridDev* grids, const PointDev* pts, double* s64all, const int* list,
+                   const int* n_list, int nz_max)
 {
   extern __shared__ double dsh[];
-  const int p = blockIdx.y, q = blockIdx.x;
-  const PointDev pt = pts[p];
-  if (!grid_in_mask(grid_mask, pt.grid)) return;
-  const GridDev& G = grids[pt.grid];
-  if (q >= G.n_z) return;
+  for (int w = blockIdx.x; w < *n_list * nz_max; w += gridDim.x) {
+    const int p = list[w / nz_max], q = w % nz_max;
+    const PointDev pt = pts[p];
+    const GridDev& G = grids[pt.grid];
+    if (q < G.n_z) direct_main(pt, G, s64all + (size_t)p * G.s64_stride, q, dsh);
+    __syncthreads();
+  }
+}
+
+__device__ void
+direct_main(const PointDev& pt, const GridDev& G, double* s64, int q, double* dsh)
+{
   const int n_t = G.n_t, nI = G.nI;
   double* wk = dsh;                 // [nI][n_t] = u_t K_i(t, q)
   double* xl = dsh + nI * n_t;      // [n_t]
@@ -1094,7 +1135,6 @@ direct_main_kernel(const GridDev* grids, const PointDev* pts, double* s64all, in
   }
   for (int t = threadIdx.x; t < n_t; t += blockDim.x) xl[t] = G.xl[t];
   __syncthreads();
-  double* s64 = s64all + (size_t)p * G.s64_stride;
   const double beta = s64[G.o_beta + q];
   const double inv2s2 = 0.5 / (pt.sigma * pt.sigma);
   for (int k = threadIdx.x; k < G.n_m; k += blockDim.x) {
@@ -1115,33 +1155,34 @@ direct_main_kernel(const GridDev* grids, const PointDev* pts, double* s64all, in
 }
 
 // W_ij(k) = sum_q cz_q K_j(q) V_i(q, k) (and the Sigma_crit-weighted W^g),
-// fixed order over q.  CTA per point.
+// fixed order over q, for the listed points in turn.
 __global__ void __launch_bounds__(256)
 direct_wreduce_kernel(const GridDev* grids, const PointDev* pts, const double* s64all,
-                      double* W, double* Wg, int w_stride, int grid_mask)
+                      double* W, double* Wg, int w_stride, const int* list, const int* n_list)
 {
-  const int p = blockIdx.x;
-  const PointDev pt = pts[p];
-  if (!grid_in_mask(grid_mask, pt.grid)) return;
-  const GridDev& G = grids[pt.grid];
-  const double* s64 = s64all + (size_t)p * G.s64_stride;
-  for (int k = threadIdx.x; k < G.n_m; k += blockDim.x) {
-    for (int i = 0; i < G.nI; ++i) {
-      double acc[kMaxZBins], accg[kMaxZBins];
-      for (int j = 0; j < G.nJ; ++j) acc[j] = accg[j] = 0.0;
-      for (int q = 0; q < G.n_z; ++q) {
-        const double v = s64[G.o_V + ((size_t)i * G.n_z + q) * G.n_m + k];
-        const double c = s64[G.o_cz + q], cs = s64[G.o_czs + q];
-        for (int j = 0; j < G.nJ; ++j) {
-          const double kj = G.Kj[j * G.n_z + q];
-          acc[j] += c * kj * v;
-          accg[j] += cs * kj * v;
+  for (int w = blockIdx.x; w < *n_list; w += gridDim.x) {
+    const int p = list[w];
+    const PointDev pt = pts[p];
+    const GridDev& G = grids[pt.grid];
+    const double* s64 = s64all + (size_t)p * G.s64_stride;
+    for (int k = threadIdx.x; k < G.n_m; k += blockDim.x) {
+      for (int i = 0; i < G.nI; ++i) {
+        double acc[kMaxZBins], accg[kMaxZBins];
+        for (int j = 0; j < G.nJ; ++j) acc[j] = accg[j] = 0.0;
+        for (int q = 0; q < G.n_z; ++q) {
+          const double v = s64[G.o_V + ((size_t)i * G.n_z + q) * G.n_m + k];
+          const double c = s64[G.o_cz + q], cs = s64[G.o_czs + q];
+          for (int j = 0; j < G.nJ; ++j) {
+            const double kj = G.Kj[j * G.n_z + q];
+            acc[j] += c * kj * v;
+            accg[j] += cs * kj * v;
+          }
         }
-      }
-      for (int j = 0; j < G.nJ; ++j) {
-        const size_t o = ((size_t)p * G.nB + i + G.nI * j) * w_stride + k;
-        W[o] = acc[j];
-        Wg[o] = accg[j];
+        for (int j = 0; j < G.nJ; ++j) {
+          const size_t o = ((size_t)p * G.nB + i + G.nI * j) * w_stride + k;
+          W[o] = acc[j];
+          Wg[o] = accg[j];
+        }
       }
     }
   }
@@ -1382,7 +1423,7 @@ finalize_kernel(const GridDev* grids, const PointDev* pts, const double* W, cons
 int gl_nodes_device(double a, double b, int n, double* xs, double* ws, cudaStream_t s);
 
 struct GridBufs {
-  DevBuf<double> xm, wm, xz, wz, xl, wl, lo_x, lo_w, zo_x, zo_w, Ki, Kj, omz;
+  DevBuf<double> xm, wm, xz, wz, xl, wl, lo_x, lo_w, zo_x, zo_w, Ki, Kj, omz, UK64;
   DevBuf<float> UK;
 };
 
@@ -1404,11 +1445,15 @@ struct y3b_engine {
   y3b::DevBuf<y3b::PointDev> pts;
   y3b::DevBuf<double> tables, s64, W, Wg, Phi, counts, shear_out;
   y3b::DevBuf<float> s32;
-  // status: code of the device-side checks | points listed for shear_phi_kernel
+  // status: code of the device-side checks | points listed for
+  // shear_phi_kernel | points listed for the direct sum
   y3b::DevBuf<int> status, order, tile_start;
   y3b::DevBuf<int> stage_ct;  // [2] lam_t stages issued / dense, last contraction
   y3b::DevBuf<int> tile_list;
   y3b::DevBuf<int> win_tile;  // [max_points][tile_cap_pp] stage windows (prep -> contraction)
+  y3b::DevBuf<double> f64_ws; // FP64 form: F, G, Y of a round of points
+  size_t f64_stride = 0;      // doubles per point
+  int f64_round = 0;          // points per round (0: the direct sum only)
   y3b::DevBuf<uint8_t> fbuf;  // F(t, k) stage blocks of the mixed form
   y3b::LikeDev like{};        // Gaussian likelihood fused into the final sums (on = 0: none)
   y3b::DevBuf<double> like_buf, logL;
@@ -1591,6 +1636,13 @@ build_grid(y3b_engine* e, int gi)
                                              b->Ki.get(), b->UK.get());
   count_launch();
   Y3B_CUDA(cudaGetLastError());
+  if (!e->cfg.hmf_fp32) {  // such an engine evaluates the mixed form only
+    Y3B_TRY(b->UK64.alloc((size_t)nki));
+    uk64_kernel<<<(nki + 255) / 256, 256, 0, s>>>(g.nI, g.n_z, g.n_t, b->wl.get(), b->Ki.get(),
+                                                  b->UK64.get());
+    count_launch();
+    Y3B_CUDA(cudaGetLastError());
+  }
   int nkj = g.nJ * g.n_z;
   SzBins szb;
   for (int j = 0; j < 8; ++j) szb.v[j] = g.sz_bin[j];
@@ -1608,25 +1660,32 @@ build_grid(y3b_engine* e, int gi)
     Y3B_CUDA(cudaMemcpy(hk.data(), b->Ki.get(), hk.size() * sizeof(double),
                         cudaMemcpyDeviceToHost));
     for (int i = 0; i < kMaxLamBins; ++i) {
-      g.kt_lo[i] = 0;
-      g.kt_hi[i] = g.n_t - 1;
+      g.kt_lo[i] = g.k64_lo[i] = 0;
+      g.kt_hi[i] = g.k64_hi[i] = g.n_t - 1;
     }
     for (int i = 0; i < g.nI; ++i) {
-      int lo = g.n_t, hi = -1;
+      int lo = g.n_t, hi = -1, lo64 = g.n_t, hi64 = -1;
       for (int q = 0; q < g.n_z; ++q) {
         const double* k = hk.data() + ((size_t)i * g.n_z + q) * g.n_t;
         double mx = 0.0;
         for (int t = 0; t < g.n_t; ++t) mx = std::max(mx, k[t]);
         if (!(mx > 0.0)) continue;
-        for (int t = 0; t < g.n_t; ++t)
+        for (int t = 0; t < g.n_t; ++t) {
           if (k[t] > 1e-12 * mx) {
             lo = std::min(lo, t);
             hi = std::max(hi, t);
           }
+          if (k[t] > 1e-30 * mx) {
+            lo64 = std::min(lo64, t);
+            hi64 = std::max(hi64, t);
+          }
+        }
       }
       if (hi >= lo) {
         g.kt_lo[i] = lo;
         g.kt_hi[i] = hi;
+        g.k64_lo[i] = lo64;
+        g.k64_hi[i] = hi64;
       }
     }
   }
@@ -1648,6 +1707,7 @@ build_grid(y3b_engine* e, int gi)
   g.wl = b->wl.get();
   g.Ki = b->Ki.get();
   g.UK = b->UK.get();
+  g.UK64 = b->UK64.get();
   g.Kj = b->Kj.get();
   g.omz = b->omz.get();
   // Scratch layouts.
@@ -1676,6 +1736,8 @@ build_grid(y3b_engine* e, int gi)
   o += pad2((size_t)g.n_z * g.n_m);
   g.o_V = o;
   o += pad2((size_t)g.nI * g.n_z * g.n_m);
+  g.o_f64 = o;
+  o += 4 + 8;  // header and 16 ints
   g.o_thdr = o;
   o += 8;
   g.o_vv = o;
@@ -1969,6 +2031,16 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
   if (cfg->with_shear)
     bytes += N * (size_t)e->nI_max * sh.n_R * e->w_stride * 8 + N * e->nB_max * sh.n_R * 8;
   const size_t budget = cfg->hbm_budget ? cfg->hbm_budget : (size_t)150 << 30;
+  // FP64 workspace: rounds of up to 128 points (100 MB at 4x nodes, so a
+  // round's factors stay in L2), fewer where the budget leaves less.
+  if (!L.hmf_f32 && bytes <= budget) {
+    for (const auto& g : e->grids)
+      e->f64_stride = std::max(e->f64_stride, f64_ws_doubles(g.n_m, g.n_z, g.n_t));
+    const size_t per = e->f64_stride * 8, fit = (budget - bytes) / per;
+    const size_t l2 = std::max<size_t>(1, ((size_t)104 << 20) / per);
+    e->f64_round = (int)std::min(std::min(N, fit), std::min<size_t>(l2, 128));
+    bytes += e->f64_round * per;
+  }
   if (bytes > budget) {
     set_error("y3b_engine_create: %zu bytes for %d points exceed the HBM budget of %zu bytes",
               bytes, cfg->max_points, budget);
@@ -1984,7 +2056,8 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
       (rc = e->order.alloc(N)) || (rc = e->tile_start.alloc(N + 1)) ||
       (rc = e->tile_list.alloc(N * (size_t)e->tile_cap_pp)) ||
       (rc = e->win_tile.alloc(N * (size_t)e->tile_cap_pp)) ||
-      (rc = e->fbuf.alloc(N * e->f_stride)))
+      (rc = e->fbuf.alloc(N * e->f_stride)) ||
+      (rc = e->f64_ws.alloc(e->f64_round * e->f64_stride)))
     return fail(rc);
   if (cfg->with_shear) {
     if ((rc = e->Phi.alloc(N * (size_t)e->nI_max * sh.n_R * e->w_stride)) ||
@@ -2087,7 +2160,8 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
   if (e->prof) ++e->prof_evals;
   PrepArgs pa{e->d_grids.get(), d_pts, d_tables, d_slot, e->lay, prec == Y3B_MIXED,
               e->s64.get(), e->s32.get(), e->status.get(), grid_mask, e->fbuf.get(), e->f_stride,
-              e->win_tile.get(), e->tile_cap_pp};
+              e->win_tile.get(), e->tile_cap_pp, e->f64_round, e->tile_start.get(),
+              e->status.get() + 2};
   ContractLaunch L{e->d_grids.get(), (int)e->grids.size(), grid_mask, d_pts, n,
                    e->order.get(), e->tile_start.get(), e->tile_list.get(), e->win_tile.get(),
                    e->tile_cap_pp, (long long)n * e->max_tiles_pp, e->cshape, e->cstages,
@@ -2125,13 +2199,25 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
   }
   StageTimer* tc = new StageTimer(e, s, 1);
   if (prec == Y3B_FP64) {
-    dim3 g1(e->nz_max, n);
-    direct_main_kernel<<<g1, 256, e->direct_smem, s>>>(e->d_grids.get(), d_pts, e->s64.get(),
-                                                       grid_mask);
+    if (e->f64_round) {
+      const F64Launch F{e->d_grids.get(), d_pts, grid_mask, 0, d_tables, d_slot, e->lay,
+                        e->s64.get(), e->f64_ws.get(), e->f64_stride, W, Wg, e->w_stride,
+                        e->n_ctas, e->cfg.with_shear && d_shear != nullptr};
+      const int rc = launch_f64(F, n, e->f64_round, (e->w_stride + kF64Rows - 1) / kF64Rows,
+                                e->nI_max, s);
+      if (rc) {
+        delete tc;
+        return rc;
+      }
+    }
+    const int *list = e->tile_start.get(), *n_list = e->status.get() + 2;
+    const int blocks = (int)std::min<long long>((long long)n * e->nz_max, 4 * e->n_ctas);
+    direct_main_kernel<<<blocks, 256, e->direct_smem, s>>>(e->d_grids.get(), d_pts, e->s64.get(),
+                                                          list, n_list, e->nz_max);
     count_launch();
     Y3B_CUDA(cudaGetLastError());
-    direct_wreduce_kernel<<<n, 256, 0, s>>>(e->d_grids.get(), d_pts, e->s64.get(), W, Wg,
-                                            e->w_stride, grid_mask);
+    direct_wreduce_kernel<<<std::min(n, 4 * e->n_ctas), 256, 0, s>>>(
+      e->d_grids.get(), d_pts, e->s64.get(), W, Wg, e->w_stride, list, n_list);
     count_launch();
     Y3B_CUDA(cudaGetLastError());
   } else {

@@ -40,6 +40,7 @@ struct GridDev {
   // lam_t nodes where richness bin i's kernel K_i(t, q) exceeds 1e-12 of its
   // maximum over t, for some z_t node q: [kt_lo[i], kt_hi[i]]
   int kt_lo[kMaxLamBins], kt_hi[kMaxLamBins];
+  int k64_lo[kMaxLamBins], k64_hi[kMaxLamBins];  // the same above 1e-30 (FP64 form)
   double lnm_lo, lnm_hi, zt_lo, zt_hi, ll_lo, ll_hi, sz0;
   double sz_bin[8];   // sigma_z(z, j) = sz0 (1 + z) + sz_bin[j]
   const double* xm;   // [n_m]  lnM nodes
@@ -49,6 +50,7 @@ struct GridDev {
   const double* xl;   // [n_t]  ln lam_t nodes
   const double* wl;
   const double* Ki;   // [nI][n_z][n_t] FP64
+  const double* UK64; // [nI][n_t][n_z] = wl_t K_i(t, q) (null with FP32 HMF tables)
   const float* UK;    // [nI][n_z][n_t_pad] = wl_t K_i(t, q) in FP32
   const double* Kj;   // [nJ][n_z]
   const double* omz;  // [n_z] survey area Omega(z_q)
@@ -56,6 +58,8 @@ struct GridDev {
   size_t s64_stride;  // doubles per point in the FP64 scratch
   size_t o_scal, o_kx, o_kt, o_kf, o_qy, o_qu;  // A0/B0, HMF cells and weights
   size_t o_cz, o_czs, o_alpha, o_beta, o_P0, o_V;
+  size_t o_f64;         // FP64 form: 1 (matrix product) or 0 (direct sum) | A0 | B0 | - |
+                        // lam_t stage window of each 64-row lnM tile (ints, first | end << 16)
   size_t o_thdr, o_vv;  // mixed form: FP64 header and row scale v_k^2 c1 of yf_kernel
   size_t o_dt64;        // mixed form: FP64 log2 D table (deep tails)
   size_t s32_stride;  // floats per point in the FP32 scratch
@@ -65,6 +69,12 @@ struct GridDev {
   size_t f_hdr, f_tinfo, f_q, f_dt32, f_rows;
   int nzp;  // n_z rounded up to 4
 };
+
+// FP64 form (fp64_form.cu): lnM rows of a tile, lam_t nodes of a stage, and
+// the largest exponent of a factor that its matrix product admits.
+constexpr int kF64Rows = 64;
+constexpr int kF64Chunk = 16;
+constexpr double kF64MaxExp = 600.0;
 
 struct PointDev {  // mirrors y3b_point
   double om, ol, ok, h0, onu, hmf_s, hmf_q;
@@ -123,6 +133,25 @@ struct ContractLaunch {
   cudaStream_t stream;
   bool shear;               // also accumulate the Sigma_crit-weighted W^g
 };
+
+struct F64Launch {
+  const GridDev* grids;  // device array
+  const PointDev* pts;   // device array
+  int grid_mask, p0;     // p0: first point of the round
+  const double* tables;
+  const int* slot;
+  TableLayout lay;
+  const double* s64;
+  double* ws;            // F, G, Y of a round's points
+  size_t ws_stride;      // doubles per point
+  double *W, *Wg;
+  int w_stride, n_ctas;
+  bool shear;
+};
+
+// Workspace doubles of one point, and the evaluation of n points in rounds.
+size_t f64_ws_doubles(int n_m, int n_z, int n_t);
+int launch_f64(const F64Launch& L, int n, int round, int row_tiles, int nI, cudaStream_t s);
 
 // The tile planner depends only on the points and their grids, so it runs on
 // L.plan_stream while the prep kernel runs; the persistent contraction over
