@@ -92,3 +92,14 @@ def test_fp64_shear_outside_the_profile_table(gpu):
                     want[b] += wm[k] * out["W"][p, b, k] * phi
         np.testing.assert_allclose(out["shear"][p], want, rtol=1e-11)
     eng.close()
+
+
+# Few samples split a grid point's theta nodes over blocks, many do not; one
+# and two theta nodes (no split at theta_lob), node counts that leave partial
+# warps of (z, lambda_true) pairs and odd z grids.
+@pytest.mark.parametrize("n,n_lt,n_zring,n_zouter,n_lnm,n_theta,n_zt_ref", [
+    (1, 60, 20, 30, 24, 10, 80), (3, 7, 5, 3, 9, 2, 40), (40, 31, 9, 15, 13, 5, 33),
+    (2, 1, 20, 30, 24, 3, 64)])
+def test_selection_bias(gpu, n, n_lt, n_zring, n_zouter, n_lnm, n_theta, n_zt_ref):
+    _compare(dict(kind="bsel", n=n, n_lt=n_lt, n_zring=n_zring, n_zouter=n_zouter, n_lnm=n_lnm,
+                  n_theta=n_theta, n_zt_ref=n_zt_ref), 1e-10)

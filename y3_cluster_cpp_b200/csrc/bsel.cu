@@ -24,14 +24,29 @@
 //   of the richness aperture, f_A the two-disk overlap fraction and xi the
 //   nonlinear correlation function at z_obs and the 3-D separation.
 //
-// Device layout: one packed FP64 block per sample (scalars and tables);
-// one kernel per (reference z node, sample) writes the per-sample tables and
-// the MOR table of the richness bins in use; one 512-thread CTA per
-// (grid point, sample) builds its grids in shared memory and does the sums.
-// Every sum runs in the reference's order (mass, lambda_true, z, theta), and
-// this file is compiled without FMA contraction, so the results follow the
-// reference's FP64 arithmetic up to the last bits of the transcendental
-// functions.
+// Device layout: one packed FP64 block per sample (scalars and tables) and
+// four kernels a batch:
+//   bsel_grid_kernel    one small block per (grid point, sample): line-of-sight
+//                       and theta grids, and the reference z nodes they read;
+//   bsel_sample_kernel  one block per (reference z node, sample): the MOR
+//                       contracted over mass, as the moments below, where read;
+//   bsel_point_kernel   one 512-thread block per (grid point, sample, group of
+//                       theta nodes): the (theta, z, lambda_true) sums;
+//   bsel_sum_kernel     the theta sums.
+// With n, b and p linear in z between reference nodes i and i + 1 (weights
+// g0 = 1 - f, g1 = f), the mass sums are polynomials in f whose coefficients
+// do not depend on the grid point:
+//   sum_M w n p   = g0 (g0 M0[i] + g1 M1[i]) + g1 (g0 M2[i+1] + g1 M0[i+1]),
+//   sum_M w n b p = g0 (g0^2 M3[i] + g0 g1 M4[i] + g1^2 M5[i])
+//                 + g1 (g0^2 M7[i+1] + g0 g1 M6[i+1] + g1^2 M3[i+1]),
+// with the moments of node j over (lambda_true) sum_M w (.) p_j of
+//   M0 n_j, M1 n_{j+1}, M2 n_{j-1}, M3 n_j b_j, M4 n_j b_{j+1} + n_{j+1} b_j,
+//   M5 n_{j+1} b_{j+1}, M6 n_{j-1} b_j + n_j b_{j-1}, M7 n_{j-1} b_{j-1}:
+// eight values replace the 24 of the mass nodes, and the point kernel reads
+// ten instead of 48 per (z, lambda_true).  Every sum has a fixed order.
+// This file is compiled without FMA contraction: the reference's separation
+// sqrt(chi_z^2 + chi_o^2 - 2 chi_z chi_o cos theta) loses ten digits, and its
+// roundings are kept (the loops that bound the kernels call fma()).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -51,9 +66,12 @@ lob_centre(int b)
 {
   return b == 0 ? 25.0 : (b == 1 ? 37.5 : (b == 2 ? 52.5 : 130.0));
 }
-constexpr int kPointThreads = 512;
-constexpr int kSampleThreads = 128;
+constexpr int kPointThreads = 512, kPointWarps = kPointThreads / 32;
+constexpr int kGridThreads = 128;
+constexpr int kSampleThreads = 256;
 constexpr int kScal = 16;  // scalars at the head of a sample block
+constexpr int kMoments = 8;
+constexpr int kGpScal = 4;  // scalars at the head of a grid point's grids
 
 // Shapes, offsets and constant tables shared by the kernels of one call.
 struct BselDims {
@@ -63,13 +81,19 @@ struct BselDims {
   // d_c | halo lnM | halo z | bias | xi r | xi z | xi
   int n_hm, n_hz, nd, n_hl, n_bz, n_xr, n_xz;
   long o_mh, o_hz, o_dn, o_dz, o_da, o_dc, o_bl, o_bz, o_bi, o_xr, o_xz, o_xi, blk;
-  // per-sample work: chi | dV | sigma_z (n_zr each) | n, b [n_zr][n_lnm] | MOR [4][n_zr][n_lnm][n_lt]
-  long w_chi, w_dv, w_sig, w_hmf, w_hmb, w_mor, mor_bin, work;
-  unsigned bins_used;
+  // per-sample moments [4][n_zr][kMoments][n_lt], bits of the reference
+  // nodes read per bin [4][need_words], and per (grid point, sample) grids:
+  // kGpScal scalars (theta_lob, chi_o, number of z nodes, fully excluded) |
+  // bracket, f, chi, c_z, theta_excl, (1 + z) / chi [nz_max each] | theta,
+  // g_theta, s(theta), cos theta [n_th each]
+  long mom_bin, mom;
+  int need_words;
+  long g_z, g_th, grid;
   // constants (device): lnM nodes / weights, lambda_true nodes / weights /
   // R_lambda per bin [4][n_lt], reference z grid, photo-z width table,
   // grid points
   const double *lnm_x, *lnm_w, *lt_x, *lt_w, *rl, *zr, *zk_z, *zk_s;
+  const double *gl_out, *gl_ring, *gl_th, *gl_th1, *gl_th2;  // nodes | weights on [-1, 1]
   const double *gp_zob, *gp_zfg, *gp_zbg;
   const int* gp_bin;
 };
@@ -80,95 +104,42 @@ chi_at(const BselDims& D, const double* B, double z)  // chi_.clamp(z) h0
   return interp1d_clamp(B + D.o_dz, B + D.o_dc, D.nd, z) * B[4];
 }
 
-// Two-disk overlap fraction f_A(theta; theta_lob, theta_lt)
-// (p_op_detail::area_overlap, p_operator_cuhre_t.hh:97-125).
+// Angle of (x, y), y >= 0, in [0, pi]: the ratio reduced to |q| <= tan(pi/8),
+// atan(q) / q a degree-11 polynomial in q^2 (Chebyshev interpolation,
+// relative error 7e-17).
 __device__ __forceinline__ double
-area_overlap(double theta, double theta_lob, double theta_lt)
+angle(double y, double x)
 {
-  if (theta > theta_lob + theta_lt) return 0.0;
-  if (theta <= fabs(theta_lob - theta_lt)) {
-    if (theta_lt <= theta_lob) return 1.0;
-    const double r = theta_lob / theta_lt;
-    return r * r;
-  }
-  const double tt = theta, ll = theta_lt, lo = theta_lob;
-  double c1 = (tt * tt + ll * ll - lo * lo) / (2.0 * tt * ll);
-  double c2 = (tt * tt + lo * lo - ll * ll) / (2.0 * tt * lo);
-  c1 = c1 < -1.0 ? -1.0 : (1.0 < c1 ? 1.0 : c1);
-  c2 = c2 < -1.0 ? -1.0 : (1.0 < c2 ? 1.0 : c2);
-  double sq = (-tt + ll + lo) * (tt + ll - lo) * (tt - ll + lo) * (tt + ll + lo);
-  sq = sq < 0.0 ? 0.0 : sq;
-  const double A = ll * ll * acos(c1) + lo * lo * acos(c2) - 0.5 * sqrt(sq);
-  return A / (kPi * ll * ll);
+  const double ax = fabs(x), mn = fmin(y, ax), mx = fmax(y, ax);
+  const bool mid = mn > 0.41421356237309503 * mx;
+  const double q = (mid ? mn - mx : mn) / (mid ? mn + mx : mx), z = q * q;
+  double s = -1.78038963948125642e-02;
+  s = fma(s, z, 3.79639031611108332e-02);
+  s = fma(s, z, -5.03504979531243929e-02);
+  s = fma(s, z, 5.84686675227513927e-02);
+  s = fma(s, z, -6.66295024603679176e-02);
+  s = fma(s, z, 7.69204519456148095e-02);
+  s = fma(s, z, -9.09089680147281282e-02);
+  s = fma(s, z, 1.11111107446570989e-01);
+  s = fma(s, z, -1.42857142792449682e-01);
+  s = fma(s, z, 1.99999999999408373e-01);
+  s = fma(s, z, -3.33333333333331205e-01);
+  double a = fma(s, z * q, q) + (mid ? 0.25 * kPi : 0.0);
+  a = y > ax ? 0.5 * kPi - a : a;
+  return x < 0.0 ? kPi - a : a;
 }
 
-// Per (reference z node, sample): chi, dV/dz, sigma_z, n(M, z), b(M, z) and
-// the shifted-Poisson MOR of every richness bin in use
-// (P_operator::set_sample, p_operator_t.hh:150-219).  A reference node
-// outside distances/z sets the domain status (the reference's Interp1D
-// throws there); the host checks this range before the launch.
-__global__ void __launch_bounds__(kSampleThreads)
-bsel_sample_kernel(BselDims D, const double* __restrict__ blocks, double* __restrict__ work,
-                   int* status)
+// Overlap area of two disks of radii o and l at distance t, partially
+// overlapping (p_op_detail::area_overlap, p_operator_cuhre_t.hh:97-125): the
+// lens angles come from the triangle (t, l, o) as angles of (4 x its area,
+// t^2 + l^2 - o^2) and (.., t^2 + o^2 - l^2), which lose no digits near
+// tangency, in place of two acos of cosines.
+__device__ __forceinline__ double
+lens_area(double t, double o, double l)
 {
-  extern __shared__ double ssm[];  // mi, lam, ln lam [n_lnm] each
-  const int iz = blockIdx.x, s = blockIdx.y, tid = threadIdx.x;
-  const double* B = blocks + (size_t)s * D.blk;
-  double* W = work + (size_t)s * D.work;
-  const double z = D.zr[iz];
-  const int NM = D.n_lnm, NL = D.n_lt;
-  if (tid == 0) {
-    W[D.w_chi + iz] = chi_at(D, B, z);
-    double dv = 0.0;
-    if (!dv_do_dz(B + D.o_dz, B + D.o_da, D.nd, B[0], B[2], B[3], B[4], z, &dv))
-      set_err(status, kDevDomain);
-    W[D.w_dv + iz] = dv;
-    W[D.w_sig + iz] = interp1d_clamp(D.zk_z, D.zk_s, kZKernelNodes, z);
-  }
-  double* mi_s = ssm;
-  double* lam_s = mi_s + NM;
-  double* llam_s = lam_s + NM;
-  const double Mmin = pow(10.0, B[7]), M1 = pow(10.0, B[8]);
-  const double alpha = B[9], eps = B[10], sig_l = B[11], zpiv = B[12];
-  const double dM1 = M1 - Mmin;
-  const double zfac = pow((1.0 + z) / (1.0 + zpiv), eps);
-  for (int iM = tid; iM < NM; iM += blockDim.x) {
-    const double x = D.lnm_x[iM];
-    W[D.w_hmf + (size_t)iz * NM + iM] =
-      interp2d_clamp(B + D.o_mh, D.n_hm, B + D.o_hz, D.n_hz, B + D.o_dn, x, z) *
-      (B[5] * (x * kLog10e - kHmfPivot) + B[6]);
-    W[D.w_hmb + (size_t)iz * NM + iM] =
-      interp2d_clamp(B + D.o_bl, D.n_hl, B + D.o_bz, D.n_bz, B + D.o_bi, x, z);
-    const double M = exp(x);
-    const double dM = fmax(M - Mmin, 0.0);
-    const double l_sat = (dM > 0.0 && dM1 > 0.0) ? pow(dM / dM1, alpha) * zfac : 0.0;
-    const double mi = (l_sat * sig_l) * (l_sat * sig_l);
-    const double lam = fmax(l_sat + mi, 1.0e-300);
-    mi_s[iM] = mi;
-    lam_s[iM] = lam;
-    llam_s[iM] = log(lam);
-  }
-  __syncthreads();
-  const int per_bin = NM * NL;
-  for (int bb = 0; bb < 4; ++bb) {
-    if (!((D.bins_used >> bb) & 1u)) continue;
-    double* dst = W + D.w_mor + (size_t)bb * D.mor_bin + (size_t)iz * per_bin;
-    const double* ltx = D.lt_x + bb * NL;
-    for (int k = tid; k < per_bin; k += blockDim.x) {
-      const int iM = k / NL, il = k - iM * NL;
-      const double x = ltx[il] + mi_s[iM];
-      dst[k] = exp(-lam_s[iM] + (x - 1.0) * llam_s[iM] - lgamma(x));
-    }
-  }
-}
-
-// Shared-memory doubles of bsel_point_kernel for the shapes in D.
-__host__ __device__ inline long
-point_smem_doubles(const BselDims& D)
-{
-  const long NZ = D.nz_max;
-  return 9 * NZ + 4L * D.n_zouter + 5L * D.n_th + D.n_xr + 2L * D.n_lt * NZ +
-         3L * D.n_th * NZ + kScal + 16 + (NZ + 1) / 2;
+  const double sq = (l + o - t) * (t + l - o) * (t - l + o) * (t + l + o);
+  const double r = sqrt(fmax(sq, 0.0)), t2 = t * t, l2 = l * l, o2 = o * o;
+  return fma(l2, angle(r, t2 + (l2 - o2)), fma(o2, angle(r, t2 + (o2 - l2)), -0.5 * r));
 }
 
 // Lower bracket of z on the reference grid: i = min(trunc(u), n - 2) with
@@ -184,297 +155,439 @@ ref_bracket(const BselDims& D, double z, double* f)
   return i;
 }
 
-// One CTA per (grid point, sample): P_operator::evaluate
-// (p_operator_t.hh:222-477) with its grids in shared memory.
-__global__ void __launch_bounds__(kPointThreads, 2)
-bsel_point_kernel(BselDims D, const double* __restrict__ blocks,
-                  const double* __restrict__ work, double* __restrict__ out)
+// z with chi(z) = target: the reference's 40-step bisection of [0.001, 2]
+// (p_operator_t.hh:621-632); the table cells of the bracket's ends bound the
+// search of each step.
+__device__ __forceinline__ double
+invert_chi(const BselDims& D, const double* B, double target)
 {
-  extern __shared__ double sm[];
-  const int g = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
-  const double* B = blocks + (size_t)s * D.blk;
-  const double* Wk = work + (size_t)s * D.work;
-  const int NZ = D.nz_max, NL = D.n_lt, NT = D.n_th, NO = D.n_zouter, NR = D.n_zring;
-  const int NM = D.n_lnm;
-  double* zs = sm;
-  double* wzs = zs + NZ;
-  double* chz = wzs + NZ;
-  double* dvz = chz + NZ;
-  double* sgz = dvz + NZ;
-  double* wzv = sgz + NZ;
-  double* thx = wzv + NZ;
-  double* ic1 = thx + NZ;
-  double* fzz = ic1 + NZ;
-  double* ufg = fzz + NZ;
-  double* wufg = ufg + NO;
-  double* ubg = wufg + NO;
-  double* wubg = ubg + NO;
-  double* ths = wubg + NO;
-  double* wths = ths + NT;
-  double* sgm = wths + NT;
-  double* omt = sgm + NT;
-  double* cst = omt + NT;
-  double* xir = cst + NT;
-  double* WP = xir + D.n_xr;
-  double* WI = WP + (size_t)NL * NZ;
-  double* pP = WI + (size_t)NL * NZ;
-  double* pI = pP + (size_t)NT * NZ;
-  double* pJ = pI + (size_t)NT * NZ;
-  double* sc = pJ + (size_t)NT * NZ;
-  int* izl = reinterpret_cast<int*>(sc + kScal + 16);  // after 8 doubles of counts and 5 chi(z)
-  // scalars: 0 zob, 1 chi_o, 2 theta_lob, 3 R_excl, 4 ln R_excl, 5 ln(chi_o - chi_fg),
-  // 6 ln(chi_bg - chi_o), 7 ring lo, 8 ring hi, 9 th_lo, 10 th_hi, 11 th_mid,
-  // 12 ln r_0, 13 1 / dln r, 14 k_sig, 15 th0_sig; ints after: n_fg, n_ring, n_bg, split, empty
-  int* cnt = reinterpret_cast<int*>(sc + kScal);
-  const int bin = D.gp_bin[g];
-  const double ddz = 1.0e-3;
+  const double* zs = B + D.o_dz;
+  const double* dc = B + D.o_dc;
+  const double z0 = zs[0], z1 = zs[D.nd - 1], h0 = B[4];
+  double lo = 0.001, hi = 2.0;
+  int c_lo = 0, c_hi = D.nd - 1;
+  for (int it = 0; it < 40; ++it) {
+    const double mid = 0.5 * (lo + hi), x = fmin(fmax(mid, z0), z1);
+    int a = c_lo, b = c_hi;
+    while (b > a + 1) {
+      const int m = (a + b) >> 1;
+      if (zs[m] > x) b = m; else a = m;
+    }
+    const double dx = zs[a + 1] - zs[a];
+    const double chi = (dx > 0.0 ? dc[a] + (x - zs[a]) / dx * (dc[a + 1] - dc[a]) : 0.0) * h0;
+    if (chi < target) {
+      lo = mid;
+      c_lo = a;
+    } else {
+      hi = mid;
+      c_hi = a + 1;
+    }
+  }
+  return 0.5 * (lo + hi);
+}
 
+// One block per (grid point, sample): P_operator::evaluate's grids
+// (p_operator_t.hh:222-430).  Latency-bound (interpolations, bisections), so
+// small blocks, many to an SM.
+__global__ void __launch_bounds__(kGridThreads)
+bsel_grid_kernel(BselDims D, const double* __restrict__ blocks, double* __restrict__ grids,
+                 unsigned* __restrict__ need)
+{
+  const int g = blockIdx.x, s = blockIdx.y, tid = threadIdx.x;
+  const double* B = blocks + (size_t)s * D.blk;
+  double* G = grids + ((size_t)s * D.n_gp + g) * D.grid;
+  double* Z = G + D.g_z;
+  double* T = G + D.g_th;
+  const int NZ = D.nz_max, NT = D.n_th, NO = D.n_zouter, NR = D.n_zring, bin = D.gp_bin[g];
+  __shared__ double cq[5], sc[16], red[kGridThreads / 32];
+  const double ddz = 1.0e-3, zob = D.gp_zob[g];
   if (tid < 5) {  // the five chi(z) this point needs, one lookup per thread
-    const double zob = D.gp_zob[g];
     const double zq[5] = {zob, D.gp_zfg[g], D.gp_zbg[g], zob + ddz, zob - ddz};
-    sc[kScal + 8 + tid] = chi_at(D, B, zq[tid]);
+    cq[tid] = chi_at(D, B, zq[tid]);
   }
   __syncthreads();
-  if (tid == 0) {
-    const double zob = D.gp_zob[g];
+  const double chi_o = cq[0];
+  if (tid == 0) {  // build_z_grid_ (p_operator_t.hh:503-583)
     const double Rlob = pow(lob_centre(bin) / 100.0, 0.2);  // p_op_detail::R_lambda
-    const double* cq = sc + kScal + 8;
-    const double chi_o = cq[0];
-    const double theta_lob = Rlob * (1.0 + zob) / chi_o;
     const double R_excl = Rlob * (1.0 + zob);
-    // build_z_grid_ (p_operator_t.hh:503-583)
-    const double zfg = D.gp_zfg[g], zbg = D.gp_zbg[g];
-    const double chi_fg = cq[1], chi_bg = cq[2];
     const double dchi_dz = (cq[3] - cq[4]) / (2.0 * ddz);
     const double dz_excl = R_excl / dchi_dz;
-    const double zr_lo = fmax(zob - dz_excl, zfg), zr_hi = fmin(zob + dz_excl, zbg);
-    const double dfg = chi_o - chi_fg, dbg = chi_bg - chi_o;
-    cnt[0] = R_excl < dfg ? NO : 0;
-    cnt[1] = zr_hi > zr_lo ? NR : 0;
-    cnt[2] = R_excl < dbg ? NO : 0;
-    sc[0] = zob;
-    sc[1] = chi_o;
-    sc[2] = theta_lob;
-    sc[3] = R_excl;
-    sc[4] = log(R_excl);
-    sc[5] = cnt[0] ? log(dfg) : 0.0;
-    sc[6] = cnt[2] ? log(dbg) : 0.0;
-    sc[7] = zr_lo;
-    sc[8] = zr_hi;
-    sc[14] = 2.5 / theta_lob;
-    sc[15] = 0.5 * theta_lob;
-    const double* xr = B + D.o_xr;
-    sc[12] = log(xr[0]);
-    sc[13] = 1.0 / log(xr[1] / xr[0]);
+    sc[0] = R_excl / chi_o;  // theta_lob
+    sc[1] = R_excl;
+    sc[2] = fmax(zob - dz_excl, D.gp_zfg[g]);
+    sc[3] = fmin(zob + dz_excl, D.gp_zbg[g]);
+    sc[4] = chi_o - cq[1];
+    sc[5] = cq[2] - chi_o;
+    sc[6] = log(R_excl);
+    sc[7] = R_excl < sc[4] ? log(sc[4]) : 0.0;
+    sc[8] = R_excl < sc[5] ? log(sc[5]) : 0.0;
   }
   __syncthreads();
-  const int n_fg = cnt[0], n_ring = cnt[1], n_bg = cnt[2];
-  const int Nz = n_fg + n_ring + n_bg;
-  const double zob = sc[0], chi_o = sc[1], theta_lob = sc[2], R_excl = sc[3];
-  {  // GL nodes of the two log-distance wings and of the ring
-    const int hO = (NO + 1) / 2, hR = (NR + 1) / 2;
-    for (int i = tid; i < 2 * hO + hR; i += nt) {
-      if (i < hO) {
-        if (n_fg) gl_node_pair(sc[4], sc[5], NO, i, ufg, wufg);
-      } else if (i < 2 * hO) {
-        if (n_bg) gl_node_pair(sc[4], sc[6], NO, i - hO, ubg, wubg);
-      } else if (n_ring) {
-        gl_node_pair(sc[7], sc[8], NR, i - 2 * hO, zs + n_fg, wzs + n_fg);
-      }
+  const double theta_lob = sc[0], R_excl = sc[1];
+  const int n_fg = R_excl < sc[4] ? NO : 0, n_ring = sc[3] > sc[2] ? NR : 0;
+  const int n_bg = R_excl < sc[5] ? NO : 0, Nz = n_fg + n_ring + n_bg;
+  unsigned* nd = need + ((size_t)s * 4 + bin) * D.need_words;
+  double tmin = 2.0 * theta_lob;
+  for (int iz = tid; iz < Nz; iz += kGridThreads) {
+    // front wing (farthest first), ring, back wing
+    double z, wz;
+    if (iz >= n_fg && iz < n_fg + n_ring) {
+      const double hl = 0.5 * (sc[3] - sc[2]);
+      z = 0.5 * (sc[2] + sc[3]) + hl * D.gl_ring[iz - n_fg];
+      wz = hl * D.gl_ring[NR + iz - n_fg];
+    } else {
+      const bool fg = iz < n_fg;
+      const int k = fg ? n_fg - 1 - iz : iz - n_fg - n_ring;
+      const double b = fg ? sc[7] : sc[8], hl = 0.5 * (b - sc[6]);
+      const double dis = exp(0.5 * (sc[6] + b) + hl * D.gl_out[k]);
+      z = invert_chi(D, B, fg ? chi_o - dis : chi_o + dis);
+      wz = hl * D.gl_out[NO + k] * dis /
+           ((chi_at(D, B, z + ddz) - chi_at(D, B, z - ddz)) / (2.0 * ddz));
     }
-  }
-  __syncthreads();
-  for (int i = tid; i < n_fg + n_bg; i += nt) {  // wing nodes: z(chi_o -+ dis)
-    const bool fg = i < n_fg;
-    const int k = fg ? i : i - n_fg;
-    const double dis = exp(fg ? ufg[k] : ubg[k]);
-    const double target = fg ? chi_o - dis : chi_o + dis;
-    double lo = 0.001, hi = 2.0;  // invert_chi_ (p_operator_t.hh:621-632)
-    for (int it = 0; it < 40; ++it) {
-      const double mid = 0.5 * (lo + hi);
-      if (chi_at(D, B, mid) < target)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    const double zi = 0.5 * (lo + hi);
-    const double dd = (chi_at(D, B, zi + ddz) - chi_at(D, B, zi - ddz)) / (2.0 * ddz);
-    const int o = fg ? n_fg - 1 - k : n_fg + n_ring + k;  // fg reversed, ring, bg
-    zs[o] = zi;
-    wzs[o] = (fg ? wufg[k] : wubg[k]) * dis / dd;
-  }
-  __syncthreads();
-  // z-node tables, photo-z weight, exclusion angle
-  for (int iz = tid; iz < Nz; iz += nt) {
-    const double z = zs[iz];
+    // the reference z tables at the bracket's nodes, linear in z
     double f;
     const int i = ref_bracket(D, z, &f);
-    izl[iz] = i;
-    fzz[iz] = f;
-    const double* cr = Wk + D.w_chi;
-    const double* dr = Wk + D.w_dv;
-    const double* sr = Wk + D.w_sig;
-    const double cz = cr[i] + f * (cr[i + 1] - cr[i]);
-    chz[iz] = cz;
-    dvz[iz] = dr[i] + f * (dr[i + 1] - dr[i]);
-    const double sg = sr[i] + f * (sr[i + 1] - sr[i]);
-    sgz[iz] = sg;
-    const double u = (z - zob) / sg;
-    wzv[iz] = fabs(u) < 1.0 ? 1.0 - u * u : 0.0;
+    const double z0 = D.zr[i], z1 = D.zr[i + 1];
+    double v0 = 0.0, v1 = 0.0;
+    dv_do_dz(B + D.o_dz, B + D.o_da, D.nd, B[0], B[2], B[3], B[4], z0, &v0);
+    dv_do_dz(B + D.o_dz, B + D.o_da, D.nd, B[0], B[2], B[3], B[4], z1, &v1);
+    const double c0 = chi_at(D, B, z0), c1 = chi_at(D, B, z1), cz = c0 + f * (c1 - c0);
+    const double s0 = interp1d_clamp(D.zk_z, D.zk_s, kZKernelNodes, z0);
+    const double s1 = interp1d_clamp(D.zk_z, D.zk_s, kZKernelNodes, z1);
+    const double u = (z - zob) / (s0 + f * (s1 - s0));
+    const double wzv = fabs(u) < 1.0 ? 1.0 - u * u : 0.0;
     double ce = (cz * cz + chi_o * chi_o - R_excl * R_excl) / (2.0 * cz * chi_o);
     ce = ce < -1.0 ? -1.0 : (1.0 < ce ? 1.0 : ce);
-    thx[iz] = ce >= 1.0 - 1e-12 ? 1e-6 : acos(ce);
-    ic1[iz] = (1.0 + z) / cz;
-  }
-  __syncthreads();
-  if (tid == 0) {  // theta range and split (p_operator_t.hh:352-395)
-    const double th_hi = 2.0 * theta_lob;
-    double th_lo = th_hi;
-    for (int iz = 0; iz < Nz; ++iz)
-      if (thx[iz] < th_lo) th_lo = thx[iz];
-    const int N1 = NT / 2, N2 = NT - N1;
-    const double th_mid = th_lo > theta_lob ? th_lo : (th_hi < theta_lob ? th_hi : theta_lob);
-    cnt[3] = !(N1 == 0 || th_mid <= th_lo || N2 == 0 || th_mid >= th_hi);
-    cnt[4] = th_lo >= th_hi;
-    sc[9] = th_lo;
-    sc[10] = th_hi;
-    sc[11] = th_mid;
-  }
-  __syncthreads();
-  double* o = out + ((size_t)s * D.n_gp + g) * 3;
-  if (cnt[4]) {  // fully excluded: the integrand is zero
-    if (tid < 3) o[tid] = 0.0;
-    return;
-  }
-  {
-    const int N1 = NT / 2, N2 = NT - N1;
-    if (cnt[3]) {
-      for (int i = tid; i < (N1 + 1) / 2 + (N2 + 1) / 2; i += nt) {
-        if (i < (N1 + 1) / 2)
-          gl_node_pair(sc[9], sc[11], N1, i, ths, wths);
-        else
-          gl_node_pair(sc[11], sc[10], N2, i - (N1 + 1) / 2, ths + N1, wths + N1);
-      }
-    } else {
-      for (int i = tid; i < (NT + 1) / 2; i += nt) gl_node_pair(sc[9], sc[10], NT, i, ths, wths);
+    const double th = ce >= 1.0 - 1e-12 ? 1e-6 : acos(ce);
+    Z[iz] = i;
+    Z[NZ + iz] = f;
+    Z[2 * NZ + iz] = cz;
+    Z[3 * NZ + iz] = wzv == 0.0 ? 0.0 : wzv * (v0 + f * (v1 - v0)) * wz;
+    // no theta passes a node outside the photo-z support
+    Z[4 * NZ + iz] = wzv == 0.0 ? 1e300 : th;
+    Z[5 * NZ + iz] = (1.0 + z) / cz;
+    if (th < tmin) tmin = th;
+    if (wzv != 0.0) {
+      atomicOr(nd + (i >> 5), 1u << (i & 31));
+      atomicOr(nd + ((i + 1) >> 5), 1u << ((i + 1) & 31));
     }
   }
-  {  // xi_NL(r, z_obs): linear in z on the evenly spaced z axis
-    const double* xz = B + D.o_xz;
-    const double u = (zob - xz[0]) * (1.0 / (xz[1] - xz[0]));
-    int j = (int)floor(u);
-    j = j < 0 ? 0 : (j > D.n_xz - 2 ? D.n_xz - 2 : j);
-    const double fz = u - j;
-    const double* r0 = B + D.o_xi + (size_t)j * D.n_xr;
-    const double* r1 = r0 + D.n_xr;
-    for (int ir = tid; ir < D.n_xr; ir += nt) xir[ir] = r0[ir] + fz * (r1[ir] - r0[ir]);
+  for (int off = 16; off > 0; off >>= 1)
+    tmin = fmin(tmin, __shfl_xor_sync(0xffffffffu, tmin, off));
+  if ((tid & 31) == 0) red[tid >> 5] = tmin;
+  __syncthreads();
+  // theta range and split (p_operator_t.hh:352-395)
+  double th_lo = red[0];
+  for (int w = 1; w < kGridThreads / 32; ++w) th_lo = fmin(th_lo, red[w]);
+  const double th_hi = 2.0 * theta_lob;
+  const int N1 = NT / 2, N2 = NT - N1;
+  const double th_mid = th_lo > theta_lob ? th_lo : (th_hi < theta_lob ? th_hi : theta_lob);
+  const bool split = !(N1 == 0 || th_mid <= th_lo || N2 == 0 || th_mid >= th_hi);
+  if (tid == 0) {
+    G[0] = theta_lob;
+    G[1] = chi_o;
+    G[2] = Nz;
+    G[3] = th_lo >= th_hi ? 1.0 : 0.0;  // fully excluded: the integrand is zero
+  }
+  for (int it = tid; it < NT; it += kGridThreads) {
+    const bool first = it < N1;
+    const double a = split && !first ? th_mid : th_lo, b = split && first ? th_mid : th_hi;
+    const double* q = split ? (first ? D.gl_th1 : D.gl_th2 - N1) : D.gl_th;
+    const int nq = split ? (first ? N1 : N2) : NT;
+    const double hl = 0.5 * (b - a), th = 0.5 * (a + b) + hl * q[it];
+    T[it] = th;
+    T[NT + it] = hl * q[nq + it] * 2.0 * kPi * sin(th);
+    T[2 * NT + it] = 1.0 / (1.0 + exp(-(2.5 / theta_lob) * (th - 0.5 * theta_lob)));
+    T[3 * NT + it] = cos(th);
+  }
+}
+
+// Shifted-Poisson density exp(-lam + (x - 1) ln lam) / Gamma(x).  With
+// y = x + 10, 1 / Gamma(x) = prod_{i<10} (x + i) / Gamma(y) and Stirling's
+// series for Gamma(y) (seven terms, remainder below 3e-17), grouped so that
+// the exponent (x - 1) ln(lam / y) + y - lam is free of large cancelling
+// terms: relative error 7e-14 rms over x and lam up to 1e3, 9e-13 for
+// exp(-lam + (x - 1) ln lam - lgamma(x)), at a third of the instructions.
+__device__ __forceinline__ double
+shifted_poisson(double x, double lam)
+{
+  const double y = x + 10.0, r = 1.0 / y, r2 = r * r, r4 = r2 * r2;
+  double s = fma(r2, 1.0 / 156.0, -691.0 / 360360.0);
+  s = fma(s, r2, 1.0 / 1188.0);
+  s = fma(s, r2, -1.0 / 1680.0);
+  s = fma(s, r2, 1.0 / 1260.0);
+  s = fma(s, r2, -1.0 / 360.0);
+  s = fma(s, r2, 1.0 / 12.0);
+  const double p = (x * (x + 1.0)) * ((x + 2.0) * (x + 3.0)) * ((x + 4.0) * (x + 5.0)) *
+                   ((x + 6.0) * (x + 7.0)) * ((x + 8.0) * (x + 9.0)) * (r4 * r4 * r2);
+  return (1.0 / kSqrt2Pi) * p * sqrt(r) * exp((x - 1.0) * log(lam * r) + ((y - lam) - s * r));
+}
+
+// Per (reference z node, sample): the moments of the shifted-Poisson MOR
+// (P_operator::set_sample, p_operator_t.hh:150-219) of every richness bin
+// whose grid points read the node.
+__global__ void __launch_bounds__(kSampleThreads)
+bsel_sample_kernel(BselDims D, const double* __restrict__ blocks,
+                   const unsigned* __restrict__ need, double* __restrict__ mom)
+{
+  extern __shared__ double ssm[];  // n, b [3][n_lnm] | mi, lam [n_lnm] | weights [n_lnm][8]
+  const int iz = blockIdx.x, s = blockIdx.y, tid = threadIdx.x;
+  const int NM = D.n_lnm, NL = D.n_lt;
+  unsigned used = 0;
+  for (int bb = 0; bb < 4; ++bb)
+    used |= ((need[((size_t)s * 4 + bb) * D.need_words + (iz >> 5)] >> (iz & 31)) & 1u) << bb;
+  if (!used) return;
+  const double* B = blocks + (size_t)s * D.blk;
+  double* n_s = ssm;
+  double* b_s = n_s + 3 * NM;
+  double* mi_s = b_s + 3 * NM;
+  double* lam_s = mi_s + NM;
+  double* wt = lam_s + NM;
+  const double z = D.zr[iz];
+  const double Mmin = pow(10.0, B[7]), M1 = pow(10.0, B[8]);
+  const double alpha = B[9], eps = B[10], sig_l = B[11], zpiv = B[12], dM1 = M1 - Mmin;
+  const double zfac = pow((1.0 + z) / (1.0 + zpiv), eps);
+  for (int k = tid; k < 7 * NM; k += kSampleThreads) {
+    const int what = k / NM, iM = k - what * NM;
+    const double x = D.lnm_x[iM];
+    if (what < 6) {  // n and b at the nodes iz - 1, iz, iz + 1
+      const double zn = D.zr[min(max(iz + what % 3 - 1, 0), D.n_zr - 1)];
+      if (what < 3)
+        n_s[k] = interp2d_clamp(B + D.o_mh, D.n_hm, B + D.o_hz, D.n_hz, B + D.o_dn, x, zn) *
+                 (B[5] * (x * kLog10e - kHmfPivot) + B[6]);
+      else
+        b_s[k - 3 * NM] =
+          interp2d_clamp(B + D.o_bl, D.n_hl, B + D.o_bz, D.n_bz, B + D.o_bi, x, zn);
+    } else {
+      const double dM = fmax(exp(x) - Mmin, 0.0);
+      const double l_sat = (dM > 0.0 && dM1 > 0.0) ? pow(dM / dM1, alpha) * zfac : 0.0;
+      const double mi = (l_sat * sig_l) * (l_sat * sig_l);
+      mi_s[iM] = mi;
+      lam_s[iM] = fmax(l_sat + mi, 1.0e-300);
+    }
   }
   __syncthreads();
-  for (int it = tid; it < NT; it += nt) {  // theta-only caches
-    const double th = ths[it];
-    const double sn = sin(th);
-    cst[it] = cos(th);
-    sgm[it] = 1.0 / (1.0 + exp(-sc[14] * (th - sc[15])));
-    omt[it] = wths[it] * 2.0 * kPi * sn;
+  for (int iM = tid; iM < NM; iM += kSampleThreads) {
+    const double w = D.lnm_w[iM];
+    const double nm = w * n_s[iM], n0 = w * n_s[NM + iM], np = w * n_s[2 * NM + iM];
+    const double bm = b_s[iM], b0 = b_s[NM + iM], bp = b_s[2 * NM + iM];
+    double* v = wt + kMoments * iM;
+    v[0] = n0;
+    v[1] = np;
+    v[2] = nm;
+    v[3] = n0 * b0;
+    v[4] = n0 * bp + np * b0;
+    v[5] = np * bp;
+    v[6] = nm * b0 + n0 * bm;
+    v[7] = nm * bm;
   }
-  // Mass sums W_P1[lt, z], W_I[lt, z] (p_operator_t.hh:433-455), z nodes in
-  // the photo-z support only; lambda_true fastest for the MOR reads.
+  __syncthreads();
+  for (int k = tid; k < 4 * NL; k += kSampleThreads) {
+    const int bb = k / NL, il = k - bb * NL;
+    if (!((used >> bb) & 1u)) continue;
+    const double lt = D.lt_x[k];
+    double acc[kMoments];
+#pragma unroll
+    for (int m = 0; m < kMoments; ++m) acc[m] = 0.0;
+#pragma unroll 2
+    for (int iM = 0; iM < NM; ++iM) {
+      const double p = shifted_poisson(lt + mi_s[iM], lam_s[iM]);
+#pragma unroll
+      for (int m = 0; m < kMoments; ++m) acc[m] = fma(wt[kMoments * iM + m], p, acc[m]);
+    }
+    double* dst = mom + (size_t)s * D.mom + bb * D.mom_bin + (size_t)iz * kMoments * NL + il;
+#pragma unroll
+    for (int m = 0; m < kMoments; ++m) dst[(size_t)m * NL] = acc[m];
+  }
+}
+
+// Shared-memory doubles of bsel_point_kernel for the shapes in D (all theta
+// nodes in one block).
+__host__ __device__ inline long
+point_smem_doubles(const BselDims& D)
+{
+  const long NZ = D.nz_max, NT = D.n_th;
+  return 2L * D.n_lt * NZ + 2L * D.n_lt + 3 * NZ + (NZ & 1) + NT * NZ + (NT * NZ + 7) / 8 +
+         2 * (NT + kPointWarps);
+}
+
+// One block per (grid point, sample, group of theta nodes): the mass sums
+// W_P1, W_I from the moments (p_operator_t.hh:433-455), then
+// sum_z sum_lt f_A W over theta > theta_excl(z) for each theta node
+// (p_operator_t.hh:457-505) -> part[..][theta] = (P, xi I).  The block's
+// (theta, z, lambda_true) terms are dealt to its warps in equal runs, z
+// fastest, so that a warp's lanes share the overlap's branch; a run's sums are
+// written per theta and added in the order of the warps.  Bound by the FP64
+// units (the overlap's two angles and square root).
+__global__ void __launch_bounds__(kPointThreads, 2)
+bsel_point_kernel(BselDims D, const double* __restrict__ blocks,
+                  const double* __restrict__ grids, const double* __restrict__ mom,
+                  double2* __restrict__ part)
+{
+  extern __shared__ __align__(16) double sm[];
+  const int g = blockIdx.x, s = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double* B = blocks + (size_t)s * D.blk;
+  const double* G = grids + ((size_t)s * D.n_gp + g) * D.grid;
+  const double* Z = G + D.g_z;
+  const double* T = G + D.g_th;
+  const int NZ = D.nz_max, NL = D.n_lt, NT = D.n_th, bin = D.gp_bin[g];
+  const int t0 = (int)((long)NT * blockIdx.z / gridDim.z);
+  const int t1 = (int)((long)NT * (blockIdx.z + 1) / gridDim.z), nt = t1 - t0;
+  double2* out = part + ((size_t)s * D.n_gp + g) * NT;
+  if (G[3] != 0.0) {
+    for (int it = t0 + tid; it < t1; it += kPointThreads) out[it] = make_double2(0.0, 0.0);
+    return;
+  }
+  const double theta_lob = G[0], chi_o = G[1];
+  const int Nz = (int)G[2], n_pair = Nz * NL;
+  double* WP = sm;                    // [NL][Nz]
+  double* WI = WP + (size_t)NL * NZ;
+  double* rl = WI + (size_t)NL * NZ;  // [NL] R_lambda(lambda_true)
+  double* ia = rl + NL;               // [NL] 1 / (pi R_lambda^2)
+  double* thx = ia + NL;              // [Nz]
+  double* ic1 = thx + NZ;             // [Nz] (1 + z) / chi
+  double* c2 = ic1 + NZ;              // [Nz] its inverse square
+  double2* red = reinterpret_cast<double2*>(c2 + NZ + (NZ & 1));
+  double* xi = reinterpret_cast<double*>(red + nt + kPointWarps);  // [nt][Nz]
+  uint8_t* on = reinterpret_cast<uint8_t*>(xi + (size_t)nt * NZ);  // [nt][Nz]
+  for (int il = tid; il < NL; il += kPointThreads) {
+    const double r = D.rl[bin * NL + il];
+    rl[il] = r;
+    ia[il] = 1.0 / (kPi * r * r);
+  }
+  for (int iz = tid; iz < Nz; iz += kPointThreads) {
+    const double c = Z[5 * NZ + iz];
+    thx[iz] = Z[4 * NZ + iz];
+    ic1[iz] = c;
+    c2[iz] = 1.0 / (c * c);
+  }
   {
     const double* ltx = D.lt_x + bin * NL;
     const double* ltw = D.lt_w + bin * NL;
-    const double* hm = Wk + D.w_hmf;
-    const double* hb = Wk + D.w_hmb;
-    const double* mor = Wk + D.w_mor + (size_t)bin * D.mor_bin;
-    for (int k = tid; k < Nz * NL; k += nt) {
+    const double* m = mom + (size_t)s * D.mom + bin * D.mom_bin;
+    for (int k = tid; k < n_pair; k += kPointThreads) {
       const int iz = k / NL, il = k - iz * NL;
-      if (wzv[iz] == 0.0) continue;
-      const double pref = wzv[iz] * dvz[iz] * wzs[iz];
-      const double lt_wlt = ltx[il] * ltw[il];
-      const int i = izl[iz];
-      const double f = fzz[iz];
-      const double* h0r = hm + (size_t)i * NM;
-      const double* h1r = h0r + NM;
-      const double* b0r = hb + (size_t)i * NM;
-      const double* b1r = b0r + NM;
-      const double* m0 = mor + (size_t)i * NM * NL + il;
-      const double* m1 = m0 + (size_t)NM * NL;
+      const double cz = Z[3 * NZ + iz];
       double aP = 0.0, aI = 0.0;
-      for (int iM = 0; iM < NM; ++iM) {
-        const double nM = h0r[iM] + f * (h1r[iM] - h0r[iM]);
-        const double bM = b0r[iM] + f * (b1r[iM] - b0r[iM]);
-        const double a = m0[(size_t)iM * NL], b = m1[(size_t)iM * NL];
-        const double pm = a + f * (b - a);
-        const double common = D.lnm_w[iM] * nM * pm;
-        aP += common;
-        aI += common * bM;
+      if (Z[4 * NZ + iz] < 1e299) {
+        const double g1 = Z[NZ + iz], g0 = 1.0 - g1;
+        const double* a = m + (size_t)(int)Z[iz] * kMoments * NL + il;  // node i
+        const double* b = a + kMoments * NL;                            // node i + 1
+        aP = g0 * (g0 * a[0] + g1 * a[NL]) + g1 * (g0 * b[2 * NL] + g1 * b[0]);
+        aI = g0 * (g0 * g0 * a[3 * NL] + g0 * g1 * a[4 * NL] + g1 * g1 * a[5 * NL]) +
+             g1 * (g0 * g0 * b[7 * NL] + g0 * g1 * b[6 * NL] + g1 * g1 * b[3 * NL]);
       }
-      WP[(size_t)il * NZ + iz] = pref * lt_wlt * aP;
-      WI[(size_t)il * NZ + iz] = pref * lt_wlt * aI;
+      const double w = cz * (ltx[il] * ltw[il]);
+      WP[il * Nz + iz] = w * aP;
+      WI[il * Nz + iz] = w * aI;
     }
   }
-  __syncthreads();
-  // (theta, z) partial sums over lambda_true (p_operator_t.hh:457-505)
-  {
-    const double* rl = D.rl + bin * NL;
-    const double r_lo = B[D.o_xr], r_hi = B[D.o_xr + D.n_xr - 1];
-    for (int k = tid; k < NT * Nz; k += nt) {
+  {  // xi_NL at z_obs and the separation (xi_lookup_, p_operator_t.hh:636-647)
+    const double* xz = B + D.o_xz;
+    const double* xr = B + D.o_xr;
+    const double uz = (D.gp_zob[g] - xz[0]) * (1.0 / (xz[1] - xz[0]));
+    int j = (int)floor(uz);
+    j = j < 0 ? 0 : (j > D.n_xz - 2 ? D.n_xz - 2 : j);
+    const double fz = uz - j, r_lo = xr[0], r_hi = xr[D.n_xr - 1];
+    const double ln0 = log(r_lo), inv = 1.0 / log(xr[1] / r_lo);
+    const double* x0 = B + D.o_xi + (size_t)j * D.n_xr;
+    const double* x1 = x0 + D.n_xr;
+    for (int k = tid; k < nt * Nz; k += kPointThreads) {
       const int it = k / Nz, iz = k - it * Nz;
-      const double theta = ths[it];
-      double sP1 = 0.0, sI1 = 0.0, sJ = 0.0;
-      if (wzv[iz] != 0.0 && theta > thx[iz]) {
-        const double cz = chz[iz];
+      const bool in = T[t0 + it] > Z[4 * NZ + iz];
+      on[k] = in;
+      double v = 0.0;
+      if (in) {
+        const double cz = Z[2 * NZ + iz];
         const double dchi =
-          sqrt(fmax(cz * cz + chi_o * chi_o - 2.0 * cz * chi_o * cst[it], 0.0));
-        // xi_lookup_ (p_operator_t.hh:636-647)
+          sqrt(fmax(cz * cz + chi_o * chi_o - 2.0 * cz * chi_o * T[3 * NT + t0 + it], 0.0));
         const double r = dchi < r_lo ? r_lo : (r_hi < dchi ? r_hi : dchi);
-        const double u = (log(r) - sc[12]) * sc[13];
+        const double u = (log(r) - ln0) * inv;
         int ir = (int)floor(u);
         ir = ir < 0 ? 0 : (ir > D.n_xr - 2 ? D.n_xr - 2 : ir);
-        const double fr = u - ir;
-        const double xi = xir[ir] + fr * (xir[ir + 1] - xir[ir]);
-        const double icz = ic1[iz];
-        for (int il = 0; il < NL; ++il) {
-          const double theta_lt = rl[il] * icz;
-          const double fA = area_overlap(theta, theta_lob, theta_lt);
-          const double wb = fA * WP[(size_t)il * NZ + iz];
-          const double wi = fA * WI[(size_t)il * NZ + iz];
-          sP1 += wb;
-          sI1 += wi * xi;
-          sJ += wi * xi;
-        }
-        sI1 = sI1 * sgm[it];
-        sJ = sJ * (1.0 - sgm[it]);
+        const double a = x0[ir] + fz * (x1[ir] - x0[ir]);
+        const double b = x0[ir + 1] + fz * (x1[ir + 1] - x0[ir + 1]);
+        v = a + (u - ir) * (b - a);
       }
-      pP[(size_t)it * NZ + iz] = sP1;
-      pI[(size_t)it * NZ + iz] = sI1;
-      pJ[(size_t)it * NZ + iz] = sJ;
+      xi[k] = v;
     }
   }
   __syncthreads();
-  // z in order per theta node, then theta in order.
-  for (int it = tid; it < NT; it += nt) {
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int iz = 0; iz < Nz; ++iz) {
-      a += pP[(size_t)it * NZ + iz];
-      b += pI[(size_t)it * NZ + iz];
-      c += pJ[(size_t)it * NZ + iz];
+  // Units of 32 (z, lambda_true) pairs; warp w takes [w U / 16, (w + 1) U / 16).
+  const int u_th = (n_pair + 31) / 32;
+  const long U = (long)nt * u_th;
+  const long ua = U * warp / kPointWarps, ub = U * (warp + 1) / kPointWarps;
+  for (long u = ua; u < ub;) {
+    const int it = (int)(u / u_th);
+    const long ue = min(ub, (long)(it + 1) * u_th);
+    const double th = T[t0 + it];
+    const double* xt = xi + (size_t)it * Nz;
+    const uint8_t* ot = on + (size_t)it * Nz;
+    int e = (int)(u - (long)it * u_th) * 32 + lane, il = e / Nz, iz = e - il * Nz;
+    double sP = 0.0, sI = 0.0;
+    for (; u < ue; ++u) {
+      if (e < n_pair && ot[iz]) {
+        const double l = rl[il] * ic1[iz];
+        double fA = 0.0;
+        if (th <= fabs(theta_lob - l)) {
+          const double q = theta_lob / l;
+          fA = l <= theta_lob ? 1.0 : q * q;
+        } else if (!(th > theta_lob + l)) {
+          fA = lens_area(th, theta_lob, l) * (ia[il] * c2[iz]);
+        }
+        sP = fma(fA, WP[e], sP);
+        sI = fma(fA * WI[e], xt[iz], sI);
+      }
+      e += 32;
+      iz += 32;
+      while (iz >= Nz) {
+        iz -= Nz;
+        ++il;
+      }
     }
-    pP[(size_t)it * NZ] = a;
-    pI[(size_t)it * NZ] = b;
-    pJ[(size_t)it * NZ] = c;
+    for (int off = 16; off > 0; off >>= 1) {
+      sP += __shfl_xor_sync(0xffffffffu, sP, off);
+      sI += __shfl_xor_sync(0xffffffffu, sI, off);
+    }
+    // The (theta, warp) pairs of the runs climb a staircase: theta + warp is
+    // a place of its own.
+    if (lane == 0) red[it + warp] = make_double2(sP, sI);
   }
   __syncthreads();
-  if (tid == 0) {
-    double P1 = 0.0, I1 = 0.0, J = 0.0;
-    for (int it = 0; it < NT; ++it) {
-      P1 += omt[it] * pP[(size_t)it * NZ];
-      I1 += omt[it] * pI[(size_t)it * NZ];
-      J += omt[it] * pJ[(size_t)it * NZ];
+  for (int it = tid; it < nt; it += kPointThreads) {
+    double a = 0.0, b = 0.0;
+    for (int w = 0; w < kPointWarps; ++w) {
+      const long lo = max(U * w / kPointWarps, (long)it * u_th);
+      const long hi = min(U * (w + 1) / kPointWarps, (long)(it + 1) * u_th);
+      if (lo < hi) {
+        a += red[it + w].x;
+        b += red[it + w].y;
+      }
     }
-    o[0] = P1;
-    o[1] = I1;
-    o[2] = J;
+    out[t0 + it] = make_double2(a, b);
   }
+}
+
+// P1, I1 and J of every (grid point, sample): theta in order.
+__global__ void __launch_bounds__(128)
+bsel_sum_kernel(BselDims D, const double* __restrict__ grids, const double2* __restrict__ part,
+                int n, double* __restrict__ out)
+{
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const double* T = grids + (size_t)k * D.grid + D.g_th;
+  const double2* P = part + (size_t)k * D.n_th;
+  double a = 0.0, b = 0.0, c = 0.0;
+  if (grids[(size_t)k * D.grid + 3] == 0.0)
+    for (int it = 0; it < D.n_th; ++it) {
+      const double w = T[D.n_th + it], sg = T[2 * D.n_th + it];
+      a += w * P[it].x;
+      b += w * (P[it].y * sg);
+      c += w * (P[it].y * (1.0 - sg));
+    }
+  out[3 * (size_t)k] = a;
+  out[3 * (size_t)k + 1] = b;
+  out[3 * (size_t)k + 2] = c;
 }
 
 }  // namespace
@@ -485,10 +598,11 @@ struct y3b_bsel {
   std::vector<double> gp_zlo, gp_zhi, gp_zob, gp_zfg, gp_zbg;
   std::vector<int> gp_bin;
   std::vector<double> lnm_x, lnm_w, lt_x, lt_w, rl, zr;  // lt_x, lt_w, rl: [4][n_lt]
-  unsigned bins_used = 0;
+  int n_sm = 1;
   int max_samples = 64;
-  y3b::DevBuf<double> d_const, d_blocks, d_work, d_out;
-  y3b::DevBuf<int> d_int;  // grid-point bins | status word
+  y3b::DevBuf<double> d_const, d_blocks, d_mom, d_grids, d_part, d_out;
+  y3b::DevBuf<int> d_int;  // grid-point bins
+  y3b::DevBuf<unsigned> d_need;  // bits of the reference z nodes read
   double* h_stage = nullptr;  // pinned: sample blocks
   size_t h_stage_cap = 0;
   double* h_out = nullptr;  // pinned: results
@@ -596,16 +710,12 @@ layout(const y3b_bsel* h, const y3b_bsel_sample& s0, BselDims& D)
   D.o_xz = o, o += D.n_xz;
   D.o_xi = o, o += (long)D.n_xr * D.n_xz;
   D.blk = (o + 1) & ~1L;
-  long w = 0;
-  D.w_chi = w, w += D.n_zr;
-  D.w_dv = w, w += D.n_zr;
-  D.w_sig = w, w += D.n_zr;
-  D.w_hmf = w, w += (long)D.n_zr * D.n_lnm;
-  D.w_hmb = w, w += (long)D.n_zr * D.n_lnm;
-  D.w_mor = (w + 1) & ~1L;
-  D.mor_bin = (long)D.n_zr * D.n_lnm * D.n_lt;
-  D.work = D.w_mor + 4 * D.mor_bin;
-  D.bins_used = h->bins_used;
+  D.mom_bin = (long)D.n_zr * kMoments * D.n_lt;
+  D.mom = 4 * D.mom_bin;
+  D.need_words = (D.n_zr + 31) / 32;
+  D.g_z = kGpScal;
+  D.g_th = D.g_z + 6L * D.nz_max;
+  D.grid = D.g_th + 4L * D.n_th;
 }
 
 }  // namespace
@@ -646,7 +756,6 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
     h->gp_bin.push_back(b);
     h->gp_zfg.push_back(bisect_fg(zob));
     h->gp_zbg.push_back(bisect_bg(zob));
-    h->bins_used |= 1u << b;
   }
   h->cfg.zo_low = h->gp_zlo.data();
   h->cfg.zo_high = h->gp_zhi.data();
@@ -677,10 +786,19 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
   put(h->gp_zob.data(), ngp);
   put(h->gp_zfg.data(), ngp);
   put(h->gp_zbg.data(), ngp);
-  int rc = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking),
+  for (int n : {cfg->n_zouter, cfg->n_zring, cfg->n_theta, cfg->n_theta / 2,
+                cfg->n_theta - cfg->n_theta / 2}) {
+    gl_nodes_host(-1.0, 1.0, n, x, w);
+    put(x.data(), n);
+    put(w.data(), n);
+  }
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int rc = cuda_status(cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, dev),
+                       "cudaDeviceGetAttribute");
+  if (!rc) rc = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking),
                        "cudaStreamCreate");
-  std::vector<int> ints(h->gp_bin);
-  ints.push_back(0);
+  const std::vector<int>& ints = h->gp_bin;
   for (int i = 0; i < 2 && !rc; ++i)
     rc = cuda_status(cudaEventCreate(&h->ev[i]), "cudaEventCreate");
   if (!rc) rc = h->d_const.upload(cst.data(), cst.size(), h->stream);
@@ -738,7 +856,8 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
       set_error("y3b_bsel_eval: sample %d has table shapes different from sample 0", k);
       return Y3B_ERR_INVALID;
     }
-    if (!(c.zt_ref_low >= t.dist_z[0] && c.zt_ref_high <= t.dist_z[t.n_dist - 1])) {
+    if (!(c.zt_ref_low >= t.dist_z[0] && c.zt_ref_high <= t.dist_z[t.n_dist - 1] &&
+          h->zr.back() <= t.dist_z[t.n_dist - 1])) {
       set_error("argument out of range in Interp1D (sample %d: the reference z grid "
                 "[%g, %g] leaves distances/z)", k, c.zt_ref_low, c.zt_ref_high);
       return Y3B_ERR_DOMAIN;
@@ -767,8 +886,12 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
   D.gp_zob = D.zk_s + kZKernelNodes;
   D.gp_zfg = D.gp_zob + ngp;
   D.gp_zbg = D.gp_zfg + ngp;
+  D.gl_out = D.gp_zbg + ngp;
+  D.gl_ring = D.gl_out + 2 * c.n_zouter;
+  D.gl_th = D.gl_ring + 2 * c.n_zring;
+  D.gl_th1 = D.gl_th + 2 * c.n_theta;
+  D.gl_th2 = D.gl_th1 + 2 * (c.n_theta / 2);
   D.gp_bin = h->d_int.get();
-  int* d_status = h->d_int.get() + ngp;
   const int chunk = std::min(n_samples, h->max_samples);
   // Pinned staging for the sample blocks and the results.
   const size_t stage = (size_t)chunk * D.blk, outn = (size_t)chunk * ngp * 3;
@@ -787,10 +910,13 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
     h->h_out_cap = outn;
   }
   Y3B_TRY(h->d_blocks.alloc(stage));
-  Y3B_TRY(h->d_work.alloc((size_t)chunk * D.work));
+  Y3B_TRY(h->d_mom.alloc((size_t)chunk * D.mom));
+  Y3B_TRY(h->d_grids.alloc((size_t)chunk * ngp * D.grid));
+  Y3B_TRY(h->d_part.alloc(2 * (size_t)chunk * ngp * c.n_theta));
+  const size_t needs = (size_t)chunk * 4 * D.need_words;
+  Y3B_TRY(h->d_need.alloc(needs));
   Y3B_TRY(h->d_out.alloc(outn));
   cudaStream_t st = h->stream;
-  Y3B_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
   h->last_kernel_ms = 0.0;
   for (int k0 = 0; k0 < n_samples; k0 += chunk) {
     const int nk = std::min(chunk, n_samples - k0);
@@ -820,12 +946,26 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
     Y3B_CUDA(cudaMemcpyAsync(h->d_blocks.get(), h->h_stage, sizeof(double) * nk * D.blk,
                              cudaMemcpyHostToDevice, st));
     Y3B_CUDA(cudaEventRecord(h->ev[0], st));
-    bsel_sample_kernel<<<dim3(D.n_zr, nk), kSampleThreads, 3 * sizeof(double) * c.n_lnm, st>>>(
-      D, h->d_blocks.get(), h->d_work.get(), d_status);
+    Y3B_CUDA(cudaMemsetAsync(h->d_need.get(), 0, needs * sizeof(unsigned), st));
+    double2* part = reinterpret_cast<double2*>(h->d_part.get());
+    bsel_grid_kernel<<<dim3(ngp, nk), kGridThreads, 0, st>>>(D, h->d_blocks.get(),
+                                                            h->d_grids.get(), h->d_need.get());
     count_launch();
     Y3B_CUDA(cudaGetLastError());
-    bsel_point_kernel<<<dim3(ngp, nk), kPointThreads, smem, st>>>(D, h->d_blocks.get(),
-                                                                 h->d_work.get(), h->d_out.get());
+    bsel_sample_kernel<<<dim3(D.n_zr, nk), kSampleThreads,
+                         (8 + kMoments) * sizeof(double) * c.n_lnm, st>>>(
+      D, h->d_blocks.get(), h->d_need.get(), h->d_mom.get());
+    count_launch();
+    Y3B_CUDA(cudaGetLastError());
+    // Few (grid point, sample) pairs: several blocks each, by theta.
+    const int split =
+      std::max(1, std::min(c.n_theta, 2 * h->n_sm / std::max(1, ngp * nk)));
+    bsel_point_kernel<<<dim3(ngp, nk, split), kPointThreads, smem, st>>>(
+      D, h->d_blocks.get(), h->d_grids.get(), h->d_mom.get(), part);
+    count_launch();
+    Y3B_CUDA(cudaGetLastError());
+    bsel_sum_kernel<<<(ngp * nk + 127) / 128, 128, 0, st>>>(D, h->d_grids.get(), part, ngp * nk,
+                                                           h->d_out.get());
     count_launch();
     Y3B_CUDA(cudaGetLastError());
     Y3B_CUDA(cudaEventRecord(h->ev[1], st));
@@ -837,5 +977,5 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
     h->last_kernel_ms += ms;
     std::memcpy(out + (size_t)k0 * ngp * 3, h->h_out, sizeof(double) * nk * ngp * 3);
   }
-  return read_device_status(d_status, st);
+  return Y3B_OK;
 }
