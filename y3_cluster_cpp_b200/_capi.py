@@ -251,7 +251,7 @@ def check(rc):
 
 
 def f64(a):
-    return np.ascontiguousarray(np.asarray(a, dtype=np.float64))
+    return np.ascontiguousarray(a, dtype=np.float64)
 
 
 def ptr(a):

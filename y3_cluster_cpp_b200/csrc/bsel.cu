@@ -67,7 +67,7 @@ lob_centre(int b)
   return b == 0 ? 25.0 : (b == 1 ? 37.5 : (b == 2 ? 52.5 : 130.0));
 }
 constexpr int kPointThreads = 512, kPointWarps = kPointThreads / 32;
-constexpr int kGridThreads = 128;
+constexpr int kGridThreads = 96;
 constexpr int kSampleThreads = 256;
 constexpr int kScal = 16;  // scalars at the head of a sample block
 constexpr int kMoments = 8;
@@ -104,42 +104,64 @@ chi_at(const BselDims& D, const double* B, double z)  // chi_.clamp(z) h0
   return interp1d_clamp(B + D.o_dz, B + D.o_dc, D.nd, z) * B[4];
 }
 
-// Angle of (x, y), y >= 0, in [0, pi]: the ratio reduced to |q| <= tan(pi/8),
-// atan(q) / q a degree-11 polynomial in q^2 (Chebyshev interpolation,
-// relative error 7e-17).
+// 1 / sqrt(v) for normal v > 0: the hardware's approximation and one step of
+// the third-order Newton iteration (error e -> 5/16 e^3).
 __device__ __forceinline__ double
-angle(double y, double x)
+rsqrt_newton(double v)
 {
-  const double ax = fabs(x), mn = fmin(y, ax), mx = fmax(y, ax);
-  const bool mid = mn > 0.41421356237309503 * mx;
-  const double q = (mid ? mn - mx : mn) / (mid ? mn + mx : mx), z = q * q;
-  double s = -1.78038963948125642e-02;
-  s = fma(s, z, 3.79639031611108332e-02);
-  s = fma(s, z, -5.03504979531243929e-02);
-  s = fma(s, z, 5.84686675227513927e-02);
-  s = fma(s, z, -6.66295024603679176e-02);
-  s = fma(s, z, 7.69204519456148095e-02);
-  s = fma(s, z, -9.09089680147281282e-02);
-  s = fma(s, z, 1.11111107446570989e-01);
-  s = fma(s, z, -1.42857142792449682e-01);
-  s = fma(s, z, 1.99999999999408373e-01);
-  s = fma(s, z, -3.33333333333331205e-01);
-  double a = fma(s, z * q, q) + (mid ? 0.25 * kPi : 0.0);
-  a = y > ax ? 0.5 * kPi - a : a;
-  return x < 0.0 ? kPi - a : a;
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+  const double e = fma(-(v * r), r, 1.0);
+  return fma(fma(0.375, e, 0.5), r * e, r);
+}
+
+// atan on [0, 1]: atan(q) / q as a degree-19 polynomial in q^2 (Chebyshev
+// interpolation of the function, truncation 3e-17).
+__device__ __forceinline__ double
+atan01(double q)
+{
+  const double z = q * q;
+  double s = -1.93423475928923002e-05;
+  s = fma(s, z, 2.14238107386039464e-04);
+  s = fma(s, z, -1.12525443022346450e-03);
+  s = fma(s, z, 3.75113848396514118e-03);
+  s = fma(s, z, -8.99108054265826059e-03);
+  s = fma(s, z, 1.67195960635073901e-02);
+  s = fma(s, z, -2.55686236443717387e-02);
+  s = fma(s, z, 3.38712670270067476e-02);
+  s = fma(s, z, -4.08112475031788546e-02);
+  s = fma(s, z, 4.66874530484852890e-02);
+  s = fma(s, z, -5.23742347191881660e-02);
+  s = fma(s, z, 5.87682811448727235e-02);
+  s = fma(s, z, -6.66576491068972266e-02);
+  s = fma(s, z, 7.69219899745829383e-02);
+  s = fma(s, z, -9.09089979321734132e-02);
+  s = fma(s, z, 1.11111105780020827e-01);
+  s = fma(s, z, -1.42857142669267329e-01);
+  s = fma(s, z, 1.99999999996479605e-01);
+  s = fma(s, z, -3.33333333333307003e-01);
+  return fma(s, z * q, q);
 }
 
 // Overlap area of two disks of radii o and l at distance t, partially
-// overlapping (p_op_detail::area_overlap, p_operator_cuhre_t.hh:97-125): the
-// lens angles come from the triangle (t, l, o) as angles of (4 x its area,
-// t^2 + l^2 - o^2) and (.., t^2 + o^2 - l^2), which lose no digits near
-// tangency, in place of two acos of cosines.
+// overlapping, |o - l| < t <= o + l (p_op_detail::area_overlap,
+// p_operator_cuhre_t.hh:97-125), from the triangle with sides t, l, o: with
+// s1 = o + l - t, s2 = t - (o - l), s3 = t + (o - l), s4 = t + l + o and
+// y = sqrt(s1 s2 s3 s4) (four times its area), the half angles at the two
+// centres have the tangents s1 s3 / y and s1 s2 / y, reciprocals s2 s4 / y and
+// s3 s4 / y.  One reciprocal square root and two polynomials in place of two
+// acos, three divisions and a square root, and no digits are lost near
+// tangency.
 __device__ __forceinline__ double
 lens_area(double t, double o, double l)
 {
-  const double sq = (l + o - t) * (t + l - o) * (t - l + o) * (t + l + o);
-  const double r = sqrt(fmax(sq, 0.0)), t2 = t * t, l2 = l * l, o2 = o * o;
-  return fma(l2, angle(r, t2 + (l2 - o2)), fma(o2, angle(r, t2 + (o2 - l2)), -0.5 * r));
+  const double d = o - l, s1 = (o + l) - t, s2 = t - d, s3 = t + d, s4 = (o + l) + t;
+  const double a = s1 * s3, b = s2 * s4, c = s1 * s2, e = s3 * s4;
+  const double sq = fmax(a * b, 1e-290), r = rsqrt_newton(sq);
+  const bool big1 = a > b, big2 = c > e;  // tangent above 1: the complement of the angle
+  const double h1 = atan01((big1 ? b : a) * r), h2 = atan01((big2 ? e : c) * r);
+  const double a1 = big1 ? 0.5 * kPi - h1 : h1, a2 = big2 ? 0.5 * kPi - h2 : h2;
+  return fma(2.0 * (l * l), a1, fma(2.0 * (o * o), a2, -0.5 * (sq * r)));
 }
 
 // Lower bracket of z on the reference grid: i = min(trunc(u), n - 2) with
@@ -189,7 +211,7 @@ invert_chi(const BselDims& D, const double* B, double target)
 // One block per (grid point, sample): P_operator::evaluate's grids
 // (p_operator_t.hh:222-430).  Latency-bound (interpolations, bisections), so
 // small blocks, many to an SM.
-__global__ void __launch_bounds__(kGridThreads)
+__global__ void __launch_bounds__(kGridThreads, 8)
 bsel_grid_kernel(BselDims D, const double* __restrict__ blocks, double* __restrict__ grids,
                  unsigned* __restrict__ need)
 {
@@ -311,7 +333,7 @@ bsel_grid_kernel(BselDims D, const double* __restrict__ blocks, double* __restri
 __device__ __forceinline__ double
 shifted_poisson(double x, double lam)
 {
-  const double y = x + 10.0, r = 1.0 / y, r2 = r * r, r4 = r2 * r2;
+  const double y = x + 10.0, q = rsqrt_newton(y), r = q * q, r2 = r * r, r4 = r2 * r2;
   double s = fma(r2, 1.0 / 156.0, -691.0 / 360360.0);
   s = fma(s, r2, 1.0 / 1188.0);
   s = fma(s, r2, -1.0 / 1680.0);
@@ -320,13 +342,13 @@ shifted_poisson(double x, double lam)
   s = fma(s, r2, 1.0 / 12.0);
   const double p = (x * (x + 1.0)) * ((x + 2.0) * (x + 3.0)) * ((x + 4.0) * (x + 5.0)) *
                    ((x + 6.0) * (x + 7.0)) * ((x + 8.0) * (x + 9.0)) * (r4 * r4 * r2);
-  return (1.0 / kSqrt2Pi) * p * sqrt(r) * exp((x - 1.0) * log(lam * r) + ((y - lam) - s * r));
+  return (1.0 / kSqrt2Pi) * p * q * exp((x - 1.0) * log(lam * r) + ((y - lam) - s * r));
 }
 
 // Per (reference z node, sample): the moments of the shifted-Poisson MOR
 // (P_operator::set_sample, p_operator_t.hh:150-219) of every richness bin
 // whose grid points read the node.
-__global__ void __launch_bounds__(kSampleThreads)
+__global__ void __launch_bounds__(kSampleThreads, 4)
 bsel_sample_kernel(BselDims D, const double* __restrict__ blocks,
                    const unsigned* __restrict__ need, double* __restrict__ mom)
 {
@@ -344,9 +366,7 @@ bsel_sample_kernel(BselDims D, const double* __restrict__ blocks,
   double* lam_s = mi_s + NM;
   double* wt = lam_s + NM;
   const double z = D.zr[iz];
-  const double Mmin = pow(10.0, B[7]), M1 = pow(10.0, B[8]);
-  const double alpha = B[9], eps = B[10], sig_l = B[11], zpiv = B[12], dM1 = M1 - Mmin;
-  const double zfac = pow((1.0 + z) / (1.0 + zpiv), eps);
+  const double Mmin = B[7], dM1 = B[8], alpha = B[9], sig_l = B[11];
   for (int k = tid; k < 7 * NM; k += kSampleThreads) {
     const int what = k / NM, iM = k - what * NM;
     const double x = D.lnm_x[iM];
@@ -360,7 +380,9 @@ bsel_sample_kernel(BselDims D, const double* __restrict__ blocks,
           interp2d_clamp(B + D.o_bl, D.n_hl, B + D.o_bz, D.n_bz, B + D.o_bi, x, zn);
     } else {
       const double dM = fmax(exp(x) - Mmin, 0.0);
-      const double l_sat = (dM > 0.0 && dM1 > 0.0) ? pow(dM / dM1, alpha) * zfac : 0.0;
+      const double l_sat = (dM > 0.0 && dM1 > 0.0)
+                             ? pow(dM / dM1, alpha) * pow((1.0 + z) / (1.0 + B[12]), B[10])
+                             : 0.0;
       const double mi = (l_sat * sig_l) * (l_sat * sig_l);
       mi_s[iM] = mi;
       lam_s[iM] = fmax(l_sat + mi, 1.0e-300);
@@ -524,17 +546,17 @@ bsel_point_kernel(BselDims D, const double* __restrict__ blocks,
     const double* xt = xi + (size_t)it * Nz;
     const uint8_t* ot = on + (size_t)it * Nz;
     int e = (int)(u - (long)it * u_th) * 32 + lane, il = e / Nz, iz = e - il * Nz;
+    const double full = kPi * theta_lob * theta_lob;
     double sP = 0.0, sI = 0.0;
     for (; u < ue; ++u) {
       if (e < n_pair && ot[iz]) {
         const double l = rl[il] * ic1[iz];
         double fA = 0.0;
-        if (th <= fabs(theta_lob - l)) {
-          const double q = theta_lob / l;
-          fA = l <= theta_lob ? 1.0 : q * q;
-        } else if (!(th > theta_lob + l)) {
-          fA = lens_area(th, theta_lob, l) * (ia[il] * c2[iz]);
-        }
+        const double inv = ia[il] * c2[iz];  // 1 / (pi l^2)
+        if (th <= fabs(theta_lob - l))
+          fA = l <= theta_lob ? 1.0 : full * inv;
+        else if (!(th > theta_lob + l))
+          fA = lens_area(th, theta_lob, l) * inv;
         sP = fma(fA, WP[e], sP);
         sI = fma(fA * WI[e], xt[iz], sI);
       }
@@ -593,6 +615,13 @@ bsel_sum_kernel(BselDims D, const double* __restrict__ grids, const double2* __r
 }  // namespace
 }  // namespace y3b
 
+namespace y3b {
+// A chunk is packed, copied and evaluated in up to kPieces pieces of at least
+// kPieceSamples samples: the host packs a piece while the device works on the
+// one before.
+constexpr int kPieces = 8, kPieceSamples = 24;
+}  // namespace y3b
+
 struct y3b_bsel {
   y3b_bsel_config cfg;
   std::vector<double> gp_zlo, gp_zhi, gp_zob, gp_zfg, gp_zbg;
@@ -608,7 +637,7 @@ struct y3b_bsel {
   double* h_out = nullptr;  // pinned: results
   size_t h_out_cap = 0;
   cudaStream_t stream = nullptr;
-  cudaEvent_t ev[2] = {nullptr, nullptr};  // around each chunk's kernels
+  cudaEvent_t ev[2 * y3b::kPieces] = {};  // around the kernels of a chunk's pieces
   double last_kernel_ms = 0.0;
   ~y3b_bsel()
   {
@@ -799,7 +828,7 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
   if (!rc) rc = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking),
                        "cudaStreamCreate");
   const std::vector<int>& ints = h->gp_bin;
-  for (int i = 0; i < 2 && !rc; ++i)
+  for (int i = 0; i < 2 * kPieces && !rc; ++i)
     rc = cuda_status(cudaEventCreate(&h->ev[i]), "cudaEventCreate");
   if (!rc) rc = h->d_const.upload(cst.data(), cst.size(), h->stream);
   if (!rc) rc = h->d_int.upload(ints.data(), ints.size(), h->stream);
@@ -919,63 +948,72 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
   cudaStream_t st = h->stream;
   h->last_kernel_ms = 0.0;
   for (int k0 = 0; k0 < n_samples; k0 += chunk) {
-    const int nk = std::min(chunk, n_samples - k0);
+    const int n_chunk = std::min(chunk, n_samples - k0);
+    const int pieces = std::max(1, std::min(kPieces, n_chunk / kPieceSamples));
     // The previous chunk's copies out of the staging buffers are done.
     Y3B_CUDA(cudaStreamSynchronize(st));
-    for (int k = 0; k < nk; ++k) {
-      const y3b_bsel_sample& s = S[k0 + k];
-      double* b = h->h_stage + (size_t)k * D.blk;
-      const double sc[kScal] = {s.cosmo.om, s.cosmo.onu, s.cosmo.ol, s.cosmo.ok, s.cosmo.h0,
-                                s.cosmo.hmf_s, s.cosmo.hmf_q, s.hod[0], s.hod[1], s.hod[2],
-                                s.hod[3], s.hod[4], s.hod[5], 0.0, 0.0, 0.0};
-      std::memcpy(b, sc, sizeof sc);
-      for (int i = 0; i < D.n_hm; ++i)  // HMF_t's log mass axis (hmf_t.hh:16-25)
-        b[D.o_mh + i] = std::log(s.t.hmf_m_h[i] * (s.cosmo.om - s.cosmo.onu));
-      std::memcpy(b + D.o_hz, s.t.hmf_z, sizeof(double) * D.n_hz);
-      std::memcpy(b + D.o_dn, s.t.dndlnmh, sizeof(double) * D.n_hz * D.n_hm);
-      std::memcpy(b + D.o_dz, s.t.dist_z, sizeof(double) * D.nd);
-      std::memcpy(b + D.o_da, s.t.dist_da, sizeof(double) * D.nd);
-      std::memcpy(b + D.o_dc, s.dist_dc, sizeof(double) * D.nd);
-      std::memcpy(b + D.o_bl, s.halo_lnM, sizeof(double) * D.n_hl);
-      std::memcpy(b + D.o_bz, s.halo_z, sizeof(double) * D.n_bz);
-      std::memcpy(b + D.o_bi, s.bias, sizeof(double) * D.n_hl * D.n_bz);
-      std::memcpy(b + D.o_xr, s.xi_r, sizeof(double) * D.n_xr);
-      std::memcpy(b + D.o_xz, s.xi_z, sizeof(double) * D.n_xz);
-      std::memcpy(b + D.o_xi, s.xi_nl, sizeof(double) * D.n_xr * D.n_xz);
-    }
-    Y3B_CUDA(cudaMemcpyAsync(h->d_blocks.get(), h->h_stage, sizeof(double) * nk * D.blk,
-                             cudaMemcpyHostToDevice, st));
-    Y3B_CUDA(cudaEventRecord(h->ev[0], st));
     Y3B_CUDA(cudaMemsetAsync(h->d_need.get(), 0, needs * sizeof(unsigned), st));
-    double2* part = reinterpret_cast<double2*>(h->d_part.get());
-    bsel_grid_kernel<<<dim3(ngp, nk), kGridThreads, 0, st>>>(D, h->d_blocks.get(),
-                                                            h->d_grids.get(), h->d_need.get());
-    count_launch();
-    Y3B_CUDA(cudaGetLastError());
-    bsel_sample_kernel<<<dim3(D.n_zr, nk), kSampleThreads,
-                         (8 + kMoments) * sizeof(double) * c.n_lnm, st>>>(
-      D, h->d_blocks.get(), h->d_need.get(), h->d_mom.get());
-    count_launch();
-    Y3B_CUDA(cudaGetLastError());
-    // Few (grid point, sample) pairs: several blocks each, by theta.
-    const int split =
-      std::max(1, std::min(c.n_theta, 2 * h->n_sm / std::max(1, ngp * nk)));
-    bsel_point_kernel<<<dim3(ngp, nk, split), kPointThreads, smem, st>>>(
-      D, h->d_blocks.get(), h->d_grids.get(), h->d_mom.get(), part);
-    count_launch();
-    Y3B_CUDA(cudaGetLastError());
-    bsel_sum_kernel<<<(ngp * nk + 127) / 128, 128, 0, st>>>(D, h->d_grids.get(), part, ngp * nk,
-                                                           h->d_out.get());
-    count_launch();
-    Y3B_CUDA(cudaGetLastError());
-    Y3B_CUDA(cudaEventRecord(h->ev[1], st));
-    Y3B_CUDA(cudaMemcpyAsync(h->h_out, h->d_out.get(), sizeof(double) * nk * ngp * 3,
+    for (int pc = 0; pc < pieces; ++pc) {
+      const int ka = (int)((long)n_chunk * pc / pieces);
+      const int nk = (int)((long)n_chunk * (pc + 1) / pieces) - ka;
+      for (int k = 0; k < nk; ++k) {
+        const y3b_bsel_sample& s = S[k0 + ka + k];
+        double* b = h->h_stage + (size_t)(ka + k) * D.blk;
+        const double Mmin = std::pow(10.0, s.hod[0]), M1 = std::pow(10.0, s.hod[1]);
+        const double sc[kScal] = {s.cosmo.om, s.cosmo.onu, s.cosmo.ol, s.cosmo.ok, s.cosmo.h0,
+                                  s.cosmo.hmf_s, s.cosmo.hmf_q, Mmin, M1 - Mmin, s.hod[2],
+                                  s.hod[3], s.hod[4], s.hod[5], 0.0, 0.0, 0.0};
+        std::memcpy(b, sc, sizeof sc);
+        for (int i = 0; i < D.n_hm; ++i)  // HMF_t's log mass axis (hmf_t.hh:16-25)
+          b[D.o_mh + i] = std::log(s.t.hmf_m_h[i] * (s.cosmo.om - s.cosmo.onu));
+        std::memcpy(b + D.o_hz, s.t.hmf_z, sizeof(double) * D.n_hz);
+        std::memcpy(b + D.o_dn, s.t.dndlnmh, sizeof(double) * D.n_hz * D.n_hm);
+        std::memcpy(b + D.o_dz, s.t.dist_z, sizeof(double) * D.nd);
+        std::memcpy(b + D.o_da, s.t.dist_da, sizeof(double) * D.nd);
+        std::memcpy(b + D.o_dc, s.dist_dc, sizeof(double) * D.nd);
+        std::memcpy(b + D.o_bl, s.halo_lnM, sizeof(double) * D.n_hl);
+        std::memcpy(b + D.o_bz, s.halo_z, sizeof(double) * D.n_bz);
+        std::memcpy(b + D.o_bi, s.bias, sizeof(double) * D.n_hl * D.n_bz);
+        std::memcpy(b + D.o_xr, s.xi_r, sizeof(double) * D.n_xr);
+        std::memcpy(b + D.o_xz, s.xi_z, sizeof(double) * D.n_xz);
+        std::memcpy(b + D.o_xi, s.xi_nl, sizeof(double) * D.n_xr * D.n_xz);
+      }
+      double* blocks = h->d_blocks.get() + (size_t)ka * D.blk;
+      double* grids = h->d_grids.get() + (size_t)ka * ngp * D.grid;
+      double* mom = h->d_mom.get() + (size_t)ka * D.mom;
+      unsigned* need = h->d_need.get() + (size_t)ka * 4 * D.need_words;
+      double2* part = reinterpret_cast<double2*>(h->d_part.get()) + (size_t)ka * ngp * c.n_theta;
+      double* o = h->d_out.get() + (size_t)ka * ngp * 3;
+      Y3B_CUDA(cudaMemcpyAsync(blocks, h->h_stage + (size_t)ka * D.blk,
+                               sizeof(double) * nk * D.blk, cudaMemcpyHostToDevice, st));
+      Y3B_CUDA(cudaEventRecord(h->ev[2 * pc], st));
+      bsel_grid_kernel<<<dim3(ngp, nk), kGridThreads, 0, st>>>(D, blocks, grids, need);
+      count_launch();
+      Y3B_CUDA(cudaGetLastError());
+      bsel_sample_kernel<<<dim3(D.n_zr, nk), kSampleThreads,
+                           (8 + kMoments) * sizeof(double) * c.n_lnm, st>>>(D, blocks, need, mom);
+      count_launch();
+      Y3B_CUDA(cudaGetLastError());
+      // Few (grid point, sample) pairs: several blocks each, by theta.
+      const int split = std::max(1, std::min(c.n_theta, 2 * h->n_sm / std::max(1, ngp * nk)));
+      bsel_point_kernel<<<dim3(ngp, nk, split), kPointThreads, smem, st>>>(D, blocks, grids, mom,
+                                                                          part);
+      count_launch();
+      Y3B_CUDA(cudaGetLastError());
+      bsel_sum_kernel<<<(ngp * nk + 127) / 128, 128, 0, st>>>(D, grids, part, ngp * nk, o);
+      count_launch();
+      Y3B_CUDA(cudaGetLastError());
+      Y3B_CUDA(cudaEventRecord(h->ev[2 * pc + 1], st));
+    }
+    Y3B_CUDA(cudaMemcpyAsync(h->h_out, h->d_out.get(), sizeof(double) * n_chunk * ngp * 3,
                              cudaMemcpyDeviceToHost, st));
     Y3B_CUDA(cudaStreamSynchronize(st));
-    float ms = 0.f;
-    Y3B_CUDA(cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]));
-    h->last_kernel_ms += ms;
-    std::memcpy(out + (size_t)k0 * ngp * 3, h->h_out, sizeof(double) * nk * ngp * 3);
+    for (int pc = 0; pc < pieces; ++pc) {
+      float ms = 0.f;
+      Y3B_CUDA(cudaEventElapsedTime(&ms, h->ev[2 * pc], h->ev[2 * pc + 1]));
+      h->last_kernel_ms += ms;
+    }
+    std::memcpy(out + (size_t)k0 * ngp * 3, h->h_out, sizeof(double) * n_chunk * ngp * 3);
   }
   return Y3B_OK;
 }

@@ -12,6 +12,7 @@ Every call runs on the GPU through ``lib/liby3b.so``; a failure raises
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import numpy as np
 
@@ -28,6 +29,14 @@ def _mor(kind, params):
     for i, v in enumerate(params):
         m.p[i] = float(v)
     return m
+
+
+def _address(a):
+    """Address of an array's data (writable, non-empty arrays the fast way)."""
+    try:
+        return C.addressof(C.c_char.from_buffer(a))
+    except (TypeError, ValueError):
+        return a.ctypes.data
 
 
 def _plob(z, coef, keep):
@@ -276,27 +285,27 @@ class BselMarg:
 
     __del__ = close
 
+    # y3b_bsel_sample after its cosmology, as _RECORD packs it.
+    _RECORD = struct.Struct("@iPiPPiPPiPPP2i3P2i3P6d")
+
     def eval(self, samples):
         n = len(samples)
+        size, head = C.sizeof(A.BselSample), C.sizeof(A.Cosmo)
         arr = (A.BselSample * max(n, 1))()
+        buf = (C.c_ubyte * C.sizeof(arr)).from_buffer(arr)
         keep = []
         for k, (cz, tables, prj, hod) in enumerate(samples):
-            t = [f64(tables[x]) for x in ("hmf_m_h", "hmf_z", "dndlnmh", "dist_z", "dist_da")]
-            p = {x: f64(prj[x]) for x in ("dist_dc", "halo_lnM", "halo_z", "bias", "xi_r",
-                                          "xi_z", "xi_nl")}
-            keep += t + list(p.values())
-            s = arr[k]
-            s.cosmo = cz
-            s.t = A.Tables(len(t[0]), ptr(t[0]), len(t[1]), ptr(t[1]), ptr(t[2]), len(t[3]),
-                           ptr(t[3]), ptr(t[4]), 0, None, None)
-            s.dist_dc = ptr(p["dist_dc"])
-            s.n_hl, s.n_hz = len(p["halo_lnM"]), len(p["halo_z"])
-            s.halo_lnM, s.halo_z, s.bias = ptr(p["halo_lnM"]), ptr(p["halo_z"]), ptr(p["bias"])
-            s.n_xr, s.n_xz = len(p["xi_r"]), len(p["xi_z"])
-            s.xi_r, s.xi_z, s.xi_nl = ptr(p["xi_r"]), ptr(p["xi_z"]), ptr(p["xi_nl"])
-            for i, key in enumerate(self.HOD_KEYS):
-                s.hod[i] = float(hod[key])
-            s.hod[5] = float(hod.get("z_pivot", 0.45))
+            v = [f64(d[x]) for d, x in
+                 [(tables, x) for x in ("hmf_m_h", "hmf_z", "dndlnmh", "dist_z", "dist_da")] +
+                 [(prj, x) for x in ("dist_dc", "halo_lnM", "halo_z", "bias", "xi_r", "xi_z",
+                                     "xi_nl")]]
+            keep.append(v)
+            mh, hz, dn, dz, da, dc, hl, bz, bi, xr, xz, xi = [_address(a) for a in v]
+            arr[k].cosmo = cz
+            self._RECORD.pack_into(
+                buf, k * size + head, len(v[0]), mh, len(v[1]), hz, dn, len(v[3]), dz, da, 0, 0, 0,
+                dc, len(v[6]), len(v[7]), hl, bz, bi, len(v[9]), len(v[10]), xr, xz, xi,
+                *[float(hod[x]) for x in self.HOD_KEYS], float(hod.get("z_pivot", 0.45)))
         out = np.empty((n, self.n_gp, 3))
         check(lib().y3b_bsel_eval(self._h, n, arr, ptr(out)))
         return out
