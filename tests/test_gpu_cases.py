@@ -103,3 +103,36 @@ def test_fp64_shear_outside_the_profile_table(gpu):
 def test_selection_bias(gpu, n, n_lt, n_zring, n_zouter, n_lnm, n_theta, n_zt_ref):
     _compare(dict(kind="bsel", n=n, n_lt=n_lt, n_zring=n_zring, n_zouter=n_zouter, n_lnm=n_lnm,
                   n_theta=n_theta, n_zt_ref=n_zt_ref), 1e-10)
+
+
+# The mixed form's stacked shear: 12 bins take whole passes of 4 x 3; one
+# point, several per warp, node sets of different sizes in one call.
+@pytest.mark.parametrize("n,radii,mixed", [(1, 1, False), (45, 15, False), (40, 4, True)])
+def test_mixed_shear(gpu, n, radii, mixed):
+    _compare(dict(kind="engine", api="device", precision="mixed", n=n, radii=radii, hmf_fp32=False,
+                  loglike=radii == 15, mixed_density=mixed, n_m=70, n_z=32, n_t=64, n_o=32,
+                  n_zo=9), 1e-4)
+
+
+@pytest.mark.parametrize("nI,nJ", [(1, 1), (3, 2), (5, 4), (8, 3)])
+def test_mixed_shear_bin_layouts(gpu, nI, nJ):
+    """Bin counts that leave partial passes of richness and z_obs bins, against
+    the engine's FP64 form (the mixed form's bound, 1e-4)."""
+    from y3_cluster_cpp_b200 import engine as E
+    from y3_cluster_cpp_b200 import synthetic
+
+    g = synthetic.grid(1, n_m=40, n_z=16, n_t=64, n_o=16, n_zo=8,
+                       lam_edges=np.geomspace(20.0, 200.0, nI + 1),
+                       zob_edges=np.linspace(0.2, 0.65, nJ + 1))
+    so = synthetic.shear_opts(n_theta=16, n_s=32, n_R=3)
+    so["lob_centers"] = np.geomspace(25.0, 130.0, nI)
+    pts = synthetic.walkers(5, seed=4, densities=(1,))
+    t = pts[0].tables
+    eng = E.Engine([g], len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]),
+                   synthetic.plob_baseline(), max_points=5, n_sci=len(t["sci_z"]), shear=so)
+    a = eng.eval(pts, E.MIXED, grid_of=lambda p: 0)
+    b = eng.eval(pts, E.FP64, grid_of=lambda p: 0)
+    for k in ("counts", "shear"):
+        assert a[k].shape == b[k].shape and np.all(np.isfinite(a[k]))
+        np.testing.assert_allclose(a[k], b[k], rtol=1e-4)
+    eng.close()

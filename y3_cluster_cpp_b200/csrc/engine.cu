@@ -1246,16 +1246,12 @@ cen_table_kernel(double u0, double du, double* row)
   if (j < kMisNx) row[j] = NfwUnit<double>::dsigma(exp(u0 + j * du));
 }
 
-// Phi_i(R, k) of the mixed form from the table, one thread per (point, k):
-// c(M), r_s and the normalisation once; per R the table position
-// u = ln R - ln r_s and its 4-point Lagrange weights, then the centred
-// profile and the miscentred one of each bin i from their rows.  A point
-// whose x = R / r_s falls outside the table reports a domain error (the
-// table covers Omega_m from 0.01 to 1 over the engine's masses and radii).
+// ln r_s and w_k times the profile's normalisation of every (point, mass):
+// S[2 p][k], S[2 p + 1][k].  Depends on the points alone, so it runs beside the
+// prep kernel.
 __global__ void __launch_bounds__(128)
-shear_tab_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_stride,
-                 ShearDev sh, const double* tab, double u0, double inv_du, double* Phi,
-                 int nI_max, int grid_mask, int* status)
+shear_mass_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_stride,
+                  ShearDev sh, int grid_mask, double* __restrict__ S)
 {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_points * w_stride) return;
@@ -1264,33 +1260,134 @@ shear_tab_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w_
   if (!grid_in_mask(grid_mask, pt.grid)) return;
   const GridDev& G = grids[pt.grid];
   if (k >= G.n_m) return;
-  const double lnM = G.xm[k];
+  const double lnM = G.xm[k], rho = kRhoCrit * pt.om;
   const double c = sh.c0 * pow(exp(lnM) / sh.c_pivot, sh.c_slope);
-  const double rho = kRhoCrit * pt.om;
-  const double rs = nfw_rs(lnM, c, rho);
-  const double norm = nfw_norm(lnM, c, rho);
-  const double ln_rs = log(rs);
-  const double* cen_row = tab + (size_t)nI_max * sh.n_R * kMisNx;
+  S[(size_t)(2 * p) * w_stride + k] = log(nfw_rs(lnM, c, rho));
+  S[(size_t)(2 * p + 1) * w_stride + k] = G.wm[k] * nfw_norm(lnM, c, rho);
+}
+
+// Stacked shear of the mixed form, N_b(R) = sum_k w_k W^g_b(k) Phi_i(R, k)
+// with Phi from the table.  A block holds the table rows of one radius in
+// shared memory (16 KB a row: lanes over k read nodes a few apart, two
+// wavefronts a load where the same reads of global memory touch a dozen
+// lines) and its warps take points in turn, lanes over k; Phi serves the
+// bin's z_obs bins as it is formed and is never stored.  As two kernels, one
+// writing [point][bin][R][k] and one summing it, 2048 points at 64 masses and
+// 15 radii took 53 + 75 us; here 51 us, about half of it the shared-memory
+// wavefronts of the table reads.  Two blocks of 256 threads an SM: with more
+// warps the sixteen sums spill (384 threads 61 us, 512 threads 75 us).  A point whose x = R / r_s falls outside the table
+// reports a domain error (it covers Omega_m from 0.01 to 1 over the engine's
+// masses and radii).
+// FULL: whole passes of kShI x kShJ bins (the wall grids of the configs), so
+// no bin is tested.
+constexpr int kShThreads = 256;
+constexpr int kShI = 4, kShJ = 3;  // richness and z_obs bins of one pass
+
+template <bool FULL>
+__global__ void __launch_bounds__(kShThreads, 2)
+shear_sum_kernel(const GridDev* grids, int n_grids, int nI, int nJ, const PointDev* pts,
+                 int n_points, int w_stride, ShearDev sh, const double* __restrict__ tab, double u0,
+                 double inv_du, const double* __restrict__ S, const double* __restrict__ Wg,
+                 int nB_max, double* __restrict__ shear, int grid_mask, int* status)
+{
+  extern __shared__ __align__(16) double rows[];  // [1 + nI][kMisNx]: centred, i = 0, 1, ..
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ int n_m_s[31];
+  const int R = blockIdx.y, lane = threadIdx.x & 31;
+  if (threadIdx.x < n_grids) n_m_s[threadIdx.x] = grids[threadIdx.x].n_m;
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&bar)),
+                 "r"((uint32_t)((nI + 1) * kMisNx * sizeof(double)))
+                 : "memory");
+    for (int i = -1; i < nI; ++i)
+      bulk_copy_g2s(rows + (size_t)(i + 1) * kMisNx,
+                    tab + (size_t)(i < 0 ? nI * sh.n_R : i * sh.n_R + R) * kMisNx,
+                    (uint32_t)(kMisNx * sizeof(double)), &bar);
+  }
+  __syncthreads();
+  {
+    long long t0 = clock64();
+    uint32_t ok = 0;
+    while (!ok) {
+      asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_addr(&bar))
+        : "memory");
+      if (!ok && clock64() - t0 > 2000000000LL) break;
+    }
+    if (__syncthreads_or(!ok)) {  // uniform exit; the copies only target this CTA's shared memory
+      if (threadIdx.x == 0) set_err(status, kDevTimeout);
+      return;
+    }
+  }
+  const double lnR = sh.lnR[R];
   bool bad = false;
-  for (int iR = 0; iR < sh.n_R; ++iR) {
-    const double tt = (sh.lnR[iR] - ln_rs - u0) * inv_du;
-    int j = (int)floor(tt);
-    if (!(tt >= 1.0 && tt <= kMisNx - 2.0)) {
-      bad = true;
-      j = min(max(j, 1), kMisNx - 3);
-    }
-    const double f = tt - j;
-    const double l0 = -f * (f - 1.0) * (f - 2.0) / 6.0, l1 = (f + 1.0) * (f - 1.0) * (f - 2.0) * 0.5;
-    const double l2 = -(f + 1.0) * f * (f - 2.0) * 0.5, l3 = (f + 1.0) * f * (f - 1.0) / 6.0;
-    const double* yc = cen_row + j;
-    const double cen =
-      (1.0 - sh.f_mis) * (l0 * __ldg(yc - 1) + l1 * __ldg(yc) + l2 * __ldg(yc + 1) + l3 * __ldg(yc + 2));
-    for (int i = 0; i < G.nI; ++i) {
-      const double* y = tab + ((size_t)i * sh.n_R + iR) * kMisNx + j;
-      const double mis = l0 * __ldg(y - 1) + l1 * __ldg(y) + l2 * __ldg(y + 1) + l3 * __ldg(y + 2);
-      Phi[(((size_t)p * nI_max + i) * sh.n_R + iR) * w_stride + k] =
-        norm * (cen + sh.f_mis * mis);
-    }
+  constexpr int nw = kShThreads / 32;
+  int p = blockIdx.x * nw + (threadIdx.x >> 5);
+  int g_next = p < n_points ? pts[p].grid : 0;  // a point ahead
+  for (; p < n_points; p += gridDim.x * nw) {
+    const int g = g_next;
+    if (p + (int)gridDim.x * nw < n_points) g_next = pts[p + gridDim.x * nw].grid;
+    if (!grid_in_mask(grid_mask, g)) continue;
+    const int n_m = n_m_s[g];
+    const double* ln_rs = S + (size_t)(2 * p) * w_stride;
+    const size_t sj = (size_t)nI * w_stride;
+    for (int i0 = 0; i0 < nI; i0 += kShI)
+      for (int j0 = 0; j0 < nJ; j0 += kShJ) {
+        const double* W = Wg + ((size_t)p * nI * nJ + i0 + nI * j0) * w_stride;
+        double acc[kShI * 4];  // [i][j], j = 3 stays zero
+#pragma unroll
+        for (int u = 0; u < kShI * 4; ++u) acc[u] = 0.0;
+        for (int k = lane; k < n_m; k += 32) {
+          double w[kShI][kShJ];
+#pragma unroll
+          for (int i = 0; i < kShI; ++i)
+#pragma unroll
+            for (int j = 0; j < kShJ; ++j)
+              w[i][j] = FULL || (i0 + i < nI && j0 + j < nJ) ? W[i * w_stride + j * sj + k] : 0.0;
+          const double tt = (lnR - ln_rs[k] - u0) * inv_du, wn = ln_rs[w_stride + k];
+          const double ft = floor(tt), f = tt - ft;
+          int jn = (int)ft;
+          if (!(tt >= 1.0 && tt <= kMisNx - 2.0)) {
+            bad = true;
+            jn = min(max(jn, 1), kMisNx - 3);
+          }
+          const double m1 = f - 1.0, m2 = f - 2.0, p1 = f + 1.0, a = f * m1, b = p1 * m2;
+          const double l0 = -a * m2 * (1.0 / 6.0), l1 = b * m1 * 0.5, l2 = -b * f * 0.5;
+          const double l3 = p1 * a * (1.0 / 6.0);
+          const double* y = rows + jn;
+          const double cen =
+            (1.0 - sh.f_mis) * (l0 * y[-1] + l1 * y[0] + l2 * y[1] + l3 * y[2]);
+#pragma unroll
+          for (int i = 0; i < kShI; ++i) {
+            if (!FULL && i0 + i >= nI) break;
+            y = rows + (size_t)(1 + i0 + i) * kMisNx + jn;
+            const double mis = l0 * y[-1] + l1 * y[0] + l2 * y[1] + l3 * y[2];
+            const double phi = wn * (cen + sh.f_mis * mis);
+#pragma unroll
+            for (int j = 0; j < kShJ; ++j) acc[4 * i + j] += w[i][j] * phi;
+          }
+        }
+        // Sixteen sums over the lanes by halving exchanges: lane 2 u ends with
+        // sum u = 4 i + j.
+#pragma unroll
+        for (int h = 8; h >= 1; h >>= 1) {
+          const bool up = (lane & (2 * h)) != 0;
+#pragma unroll
+          for (int u = 0; u < h; ++u) {
+            const double send = up ? acc[u] : acc[u + h];
+            acc[u] = (up ? acc[u + h] : acc[u]) + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+          }
+        }
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+        const int i = i0 + (lane >> 3), j = (lane >> 1) & 3;
+        if ((lane & 1) == 0 && j < kShJ && (FULL || (i < nI && j0 + j < nJ)))
+          shear[((size_t)p * nB_max + i + nI * (j0 + j)) * sh.n_R + R] = acc[0];
+      }
   }
   if (bad) set_err(status, kDevDomain);
 }
@@ -1350,8 +1447,9 @@ shear_tab64_kernel(const GridDev* grids, const PointDev* pts, int n_points, int 
       norm * (cen + sh.f_mis * read(tab + ((size_t)i * sh.n_R + iR) * kMisNx));
 }
 
-// N_b = sum_k w_k W_b(k); N_b(R) = sum_k w_k W^g_b(k) Phi_i(R, k).  CTA per
-// point, warp per output, fixed xor-tree order.
+// N_b = sum_k w_k W_b(k) and, where Phi is given (the FP64 form), N_b(R) =
+// sum_k w_k W^g_b(k) Phi_i(R, k).  CTA per point, warp per output, fixed
+// xor-tree order.
 __global__ void __launch_bounds__(256)
 finalize_kernel(const GridDev* grids, const PointDev* pts, const double* W, const double* Wg,
                 const double* Phi, int w_stride, int nB_max, int nI_max, int n_R,
@@ -1411,6 +1509,10 @@ finalize_kernel(const GridDev* grids, const PointDev* pts, const double* W, cons
       }
     }
   }
+  // The mixed form's shear is summed before this kernel.
+  if (shear && !Phi && like.on && logL)
+    for (int u = threadIdx.x; u < G.nB * n_R; u += blockDim.x)
+      s_sh[u] = shear[(size_t)p * nB_max * n_R + u];
   // The point's Gaussian likelihood, in the block that produced its counts
   // and shear (likelihood_cp.py:132-200): no second pass over them.
   if (like.on && logL) {
@@ -1495,8 +1597,9 @@ struct y3b_engine {
   std::vector<GraphKey> seen;         // recent evaluations without a graph
   unsigned long long graph_clock = 0;
   size_t s64_stride = 0, s32_stride = 0;
+  size_t phi_rows = 0;        // rows of w_stride doubles per point in Phi: max(nI n_R, 2)
   int w_stride = 0, nB_max = 0, nI_max = 0, nz_max = 0, nt_max = 0;
-  size_t prep_smem = 0, yf_smem = 0, direct_smem = 0;
+  size_t prep_smem = 0, yf_smem = 0, direct_smem = 0, shear_smem = 0;
   size_t device_bytes = 0;
   int last_n = 0;
   std::vector<std::array<double, 2>> zt_node_range;  // per grid: min, max z_t node
@@ -1999,6 +2102,8 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
     e->mis_u0 = std::log(x_lo / 1.5);
     e->mis_du = (std::log(x_hi * 1.5) - e->mis_u0) / (kMisNx - 1);
     const int n_pairs = e->nI_max * sh.n_R;
+    e->phi_rows = std::max(n_pairs, 2);
+    e->shear_smem = (size_t)(e->nI_max + 1) * kMisNx * sizeof(double);
     if ((rc = e->mis_tab.alloc((size_t)(n_pairs + 1) * kMisNx))) return fail(rc);
     std::vector<double> ratio(n_pairs);  // x_mis / x of each (i, R)
     for (int i = 0; i < e->nI_max; ++i)
@@ -2029,7 +2134,7 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
                                           kFStageBytes);
   bytes += N * e->f_stride;
   if (cfg->with_shear)
-    bytes += N * (size_t)e->nI_max * sh.n_R * e->w_stride * 8 + N * e->nB_max * sh.n_R * 8;
+    bytes += N * e->phi_rows * e->w_stride * 8 + N * e->nB_max * sh.n_R * 8;
   const size_t budget = cfg->hbm_budget ? cfg->hbm_budget : (size_t)150 << 30;
   // FP64 workspace: rounds of up to 128 points (100 MB at 4x nodes, so a
   // round's factors stay in L2), fewer where the budget leaves less.
@@ -2060,7 +2165,7 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
       (rc = e->f64_ws.alloc(e->f64_round * e->f64_stride)))
     return fail(rc);
   if (cfg->with_shear) {
-    if ((rc = e->Phi.alloc(N * (size_t)e->nI_max * sh.n_R * e->w_stride)) ||
+    if ((rc = e->Phi.alloc(N * e->phi_rows * e->w_stride)) ||
         (rc = e->shear_out.alloc(N * e->nB_max * (size_t)sh.n_R)))
       return fail(rc);
   }
@@ -2080,6 +2185,14 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
                                 (int)cudaSharedmemCarveoutMaxShared));
   Y3B_CUDA(cudaFuncSetAttribute(yf_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 (int)cudaSharedmemCarveoutMaxShared));
+  if (e->shear_smem) {
+    Y3B_CUDA(cudaFuncSetAttribute(shear_sum_kernel<true>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)e->shear_smem));
+    Y3B_CUDA(cudaFuncSetAttribute(shear_sum_kernel<false>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)e->shear_smem));
+  }
   Y3B_CUDA(cudaFuncSetAttribute(direct_main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)e->direct_smem));
   *out = e;
@@ -2147,8 +2260,8 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
 {
   double* W = e->W.get() + w_off * e->nB_max * e->w_stride;
   double* Wg = e->Wg.get() + w_off * e->nB_max * e->w_stride;
-  double* Phi = e->Phi.get() ? e->Phi.get() + w_off * e->nI_max * e->shear.n_R * e->w_stride
-                             : nullptr;
+  // Phi of the FP64 form; ln r_s and the mass weights of the mixed form's shear.
+  double* Phi = e->Phi.get() ? e->Phi.get() + w_off * e->phi_rows * e->w_stride : nullptr;
   if (prec == Y3B_FP64 && e->lay.hmf_f32) {
     set_error("an engine with FP32 dndlnmh tables (hmf_fp32) evaluates the mixed form only");
     return Y3B_ERR_INVALID;
@@ -2177,7 +2290,14 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
     Y3B_TRY(contract_check(L));
     Y3B_CUDA(cudaEventRecord(e->plan_fork, s));
     Y3B_CUDA(cudaStreamWaitEvent(e->pstream, e->plan_fork, 0));
-    const int prc = launch_plan(L);
+    int prc = launch_plan(L);
+    if (!prc && e->cfg.with_shear && d_shear) {
+      shear_mass_kernel<<<(unsigned)(((long long)n * e->w_stride + 127) / 128), 128, 0,
+                          e->pstream>>>(e->d_grids.get(), d_pts, n, e->w_stride, e->shear,
+                                        grid_mask, Phi);
+      count_launch();
+      prc = cuda_status(cudaGetLastError(), "shear_mass_kernel");
+    }
     Y3B_CUDA(cudaEventRecord(e->plan_join, e->pstream));
     if (prc) {  // join before returning, so that a capture in progress stays whole
       cudaStreamWaitEvent(s, e->plan_join, 0);
@@ -2243,9 +2363,14 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
                                                      e->w_stride, e->shear, e->quad.view(), Phi,
                                                      e->nI_max);
     } else {
-      shear_tab_kernel<<<blocks, 128, 0, s>>>(
-        e->d_grids.get(), d_pts, n, e->w_stride, e->shear, e->mis_tab.get(), e->mis_u0,
-        1.0 / e->mis_du, Phi, e->nI_max, grid_mask, e->status.get());
+      // Two blocks an SM over the radii, a warp at least one point.
+      const int groups = std::max(1, std::min((n + kShThreads / 32 - 1) / (kShThreads / 32),
+                                              2 * e->n_ctas / e->shear.n_R));
+      auto kernel = e->nI_max % kShI == 0 && e->grids[0].nJ % kShJ == 0 ? shear_sum_kernel<true>
+                                                                       : shear_sum_kernel<false>;
+      kernel<<<dim3(groups, e->shear.n_R), kShThreads, e->shear_smem, s>>>(
+        e->d_grids.get(), (int)e->grids.size(), e->nI_max, e->grids[0].nJ, d_pts, n, e->w_stride,
+        e->shear, e->mis_tab.get(), e->mis_u0, 1.0 / e->mis_du, Phi, Wg, e->nB_max, d_shear, grid_mask, e->status.get());
     }
     count_launch();
     Y3B_CUDA(cudaGetLastError());
@@ -2255,7 +2380,8 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
     // The likelihood needs the shear when its data vector has one.
     const bool like = e->like.on && (e->like.n_R == 0 || shear);
     finalize_kernel<<<n, 256, 0, s>>>(e->d_grids.get(), d_pts, W, Wg,
-                                      shear ? Phi : nullptr, e->w_stride, e->nB_max,
+                                      shear && prec == Y3B_FP64 ? Phi : nullptr, e->w_stride,
+                                      e->nB_max,
                                       e->nI_max, e->shear.n_R, d_counts,
                                       shear ? d_shear : nullptr, grid_mask, e->like,
                                       like ? e->logL.get() + w_off : nullptr);
