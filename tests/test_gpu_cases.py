@@ -136,3 +136,17 @@ def test_mixed_shear_bin_layouts(gpu, nI, nJ):
         assert a[k].shape == b[k].shape and np.all(np.isfinite(a[k]))
         np.testing.assert_allclose(a[k], b[k], rtol=1e-4)
     eng.close()
+
+
+# The mixed form's lnM tiles: one group of 32 rows, two, four, and a second
+# tile with a remainder; z rows that leave warps of the factor kernel short or
+# without work; FP32 and FP64 HMF tables.
+@pytest.mark.parametrize("n_m,n_z,n_t,hmf_fp32", [(20, 16, 32, False), (32, 16, 64, True),
+                                                  (33, 48, 40, False), (64, 32, 64, True),
+                                                  (65, 80, 96, False), (128, 16, 33, True),
+                                                  (129, 112, 64, False), (161, 128, 160, True),
+                                                  (193, 32, 256, False)])
+def test_mixed_row_groups(gpu, n_m, n_z, n_t, hmf_fp32):
+    _compare(dict(kind="engine", api="device", precision="mixed", n=3, radii=0, hmf_fp32=hmf_fp32,
+                  loglike=False, mixed_density=False, n_m=n_m, n_z=n_z, n_t=n_t, n_o=32, n_zo=9),
+             1e-4)

@@ -806,11 +806,26 @@ yf_smem_bytes(const TableLayout& L, int nzp_max, int n_t_pad_max)
          (size_t)n_t_pad_max * 4;
 }
 
+// An HMF z row at tile row r: linear in mass, scaled by kf_k / (sqrt(2 pi) s)
+// (the product kept apart from the differences that follow).
+__device__ __forceinline__ float
+hmf_row(const float* h, const int* rx, const float* rt, const float* rn, int r)
+{
+  const float* hx = h + rx[r];
+  return __fmul_rn(fmaf(rt[r], hx[1] - hx[0], hx[0]), rn[r]);
+}
+
 // Mixed form, one CTA per (point, 128-row lnM tile): Y(k, q) of the tile's
 // rows and its F(t, k) stage blocks, from the inputs the prep kernel wrote,
 // staged into shared memory by bulk copies on one mbarrier (the HMF grid
 // too when the packed tables hold it in FP32; an FP64 grid is converted
 // while the copies fly).
+//
+// Bound by instruction issue and the latency of a CTA's staging at small
+// grids, and by the stores of Y and F (540 MB) beside the issue at large ones.
+// Rows in groups of 32: a tile of at most 32 or 64 rows takes no work for the
+// others, which are stored as zeros.  2048 points at 64 lnM x 32 z x 64 lam_t
+// nodes, FP64 tables: 72 -> 62 us; at 256 x 128 x 256, FP32 tables: 187 -> 183.
 __global__ void __launch_bounds__(256, 3)
 yf_kernel(PrepArgs a)
 {
@@ -851,8 +866,7 @@ yf_kernel(PrepArgs a)
   // which land while the F blocks are written.
   __shared__ __align__(8) uint64_t bar, bar2;
   __shared__ int timed_out;
-  int bad = 0;
-  const size_t n_dn = (size_t)n_hz * n_hm;
+  const int n_dn = n_hz * n_hm;
   const uint32_t h_bytes = L.hmf_f32 ? (uint32_t)yf_h32_bytes(L) : 0u;
   const uint32_t bytes = kYfRowFields * kGemmRows * 4 + kGemmRows * 8 + 16 + kYfHdr * 4 + 64 +
                          12u * nzp + 4u * n_t_pad;
@@ -900,6 +914,32 @@ yf_kernel(PrepArgs a)
       }
     }
   };
+  // Non-finite HMF entries show in the largest magnitude of the FP32 bits.
+  uint32_t top = 0;
+  if (!L.hmf_f32) {  // FP64 grid: convert while the copies are in flight
+    const double2* __restrict__ d2 = reinterpret_cast<const double2*>(src + L.off[2]);
+    const int n2 = n_dn / 2;
+    for (int i0 = tid; i0 < n2; i0 += 4 * blockDim.x) {
+      double2 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * blockDim.x;
+        v[u] = i < n2 ? __ldg(d2 + i) : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * blockDim.x;
+        const float2 f = make_float2((float)v[u].x, (float)v[u].y);
+        if (i < n2) reinterpret_cast<float2*>(h32)[i] = f;
+        top = max(top, max(__float_as_uint(f.x) & 0x7fffffffu, __float_as_uint(f.y) & 0x7fffffffu));
+      }
+    }
+    if ((n_dn & 1) && tid == 0) {
+      const float f = (float)__ldg(src + L.off[2] + n_dn - 1);
+      h32[n_dn - 1] = f;
+      top = max(top, __float_as_uint(f) & 0x7fffffffu);
+    }
+  }
   wait_bar(&bar);
   __syncthreads();
   if (timed_out) {  // uniform exit; the copies only target this CTA's shared memory
@@ -919,10 +959,14 @@ yf_kernel(PrepArgs a)
   const float* row_am = rows + 4 * kGemmRows;
   const float* row_vs2 = rows + 5 * kGemmRows;
   const float2 sc2 = make_float2(sc1, sc1);
+  const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5, n8 = 2 * (w_hi - w_lo);
+  // Groups of 32 rows that take work: 1, 2 or 4 (2^lg).
+  const int n_row = n_m - mt0 * kGemmRows;
+  const int lg = n_row > 64 ? 2 : n_row > 32 ? 1 : 0, groups = 1 << lg;
   uint8_t* fb = a.fbuf + (size_t)p * a.f_stride;
   const int nk = n_t_pad / 16;
-  for (int it = w_lo * 2 * kGemmRows + tid; it < w_hi * 2 * kGemmRows; it += blockDim.x) {
-    const int r = it % kGemmRows, t8 = it / kGemmRows;
+  for (int it = warp; it < n8 << lg; it += nw) {
+    const int t8 = 2 * w_lo + (it >> lg), r = 32 * (it & (groups - 1)) + lane;
     const float am = row_am[r], vs = row_vs2[r];
     const float2 nam2 = make_float2(-am, -am), vs2 = make_float2(vs, vs);
     const float4 d0 = *reinterpret_cast<const float4*>(dt_f + t8 * 8);
@@ -939,166 +983,168 @@ yf_kernel(PrepArgs a)
     uint8_t* st = fb + ((size_t)mt0 * nk + (t8 >> 1)) * kFStageBytes + (t8 & 1) * 2048 + r * 16;
     store_split8(st, st + kFStageBytes / 2, v);
   }
-  if (!L.hmf_f32) {  // FP64 grid: convert while the copies are in flight
-    const double* __restrict__ dng = src + L.off[2];
-    const int nn = (int)n_dn;
-    for (int i0 = tid; i0 < nn; i0 += 4 * blockDim.x) {
-      double v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * blockDim.x;
-        v[u] = i < nn ? __ldg(dng + i) : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * blockDim.x;
-        if (i < nn) h32[i] = (float)v[u];
-        bad |= !isfinite(v[u]) || !isfinite((float)v[u]);
-      }
+  if (groups < 4)
+    for (int it = warp; it < n8 * 4; it += nw) {
+      if ((it & 3) < groups) continue;
+      const int t8 = 2 * w_lo + (it >> 2), r = 32 * (it & 3) + lane;
+      uint8_t* st = fb + ((size_t)mt0 * nk + (t8 >> 1)) * kFStageBytes + (t8 & 1) * 2048 + r * 16;
+      *reinterpret_cast<uint4*>(st) = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(st + kFStageBytes / 2) = make_uint4(0, 0, 0, 0);
     }
-  }
   wait_bar(&bar2);
   __syncthreads();
   if (timed_out) {
     if (tid == 0) set_err(a.status, kDevTimeout);
     return;
   }
-  if (L.hmf_f32)
-    for (int i = tid; i < (int)n_dn; i += blockDim.x) bad |= !isfinite(h32[i]);
-  if (__syncthreads_or(bad)) {
+  if (L.hmf_f32) {
+    const uint4* h4 = reinterpret_cast<const uint4*>(h32);
+    for (int j = tid; j < n_dn / 4; j += blockDim.x) {
+      const uint4 v = h4[j];
+      top = max(max(top, max(v.x & 0x7fffffffu, v.y & 0x7fffffffu)),
+                max(v.z & 0x7fffffffu, v.w & 0x7fffffffu));
+    }
+    if (tid < (n_dn & 3)) top = max(top, __float_as_uint(h32[(n_dn & ~3) + tid]) & 0x7fffffffu);
+  }
+  if (__syncthreads_or(top >= 0x7f800000u)) {
     if (tid == 0) set_err(a.status, kDevNonFinite);
     return;
   }
-  const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
   const float c2 = fh[0], mu_sat_lo = fh[1], mu_sat_hi = fh[2];
   const float mu0c = fh[4], inv_hmu_f = fh[5];
-  // Y(k, q) = n(M_k, z_q) kf_k H(k, q) 2^-(v_k^2 c1) / (sqrt(2 pi) s D_kq).
-  // Warp w takes a contiguous run of z rows and lane the tile rows
-  // lane + 32 j (j < 4).  Each lane keeps, in registers, the two HMF z rows
-  // around the current z_q interpolated in mass and scaled by
-  // kf_k / (sqrt(2 pi) s), and advances them with q (the z nodes ascend).  A
-  // z row whose tile cells all have mu more than 5.6 sigma inside the domain
-  // (D = 1 in FP32) is FP32 only.  Otherwise an unsaturated cell takes
-  // log2 D from the table by a cubic Hermite in FP32 where D >= 2^-16 (its
-  // relative error there ~1e-6); deeper in a tail, and in rows that carry a
-  // scale, by the Hermite of the FP64 table (read through L1), and forms
-  // 2^(log2 H - v^2 c1 - log2 D) in FP64, applied as an exact power of two
-  // times 2^(fraction) in FP32.
-  {
+  // Y(k, q) = n(M_k, z_q) kf_k H(k, q) 2^-(v_k^2 c1) / (sqrt(2 pi) s D_kq) of
+  // the tile's first 32 J rows.  Warp w takes a contiguous run of z rows and
+  // lane the tile rows lane + 32 j (j < J).  Each lane keeps, in registers,
+  // the HMF z row below the current z_q interpolated in mass and scaled by
+  // kf_k / (sqrt(2 pi) s), and its difference to the one above, and advances
+  // them with q (the z nodes ascend).  A z row whose tile cells all have mu
+  // more than 5.6 sigma inside the domain (D = 1 in FP32) takes no table.
+  // Otherwise an unsaturated cell takes log2 D from the table by a cubic
+  // Hermite in FP32 where D >= 2^-16 (its relative error there ~1e-6); deeper
+  // in a tail, and in rows that carry a scale, by the Hermite of the FP64
+  // table (read through L1), and forms 2^(log2 H - v^2 c1 - log2 D) in FP64,
+  // applied as an exact power of two times 2^(fraction) in FP32.  Those cells
+  // follow in a pass of their own after every eight z rows: without their
+  // FP64 code the main loop keeps all of its state in registers.
+  auto y_rows = [&](auto rows_of) {
+    constexpr int J = decltype(rows_of)::value;
     const float* rt_s = rows;
     const int* rx_s = reinterpret_cast<const int*>(rows + kGemmRows);
     const float* rn_s = rows + 2 * kGemmRows;
     const float* ra_s = rows + 3 * kGemmRows;
     const float* rvf_s = rows + 6 * kGemmRows;
+    const float tmin = __int_as_float(tinfo[0]), tmax = __int_as_float(tinfo[1]);
+    const bool scaled = tinfo[2] != 0;
     // Runs of whole pairs of z rows (n_z is a multiple of 16): Y is stored
     // [lnM tile][z / 2][128 rows][2], one float2 per lane and row.
     const int qs = ((n_z / 2 + nw - 1) / nw) * 2, qa = warp * qs, qb_end = min(n_z, qa + qs);
-    float rn[4], rk[4], R0[4], R1[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      rn[j] = rn_s[lane + 32 * j];
-      rk[j] = ra_s[lane + 32 * j];
-      R0[j] = R1[j] = 0.f;
-    }
-    const float tmin = __int_as_float(tinfo[0]), tmax = __int_as_float(tinfo[1]);
-    const bool scaled = tinfo[2] != 0;
     float* __restrict__ yblk = s32 + Gp->f_Yt + (size_t)mt0 * n_z * kGemmRows;
+    float rk[J], R0[J], R1[J], dR[J];
+    unsigned own = 0, sc_rows = 0;  // bit j: the tile has the row; it carries a scale
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int r = lane + 32 * j;
+      rk[j] = ra_s[r];
+      R0[j] = R1[j] = dR[j] = 0.f;
+      own |= (r < n_row ? 1u : 0u) << j;
+      sc_rows |= (rvf_s[r] != 0.f ? 1u : 0u) << j;
+    }
     int ycur = -2;
-    for (int q0 = qa; q0 < qb_end; q0 += 2) {
-    float yv[4][2];
+    for (int q0 = qa; q0 < qb_end; q0 += 8) {
+      const int q1 = min(q0 + 8, qb_end);
+      unsigned deep = 0u;  // bit 4 (q - q0) + j: left to the FP64 pass
+      for (int qp = q0; qp < q1; qp += 2) {
+        float yv[J][2];
 #pragma unroll
-    for (int dq = 0; dq < 2; ++dq) {
-      const int q = q0 + dq;
-      const int yq = qy[q];
-      if (yq != ycur) {  // warp-uniform
-        const float* h1 = h32 + (size_t)(yq + 1) * n_hm;
-        if (yq == ycur + 1) {
+        for (int dq = 0; dq < 2; ++dq) {
+          const int q = qp + dq;
+          const int yq = qy[q];
+          if (yq != ycur) {  // warp-uniform
+            const float* h1 = h32 + (size_t)(yq + 1) * n_hm;
+            if (yq == ycur + 1) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int x = rx_s[lane + 32 * j];
-            R0[j] = R1[j];
-            R1[j] = fmaf(rt_s[lane + 32 * j], h1[x + 1] - h1[x], h1[x]) * rn[j];
-          }
-        } else {
-          const float* h0 = h1 - n_hm;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int x = rx_s[lane + 32 * j];
-            const float t = rt_s[lane + 32 * j];
-            R0[j] = fmaf(t, h0[x + 1] - h0[x], h0[x]) * rn[j];
-            R1[j] = fmaf(t, h1[x + 1] - h1[x], h1[x]) * rn[j];
-          }
-        }
-        ycur = yq;
-      }
-      const float u = qu[q], bb = qb[q];
-      const float hx = -bb * c2, hy = -0.5f * bb * bb * c2;  // H = 2^(a hx + hy)
-      const float sat_lo = mu_sat_lo - bb, sat_hi = mu_sat_hi - bb;
-      float y[4], nv[4], e[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        nv[j] = fmaf(u, R1[j] - R0[j], R0[j]);
-        e[j] = scaled ? fmaf(rk[j], hx, hy) - rvf_s[lane + 32 * j] : fmaf(rk[j], hx, hy);
-        y[j] = nv[j] * fast_exp2(e[j]);
-      }
-      if (!(tmin > sat_lo && tmax < sat_hi)) {  // some cell of this z row is unsaturated
-        // The lane's four cells side by side and without branches (their
-        // chains interleave): the FP32 Hermite of log2 D for each, kept
-        // where the cell is unsaturated.  Deep-tail cells and rows that
-        // carry a scale follow in the rare FP64 pass below.
-        unsigned deep = 0u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = lane + 32 * j;
-          const bool sl = mt0 * kGemmRows + r < n_m && !(rk[j] > sat_lo && rk[j] < sat_hi);
-          const float uu = (rk[j] + bb - mu0c) * inv_hmu_f;
-          const int jj = min(max((int)floorf(uu), 0), kDTab - 2);
-          const float t = uu - (float)jj;
-          const float4 cf = *reinterpret_cast<const float4*>(dt32 + 4 * jj);
-          const float l2d = fmaf(fmaf(fmaf(cf.w, t, cf.z), t, cf.y), t, cf.x);
-          const float ys = nv[j] * fast_exp2(e[j] - l2d);
-          const bool shallow = l2d >= -16.f && (!scaled || rvf_s[r] == 0.f);
-          y[j] = sl && shallow ? ys : y[j];
-          deep |= (sl && !shallow) ? 1u << j : 0u;
-        }
-        if (deep) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (!(deep & (1u << j))) continue;
-            const int r = lane + 32 * j;
-            const int k = mt0 * kGemmRows + r;
-            const double alpha = __ldg(s64 + Gp->o_alpha + k), beta = __ldg(s64 + Gp->o_beta + q);
-            const double mu = alpha + beta;
-            const double ud = (mu - th[2]) * th[3];
-            const int jd = min(max((int)floor(ud), 0), kDTab - 2);
-            const double td = ud - jd, td2 = td * td, td3 = td2 * td;
-            const double* d64 = s64 + Gp->o_dt64;
-            const double l2 = (2.0 * td3 - 3.0 * td2 + 1.0) * __ldg(d64 + jd) +
-                              (td3 - 2.0 * td2 + td) * __ldg(d64 + kDTab + jd) +
-                              (3.0 * td2 - 2.0 * td3) * __ldg(d64 + jd + 1) +
-                              (td3 - td2) * __ldg(d64 + kDTab + jd + 1);
-            const double ad = alpha - th[0], bd = beta - th[1];
-            const double ex = -(ad * bd + 0.5 * bd * bd) * th[4] - row_vv[r] - l2;
-            const double ei = rint(ex);
-            const float yf = mul_pow2(nv[j] * fast_exp2((float)(ex - ei)), ei);
-            if (!(fabsf(yf) <= 3.402823466e38f)) {  // not representable: report, never a NaN
-              set_err(a.status, kDevRange);
-              y[j] = 0.f;
+              for (int j = 0; j < J; ++j) R0[j] = R1[j];
             } else {
-              y[j] = yf;
+#pragma unroll
+              for (int j = 0; j < J; ++j) R0[j] = hmf_row(h1 - n_hm, rx_s, rt_s, rn_s, lane + 32 * j);
             }
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+              R1[j] = hmf_row(h1, rx_s, rt_s, rn_s, lane + 32 * j);
+              dR[j] = R1[j] - R0[j];
+            }
+            ycur = yq;
           }
+          const float u = qu[q], bb = qb[q];
+          const float hx = -bb * c2, hy = -0.5f * bb * bb * c2;  // H = 2^(a hx + hy)
+          const float sat_lo = mu_sat_lo - bb, sat_hi = mu_sat_hi - bb;
+          float e[J];
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            e[j] = fmaf(rk[j], hx, hy);
+            if (scaled) e[j] -= rvf_s[lane + 32 * j];
+          }
+          if (!(tmin > sat_lo && tmax < sat_hi)) {  // some cell of this z row is unsaturated
+            unsigned low = 0u;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+              const bool sl = (own >> j & 1u) && !(rk[j] > sat_lo && rk[j] < sat_hi);
+              const float uu = (rk[j] + bb - mu0c) * inv_hmu_f;
+              const int jj = min(max((int)floorf(uu), 0), kDTab - 2);
+              const float t = uu - (float)jj;
+              const float4 cf = *reinterpret_cast<const float4*>(dt32 + 4 * jj);
+              const float l2d = fmaf(fmaf(fmaf(cf.w, t, cf.z), t, cf.y), t, cf.x);
+              if (sl) {
+                e[j] -= l2d;
+                low |= l2d >= -16.f ? (sc_rows & (1u << j)) : 1u << j;
+              }
+            }
+            deep |= low << (4 * (q - q0));
+          }
+#pragma unroll
+          for (int j = 0; j < J; ++j) yv[j][dq] = fmaf(u, dR[j], R0[j]) * fast_exp2(e[j]);
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<float2*>(yblk + ((size_t)(qp >> 1) * kGemmRows + lane + 32 * j) * 2) =
+            j < J ? make_float2(yv[j % J][0], yv[j % J][1]) : make_float2(0.f, 0.f);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) yv[j][dq] = y[j];
+      for (unsigned any = __reduce_or_sync(0xffffffffu, deep); any; any &= any - 1) {
+        const int b = __ffs(any) - 1;
+        if (!(deep >> b & 1u)) continue;
+        const int q = q0 + (b >> 2), r = lane + 32 * (b & 3), k = mt0 * kGemmRows + r;
+        const float* h0 = h32 + (size_t)qy[q] * n_hm;
+        const float L0 = hmf_row(h0, rx_s, rt_s, rn_s, r);
+        const float nv = fmaf(qu[q], hmf_row(h0 + n_hm, rx_s, rt_s, rn_s, r) - L0, L0);
+        const double alpha = __ldg(s64 + Gp->o_alpha + k), beta = __ldg(s64 + Gp->o_beta + q);
+        const double mu = alpha + beta;
+        const double ud = (mu - th[2]) * th[3];
+        const int jd = min(max((int)floor(ud), 0), kDTab - 2);
+        const double td = ud - jd, td2 = td * td, td3 = td2 * td;
+        const double* d64 = s64 + Gp->o_dt64;
+        const double l2 = (2.0 * td3 - 3.0 * td2 + 1.0) * __ldg(d64 + jd) +
+                          (td3 - 2.0 * td2 + td) * __ldg(d64 + kDTab + jd) +
+                          (3.0 * td2 - 2.0 * td3) * __ldg(d64 + jd + 1) +
+                          (td3 - td2) * __ldg(d64 + kDTab + jd + 1);
+        const double ad = alpha - th[0], bd = beta - th[1];
+        const double ex = -(ad * bd + 0.5 * bd * bd) * th[4] - row_vv[r] - l2;
+        const double ei = rint(ex);
+        float yf = mul_pow2(nv * fast_exp2((float)(ex - ei)), ei);
+        if (!(fabsf(yf) <= 3.402823466e38f)) {  // not representable: report, never a NaN
+          set_err(a.status, kDevRange);
+          yf = 0.f;
+        }
+        yblk[((size_t)(q >> 1) * kGemmRows + r) * 2 + (q & 1)] = yf;
+      }
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float2*>(yblk + ((size_t)(q0 >> 1) * kGemmRows + lane + 32 * j) * 2) =
-        make_float2(yv[j][0], yv[j][1]);
-    }
-  }
+  };
+  // Rows in groups of 32: tiles of up to 32, 64 or 128 rows.
+  if (lg == 0)
+    y_rows(std::integral_constant<int, 1>{});
+  else if (lg == 1)
+    y_rows(std::integral_constant<int, 2>{});
+  else
+    y_rows(std::integral_constant<int, 4>{});
 }
 
 // ---------------------------------------------------------------------------
