@@ -181,9 +181,19 @@ constexpr int kEvalChunks = 8;  // chunks of a large host-buffer evaluation
 //   FP64 form: the HMF cells and weights, the matrix product's header and
 //         windows; P0 = n(M_k,z_q) / (sqrt(2 pi) s D_kq) for the points it
 //         does not admit, which are listed for the direct sum;
-//   mixed form: a_k, b_q, delta_t, c1, c2, C_j(q), C^g_j(q) for the
+//   mixed form: b_q, delta_t, c1, c2, C_j(q), C^g_j(q) for the
 //         contraction, the lam_t windows, and yf_kernel's inputs (row
 //         blocks, z rows, the log2 D table).
+//
+// Bound by latency: a chain of short phases (a search, a logarithm, three
+// divisions and a square root per z node, then the table, then the windows),
+// so the phases are kept few and wide.  lnM and z nodes go in one pass, the
+// ranges of alpha and beta come from their end nodes (both are monotone), the
+// windows from ballots over the lam_t nodes, the table's all-zero intervals
+// are not written.  128 threads: 256 or 512 do not shorten the chain (one
+// point: 14.6, 14.8, 15.4 us) and leave fewer points in flight (2048 points:
+// 47, 72, 117 us).  Prep and yf_kernel together, 2048 points at 64 lnM x 32 z
+// nodes: 126 -> 108 us; at 256 x 128: 239 -> 232; one point: 28.4 -> 24.
 // Shared memory: table block | the grid's lnM and z_t nodes, z_t weights,
 // Omega(z_t) and K_j(z_t) (staged with it) | per-k and per-q vectors |
 // FP32 delta_t.
@@ -213,8 +223,17 @@ prep_kernel(PrepArgs a)
     if (threadIdx.x == 0) set_err(a.status, kDevShape);  // no such grid
     return;
   }
-  const GridDev* __restrict__ Gp = a.grids + pt.grid;
-  const int n_m = Gp->n_m, n_z = Gp->n_z, n_m_pad = Gp->n_m_pad, tid = threadIdx.x;
+  // The grid's record in shared memory: each of its cache lines would
+  // otherwise cost a trip to L2 at its first use, one after another.
+  const int tid = threadIdx.x;
+  __shared__ GridDev grid;
+  static_assert(sizeof(GridDev) % 8 == 0);
+  for (int i = tid; i < (int)sizeof(GridDev) / 8; i += blockDim.x)
+    reinterpret_cast<uint64_t*>(&grid)[i] =
+      __ldg(reinterpret_cast<const unsigned long long*>(a.grids + pt.grid) + i);
+  __syncthreads();
+  const GridDev* Gp = &grid;
+  const int n_m = Gp->n_m, n_z = Gp->n_z, n_m_pad = Gp->n_m_pad;
   const TableLayout& L = a.lay;
   const int n_hm = L.n_hm, n_hz = L.n_hz;
   // The small tables (HMF axes, distances, Sigma_crit) are staged in shared
@@ -241,47 +260,45 @@ prep_kernel(PrepArgs a)
   __shared__ __align__(8) uint64_t bar;
   __shared__ int timed_out;
   int bad = 0;  // a non-finite table entry seen by this thread
-  __shared__ double red[6];
   __shared__ int swin[16];  // lam_t stage window per lnM tile (n_m <= 1024)
 
+  if (a.mixed)
+    for (int t = tid * 16; t < Gp->n_t; t += blockDim.x * 16)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(Gp->xl + t));
   const double* src = a.tables + (size_t)(a.slot ? a.slot[p] : p) * L.stride;
   const uint32_t bytes =
     (uint32_t)((head + tail + n_m2 + (size_t)(3 + nJ) * n_z) * sizeof(double));
-  if (tid == 0) {
-    timed_out = 0;
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid == 0) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&bar)),
-                 "r"(bytes)
-                 : "memory");
-    asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-        "r"(smem_addr(tab)),
-      "l"(src), "r"((uint32_t)(head * sizeof(double))), "r"(smem_addr(&bar))
-      : "memory");
-    if (tail)
-      asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
-        "[%3];" ::"r"(smem_addr(tab + head)),
-        "l"(src + L.off[3]), "r"((uint32_t)(tail * sizeof(double))), "r"(smem_addr(&bar))
-        : "memory");
-    bulk_copy_g2s(g_xm, Gp->xm, (uint32_t)(n_m2 * 8), &bar);
-    bulk_copy_g2s(g_xz, Gp->xz, (uint32_t)(n_z * 8), &bar);
-    bulk_copy_g2s(g_wz, Gp->wz, (uint32_t)(n_z * 8), &bar);
-    bulk_copy_g2s(g_omz, Gp->omz, (uint32_t)(n_z * 8), &bar);
-    bulk_copy_g2s(g_Kj, Gp->Kj, (uint32_t)((size_t)nJ * n_z * 8), &bar);
+  if (tid < 32) {  // warp 0: one copy per lane
+    if (tid == 0) {
+      timed_out = 0;
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar)) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&bar)),
+                   "r"(bytes)
+                   : "memory");
+    }
+    __syncwarp();
+    const void* from = src;
+    double* to = tab;
+    size_t len = head;
+    if (tid == 1) from = src + L.off[3], to = tab + head, len = tail;
+    if (tid == 2) from = Gp->xm, to = g_xm, len = n_m2;
+    if (tid == 3) from = Gp->xz, to = g_xz, len = n_z;
+    if (tid == 4) from = Gp->wz, to = g_wz, len = n_z;
+    if (tid == 5) from = Gp->omz, to = g_omz, len = n_z;
+    if (tid == 6) from = Gp->Kj, to = g_Kj, len = (size_t)nJ * n_z;
+    if (tid < 7 && len) bulk_copy_g2s(to, from, (uint32_t)(len * 8), &bar);
     // The mixed form's HMF grid is read next by yf_kernel (both of the
     // point's lnM tiles): start bringing it into L2 now.
-    if (a.mixed) {
+    if (tid == 7 && a.mixed) {
       const size_t n_dn = (size_t)n_hz * n_hm;
       const uint32_t hb = (uint32_t)(L.hmf_f32 ? ((n_dn + 1) / 2 + 1) / 2 * 16 : (n_dn * 8 + 15) & ~size_t(15));
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + L.off[2]), "r"(hb)
                    : "memory");
     }
   }
+  __syncthreads();
+  const double lnMpiv = log(pt.Mpiv);
   {
     long long t0 = clock64();
     uint32_t ok = 0;
@@ -333,23 +350,29 @@ prep_kernel(PrepArgs a)
   __syncthreads();
   double* s64 = a.s64 + (size_t)p * Gp->s64_stride;
   float* s32 = a.s32 + (size_t)p * Gp->s32_stride;
-  const double lnMpiv = log(pt.Mpiv);
   const double* xm = g_xm;
   const double* xz = g_xz;
-  for (int k = tid; k < n_m; k += blockDim.x) {
-    const double x = xm[k];
-    const double alpha = pt.B * (x - lnMpiv);
-    k_alpha[k] = alpha;
-    s64[Gp->o_alpha + k] = alpha;
-    const double xx = fmin(fmax(x, mh[0]), mh[n_hm - 1]);
-    const int xi = bsearch_cell(mh, n_hm, xx);
-    k_x[k] = xi;
-    k_t[k] = (xx - mh[xi]) / (mh[xi + 1] - mh[xi]);
-    k_f[k] = pt.hmf_s * (x * kLog10e - kHmfPivot) + pt.hmf_q;
-  }
+  // The lnM and z_t vectors in one pass, from a warp's edge on for the latter
+  // (at 64 lnM x 32 z nodes both fit one pass of the block).
   const size_t o_cz = Gp->o_cz, o_czs = Gp->o_czs, o_beta = Gp->o_beta;
   const double* Kj = g_Kj;
-  for (int q = tid; q < n_z; q += blockDim.x) {
+  const int n_m32 = (n_m + 31) & ~31;
+  for (int i = tid; i < n_m32 + n_z; i += blockDim.x) {
+    if (i < n_m32) {
+      const int k = i;
+      if (k >= n_m) continue;
+      const double x = xm[k];
+      const double alpha = pt.B * (x - lnMpiv);
+      k_alpha[k] = alpha;
+      s64[Gp->o_alpha + k] = alpha;
+      const double xx = fmin(fmax(x, mh[0]), mh[n_hm - 1]);
+      const int xi = bsearch_cell(mh, n_hm, xx);
+      k_x[k] = xi;
+      k_t[k] = (xx - mh[xi]) / (mh[xi + 1] - mh[xi]);
+      k_f[k] = pt.hmf_s * (x * kLog10e - kHmfPivot) + pt.hmf_q;
+      continue;
+    }
+    const int q = i - n_m32;
     const double z = xz[q];
     const double beta = pt.A + pt.C * log1p(z);
     q_beta[q] = beta;
@@ -375,50 +398,13 @@ prep_kernel(PrepArgs a)
     }
   }
   __syncthreads();
-  {  // centres of the alpha and beta ranges: block min/max
-    double amin = 1e300, amax = -1e300, bmin = 1e300, bmax = -1e300;
-    for (int k = tid; k < n_m; k += blockDim.x) {
-      amin = fmin(amin, k_alpha[k]);
-      amax = fmax(amax, k_alpha[k]);
-    }
-    for (int q = tid; q < n_z; q += blockDim.x) {
-      bmin = fmin(bmin, q_beta[q]);
-      bmax = fmax(bmax, q_beta[q]);
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-      amin = fmin(amin, __shfl_xor_sync(0xffffffffu, amin, off));
-      amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-      bmin = fmin(bmin, __shfl_xor_sync(0xffffffffu, bmin, off));
-      bmax = fmax(bmax, __shfl_xor_sync(0xffffffffu, bmax, off));
-    }
-    __shared__ double wred[4][32];
-    const int w = tid >> 5, nw = blockDim.x >> 5;
-    if ((tid & 31) == 0) {
-      wred[0][w] = amin;
-      wred[1][w] = amax;
-      wred[2][w] = bmin;
-      wred[3][w] = bmax;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      for (int i = 1; i < nw; ++i) {
-        amin = fmin(amin, wred[0][i]);
-        amax = fmax(amax, wred[1][i]);
-        bmin = fmin(bmin, wred[2][i]);
-        bmax = fmax(bmax, wred[3][i]);
-      }
-      red[0] = 0.5 * (amin + amax);
-      red[1] = 0.5 * (bmin + bmax);
-      red[2] = amin + bmin;  // range of mu = alpha_k + beta_q
-      red[3] = amax + bmax;
-      red[4] = bmin;
-      red[5] = bmax;
-      s64[Gp->o_scal] = red[0];
-      s64[Gp->o_scal + 1] = red[1];
-    }
-  }
-  __syncthreads();
-  const double A0 = red[0], B0 = red[1];
+  // Centres and ranges of alpha and beta: both are monotone in their nodes.
+  const double a_lo = fmin(1e300, fmin(k_alpha[0], k_alpha[n_m - 1]));
+  const double a_hi = fmax(-1e300, fmax(k_alpha[0], k_alpha[n_m - 1]));
+  const double b_lo = fmin(1e300, fmin(q_beta[0], q_beta[n_z - 1]));
+  const double b_hi = fmax(-1e300, fmax(q_beta[0], q_beta[n_z - 1]));
+  const double mu_lo = a_lo + b_lo, mu_hi = a_hi + b_hi;  // range of mu = alpha_k + beta_q
+  const double A0 = 0.5 * (a_lo + a_hi), B0 = 0.5 * (b_lo + b_hi);
   const double sig = pt.sigma, inv_s = 1.0 / sig;
   const double norm0 = 1.0 / (kSqrt2Pi * sig);
   const double ll_lo = Gp->ll_lo, ll_hi = Gp->ll_hi;
@@ -434,10 +420,10 @@ prep_kernel(PrepArgs a)
     // 4e-17 of its peak.
     constexpr double kSnap = 1048576.0, kWin64 = 8.7;
     const double a0 = rint(A0 * kSnap) / kSnap, b0 = rint(B0 * kSnap) / kSnap, l0 = a0 + b0;
-    const double am = 0.5 * ((red[3] - red[2]) - (red[5] - red[4])) + 1e-6;
-    const double bm = 0.5 * (red[5] - red[4]) + 1e-6;
+    const double am = 0.5 * ((mu_hi - mu_lo) - (b_hi - b_lo)) + 1e-6;
+    const double bm = 0.5 * (b_hi - b_lo) + 1e-6;
     const double dm = fmax(fabs(xl0 - l0), fabs(xl1 - l0));
-    const double vm = fmax(fmax(xl0 - red[2], red[3] - xl1), 0.0);
+    const double vm = fmax(fmax(xl0 - mu_lo, mu_hi - xl1), 0.0);
     const double ex = (bm * (dm + am + 0.5 * bm) + 0.5 * vm * vm) * inv_s * inv_s;
     const bool product = a.f64_rounds && ex <= kF64MaxExp;
     double* hdr = s64 + Gp->o_f64;
@@ -471,8 +457,8 @@ prep_kernel(PrepArgs a)
           hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
         }
         if (lane) continue;
-        lo += red[4];
-        hi += red[5];
+        lo += b_lo;
+        hi += b_hi;
         const double e_lo = fmin(fmax(lo, ll_lo), ll_hi) - lo, w2 = kWin64 * sig * kWin64 * sig;
         const double e_hi = fmin(fmax(hi, ll_lo), ll_hi) - hi;
         const double x_lo = lo - sqrt(e_lo * e_lo + w2), x_hi = hi + sqrt(e_hi * e_hi + w2);
@@ -512,11 +498,14 @@ prep_kernel(PrepArgs a)
   // per-tile row blocks, the z rows, the log2 D table and the windows.
   const double L0 = A0 + B0;
   const int n_t = Gp->n_t, n_t_pad = Gp->n_t_pad, n_mt = n_m_pad / kGemmRows;
-  for (int k = tid; k < n_m_pad; k += blockDim.x)
-    s32[Gp->f_a + k] = k < n_m ? (float)(k_alpha[k] - A0) : 0.f;
   for (int q = tid; q < n_z; q += blockDim.x) s32[Gp->f_b + q] = (float)(q_beta[q] - B0);
-  for (int t = tid; t < n_t_pad; t += blockDim.x)
-    s32[Gp->f_delta + t] = t < n_t ? (float)(Gp->xl[t] - L0) : 0.f;
+  float* dt_f = reinterpret_cast<float*>(
+    (reinterpret_cast<uintptr_t>(q_y + n_z) + 15) & ~uintptr_t(15));  // [n_t_pad]
+  for (int t = tid; t < n_t_pad; t += blockDim.x) {
+    const float d = t < n_t ? (float)(Gp->xl[t] - L0) : 0.f;
+    dt_f[t] = d;
+    s32[Gp->f_delta + t] = d;
+  }
   constexpr double kLog2e = 1.4426950408889634;
   const double c1d = kLog2e * 0.5 / (sig * sig), c2d = kLog2e / (sig * sig);
   const float sc1 = sqrtf((float)c1d);
@@ -532,10 +521,10 @@ prep_kernel(PrepArgs a)
   // far mu lies outside the domain) and dlnD/dmu = (phi(a) - phi(b)) / (s D),
   // taken in logs.  Only nodes next to a mu that fails the FP32 saturation
   // test are read (the test's margin is 1e-3 plus FP32 rounding, and the
-  // nodes used lie within hmu of mu): the interior nodes hold 0 without an
-  // erfc.
-  const double mu0 = red[2];
-  const double hmu = red[3] > red[2] ? (red[3] - red[2]) / (kDTab - 1) : 1.0;
+  // nodes used lie within hmu of mu): the interior nodes are 0 without an
+  // erfc, and intervals between two of them are not written.
+  const double mu0 = mu_lo;
+  const double hmu = mu_hi > mu_lo ? (mu_hi - mu_lo) / (kDTab - 1) : 1.0;
   const double inv_hmu = 1.0 / hmu;
   {
     float* dt32 = s32 + Gp->f_dt32;
@@ -545,10 +534,6 @@ prep_kernel(PrepArgs a)
     const int j_sat1 =
       (int)fmin(fmax(floor((ll_hi - 5.6 * sig - 0.01 - mu0) * inv_hmu) - 2.0, 0.0), (double)kDTab);
     const int n_lo = min(j_sat0 + 1, kDTab), n_hi = kDTab - max(j_sat1, n_lo);
-    for (int j = n_lo + tid; j < kDTab - n_hi; j += blockDim.x) {
-      dtS[j] = 0.0;
-      dtS[kDTab + j] = 0.0;
-    }
     // Nodes evaluated in FP32 (transcendentals an order of magnitude faster
     // than FP64 here); where log2 D < -12 (the FP32 value's absolute error
     // would pass 1e-6) the node is evaluated again in FP64 for both tables.
@@ -579,9 +564,12 @@ prep_kernel(PrepArgs a)
     // cubic Hermite in t = (mu - mu_j) / h as coefficients
     // c0 + c1 t + c2 t^2 + c3 t^3 (one 16-byte load and three FMAs per
     // cell), formed in FP64.
-    for (int j = tid; j < kDTab; j += blockDim.x) {
-      const int j1 = min(j + 1, kDTab - 1);
-      const double T0 = dtS[j], T1 = dtS[j1], D0 = dtS[kDTab + j], D1 = dtS[kDTab + j1];
+    const int j_hi = kDTab - n_hi, skip = max(j_hi - 1 - n_lo, 0);  // intervals left out
+    for (int r = tid; r < kDTab - skip; r += blockDim.x) {
+      const int j = r < n_lo ? r : r + skip, j1 = min(j + 1, kDTab - 1);
+      const bool in0 = j >= n_lo && j < j_hi, in1 = j1 >= n_lo && j1 < j_hi;
+      const double T0 = in0 ? 0.0 : dtS[j], T1 = in1 ? 0.0 : dtS[j1];
+      const double D0 = in0 ? 0.0 : dtS[kDTab + j], D1 = in1 ? 0.0 : dtS[kDTab + j1];
       dt64[j] = T0;
       dt64[kDTab + j] = D0;
       *reinterpret_cast<float4*>(dt32 + 4 * j) =
@@ -622,9 +610,6 @@ prep_kernel(PrepArgs a)
       qb[q] = q < n_z ? (float)(q_beta[q] - B0) : 0.f;
     }
   }
-  float* dt_f = reinterpret_cast<float*>(
-    (reinterpret_cast<uintptr_t>(q_y + n_z) + 15) & ~uintptr_t(15));  // [n_t_pad]
-  for (int t = tid; t < n_t_pad; t += blockDim.x) dt_f[t] = t < n_t ? (float)(Gp->xl[t] - L0) : 0.f;
   __shared__ float tile_af[16];  // per lnM tile: min and max of its rows' FP32 a_k
   __shared__ int tile_sc[8];     // per lnM tile: some row carries a scale
   for (int mt = tid; mt < 8; mt += blockDim.x) tile_sc[mt] = 0;
@@ -646,51 +631,37 @@ prep_kernel(PrepArgs a)
     constexpr double kWin = 5.0;
     const int nk = n_t_pad / 16;
     for (int mt = warp; mt < n_mt; mt += nw) {
-      double amn = 1e300, amx = -1e300;
-      for (int k = mt * kGemmRows + lane; k < min(n_m, (mt + 1) * kGemmRows); k += 32) {
-        amn = fmin(amn, k_alpha[k]);
-        amx = fmax(amx, k_alpha[k]);
-      }
-      for (int off = 16; off > 0; off >>= 1) {
-        amn = fmin(amn, __shfl_xor_sync(0xffffffffu, amn, off));
-        amx = fmax(amx, __shfl_xor_sync(0xffffffffu, amx, off));
-      }
-      if (lane == 0) {
-        int lo = 0, hi = nk;
-        if (amx >= amn) {
-          const double mu_lo = amn + red[4], mu_hi = amx + red[5];
-          const double e_lo = fmin(fmax(mu_lo, ll_lo), ll_hi) - mu_lo;
-          const double e_hi = fmin(fmax(mu_hi, ll_lo), ll_hi) - mu_hi;
-          const double w2 = (kWin * sig) * (kWin * sig);
-          const float dlo = (float)(mu_lo - sqrt(e_lo * e_lo + w2) - L0);
-          const float dhi = (float)(mu_hi + sqrt(e_hi * e_hi + w2) - L0);
-          int a = 0, b = n_t;  // first t with delta_t >= dlo (nodes ascend)
-          while (a < b) {
-            const int m = (a + b) >> 1;
-            if (dt_f[m] < dlo) a = m + 1; else b = m;
-          }
-          const int t_lo = a;
-          a = t_lo;
-          b = n_t;  // first t with delta_t > dhi
-          while (a < b) {
-            const int m = (a + b) >> 1;
-            if (dt_f[m] <= dhi) a = m + 1; else b = m;
-          }
-          const int t_hi = a;
-          // Stages [t_lo / 16, ceil(t_hi / 16)), the count rounded up to
-          // pairs (at least one pair; nk is even) and kept inside [0, nk).
-          const int s_lo = t_lo / 16, s_hi = (t_hi + 15) / 16;
-          const int cnt = max(2, (s_hi - s_lo + 1) & ~1);
-          lo = min(s_lo, nk - cnt);
-          hi = lo + cnt;
+      const double ka = k_alpha[mt * kGemmRows], kb = k_alpha[min(n_m, (mt + 1) * kGemmRows) - 1];
+      const double amn = fmin(1e300, fmin(ka, kb)), amx = fmax(-1e300, fmax(ka, kb));
+      int lo = 0, hi = nk;
+      if (amx >= amn) {
+        const double m_lo = amn + b_lo, m_hi = amx + b_hi;
+        const double e_lo = fmin(fmax(m_lo, ll_lo), ll_hi) - m_lo;
+        const double e_hi = fmin(fmax(m_hi, ll_lo), ll_hi) - m_hi;
+        const double w2 = (kWin * sig) * (kWin * sig);
+        const float dlo = (float)(m_lo - sqrt(e_lo * e_lo + w2) - L0);
+        const float dhi = (float)(m_hi + sqrt(e_hi * e_hi + w2) - L0);
+        int t_lo = 0, t_hi = 0;  // nodes below dlo, nodes up to dhi (they ascend)
+        for (int t0 = 0; t0 < n_t; t0 += 32) {
+          const bool in = t0 + lane < n_t;
+          const float d = dt_f[in ? t0 + lane : 0];
+          t_lo += __popc(__ballot_sync(0xffffffffu, in && d < dlo));
+          t_hi += __popc(__ballot_sync(0xffffffffu, in && d <= dhi));
         }
-        swin[2 * mt] = lo;
-        swin[2 * mt + 1] = hi;
-        // The tile's range of a_k = alpha_k - A0 as FP32: rounding is
-        // monotone, so these are the min and max of its rows' FP32 a_k.
-        tile_af[2 * mt] = (float)(amn - A0);
-        tile_af[2 * mt + 1] = (float)(amx - A0);
+        // Stages [t_lo / 16, ceil(t_hi / 16)), the count rounded up to
+        // pairs (at least one pair; nk is even) and kept inside [0, nk).
+        const int s_lo = t_lo / 16, s_hi = (t_hi + 15) / 16;
+        const int cnt = max(2, (s_hi - s_lo + 1) & ~1);
+        lo = min(s_lo, nk - cnt);
+        hi = lo + cnt;
       }
+      if (lane) continue;
+      swin[2 * mt] = lo;
+      swin[2 * mt + 1] = hi;
+      // The tile's range of a_k = alpha_k - A0 as FP32: rounding is
+      // monotone, so these are the min and max of its rows' FP32 a_k.
+      tile_af[2 * mt] = (float)(amn - A0);
+      tile_af[2 * mt + 1] = (float)(amx - A0);
     }
   }
   __syncthreads();
@@ -782,8 +753,8 @@ prep_kernel(PrepArgs a)
     double dmax = 0.0;
     const int t0 = h_lo * 16, t1 = min(h_hi * 16, n_t) - 1;
     if (t1 >= t0) dmax = fmax(fabs((double)dt_f[t0]), fabs((double)dt_f[t1]));
-    const double bmax = 0.5 * (red[5] - red[4]);
-    const double amax = 0.5 * ((red[3] - red[2]) - (red[5] - red[4]));
+    const double bmax = 0.5 * (b_hi - b_lo);
+    const double amax = 0.5 * ((mu_hi - mu_lo) - (b_hi - b_lo));
     const double e = c2d * bmax * fmax(dmax, amax + 0.5 * bmax);
     if (!(e <= kMaxExp2)) set_err(a.status, kDevRange);
   }
@@ -1861,8 +1832,6 @@ build_grid(y3b_engine* e, int gi)
   g.omz = b->omz.get();
   // Scratch layouts.
   size_t o = 0;
-  g.o_scal = o;
-  o += 4;
   g.o_kx = o;
   o += pad2(g.n_m);
   g.o_kt = o;
@@ -1898,8 +1867,6 @@ build_grid(y3b_engine* e, int gi)
   // the bulk copies of yf_kernel and the contraction start aligned.
   g.nzp = (g.n_z + 3) & ~3;
   size_t f = 0;
-  g.f_a = f;
-  f += g.n_m_pad;
   g.f_b = f;
   f += g.nzp;
   g.f_delta = f;
