@@ -150,3 +150,24 @@ def test_mixed_row_groups(gpu, n_m, n_z, n_t, hmf_fp32):
     _compare(dict(kind="engine", api="device", precision="mixed", n=3, radii=0, hmf_fp32=hmf_fp32,
                   loglike=False, mixed_density=False, n_m=n_m, n_z=n_z, n_t=n_t, n_o=32, n_zo=9),
              1e-4)
+
+
+# The miscentred profile at 24 Chebyshev nodes in lnM (grids above 32 masses on
+# at most nine e-folds) and at every mass on the rule's other side, against the
+# closed-form profile's quadrature at every mass, which cancels to about 1e-12
+# of itself near r_s: 1e-10.
+@pytest.mark.parametrize("n_lnm,lo,hi", [(33, 29.9336, 36.73), (96, 27.9, 36.9), (200, 31.0, 31.5),
+                                         (96, 27.8, 36.9), (32, 29.9336, 36.73)])
+def test_miscentred_profile_nodes(gpu, n_lnm, lo, hi):
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+
+    s = cases._module_inputs(dict(mor="lognormal", tab_m=40, tab_z=24, n_q=17, radii=4), 3)
+    sel = E.sel_function(s["cfg"], s["kind"], s["mor"], *s["plob"])
+    h = E.SelGL(n_lnm=n_lnm, n_z=19, lnm_low=lo, lnm_high=hi).build(s["cz"], s["tab"], sel)
+    w = h.weights()
+    got = h.shear(s["bins"], s["r"], s["halo"], f_mis=1.0)
+    rmis = 0.17 * (np.array((25.0, 37.5, 52.5, 130.0))[s["bins"] % 4] / 100.0) ** 0.2
+    prof = E.nfw_mis("dsigma", s["r"][:, None], rmis[:, None], w["lnm_x"], 4.0, cases.RHO_CRIT)
+    want = s["om"] * np.sum(w["lnm_w"] * w["W"][s["bins"]] * prof, axis=1)
+    np.testing.assert_allclose(got, want, rtol=1e-10, atol=1e-10 * np.max(np.abs(want)))
