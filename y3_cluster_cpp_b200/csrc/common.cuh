@@ -59,15 +59,21 @@ bsearch_cell(const T* xs, int n, T x)
   return ilo;
 }
 
+// Linear interpolation in cell i.
+__device__ __forceinline__ double
+interp1d_cell(const double* xs, const double* ys, int i, double x)
+{
+  const double dx = xs[i + 1] - xs[i];
+  return dx > 0.0 ? ys[i] + (x - xs[i]) / dx * (ys[i + 1] - ys[i]) : 0.0;
+}
+
 // Unclamped linear interpolation; returns false outside [xs[0], xs[n-1]]
 // (the reference throws std::domain_error there, interp_1d.cc:76-77).
 __device__ __forceinline__ bool
 interp1d(const double* xs, const double* ys, int n, double x, double* out)
 {
   if (!(x >= xs[0] && x <= xs[n - 1])) return false;
-  int i = bsearch_cell(xs, n, x);
-  double dx = xs[i + 1] - xs[i];
-  *out = (dx > 0.0) ? ys[i] + (x - xs[i]) / dx * (ys[i + 1] - ys[i]) : 0.0;
+  *out = interp1d_cell(xs, ys, bsearch_cell(xs, n, x), x);
   return true;
 }
 
@@ -80,21 +86,34 @@ interp1d_clamp(const double* xs, const double* ys, int n, double x)
   return out;
 }
 
-// Clamped bilinear interpolation; zs[j * nx + i] (y slow).
-__device__ __forceinline__ double
-interp2d_clamp(const double* xs, int nx, const double* ys, int ny,
-               const double* zs, double x, double y)
+// Cell of x clamped to the axis, and the position inside it.
+__device__ __forceinline__ int
+clamp_cell(const double* xs, int n, double x, double* t)
 {
-  double xx = fmin(fmax(x, xs[0]), xs[nx - 1]);
-  double yy = fmin(fmax(y, ys[0]), ys[ny - 1]);
-  int xi = bsearch_cell(xs, nx, xx);
-  int yi = bsearch_cell(ys, ny, yy);
-  double t = (xx - xs[xi]) / (xs[xi + 1] - xs[xi]);
-  double u = (yy - ys[yi]) / (ys[yi + 1] - ys[yi]);
+  const double xx = fmin(fmax(x, xs[0]), xs[n - 1]);
+  const int i = bsearch_cell(xs, n, xx);
+  *t = (xx - xs[i]) / (xs[i + 1] - xs[i]);
+  return i;
+}
+
+// Bilinear interpolation in cell (xi, yi); zs[j * nx + i] (y slow).
+__device__ __forceinline__ double
+bilinear_at(const double* zs, int nx, int xi, int yi, double t, double u)
+{
   const double* r0 = zs + (size_t)yi * nx + xi;
   const double* r1 = r0 + nx;
   return (1.0 - t) * (1.0 - u) * r0[0] + t * (1.0 - u) * r0[1] +
          (1.0 - t) * u * r1[0] + t * u * r1[1];
+}
+
+// Clamped bilinear interpolation.
+__device__ __forceinline__ double
+interp2d_clamp(const double* xs, int nx, const double* ys, int ny,
+               const double* zs, double x, double y)
+{
+  double t, u;
+  const int xi = clamp_cell(xs, nx, x, &t), yi = clamp_cell(ys, ny, y, &u);
+  return bilinear_at(zs, nx, xi, yi, t, u);
 }
 
 // 2^x on the MUFU unit (PTX ex2.approx.ftz.f32; ~2 ulp, subnormals flush

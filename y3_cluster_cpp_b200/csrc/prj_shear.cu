@@ -114,7 +114,10 @@ dsigma_single_table(const PrjTable& T, double R, double Rmis, double lnM)
 // Per slice: the theta and z grids and the sums over the line of sight.
 // One block; the node counts are a few dozen to a few hundred, so the block
 // is bound by the latency of its phases (interpolations, the 40-step chi(z)
-// bisections), which run one node a thread.
+// bisections), which run one node a thread.  24 masses, 60 z nodes, 12 slices:
+// 64 -> 41 us with bisections that narrow their table search with the interval,
+// the table cells of a mass and of a z node found once, and the scalar set-up on
+// three warps.
 constexpr int kSliceThreads = 512;
 
 __global__ void __launch_bounds__(kSliceThreads)
@@ -147,8 +150,10 @@ prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ s
     for (int i = tid; i < D.n_xr; i += nt_thr) S[D.s_xi + i] = (1.0 - u) * r0[i] + u * r1[i];
   }
   __syncthreads();
+  // Three chains of scalar work, a warp's first thread each.
+  const double D_A = chis[0] / (1.0 + zob);
   if (tid == 0) {
-    const double chi_o = chis[0], D_A = chi_o / (1.0 + zob);
+    const double chi_o = chis[0];
     const double Rl = pow(D.sl_lob[sl] / 100.0, 0.2), R_excl = Rl * (1.0 + zob);
     // theta breakpoints (sp_detail::build_theta_grid, sigma_prj_t.hh:95-180):
     // the radii ascend, so the sorted list is a merge of theta_R with the
@@ -195,6 +200,8 @@ prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ s
     if (n == 0) put(lower);
     if (last < th_max) put(th_max);
     n_bd_s = n;
+  } else if (tid == 32) {
+    const double Rl = pow(D.sl_lob[sl] / 100.0, 0.2), th_lam = Rl * (1.0 + zob) / chis[0];
     // b_sel asymptotes linear in z_obs (sigma_prj_frozen_t.hh:200-217)
     const double* bz = B + D.o_bzob;
     const int nzb = D.n_bzob, nlb = D.n_blob, lb = D.sl_lb[sl];
@@ -209,6 +216,9 @@ prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ s
     sc[1] = (1.0 - f) * bl[j0 * nlb + lb] + f * bl[j1 * nlb + lb];
     sc[2] = 2.5 / th_lam;
     sc[3] = 0.5 * th_lam;
+  } else if (tid == 64) {
+    const double chi_o = chis[0];
+    const double R_excl = pow(D.sl_lob[sl] / 100.0, 0.2) * (1.0 + zob);
     // line-of-sight ranges (sigma_prj_frozen_t.hh:380-455)
     const double dchi_dz = (chis[3] - chis[4]) / (2.0 * dz1);
     const double dz_ex = R_excl / dchi_dz;
@@ -254,13 +264,27 @@ prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ s
       const double a = log(R_excl), b = log(fg ? sc[7] : sc[8]), hl = 0.5 * (b - a);
       const double dis = exp(0.5 * (a + b) + hl * D.gl_out[q]);
       const double target = fg ? chi_o - dis : chi_o + dis;
-      double lo = 0.001, hi = 2.0;  // sigma_prj_frozen_t.hh:458-468
+      // sigma_prj_frozen_t.hh:458-468; the cells of the two ends bracket the
+      // one of the midpoint, so its search shrinks with the interval.
+      double lo = 0.001, hi = 2.0;
+      int c_lo = 0, c_hi = D.nd - 1;
       for (int it = 0; it < 40; ++it) {
-        const double mid = 0.5 * (lo + hi);
-        if (chi(mid) < target)
+        const double mid = 0.5 * (lo + hi), x = fmin(fmax(mid, dz[0]), dz[D.nd - 1]);
+        int a = c_lo, b = c_hi;
+        while (b > a + 1) {
+          const int m = (a + b) >> 1;
+          if (dz[m] > x)
+            b = m;
+          else
+            a = m;
+        }
+        if (interp1d_cell(dz, B + D.o_dc, a, x) * h0 < target) {
           lo = mid;
-        else
+          c_lo = a;
+        } else {
           hi = mid;
+          c_hi = a + 1;
+        }
       }
       z = 0.5 * (lo + hi);
       wz = hl * D.gl_out[D.n_zouter + q] * dis / ((chi(z + dz1) - chi(z - dz1)) / (2.0 * dz1));
@@ -284,34 +308,53 @@ prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ s
   if (tid == 0) nt_out[sl] = n_th;
   __syncthreads();
   // n and b at every z node of non-zero weight and, in the last item, at
-  // z_obs: one warp a node, lanes over the masses.
-  for (int i = warp; i <= D.nz; i += nw) {
-    const bool anchor = i == D.nz;
-    const double c = anchor ? 1.0 : S[D.s_zc + i], z = anchor ? zob : (c != 0.0 ? S[D.s_z + i] : 0.0);
-    double num = 0.0;
-    for (int k = lane; k < D.n_lnm; k += 32) {
-      if (c == 0.0) {  // the reference skips these nodes entirely
-        S[D.s_wz + (size_t)i * D.n_lnm + k] = 0.0;
-        continue;
+  // z_obs: one warp a node, lanes over the masses.  A lane keeps the mass
+  // cells of both tables over its warp's nodes, whose z cells the lanes find
+  // side by side, one node each.
+  const double *hz = B + D.o_hz, *bl = B + D.o_bl, *bz = B + D.o_bz;
+  for (int i0 = warp; i0 <= D.nz; i0 += 32 * nw) {
+    const int il = i0 + nw * lane;  // this lane's node
+    double c_l = 0.0, z_l = zob, uh_l, ub_l;
+    if (il == D.nz) {
+      c_l = 1.0;
+    } else if (il < D.nz) {
+      c_l = S[D.s_zc + il];
+      if (c_l != 0.0) z_l = S[D.s_z + il];
+    }
+    const int jh_l = clamp_cell(hz, D.n_hz, z_l, &uh_l), jb_l = clamp_cell(bz, D.n_bz, z_l, &ub_l);
+    for (int k0 = 0; k0 < D.n_lnm; k0 += 32) {
+      const int k = k0 + lane;
+      const bool in = k < D.n_lnm;
+      const double x = D.lnm_x[in ? k : 0], w = D.lnm_w[in ? k : 0];
+      const double an = in ? D.anchor[k] : 0.0, f = B[5] * (x * kLog10e - kHmfPivot) + B[6];
+      double th, tb;
+      const int xh = clamp_cell(S + D.s_mh, D.n_hm, x, &th), xb = clamp_cell(bl, D.n_bl, x, &tb);
+      for (int m = 0; m < 32 && i0 + nw * m <= D.nz; ++m) {
+        const int i = i0 + nw * m, jh = __shfl_sync(0xffffffffu, jh_l, m);
+        const int jb = __shfl_sync(0xffffffffu, jb_l, m);
+        const double c = __shfl_sync(0xffffffffu, c_l, m), uh = __shfl_sync(0xffffffffu, uh_l, m);
+        const double ub = __shfl_sync(0xffffffffu, ub_l, m);
+        const bool anchor = i == D.nz;
+        double num = 0.0;
+        if (c == 0.0) {  // the reference skips these nodes entirely
+          if (in) S[D.s_wz + (size_t)i * D.n_lnm + k] = 0.0;
+        } else {
+          const double n = bilinear_at(B + D.o_dn, D.n_hm, xh, jh, th, uh) * f;
+          const double b = bilinear_at(B + D.o_bi, D.n_bl, xb, jb, tb, ub);
+          num = an * n * b;
+          if (in && anchor)
+            S[D.s_wcl + k] = w * n * b;
+          else if (in)
+            S[D.s_wz + (size_t)i * D.n_lnm + k] = c * n * w;
+        }
+        for (int off = 16; off > 0; off >>= 1) num += __shfl_xor_sync(0xffffffffu, num, off);
+        if (lane == 0) {  // the mass chunks in order
+          double* to = anchor ? &sc[9] : &S[D.s_ab + i];
+          *to = (k0 ? *to : 0.0) + num;
+        }
       }
-      const double x = D.lnm_x[k];
-      const double n = interp2d_clamp(S + D.s_mh, D.n_hm, B + D.o_hz, D.n_hz, B + D.o_dn, x, z) *
-                       (B[5] * (x * kLog10e - kHmfPivot) + B[6]);
-      const double b =
-        interp2d_clamp(B + D.o_bl, D.n_bl, B + D.o_bz, D.n_bz, B + D.o_bi, x, z);
-      num += D.anchor[k] * n * b;
-      if (anchor)
-        S[D.s_wcl + k] = D.lnm_w[k] * n * b;
-      else
-        S[D.s_wz + (size_t)i * D.n_lnm + k] = c * n * D.lnm_w[k];
     }
-    for (int off = 16; off > 0; off >>= 1) num += __shfl_xor_sync(0xffffffffu, num, off);
-    if (lane == 0) {
-      if (anchor)
-        sc[9] = num + 1.0e-300;
-      else
-        S[D.s_ab + i] = num;
-    }
+    if (lane == 0 && i0 <= D.nz && (D.nz - i0) % nw == 0 && (D.nz - i0) / nw < 32) sc[9] += 1.0e-300;
   }
   __syncthreads();
   for (int i = tid; i < D.nz; i += nt_thr) {
