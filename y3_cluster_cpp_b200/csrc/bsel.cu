@@ -629,9 +629,8 @@ struct y3b_bsel {
   std::vector<double> lnm_x, lnm_w, lt_x, lt_w, rl, zr;  // lt_x, lt_w, rl: [4][n_lt]
   int n_sm = 1;
   int max_samples = 64;
-  y3b::DevBuf<double> d_const, d_blocks, d_mom, d_grids, d_part, d_out;
+  y3b::DevBuf<double> d_const, d_blocks, d_work, d_out;
   y3b::DevBuf<int> d_int;  // grid-point bins
-  y3b::DevBuf<unsigned> d_need;  // bits of the reference z nodes read
   double* h_stage = nullptr;  // pinned: sample blocks
   size_t h_stage_cap = 0;
   double* h_out = nullptr;  // pinned: results
@@ -939,11 +938,16 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
     h->h_out_cap = outn;
   }
   Y3B_TRY(h->d_blocks.alloc(stage));
-  Y3B_TRY(h->d_mom.alloc((size_t)chunk * D.mom));
-  Y3B_TRY(h->d_grids.alloc((size_t)chunk * ngp * D.grid));
-  Y3B_TRY(h->d_part.alloc(2 * (size_t)chunk * ngp * c.n_theta));
+  // One work block: theta sums | grids | moments | bits of the reference z
+  // nodes read.
+  const size_t n_part = 2 * (size_t)chunk * ngp * c.n_theta;
+  const size_t n_grids = (size_t)chunk * ngp * D.grid, n_mom = (size_t)chunk * D.mom;
   const size_t needs = (size_t)chunk * 4 * D.need_words;
-  Y3B_TRY(h->d_need.alloc(needs));
+  Y3B_TRY(h->d_work.alloc(n_part + n_grids + n_mom + (needs + 1) / 2));
+  double* const w_part = h->d_work.get();
+  double* const w_grids = w_part + n_part;
+  double* const w_mom = w_grids + n_grids;
+  unsigned* const w_need = reinterpret_cast<unsigned*>(w_mom + n_mom);
   Y3B_TRY(h->d_out.alloc(outn));
   cudaStream_t st = h->stream;
   h->last_kernel_ms = 0.0;
@@ -952,7 +956,7 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
     const int pieces = std::max(1, std::min(kPieces, n_chunk / kPieceSamples));
     // The previous chunk's copies out of the staging buffers are done.
     Y3B_CUDA(cudaStreamSynchronize(st));
-    Y3B_CUDA(cudaMemsetAsync(h->d_need.get(), 0, needs * sizeof(unsigned), st));
+    Y3B_CUDA(cudaMemsetAsync(w_need, 0, needs * sizeof(unsigned), st));
     for (int pc = 0; pc < pieces; ++pc) {
       const int ka = (int)((long)n_chunk * pc / pieces);
       const int nk = (int)((long)n_chunk * (pc + 1) / pieces) - ka;
@@ -979,10 +983,10 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
         std::memcpy(b + D.o_xi, s.xi_nl, sizeof(double) * D.n_xr * D.n_xz);
       }
       double* blocks = h->d_blocks.get() + (size_t)ka * D.blk;
-      double* grids = h->d_grids.get() + (size_t)ka * ngp * D.grid;
-      double* mom = h->d_mom.get() + (size_t)ka * D.mom;
-      unsigned* need = h->d_need.get() + (size_t)ka * 4 * D.need_words;
-      double2* part = reinterpret_cast<double2*>(h->d_part.get()) + (size_t)ka * ngp * c.n_theta;
+      double* grids = w_grids + (size_t)ka * ngp * D.grid;
+      double* mom = w_mom + (size_t)ka * D.mom;
+      unsigned* need = w_need + (size_t)ka * 4 * D.need_words;
+      double2* part = reinterpret_cast<double2*>(w_part) + (size_t)ka * ngp * c.n_theta;
       double* o = h->d_out.get() + (size_t)ka * ngp * 3;
       Y3B_CUDA(cudaMemcpyAsync(blocks, h->h_stage + (size_t)ka * D.blk,
                                sizeof(double) * nk * D.blk, cudaMemcpyHostToDevice, st));
