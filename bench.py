@@ -463,7 +463,7 @@ def module_latency(n_calls=40):
 
 def prj_latency(n_calls=30):
     """Per-sample latency of the frozen-physics projection shear
-    (y3b_prj_eval: host grids, table upload, device sums, 12 slices x 10
+    (y3b_prj_eval: table upload, device grids and sums, 12 slices x 10
     radii, default options, direct single-kernel quadrature), next to the
     reference's published 82 ms per sample."""
     import numpy as np
@@ -653,9 +653,9 @@ def serving_run(a, rank, dev):
             "fp64_per_request": {"throughput": fp64_tp, "unit": UNIT,
                                  **serve.percentiles_ms(np.asarray(lat64)),
                                  "capacity": fp64_capacity,
-                                 "form": "FP64 direct nested GL (one exp per lnM, z_t, lam_t "
-                                         "node, no factorisation), one engine call per "
-                                         "request, host tables"},
+                                 "form": "FP64 form (factorised lam_t sum on the FP64 tensor "
+                                         "cores), one engine call per request, host "
+                                         "tables"},
             "saturated": {"outstanding_requests": outstanding, "throughput": sat_tp,
                           "unit": UNIT, **serve.percentiles_ms(sat["latency_s"]),
                           "launches": sat_launches,
@@ -902,7 +902,7 @@ def run_ours(a):
                        "parallelism": f"walker-sharded x{world}"},
             "max_rel_err_vs_fp64": max_rel,
             "plain_fp64": {"value": plain_fp64, "unit": UNIT,
-                           "mode": "FP64 direct quadrature, one point per call"},
+                           "mode": "FP64 form, one point per call"},
             "fp64_batched": {"value": fp64_batched, "unit": UNIT},
             "speedup_vs_plain_fp64": value / world / plain_fp64,
             "roofline": {"bound": "tensor", "achieved": achieved_tf, "peak": peak_tf,

@@ -271,8 +271,8 @@ void y3b_prj_destroy(y3b_prj* h);
 /* Module options (p_operator_t.hh:95-110): node counts (defaults n_lt 60,
  * n_zring 20, n_zouter 30, n_lnm 24, n_theta 10, n_zt_ref 80), the reference
  * z grid [zt_ref_low, zt_ref_high] (0.05, 0.90) and the mass range (required).
- * max_samples bounds one device batch (the MOR table takes
- * 4 n_zt_ref n_lnm n_lt doubles per sample); eval splits larger calls. */
+ * max_samples bounds one device batch (the mass moments take
+ * 32 n_zt_ref n_lt doubles per sample); eval splits larger calls. */
 typedef struct {
   int n_lt, n_zring, n_zouter, n_lnm, n_theta, n_zt_ref;
   double zt_ref_low, zt_ref_high, lnm_low, lnm_high;
@@ -307,8 +307,9 @@ int y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out);
  * Host buffers; FP64 throughout.  Y3B_ERR_DOMAIN if the reference z grid
  * leaves distances/z (the reference's Interp1D throws there). */
 int y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* samples, double* out);
-/* Device time of the last y3b_bsel_eval's kernels (CUDA events around each
- * chunk's two kernels, summed; the copies and host packing excluded). */
+/* Device time of the last y3b_bsel_eval's kernels (CUDA events around the
+ * kernels of each piece of a batch, summed; the copies and host packing
+ * excluded). */
 int y3b_bsel_kernel_ms(const y3b_bsel* h, double* ms);
 void y3b_bsel_destroy(y3b_bsel* h);
 

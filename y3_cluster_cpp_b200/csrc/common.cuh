@@ -331,56 +331,6 @@ struct NfwUnit<double> {
   }
 };
 
-template <>
-struct NfwUnit<float> {
-  // FP32 variant: same branches; the series near x = 1 is truncated at the
-  // terms that matter in single precision (|w| < 0.05, 8 terms).
-  static __device__ __forceinline__ float g(float x)
-  {
-    float w = 1.0f - x * x;
-    if (fabsf(w) < 0.05f) {
-      float s = 1.0f / 15.0f;
-#pragma unroll
-      for (int n = 6; n >= 0; --n) s = 1.0f / (2 * n + 1) + w * s;
-      return s;
-    }
-    if (x < 1.0f) {
-      float y = sqrtf(w);
-      return atanhf(y) / y;
-    }
-    float y = sqrtf(-w);
-    return atanf(y) / y;
-  }
-  static __device__ __forceinline__ float sigma(float x)
-  {
-    float w = 1.0f - x * x;
-    if (fabsf(w) < 0.05f) {
-      float s = 1.0f / 17.0f;
-#pragma unroll
-      for (int n = 6; n >= 0; --n) s = 1.0f / (2 * n + 3) + w * s;
-      return s;
-    }
-    return (g(x) - 1.0f) / w;
-  }
-  static __device__ __forceinline__ float sigma_bar(float x)
-  {
-    if (x < 0.5f) {
-      float y = sqrtf(1.0f - x * x);
-      float x2 = x * x;
-      return (2.0f / y) * (logf(2.0f / x) / (1.0f + y) +
-                           log1pf(-x2 / (2.0f * (1.0f + y))) / x2);
-    }
-    return 2.0f * (g(x) + logf(0.5f * x)) / (x * x);
-  }
-  static __device__ __forceinline__ float dsigma(float x)
-  {
-    const float w = 1.0f - x * x;
-    if (x < 0.5f || fabsf(w) < 0.05f) return sigma_bar(x) - sigma(x);
-    const float gx = g(x);
-    return 2.0f * (gx + logf(0.5f * x)) / (x * x) - (gx - 1.0f) / w;
-  }
-};
-
 // Single-offset miscentred DeltaSigma (the "single" kernel of
 // NFW_DSIGMA_MIS, nfw_dsigma_mis.hh:53-55) in units of 2 r_s delta_c rho:
 // the mean tangential shear on the circle of radius x around the offset

@@ -11,7 +11,9 @@
 //
 // Two precisions share the per-point prep (FP64 tables, z factors, MOR
 // normalisation D_kq by an erf difference):
-//   * FP64 "plain" form: one exp per (k, q, t) in FP64 (direct_main_kernel).
+//   * FP64 form: the lambda_t sum as a matrix product on the FP64 tensor
+//     cores (fp64_form.cu); points whose factors leave its range take one
+//     exp per (k, q, t) (direct_main_kernel).
 //   * mixed form: the lambda_t sum as a split-BF16 tcgen05 GEMM
 //     (mixed_gemm.cu) with FP32 integrands and FP64 final sums.
 // Reductions are fixed-order trees; reruns are bit-identical.
@@ -1119,7 +1121,7 @@ yf_kernel(PrepArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// FP64 plain form, for the points that the matrix product (fp64_form.cu) does
+// The FP64 form's direct sum, for the points that the matrix product (fp64_form.cu) does
 // not admit, listed by the prep kernel.  CTA = (listed point, z node q) in
 // turn; thread k sums over lam_t with one FP64 exp per node:
 // V_i(q, k) = P0_kq sum_t u_t K_i(t, q) exp(-(l_t - mu)^2/2s^2) (with the edge
