@@ -171,3 +171,10 @@ def test_miscentred_profile_nodes(gpu, n_lnm, lo, hi):
     prof = E.nfw_mis("dsigma", s["r"][:, None], rmis[:, None], w["lnm_x"], 4.0, cases.RHO_CRIT)
     want = s["om"] * np.sum(w["lnm_w"] * w["W"][s["bins"]] * prof, axis=1)
     np.testing.assert_allclose(got, want, rtol=1e-10, atol=1e-10 * np.max(np.abs(want)))
+
+
+# The profile at 16 Chebyshev nodes in lnM starts at 17 masses.  By the rule's
+# bound its error is 1e-13 of the profile; 1e-9 is the restatement's.
+@pytest.mark.parametrize("n_lnm,radii", [(16, 3), (17, 3), (24, 10), (40, 2)])
+def test_projection_shear_profile_nodes(gpu, n_lnm, radii):
+    _compare(dict(kind="prj", radii=radii, n_lnm=n_lnm, n_per_seg=6, n_zring=8, n_zouter=8), 1e-9)

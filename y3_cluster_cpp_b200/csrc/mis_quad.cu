@@ -1,6 +1,8 @@
 // mis_quad.cu -- the miscentred DeltaSigma of (R, R_mis) pairs at many scale
 // radii: one quadrature geometry per pair, shared by its scale radii.
 #include <algorithm>
+#include <cmath>
+#include <vector>
 
 #include "mis_quad.cuh"
 
@@ -136,6 +138,35 @@ cos_kernel(const double* x, int n, double* out)
 }
 
 }  // namespace
+
+// Node positions on [lo, hi], then the barycentric interpolation matrix
+// [node][mass].
+std::vector<double>
+cheb_rows(int N, double lo, double hi, const std::vector<double>& x)
+{
+  const size_t nx = x.size();
+  const long double mid = 0.5L * ((long double)lo + hi), half = 0.5L * ((long double)hi - lo);
+  std::vector<double> v(N + N * nx);
+  std::vector<long double> wt(N), c(N);
+  for (int j = 0; j < N; ++j) {
+    const long double a = (2 * j + 1) * 3.14159265358979323846264338327950288L / (2 * N);
+    v[j] = (double)(mid + half * std::cos(a));
+    wt[j] = (j & 1 ? -1.0L : 1.0L) * std::sin(a);
+  }
+  for (size_t k = 0; k < nx; ++k) {
+    long double sum = 0.0L;
+    int hit = -1;
+    for (int j = 0; j < N; ++j) {
+      const long double d = (long double)x[k] - v[j];
+      if (d == 0.0L) hit = j;
+      c[j] = hit >= 0 ? 0.0L : wt[j] / d;
+      sum += c[j];
+    }
+    for (int j = 0; j < N; ++j)
+      v[N + j * nx + k] = hit >= 0 ? (j == hit ? 1.0 : 0.0) : (double)(c[j] / sum);
+  }
+  return v;
+}
 
 int
 cos_device(const double* x, int n, double* out, cudaStream_t s)

@@ -14,6 +14,8 @@
 // offset ring crosses the aperture.
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 #include "host_common.h"
 #include "nfw_table.cuh"
@@ -22,6 +24,9 @@ namespace y3b {
 
 int gl_nodes_device(double a, double b, int n, double* xs, double* ws, cudaStream_t s);
 int cos_device(const double* x, int n, double* out, cudaStream_t s);
+
+// N Chebyshev nodes on [lo, hi], then the interpolation matrix [N][x.size()].
+std::vector<double> cheb_rows(int N, double lo, double hi, const std::vector<double>& x);
 
 // Miscentred profile quadrature nodes in s: two GL panels split at the
 // ring-crossing kink s_k = x / x_mis (R / R_mis, mass independent).

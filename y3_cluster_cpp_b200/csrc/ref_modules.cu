@@ -689,36 +689,6 @@ namespace y3b {
 constexpr int kChebMinMasses = 32;
 constexpr double kChebMaxRange = 9.0;
 
-// Node positions on [lo, hi], then the barycentric interpolation matrix
-// [node][mass].
-std::vector<double>
-cheb_rows(double lo, double hi, const std::vector<double>& x)
-{
-  constexpr int N = kChebNodes;
-  const size_t nx = x.size();
-  const long double mid = 0.5L * ((long double)lo + hi), half = 0.5L * ((long double)hi - lo);
-  std::vector<double> v(N + N * nx);
-  long double wt[N];
-  for (int j = 0; j < N; ++j) {
-    const long double a = (2 * j + 1) * 3.14159265358979323846264338327950288L / (2 * N);
-    v[j] = (double)(mid + half * std::cos(a));
-    wt[j] = (j & 1 ? -1.0L : 1.0L) * std::sin(a);
-  }
-  for (size_t k = 0; k < nx; ++k) {
-    long double c[N], sum = 0.0L;
-    int hit = -1;
-    for (int j = 0; j < N; ++j) {
-      const long double d = (long double)x[k] - v[j];
-      if (d == 0.0L) hit = j;
-      c[j] = hit >= 0 ? 0.0L : wt[j] / d;
-      sum += c[j];
-    }
-    for (int j = 0; j < N; ++j)
-      v[N + j * nx + k] = hit >= 0 ? (j == hit ? 1.0 : 0.0) : (double)(c[j] / sum);
-  }
-  return v;
-}
-
 }  // namespace y3b
 
 struct y3b_selgl {
@@ -788,7 +758,7 @@ y3b_selgl_create(const y3b_selgl_config* cfg, y3b_selgl** out)
   if (rc == Y3B_OK) rc = y3b::cuda_status(cudaStreamSynchronize(h->stream), "sync");
   if (rc == Y3B_OK && cfg->n_lnm > y3b::kChebMinMasses &&
       cfg->lnm_high - cfg->lnm_low <= y3b::kChebMaxRange) {
-    const std::vector<double> v = y3b::cheb_rows(cfg->lnm_low, cfg->lnm_high, h->h_lnm_x);
+    const std::vector<double> v = y3b::cheb_rows(y3b::kChebNodes, cfg->lnm_low, cfg->lnm_high, h->h_lnm_x);
     rc = h->cheb.upload(v.data(), v.size(), h->stream);
     if (rc == Y3B_OK) rc = y3b::cuda_status(cudaStreamSynchronize(h->stream), "sync");
   }
