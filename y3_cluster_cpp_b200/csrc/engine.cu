@@ -1121,9 +1121,9 @@ yf_kernel(PrepArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// The FP64 form's direct sum, for the points that the matrix product (fp64_form.cu) does
-// not admit, listed by the prep kernel.  CTA = (listed point, z node q) in
-// turn; thread k sums over lam_t with one FP64 exp per node:
+// The FP64 form's direct sum, for the points that the matrix product
+// (fp64_form.cu) does not admit, listed by the prep kernel.  CTA = (listed
+// point, z node q) in turn; thread k sums over lam_t with one FP64 exp per node:
 // V_i(q, k) = P0_kq sum_t u_t K_i(t, q) exp(-(l_t - mu)^2/2s^2) (with the edge
 // factor exp(-v^2 / 2 s^2) moved into P0 for mu outside the nodes' span).
 __device__ void direct_main(const PointDev& pt, const GridDev& G, double* s64, int q, double* dsh);

@@ -27,8 +27,8 @@
 // prj_slice_kernel (one block per slice: both grids, the line-of-sight sums),
 // prj_psi_kernel (one warp per theta node), prj_profile_kernel (one warp per
 // (grid point, theta node): the profile of every mass or Chebyshev node,
-// contracted with the slice's mass weights) and prj_sum_kernel (one block per grid point: the
-// theta sums).  Every sum has a fixed order.
+// contracted with the slice's mass weights) and prj_sum_kernel (one block per
+// grid point: the theta sums).  Every sum has a fixed order.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
