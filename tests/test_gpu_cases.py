@@ -178,3 +178,41 @@ def test_miscentred_profile_nodes(gpu, n_lnm, lo, hi):
 @pytest.mark.parametrize("n_lnm,radii", [(16, 3), (17, 3), (24, 10), (40, 2)])
 def test_projection_shear_profile_nodes(gpu, n_lnm, radii):
     _compare(dict(kind="prj", radii=radii, n_lnm=n_lnm, n_per_seg=6, n_zring=8, n_zouter=8), 1e-9)
+
+
+@pytest.mark.parametrize("hmf_fp32", [False, True])
+def test_points_given_up_by_their_tables(gpu, hmf_fp32):
+    """A non-finite table entry of a point whose scratch holds another grid's
+    values (the engine ran the larger grid before, in every form it has) gives
+    the domain error, and the next call gives what a fresh engine gives."""
+    from y3_cluster_cpp_b200 import _capi, synthetic
+    from y3_cluster_cpp_b200 import engine as E
+
+    grids = [synthetic.grid(4), synthetic.grid(1, n_m=33, n_z=16, n_t=40, n_o=16, n_zo=8)]
+    so = synthetic.shear_opts(n_theta=16, n_s=32, n_R=3)
+    pts = synthetic.walkers(3, seed=8, densities=(1,))
+    t = pts[0].tables
+    precs = (E.MIXED,) if hmf_fp32 else (E.MIXED, E.FP64)
+
+    def engine():
+        return E.Engine(grids, len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]),
+                        synthetic.plob_baseline(), max_points=3, n_sci=len(t["sci_z"]), shear=so,
+                        hmf_fp32=hmf_fp32)
+
+    eng, fresh = engine(), engine()
+    want = {p: fresh.eval(pts, p, grid_of=lambda _: 1) for p in precs}
+    for where in ("dndlnmh", "dist_da", "hmf_z"):
+        for p in precs:
+            eng.eval(pts, p, grid_of=lambda _: 0)
+        bad = synthetic.walkers(3, seed=8, densities=(1,))
+        bad[1].tables[where] = np.array(bad[1].tables[where], copy=True)
+        bad[1].tables[where].flat[3] = np.nan
+        for p in precs:
+            with pytest.raises(_capi.Y3BError) as err:
+                eng.eval(bad, p, grid_of=lambda _: 1)
+            assert err.value.status == _capi.ERR_DOMAIN
+            got = eng.eval(pts, p, grid_of=lambda _: 1)
+            for k in ("counts", "shear"):
+                np.testing.assert_array_equal(got[k], want[p][k])
+    eng.close()
+    fresh.close()

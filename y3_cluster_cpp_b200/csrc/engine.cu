@@ -263,6 +263,26 @@ prep_kernel(PrepArgs a)
   __shared__ int timed_out;
   int bad = 0;  // a non-finite table entry seen by this thread
   __shared__ int swin[16];  // lam_t stage window per lnM tile (n_m <= 1024)
+  double* s64 = a.s64 + (size_t)p * Gp->s64_stride;
+  float* s32 = a.s32 + (size_t)p * Gp->s32_stride;
+  // Leaves the point unprepared: its scratch holds an earlier call's values,
+  // maybe of another grid, and the kernels that follow take cells and windows
+  // from there.  The FP64 form's header says no work, the mixed form's tiles
+  // an empty window to yf_kernel (no F, no Y) and the first pair of stages to
+  // the contraction, whose values go nowhere: the call reports the error.
+  auto give_up = [&](int code) {
+    if (tid != 0) return;
+    set_err(a.status, code);
+    if (!a.mixed) {
+      s64[Gp->o_f64] = 0.0;
+      return;
+    }
+    for (int mt = 0; mt < n_m_pad / kGemmRows; ++mt) {
+      for (int bg = 0; bg < Gp->n_bg; ++bg)
+        a.win_tile[(size_t)p * a.win_stride + mt * Gp->n_bg + bg] = 2 << 16;
+      s32[Gp->f_tinfo + 4 * mt + 3] = __int_as_float(0);
+    }
+  };
 
   if (a.mixed)
     for (int t = tid * 16; t < Gp->n_t; t += blockDim.x * 16)
@@ -319,7 +339,7 @@ prep_kernel(PrepArgs a)
   }
   __syncthreads();
   if (timed_out) {  // uniform exit; the copy only targets this CTA's shared memory
-    if (tid == 0) set_err(a.status, kDevTimeout);
+    give_up(kDevTimeout);
     return;
   }
   // Every table entry must be finite: the staged sections (not their
@@ -336,7 +356,7 @@ prep_kernel(PrepArgs a)
       for (int i = tid; i < n_hz * n_hm; i += blockDim.x) bad |= !isfinite(__ldg(dng + i));
     }
     if (__syncthreads_or(bad)) {
-      if (tid == 0) set_err(a.status, kDevNonFinite);
+      give_up(kDevNonFinite);
       return;
     }
   }
@@ -350,8 +370,6 @@ prep_kernel(PrepArgs a)
   // HMF mass axis ln(m_h (Omega_M - Omega_nu)) (hmf_t.hh:15-25), in place.
   for (int i = tid; i < n_hm; i += blockDim.x) mh[i] = log(mh[i] * (pt.om - pt.onu));
   __syncthreads();
-  double* s64 = a.s64 + (size_t)p * Gp->s64_stride;
-  float* s32 = a.s32 + (size_t)p * Gp->s32_stride;
   const double* xm = g_xm;
   const double* xz = g_xz;
   // The lnM and z_t vectors in one pass, from a warp's edge on for the latter
@@ -920,6 +938,11 @@ yf_kernel(PrepArgs a)
     if (tid == 0) set_err(a.status, kDevTimeout);
     return;
   }
+  const int win = tinfo[3], w_lo = win & 0xFFFF, w_hi = win >> 16;
+  if (w_hi == 0) {  // the prep kernel left the point unprepared (and reported it)
+    wait_bar(&bar2);
+    return;
+  }
   const float sc1 = fh[3];
   // F'(t, k) for the contraction (the row scale above), split into bf16
   // hi + lo and written in its shared-memory stage layout: block
@@ -928,7 +951,6 @@ yf_kernel(PrepArgs a)
   // exponent is >= 0 on every real node; the padded nodes past n_t (whose G
   // is zero) take its magnitude, so F' <= 1 stays finite there too.  Only
   // the stages inside the tile's window are ever read.
-  const int win = tinfo[3], w_lo = win & 0xFFFF, w_hi = win >> 16;
   const float* row_am = rows + 4 * kGemmRows;
   const float* row_vs2 = rows + 5 * kGemmRows;
   const float2 sc2 = make_float2(sc1, sc1);

@@ -57,7 +57,7 @@ f64_factor_kernel(F64Launch L)
   const GridDev* __restrict__ Gp = L.grids + pt.grid;
   const double* __restrict__ s64 = L.s64 + (size_t)p * Gp->s64_stride;
   const double* hdr = s64 + Gp->o_f64;
-  if (hdr[0] == 0.0) return;  // direct sum
+  if (hdr[0] == 0.0) return;  // direct sum, or left unprepared
   const int n_m = Gp->n_m, n_z = Gp->n_z, n_t = Gp->n_t;
   const F64Ws w = f64_ws(n_m, n_z, n_t);
   double* ws = L.ws + (size_t)blockIdx.y * L.ws_stride;
