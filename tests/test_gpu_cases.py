@@ -216,3 +216,34 @@ def test_points_given_up_by_their_tables(gpu, hmf_fp32):
                 np.testing.assert_array_equal(got[k], want[p][k])
     eng.close()
     fresh.close()
+
+
+def test_fp64_bins_far_from_every_mass(gpu):
+    """Mass-richness relations that leave richness bins many sigma above every
+    mass, with a P(lambda_o | lambda_t) without projection tail: small positive
+    counts, not zero, down to the bins that no factor holds.  An exponent of
+    up to 600 is rounded to 1e-13 of itself on both sides, mu (in 1 / sigma per
+    sigma) to 3e-13: 1e-11."""
+    import oracle
+    from y3_cluster_cpp_b200 import engine as E
+    from y3_cluster_cpp_b200 import synthetic
+
+    pz, pc = synthetic.plob_baseline()
+    pc = np.array(pc).reshape(8, -1)
+    pc[7] = 0.0
+    g = synthetic.grid(1, n_m=64, n_z=16, n_t=256, n_o=32, n_zo=8)
+    pts = []
+    for sigma in (0.05, 0.1, 0.2):
+        for A in (-0.5, 0.5, 1.5, 2.5, 3.2):
+            p = synthetic.fiducial(1)
+            p.A, p.sigma = A, sigma
+            pts.append(p)
+    t = pts[0].tables
+    eng = E.Engine([g], len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]), (pz, pc.ravel()),
+                   max_points=len(pts))
+    got = eng.eval(pts, E.FP64, grid_of=lambda _: 0)["counts"]
+    want = np.array([oracle.direct_eval(g, pz, pc.ravel(), p.mor, oracle.cosmo(p.om, p.h0),
+                                        p.tables)[0] for p in pts])
+    assert np.all(want > 0) and want.min() < 1e-200
+    np.testing.assert_allclose(got, want, rtol=1e-11)
+    eng.close()

@@ -343,17 +343,13 @@ prep_kernel(PrepArgs a)
     return;
   }
   // Every table entry must be finite: the staged sections (not their
-  // alignment padding) and, for the FP64 form, the HMF grid in global memory
-  // (yf_kernel checks the mixed form's copy of it).
+  // alignment padding) here, the HMF grid in global memory where it is read
+  // (below for the FP64 form, yf_kernel for the mixed form).
   {
     const int len[7] = {n_hm, n_hz, 0, L.n_dist, L.n_dist, L.n_sci, L.n_sci};
     for (int sct = 0; sct < 7; ++sct) {
       const double* base = sct < 2 ? tab + L.off[sct] : tab + head + (L.off[sct] - L.off[3]);
       for (int i = tid; i < len[sct]; i += blockDim.x) bad |= !isfinite(base[i]);
-    }
-    if (!a.mixed) {
-      const double* __restrict__ dng = src + L.off[2];
-      for (int i = tid; i < n_hz * n_hm; i += blockDim.x) bad |= !isfinite(__ldg(dng + i));
     }
     if (__syncthreads_or(bad)) {
       give_up(kDevNonFinite);
@@ -432,20 +428,79 @@ prep_kernel(PrepArgs a)
     double* __restrict__ P0 = s64 + Gp->o_P0;
     const double xl0 = Gp->xl[0], xl1 = Gp->xl[Gp->n_t - 1];
     // Matrix-product form (fp64_form.cu): centres on multiples of 2^-20 (the
-    // differences from them are exact), the exponents of its factors G and
-    // H and of the edge factor exp(v^2 / 2 s^2) together below kF64MaxExp
-    // (F = S / (G H) then stays in range too where the product matters), and
-    // the lam_t window of each 64-row tile: outside mu -+ sqrt(e^2 + (8.7 s)^2),
-    // e the distance of mu to the domain, the renormalised density is below
-    // 4e-17 of its peak.
-    constexpr double kSnap = 1048576.0, kWin64 = 8.7;
+    // differences from them are exact); the exponents of its factors G and
+    // H and of the edge factor exp(v^2 / 2 s^2) together below kF64MaxExp, so
+    // that F = S / (G H) holds every term above exp(-(708 - kF64MaxExp)) of
+    // the density's peak.  Terms below exp(-room) of it may be left out:
+    // a bin's sum is at least what the mass nearest to its kernel gives, a gap
+    // of g sigma away, exp(-g^2 / 2) of a peak, times the smallest HMF value
+    // against the largest, times 1/100 for the kernel's shoulder (kp_lo,
+    // kp_hi), so room = g^2 / 2 + ln(ratio) + kF64Bits, which takes in 2^-56,
+    // the 1/100 and a factor of 1e6 for the weights of the nodes.  Where room
+    // passes kF64MaxRoom (bins out of every mass's reach, tables that span
+    // more or touch zero) the point takes the direct sum.
+    constexpr double kSnap = 1048576.0, kF64Bits = 57.0;
     const double a0 = rint(A0 * kSnap) / kSnap, b0 = rint(B0 * kSnap) / kSnap, l0 = a0 + b0;
     const double am = 0.5 * ((mu_hi - mu_lo) - (b_hi - b_lo)) + 1e-6;
     const double bm = 0.5 * (b_hi - b_lo) + 1e-6;
     const double dm = fmax(fabs(xl0 - l0), fabs(xl1 - l0));
     const double vm = fmax(fmax(xl0 - mu_lo, mu_hi - xl1), 0.0);
     const double ex = (bm * (dm + am + 0.5 * bm) + 0.5 * vm * vm) * inv_s * inv_s;
-    const bool product = a.f64_rounds && ex <= kF64MaxExp;
+    // The HMF grid: finite everywhere, and the extremes of the cells in use.
+    double n_lo = 1e300, n_hi = 0.0;
+    {
+      const int warp = tid >> 5, lane = tid & 31, nw = kPrepThreads / 32;
+      const int x0 = k_x[0], x1 = k_x[n_m - 1] + 1, y0 = q_y[0], y1 = q_y[n_z - 1] + 1;
+      for (int y = warp; y < n_hz; y += 2 * nw) {  // two rows, 128 columns at a time
+        const bool two = y + nw < n_hz, in0 = y >= y0 && y <= y1, in1 = y + nw >= y0 && y + nw <= y1;
+        const double* r0 = dn + (size_t)y * n_hm;
+        const double* r1 = r0 + (two ? (size_t)nw * n_hm : 0);
+        for (int xb = lane; xb < n_hm; xb += 128) {
+          double v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            v[u] = __ldg((u < 4 ? r0 : r1) + min(xb + 32 * (u & 3), n_hm - 1));
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int x = xb + 32 * (u & 3);
+            bad |= !isfinite(v[u]);
+            if (x >= x0 && x <= x1 && (u < 4 ? in0 : in1 && two)) {
+              n_lo = fmin(n_lo, v[u]);
+              n_hi = fmax(n_hi, v[u]);
+            }
+          }
+        }
+      }
+      for (int off = 16; off > 0; off >>= 1) {
+        n_lo = fmin(n_lo, __shfl_xor_sync(0xffffffffu, n_lo, off));
+        n_hi = fmax(n_hi, __shfl_xor_sync(0xffffffffu, n_hi, off));
+      }
+      __shared__ double n_s[2][kPrepThreads / 32];
+      if (lane == 0) {
+        n_s[0][warp] = n_lo;
+        n_s[1][warp] = n_hi;
+      }
+      if (__syncthreads_or(bad)) {
+        give_up(kDevNonFinite);
+        return;
+      }
+      for (int w = 0; w < nw; ++w) {
+        n_lo = fmin(n_lo, n_s[0][w]);
+        n_hi = fmax(n_hi, n_s[1][w]);
+      }
+    }
+    bool product = a.f64_rounds && ex <= kF64MaxExp;
+    double room = 0.0;
+    if (product) {  // uniform
+      double gap = 0.0;
+      for (int i = 0; i < Gp->nI; ++i) {  // at every z_t node
+        gap = fmax(gap, Gp->xl[Gp->kp_lo[i]] - (a_hi + b_lo));
+        gap = fmax(gap, (a_lo + b_hi) - Gp->xl[Gp->kp_hi[i]]);
+      }
+      const double f0 = k_f[0], f1 = k_f[n_m - 1];  // linear in between
+      room = kF64Bits + 0.5 * gap * gap * inv_s * inv_s + log(n_hi / n_lo) + fabs(log(f1 / f0));
+      product = n_lo > 0.0 && room <= kF64MaxRoom;
+    }
     double* hdr = s64 + Gp->o_f64;
     if (tid == 0) {
       hdr[0] = product ? 1.0 : 0.0;
@@ -479,7 +534,9 @@ prep_kernel(PrepArgs a)
         if (lane) continue;
         lo += b_lo;
         hi += b_hi;
-        const double e_lo = fmin(fmax(lo, ll_lo), ll_hi) - lo, w2 = kWin64 * sig * kWin64 * sig;
+        // outside mu -+ sqrt(e^2 + 2 room s^2), e the distance of mu to the
+        // domain, the renormalised density is below exp(-room) of its peak
+        const double e_lo = fmin(fmax(lo, ll_lo), ll_hi) - lo, w2 = 2.0 * room * sig * sig;
         const double e_hi = fmin(fmax(hi, ll_lo), ll_hi) - hi;
         const double x_lo = lo - sqrt(e_lo * e_lo + w2), x_hi = hi + sqrt(e_hi * e_hi + w2);
         const double* xl = Gp->xl;
@@ -1804,32 +1861,41 @@ build_grid(y3b_engine* e, int gi)
     Y3B_CUDA(cudaMemcpy(hk.data(), b->Ki.get(), hk.size() * sizeof(double),
                         cudaMemcpyDeviceToHost));
     for (int i = 0; i < kMaxLamBins; ++i) {
-      g.kt_lo[i] = g.k64_lo[i] = 0;
-      g.kt_hi[i] = g.k64_hi[i] = g.n_t - 1;
+      g.kt_lo[i] = g.k64_lo[i] = g.kp_lo[i] = 0;
+      g.kt_hi[i] = g.k64_hi[i] = g.kp_hi[i] = g.n_t - 1;
     }
     for (int i = 0; i < g.nI; ++i) {
-      int lo = g.n_t, hi = -1, lo64 = g.n_t, hi64 = -1;
+      int lo = g.n_t, hi = -1, lo64 = g.n_t, hi64 = -1, p_lo = 0, p_hi = g.n_t - 1;
       for (int q = 0; q < g.n_z; ++q) {
         const double* k = hk.data() + ((size_t)i * g.n_z + q) * g.n_t;
         double mx = 0.0;
         for (int t = 0; t < g.n_t; ++t) mx = std::max(mx, k[t]);
         if (!(mx > 0.0)) continue;
+        int first = g.n_t, last = -1;
         for (int t = 0; t < g.n_t; ++t) {
           if (k[t] > 1e-12 * mx) {
             lo = std::min(lo, t);
             hi = std::max(hi, t);
           }
-          if (k[t] > 1e-30 * mx) {
+          if (k[t] > 1e-100 * mx) {
             lo64 = std::min(lo64, t);
             hi64 = std::max(hi64, t);
           }
+          if (k[t] >= 1e-2 * mx) {
+            first = std::min(first, t);
+            last = t;
+          }
         }
+        p_lo = std::max(p_lo, first);
+        p_hi = std::min(p_hi, last);
       }
       if (hi >= lo) {
         g.kt_lo[i] = lo;
         g.kt_hi[i] = hi;
         g.k64_lo[i] = lo64;
         g.k64_hi[i] = hi64;
+        g.kp_lo[i] = p_lo;
+        g.kp_hi[i] = p_hi;
       }
     }
   }

@@ -40,7 +40,8 @@ struct GridDev {
   // lam_t nodes where richness bin i's kernel K_i(t, q) exceeds 1e-12 of its
   // maximum over t, for some z_t node q: [kt_lo[i], kt_hi[i]]
   int kt_lo[kMaxLamBins], kt_hi[kMaxLamBins];
-  int k64_lo[kMaxLamBins], k64_hi[kMaxLamBins];  // the same above 1e-30 (FP64 form)
+  int k64_lo[kMaxLamBins], k64_hi[kMaxLamBins];  // the same above 1e-100 (FP64 form)
+  int kp_lo[kMaxLamBins], kp_hi[kMaxLamBins];    // the same above 1e-2, for every z_t node
   double lnm_lo, lnm_hi, zt_lo, zt_hi, ll_lo, ll_hi, sz0;
   double sz_bin[8];   // sigma_z(z, j) = sz0 (1 + z) + sz_bin[j]
   const double* xm;   // [n_m]  lnM nodes
@@ -71,10 +72,13 @@ struct GridDev {
 };
 
 // FP64 form (fp64_form.cu): lnM rows of a tile, lam_t nodes of a stage, and
-// the largest exponent of a factor that its matrix product admits.
+// the largest exponent of its factors G and H that its matrix product admits.
 constexpr int kF64Rows = 64;
 constexpr int kF64Chunk = 16;
-constexpr double kF64MaxExp = 600.0;
+constexpr double kF64MaxExp = 400.0;
+// ... and the largest exponent of the terms that it may have to keep: below
+// that of the kernels' cut (1e-100) and 708 - kF64MaxExp.
+constexpr double kF64MaxRoom = 230.0;
 
 struct PointDev {  // mirrors y3b_point
   double om, ol, ok, h0, onu, hmf_s, hmf_q;

@@ -10,8 +10,8 @@
 // at the part's 37 TFLOP/s.  The centres are multiples of 2^-20, so delta, a
 // and b are exact differences and the identity holds to the rounding of the
 // exponentials' arguments; FP64's exponent range holds the factors wherever
-// the point passes the prep kernel's bound (kF64MaxExp), the others keep the
-// direct sum (direct_main_kernel).  48 points at 4x nodes: 147 us a call,
+// the point passes the prep kernel's bounds (kF64MaxExp, kF64MaxRoom), the others keep the
+// direct sum (direct_main_kernel).  48 points at 4x nodes: 172 us a call,
 // 1841 us with the direct sum; results within 2e-16 of each other.
 //
 // The points of a call are taken in rounds that fit the workspace (F, G and Y
