@@ -7,18 +7,21 @@
 // so S_i(k,q) = H sum_t F(t,k) [u_t K_i(t,q) G(t,q)] needs one exponential
 // per (t,k), (t,q) and (k,q) instead of one per (k,q,t): 131 thousand in
 // place of 8.4 million a point at 4x nodes, and 34 M multiply-adds that run
-// at the part's 37 TFLOP/s.  The centres are multiples of 2^-20, so delta, a
-// and b are exact differences and the identity holds to the rounding of the
-// exponentials' arguments; FP64's exponent range holds the factors wherever
-// the point passes the prep kernel's bounds (kF64MaxExp, kF64MaxRoom), the others keep the
-// direct sum (direct_main_kernel).  48 points at 4x nodes: 172 us a call,
-// 1841 us with the direct sum; results within 2e-16 of each other.
+// at the part's 37 TFLOP/s.  The factors' exponents carry their rounding errors
+// (fp64_factors.cuh), and L0 = A0 + B0 exactly, so that the identity holds to
+// the last places of a factor: a cell is within 1.3e-15 of the exact
+// sum, the direct sum, which rounds mu, within 9e-15 (s from 0.06 to 0.24).
+// FP64's exponent range holds the factors wherever the point passes the prep
+// kernel's bounds (kF64MaxExp, kF64MaxRoom), the others keep the direct sum
+// (direct_main_kernel).  48 points at 4x nodes: 178 us a call, 1841 us with
+// the direct sum.
 //
 // The points of a call are taken in rounds that fit the workspace (F, G and Y
 // of a round stay in L2); f64_factor_kernel writes them, f64_gemm_kernel
 // contracts lambda_t and z_t and writes the mass weights W_ij(k).
 #include "common.cuh"
 #include "engine_internal.h"
+#include "fp64_factors.cuh"
 #include "host_common.h"
 #include "mor_norm.cuh"
 
@@ -45,9 +48,10 @@ f64_ws(int n_m, int n_z, int n_t)
   return w;
 }
 
-// F, G and Y(k, q) = n(M_k, z_q) H(k, q) / (sqrt(2 pi) s D_kq), one element a
-// thread; F and G only on the windows' lam_t stages (zero past the last node
-// and row).
+// F, G and Y(k, q) = n(M_k, z_q) H(k, q) / (sqrt(2 pi) s D_kq); F and G only on
+// the windows' lam_t stages (zero past the last node and row).  Bound by the
+// FP64 units: an exponential and some thirty operations for its exponent an
+// element, so that what depends on the column alone is formed once a column.
 __global__ void __launch_bounds__(kFactorThreads)
 f64_factor_kernel(F64Launch L)
 {
@@ -62,53 +66,55 @@ f64_factor_kernel(F64Launch L)
   const F64Ws w = f64_ws(n_m, n_z, n_t);
   double* ws = L.ws + (size_t)blockIdx.y * L.ws_stride;
   const double A0 = hdr[1], B0 = hdr[2], L0 = A0 + B0, inv_s = 1.0 / pt.sigma;
-  const double c = 0.5 * inv_s * inv_s;
+  const Dd c = f64_half_inv_var(pt.sigma);
   const double* alpha = s64 + Gp->o_alpha;
   const double* beta = s64 + Gp->o_beta;
   const int* win = reinterpret_cast<const int*>(hdr + 4);
   const int step = gridDim.x * kFactorThreads, i0 = blockIdx.x * kFactorThreads + threadIdx.x;
-  const int nF = w.n_tp * w.n_mp, nG = w.n_tp * n_z, nY = n_m * n_z;
   int h_lo = w.n_tp, h_hi = 0;  // hull of the tiles' windows
   for (int m = 0; m < w.n_mp / kF64Rows; ++m) {
     h_lo = min(h_lo, (win[m] & 0xFFFF) * kF64Chunk);
     h_hi = max(h_hi, (win[m] >> 16) * kF64Chunk);
   }
-  for (int i = i0; i < nF; i += step) {
-    const int t = i / w.n_mp, k = i - t * w.n_mp, v = win[k / kF64Rows];
-    if (t < (v & 0xFFFF) * kF64Chunk || t >= (v >> 16) * kF64Chunk) continue;
-    double f = 0.0;
-    if (t < n_t && k < n_m) {
-      const double d = (Gp->xl[t] - L0) - (alpha[k] - A0);
-      f = exp(-d * d * c);
-    }
-    ws[i] = f;
+  // A thread keeps its column (k of F, q of G and Y) and takes rows apart by
+  // the rows that the threads cover at once.
+  int P = min(step, w.n_mp), R = step / P, r0 = i0 / P;
+  for (int k = i0 - r0 * P; r0 < R && k < w.n_mp; k += P) {
+    const int v = win[k / kF64Rows], t_end = (v >> 16) * kF64Chunk;
+    const bool in = k < n_m;
+    const Dd a = dd_diff(alpha[in ? k : 0], A0);
+    for (int t = (v & 0xFFFF) * kF64Chunk + r0; t < t_end; t += R)
+      ws[(size_t)t * w.n_mp + k] =
+        in && t < n_t ? f64_F(dd_diff(Gp->xl[t], L0), a, c) : 0.0;
   }
-  for (int i = i0; i < nG; i += step) {
-    const int t = i / n_z, q = i - t * n_z;
-    if (t < h_lo || t >= h_hi) continue;
-    ws[w.g + i] = t < n_t ? exp((Gp->xl[t] - L0) * (beta[q] - B0) * (2.0 * c)) : 0.0;
+  P = min(step, n_z);
+  R = step / P;
+  r0 = i0 / P;
+  for (int q = i0 - r0 * P; r0 < R && q < n_z; q += P) {
+    const Dd b = dd_diff(beta[q], B0);
+    for (int t = h_lo + r0; t < h_hi; t += R)
+      ws[w.g + (size_t)t * n_z + q] = t < n_t ? f64_G(dd_diff(Gp->xl[t], L0), b, c) : 0.0;
   }
   const double* dn = L.tables + (size_t)(L.slot ? L.slot[p] : p) * L.lay.stride + L.lay.off[2];
   const double norm0 = inv_s / kSqrt2Pi;
-  for (int i = i0; i < nY; i += step) {
-    const int k = i / n_z, q = i - k * n_z;
-    const double t = s64[Gp->o_kt + k], u = s64[Gp->o_qu + q];
-    const double* r0 = dn + (size_t)s64[Gp->o_qy + q] * L.lay.n_hm + (int)s64[Gp->o_kx + k];
-    const double* r1 = r0 + L.lay.n_hm;
-    const double n = ((1.0 - t) * (1.0 - u) * r0[0] + t * (1.0 - u) * r0[1] +
-                      (1.0 - t) * u * r1[0] + t * u * r1[1]) *
-                     s64[Gp->o_kf + k] * norm0;
-    const double mu = alpha[k] + beta[q], a = alpha[k] - A0, b = beta[q] - B0;
-    const double lo = (Gp->ll_lo - mu) * inv_s, hi = (Gp->ll_hi - mu) * inv_s;
-    const double h = -b * (2.0 * a + b) * c;
-    double y;
-    if (lo < -8.5 && hi > 8.5)
-      y = n * exp(h);
-    else if (lo <= 0.0 && hi >= 0.0)
-      y = n * exp(h) / mor_norm_slow(lo, hi);
-    else
-      y = n * exp(h - ln_mor_norm(lo, hi));
-    ws[w.y + i] = y;
+  for (int q = i0 - r0 * P; r0 < R && q < n_z; q += P) {
+    const Dd b = dd_diff(beta[q], B0);
+    const double u = s64[Gp->o_qu + q];
+    const double* row = dn + (size_t)s64[Gp->o_qy + q] * L.lay.n_hm;
+    for (int k = r0; k < n_m; k += R) {
+      const double t = s64[Gp->o_kt + k];
+      const double* d0 = row + (int)s64[Gp->o_kx + k];
+      const double* d1 = d0 + L.lay.n_hm;
+      const double n = ((1.0 - t) * (1.0 - u) * d0[0] + t * (1.0 - u) * d0[1] +
+                        (1.0 - t) * u * d1[0] + t * u * d1[1]) *
+                       s64[Gp->o_kf + k] * norm0;
+      const double mu = alpha[k] + beta[q];
+      const double lo = (Gp->ll_lo - mu) * inv_s, hi = (Gp->ll_hi - mu) * inv_s;
+      const bool in = lo <= 0.0 && hi >= 0.0;
+      double y = n * f64_H(dd_diff(alpha[k], A0), b, c, in ? 0.0 : ln_mor_norm(lo, hi));
+      if (in && !(lo < -8.5 && hi > 8.5)) y /= mor_norm_slow(lo, hi);
+      ws[w.y + (size_t)k * n_z + q] = y;
+    }
   }
 }
 
@@ -126,7 +132,7 @@ dmma(double* c, double a, double b)
 // lam_t nodes are double-buffered: F by 16-byte async copies, B = G u K_i
 // formed in registers a chunk ahead.  Leading dimensions of 4 modulo 16
 // doubles keep the fragment loads free of bank conflicts.  Bound by the FP64
-// units: 26 KB of shared memory and ~100 registers leave four blocks an SM.
+// units: 30 KB of shared memory and 128 registers leave four blocks an SM.
 constexpr int kCols = 32, kLdF = kF64Rows + 4, kLdB = kCols + 4, kLdS = kCols + 1;
 
 __global__ void __launch_bounds__(128, 4)
