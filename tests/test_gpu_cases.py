@@ -247,3 +247,27 @@ def test_fp64_bins_far_from_every_mass(gpu):
     assert np.all(want > 0) and want.min() < 1e-200
     np.testing.assert_allclose(got, want, rtol=1e-11)
     eng.close()
+
+
+@pytest.mark.parametrize("n_lnm", [21, 24, 40])
+@pytest.mark.parametrize("peak", [30.5, 33.1, 35.5])
+def test_projection_profile_nodes_against_every_mass(gpu, n_lnm, peak):
+    """The profile at Chebyshev nodes of lnM (six e-folds, the widest range of
+    the rule) against the profile at every mass (the next double above it),
+    with an HMF of one narrow peak, so that few masses carry the sums and the
+    interpolation's error is not averaged.  The mass nodes of the two differ by
+    1e-16 of themselves; interpolation and the ring sums' rounding leave 1e-14
+    of a profile: 5e-14 of the largest output of each channel."""
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+
+    om, t, p, grid = cases._prj_inputs(dict(radii=6), 5)
+    lnm = np.log(t["hmf_m_h"] * om)
+    t = dict(t, dndlnmh=t["dndlnmh"] * (np.abs(lnm - peak) < 0.15))
+    kw = dict(n_lnm=n_lnm, n_per_seg=6, n_zring=8, n_zouter=8, lnm_low=30.0)
+    cz = E.cosmo(om, cases.H0)
+    nodes = E.PrjShear(grid, lnm_high=36.0, **kw).eval(cz, t, p)
+    every = E.PrjShear(grid, lnm_high=np.nextafter(36.0, 40.0), **kw).eval(cz, t, p)
+    for c in range(3):
+        np.testing.assert_allclose(nodes[:, c], every[:, c], rtol=0,
+                                   atol=5e-14 * np.max(np.abs(every[:, c])))

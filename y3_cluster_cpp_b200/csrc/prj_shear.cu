@@ -99,13 +99,17 @@ constexpr double kRuleLn0 = 0.609, kRuleLn1 = 0.1587, kRuleLn2 = 0.0401;
 // The profile of a ring is analytic in ln r_s = lnM / 3 + const, |Im| < pi
 // (it sums the NFW DeltaSigma at distances proportional to 1 / r_s), and
 // enters only through sums over the masses with the slice's weights.  Where
-// it saves a group of eight masses (more than 16 of them, on at most six
-// e-folds) the profile is taken at 16 Chebyshev nodes of lnM and the weights
-// are projected on the nodes instead: the interpolant's error is
-// rho^-16 <= 1e-13 there (rho = h + sqrt(h^2 + 1), h = 6 pi / range), relative
-// since it is the profile per unit mass that is interpolated.
-// 24 masses, 120 grid points: 97 -> 67 us.
-constexpr int kProfNodes = 16;
+// it saves a group of masses (more than 20 of them, on at most six e-folds)
+// the profile is taken at 20 Chebyshev nodes of lnM and the weights are
+// projected on the nodes instead.  It is the profile per unit mass that is
+// interpolated, which spans the range within two decades: the interpolant
+// converges as rho^-n (rho = h + sqrt(h^2 + 1), h = 6 pi / range, 6.4 at six
+// e-folds) from a constant of some tens, the branch points of the ring's many
+// distances.  At six e-folds, over radii from 0.05 to 30 and R_mis from
+// R / 100 to 100 R, the error of a mass is at most 5.6e-15 of its ring's sum
+// of |terms| (1.6e-11 with 16 nodes, 1e-15 the sum's own rounding).
+// 24 masses, 120 grid points: 97 -> 82 us (16 nodes: 67).
+constexpr int kProfNodes = 20;
 constexpr double kProfRange = 6.0;
 
 struct PrjQuad {
@@ -473,8 +477,9 @@ ring_masses_closed(const PrjQuad& Q, const double* __restrict__ rule, int n, dou
 // tangential shear on the circle of radius R around the offset centre,
 // (1/pi) int dt DSigma(d / r_s) (2 a^2 / d^2 - 1), d^2 = R^2 + Rm^2 -
 // 2 R Rm cos t, a = R - Rm cos t.  The geometry is shared by the masses,
-// which only scale d; eight masses accumulate side by side and are summed
-// over the lanes by halving exchanges (nine 64-bit shuffles for eight sums).
+// which only scale d; eight masses (four at the end, where they suffice)
+// accumulate side by side and are summed over the lanes by halving exchanges
+// (nine 64-bit shuffles for eight sums).
 template <int NJ>
 __device__ __forceinline__ double2
 ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double Rm, int n_lnm,
@@ -489,33 +494,37 @@ ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double 
     D2[j] = s2 - c2 * ct;
     A[j] = rule[kRuleTot + lane + 32 * j] * (2.0 * a * a / D2[j] - 1.0) / kPiP;
   }
-  for (int k0 = 0; k0 < n_lnm; k0 += 8) {
-    double acc[8];
+  auto group = [&](auto masses, int k0) {
+    constexpr int U = decltype(masses)::value, S = 32 / U;  // a sum ends on S lanes
+    double acc[U];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < U; ++u) {
       const double q = __ldg(Q.mass + min(k0 + u, n_lnm - 1));
       acc[u] = 0.0;
 #pragma unroll
       for (int j = 0; j < NJ; ++j) acc[u] += A[j] * nfw_dsigma_w(Q.nfw, D2[j] * q, outside);
     }
 #pragma unroll
-    for (int h = 4; h >= 1; h >>= 1) {
-      const bool up = (lane & (4 * h)) != 0;
+    for (int h = U / 2; h >= 1; h >>= 1) {
+      const bool up = (lane & (S * h)) != 0;
 #pragma unroll
       for (int u = 0; u < h; ++u) {
         const double send = up ? acc[u] : acc[u + h];
-        acc[u] = (up ? acc[u + h] : acc[u]) + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+        acc[u] = (up ? acc[u + h] : acc[u]) + __shfl_xor_sync(0xffffffffu, send, S * h);
       }
     }
-    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
-    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-    const int k = k0 + (lane >> 2);
-    if ((lane & 3) == 0 && k < n_lnm) {
+#pragma unroll
+    for (int off = S / 2; off >= 1; off >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    const int k = k0 + lane / S;
+    if (lane % S == 0 && k < n_lnm) {
       const double v = Q.mass[n_lnm + k] * acc[0];
       ar += w[k] * v;
       ac += wc[k] * v;
     }
-  }
+  };
+  int k0 = 0;
+  for (; k0 + 4 < n_lnm; k0 += 8) group(std::integral_constant<int, 8>{}, k0);
+  if (k0 < n_lnm) group(std::integral_constant<int, 4>{}, k0);
   if (__any_sync(0xffffffffu, outside))
     return ring_masses_closed(Q, rule, 32 * NJ, R, Rm, n_lnm, w, wc, lane);
   for (int off = 16; off >= 4; off >>= 1) {
@@ -528,7 +537,8 @@ ring_masses(const PrjQuad& Q, const double* __restrict__ rule, double R, double 
 // The same contractions by quadrature, one warp per (grid point, theta
 // node): the lanes take the ring's nodes, so the profile's table reads of a
 // warp fall on few, neighbouring segments.  12 slices x 10 radii x ~130
-// theta x 24 masses: 98 us, bound by those reads (L1).
+// theta x 20 nodes (24 masses): 82 us, bound by those reads (L1); 98 us with
+// a profile at every mass.
 __global__ void __launch_bounds__(256, 3)
 prj_profile_kernel(PrjDims D, PrjQuad Q, const double* __restrict__ scratch,
                    const int* __restrict__ nt, double2* __restrict__ P)
