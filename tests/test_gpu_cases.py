@@ -271,3 +271,29 @@ def test_projection_profile_nodes_against_every_mass(gpu, n_lnm, peak):
     for c in range(3):
         np.testing.assert_allclose(nodes[:, c], every[:, c], rtol=0,
                                    atol=5e-14 * np.max(np.abs(every[:, c])))
+
+
+@pytest.mark.parametrize("peak", [28.2, 30.0, 36.5])
+@pytest.mark.parametrize("n_lnm", [33, 96])
+def test_miscentred_profile_nodes_against_every_mass(gpu, n_lnm, peak):
+    """The module's profile at Chebyshev nodes of lnM (nine e-folds, the widest
+    range of the rule) against the profile at every mass (the next double above
+    it), with a selection of one narrow mass peak.  Per unit number count: the
+    mass nodes of the two differ by their rounding, which the selection's ramps
+    turn into 4e-14 of the mass weights, alike for every radius.  The sums of
+    the two sides are rounded alike; 2e-14 of each value is ten times the
+    interpolation."""
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+
+    s = cases._module_inputs(dict(mor="lognormal", tab_m=40, tab_z=24, n_q=17, radii=6), 3)
+    lnm, z = np.linspace(28.0, 37.0, 181), np.linspace(0.05, 0.8, 9)
+    S = np.tile((np.abs(lnm - peak) < 0.2).astype(float), (12, 9, 1))
+    got = []
+    for hi in (37.0, np.nextafter(37.0, 40.0)):
+        h = E.SelGL(n_lnm=n_lnm, n_z=19, lnm_low=28.0, lnm_high=hi).build(s["cz"], s["tab"],
+                                                                          (lnm, z, S))
+        got.append(h.shear(s["bins"], s["r"], s["halo"], f_mis=1.0) /
+                   h.weights()["norm"][s["bins"]])
+    assert np.all(got[1] != 0)
+    np.testing.assert_allclose(got[0], got[1], rtol=2e-14)
