@@ -297,3 +297,32 @@ def test_miscentred_profile_nodes_against_every_mass(gpu, n_lnm, peak):
                    h.weights()["norm"][s["bins"]])
     assert np.all(got[1] != 0)
     np.testing.assert_allclose(got[0], got[1], rtol=2e-14)
+
+
+def test_engines_of_different_bin_counts_side_by_side(gpu):
+    """An engine made later, with smaller tiles and tables, takes no shared
+    memory away from the launches of an earlier one."""
+    from y3_cluster_cpp_b200 import engine as E
+    from y3_cluster_cpp_b200 import synthetic
+
+    pts = synthetic.walkers(3, seed=4, densities=(1,))
+    t = pts[0].tables
+
+    def engine(nI, n_z):
+        g = synthetic.grid(1, n_m=40, n_z=n_z, n_t=64, n_o=16, n_zo=8,
+                           lam_edges=np.geomspace(20.0, 200.0, nI + 1))
+        so = synthetic.shear_opts(n_theta=16, n_s=32, n_R=3)
+        so["lob_centers"] = np.geomspace(25.0, 130.0, nI)
+        return E.Engine([g], len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]),
+                        synthetic.plob_baseline(), max_points=3, n_sci=len(t["sci_z"]), shear=so)
+
+    first = engine(8, 128)
+    want = first.eval(pts, E.MIXED, grid_of=lambda p: 0)
+    second = engine(1, 16)
+    second.eval(pts, E.MIXED, grid_of=lambda p: 0)
+    for prec in (E.MIXED, E.FP64):
+        got = first.eval(pts, prec, grid_of=lambda p: 0)
+        for k in ("counts", "shear"):
+            np.testing.assert_allclose(got[k], want[k], rtol=0 if prec == E.MIXED else 1e-4)
+    first.close()
+    second.close()

@@ -744,6 +744,7 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
   cudaGetDevice(&dev);
   int rc = cuda_status(cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, dev),
                        "cudaDeviceGetAttribute");
+  if (!rc) rc = allow_max_smem(bsel_point_kernel);
   if (!rc) rc = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking),
                        "cudaStreamCreate");
   const std::vector<int>& ints = h->gp_bin;
@@ -819,8 +820,6 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
               "(at most 227 KB)", smem);
     return Y3B_ERR_INVALID;
   }
-  Y3B_CUDA(cudaFuncSetAttribute(bsel_point_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
   const double* cd = h->d_const.get();
   const int NL = c.n_lt, ngp = c.n_gp;
   D.lnm_x = cd;

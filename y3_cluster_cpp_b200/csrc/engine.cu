@@ -2278,26 +2278,16 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
   if (!rc) rc = e->d_grids.upload(e->grids.data(), e->grids.size(), e->stream);
   if (!rc) rc = cuda_status(cudaStreamSynchronize(e->stream), "sync");
   if (rc) return fail(rc);
-  Y3B_CUDA(cudaFuncSetAttribute(prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)e->prep_smem));
-  Y3B_CUDA(cudaFuncSetAttribute(yf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)e->yf_smem));
+  if ((rc = allow_max_smem(prep_kernel)) || (rc = allow_max_smem(yf_kernel)) ||
+      (rc = allow_max_smem(direct_main_kernel)) || (rc = allow_max_smem(shear_sum_kernel<true>)) ||
+      (rc = allow_max_smem(shear_sum_kernel<false>)))
+    return fail(rc);
   // Several 256-thread CTAs per SM (three for yf_kernel, the register limit,
   // at ~37 KB each at 256 lnM x 128 z nodes): ask for the largest carveout.
   Y3B_CUDA(cudaFuncSetAttribute(prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 (int)cudaSharedmemCarveoutMaxShared));
   Y3B_CUDA(cudaFuncSetAttribute(yf_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 (int)cudaSharedmemCarveoutMaxShared));
-  if (e->shear_smem) {
-    Y3B_CUDA(cudaFuncSetAttribute(shear_sum_kernel<true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)e->shear_smem));
-    Y3B_CUDA(cudaFuncSetAttribute(shear_sum_kernel<false>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)e->shear_smem));
-  }
-  Y3B_CUDA(cudaFuncSetAttribute(direct_main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)e->direct_smem));
   *out = e;
   return Y3B_OK;
 }

@@ -44,6 +44,20 @@ cuda_status(cudaError_t e, const char* what)
 
 #define Y3B_CUDA(expr) Y3B_TRY(::y3b::cuda_status((expr), #expr))
 
+// Lets launches of a kernel take all of an SM's shared memory.  The limit
+// belongs to the kernel on the device, not to a handle: at one handle's size
+// it would refuse the launches of another handle that needs more.
+template <typename K>
+int
+allow_max_smem(K* kernel)
+{
+  cudaFuncAttributes a;
+  Y3B_CUDA(cudaFuncGetAttributes(&a, kernel));
+  return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          227 * 1024 - (int)a.sharedSizeBytes),
+                     "cudaFuncAttributeMaxDynamicSharedMemorySize");
+}
+
 // Checks that a usable sm_100 device is current.
 int require_device();
 

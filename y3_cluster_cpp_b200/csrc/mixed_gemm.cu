@@ -941,15 +941,6 @@ contract_smem_bytes(const ContractShape& c)
 
 template <int NJ, bool SHEAR>
 static int
-set_attr_nj(size_t smem)
-{
-  Y3B_CUDA(cudaFuncSetAttribute(contract_kernel<NJ, SHEAR>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  return Y3B_OK;
-}
-
-template <int NJ, bool SHEAR>
-static int
 launch_nj(const ContractLaunch& L, size_t smem)
 {
   auto k = contract_kernel<NJ, SHEAR>;
@@ -986,14 +977,15 @@ launch_shear(const ContractLaunch& L, size_t smem)
 int
 contract_prepare(const ContractShape& c)
 {
-  const size_t smem = contract_smem_bytes(c);
-  if (smem == (size_t)-1) {
+  if (contract_smem_bytes(c) == (size_t)-1) {
     set_error("contract: the grids need more shared memory than one CTA has");
     return Y3B_ERR_UNSUPPORTED;
   }
   switch (c.nJ) {
 #define Y3B_ATTR(n) \
-  case n: Y3B_TRY((set_attr_nj<n, false>(smem))); return set_attr_nj<n, true>(smem);
+  case n: \
+    Y3B_TRY(allow_max_smem(contract_kernel<n, false>)); \
+    return allow_max_smem(contract_kernel<n, true>);
     Y3B_ATTR(1) Y3B_ATTR(2) Y3B_ATTR(3) Y3B_ATTR(4) Y3B_ATTR(5) Y3B_ATTR(6) Y3B_ATTR(7)
     Y3B_ATTR(8)
 #undef Y3B_ATTR

@@ -840,9 +840,7 @@ y3b_selgl_build(y3b_selgl* h, const y3b_cosmo* c, const y3b_tables* t,
                     d + o_da, include_sci ? d + o_sz : nullptr,
                     include_sci ? d + o_sv : nullptr};
   const size_t shm = build_smem_bytes(h->cfg.n_z);
-  if (shm > 48 * 1024)
-    Y3B_CUDA(cudaFuncSetAttribute(selgl_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)shm));
+  if (shm > 48 * 1024) Y3B_TRY(allow_max_smem(selgl_build_kernel));
   selgl_build_kernel<<<nb, kBuildThreads, shm, s>>>(
     h->cfg.n_lnm, h->cfg.n_z, h->lnm_x.get(), h->lnm_w.get(), h->z_x.get(), h->z_w.get(),
     h->cfg.lnm_low, h->cfg.lnm_high, *c, td, include_sci, sel->n_lnm, d + o_sl, sel->n_z,
