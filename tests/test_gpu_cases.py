@@ -326,3 +326,11 @@ def test_engines_of_different_bin_counts_side_by_side(gpu):
             np.testing.assert_allclose(got[k], want[k], rtol=0 if prec == E.MIXED else 1e-4)
     first.close()
     second.close()
+
+
+# The masses' factors stand in shared memory 320 at a time: whole tiles, a
+# remainder, several tiles, and more (bin, lambda_true) pairs than threads.
+@pytest.mark.parametrize("n_lnm,n_lt", [(320, 5), (321, 5), (400, 70), (1900, 3)])
+def test_selection_bias_many_masses(gpu, n_lnm, n_lt):
+    _compare(dict(kind="bsel", n=2, n_lt=n_lt, n_zring=4, n_zouter=3, n_lnm=n_lnm, n_theta=3,
+                  n_zt_ref=12), 1e-10)

@@ -267,76 +267,92 @@ bsel_grid_kernel(BselDims D, const double* __restrict__ blocks, double* __restri
 
 // Per (reference z node, sample): the moments of the shifted-Poisson MOR
 // (P_operator::set_sample, p_operator_t.hh:150-219) of every richness bin
-// whose grid points read the node.
+// whose grid points read the node.  The masses' factors stand in shared
+// memory, kMassTile at a time (128 bytes a mass, below 48 KB for any count).
+constexpr int kMassTile = 320;
+
 __global__ void __launch_bounds__(kSampleThreads, 4)
 bsel_sample_kernel(BselDims D, const double* __restrict__ blocks,
                    const unsigned* __restrict__ need, double* __restrict__ mom)
 {
-  extern __shared__ double ssm[];  // n, b [3][n_lnm] | mi, lam [n_lnm] | weights [n_lnm][8]
+  extern __shared__ double ssm[];  // n, b [3][tile] | mi, lam [tile] | weights [tile][8]
   const int iz = blockIdx.x, s = blockIdx.y, tid = threadIdx.x;
-  const int NM = D.n_lnm, NL = D.n_lt;
+  const int NM = D.n_lnm, NL = D.n_lt, NT = min(NM, kMassTile);
   unsigned used = 0;
   for (int bb = 0; bb < 4; ++bb)
     used |= ((need[((size_t)s * 4 + bb) * D.need_words + (iz >> 5)] >> (iz & 31)) & 1u) << bb;
   if (!used) return;
   const double* B = blocks + (size_t)s * D.blk;
   double* n_s = ssm;
-  double* b_s = n_s + 3 * NM;
-  double* mi_s = b_s + 3 * NM;
-  double* lam_s = mi_s + NM;
-  double* wt = lam_s + NM;
+  double* b_s = n_s + 3 * NT;
+  double* mi_s = b_s + 3 * NT;
+  double* lam_s = mi_s + NT;
+  double* wt = lam_s + NT;
   const double z = D.zr[iz];
   const double Mmin = B[7], dM1 = B[8], alpha = B[9], sig_l = B[11];
-  for (int k = tid; k < 7 * NM; k += kSampleThreads) {
-    const int what = k / NM, iM = k - what * NM;
-    const double x = D.lnm_x[iM];
-    if (what < 6) {  // n and b at the nodes iz - 1, iz, iz + 1
-      const double zn = D.zr[min(max(iz + what % 3 - 1, 0), D.n_zr - 1)];
-      if (what < 3)
-        n_s[k] = interp2d_clamp(B + D.o_mh, D.n_hm, B + D.o_hz, D.n_hz, B + D.o_dn, x, zn) *
-                 (B[5] * (x * kLog10e - kHmfPivot) + B[6]);
-      else
-        b_s[k - 3 * NM] =
-          interp2d_clamp(B + D.o_bl, D.n_hl, B + D.o_bz, D.n_bz, B + D.o_bi, x, zn);
-    } else {
-      const double dM = fmax(exp(x) - Mmin, 0.0);
-      const double l_sat = (dM > 0.0 && dM1 > 0.0)
-                             ? pow(dM / dM1, alpha) * pow((1.0 + z) / (1.0 + B[12]), B[10])
-                             : 0.0;
-      const double mi = (l_sat * sig_l) * (l_sat * sig_l);
-      mi_s[iM] = mi;
-      lam_s[iM] = fmax(l_sat + mi, 1.0e-300);
+  auto factors = [&](int m0, int nm_t) {  // of masses m0 .. m0 + nm_t - 1
+    for (int k = tid; k < 7 * nm_t; k += kSampleThreads) {
+      const int what = k / nm_t, iM = k - what * nm_t;
+      const double x = D.lnm_x[m0 + iM];
+      if (what < 6) {  // n and b at the nodes iz - 1, iz, iz + 1
+        const double zn = D.zr[min(max(iz + what % 3 - 1, 0), D.n_zr - 1)];
+        if (what < 3)
+          n_s[what * NT + iM] =
+            interp2d_clamp(B + D.o_mh, D.n_hm, B + D.o_hz, D.n_hz, B + D.o_dn, x, zn) *
+            (B[5] * (x * kLog10e - kHmfPivot) + B[6]);
+        else
+          b_s[(what - 3) * NT + iM] =
+            interp2d_clamp(B + D.o_bl, D.n_hl, B + D.o_bz, D.n_bz, B + D.o_bi, x, zn);
+      } else {
+        const double dM = fmax(exp(x) - Mmin, 0.0);
+        const double l_sat = (dM > 0.0 && dM1 > 0.0)
+                               ? pow(dM / dM1, alpha) * pow((1.0 + z) / (1.0 + B[12]), B[10])
+                               : 0.0;
+        const double mi = (l_sat * sig_l) * (l_sat * sig_l);
+        mi_s[iM] = mi;
+        lam_s[iM] = fmax(l_sat + mi, 1.0e-300);
+      }
     }
-  }
-  __syncthreads();
-  for (int iM = tid; iM < NM; iM += kSampleThreads) {
-    const double w = D.lnm_w[iM];
-    const double nm = w * n_s[iM], n0 = w * n_s[NM + iM], np = w * n_s[2 * NM + iM];
-    const double bm = b_s[iM], b0 = b_s[NM + iM], bp = b_s[2 * NM + iM];
-    double* v = wt + kMoments * iM;
-    v[0] = n0;
-    v[1] = np;
-    v[2] = nm;
-    v[3] = n0 * b0;
-    v[4] = n0 * bp + np * b0;
-    v[5] = np * bp;
-    v[6] = nm * b0 + n0 * bm;
-    v[7] = nm * bm;
-  }
-  __syncthreads();
-  for (int k = tid; k < 4 * NL; k += kSampleThreads) {
-    const int bb = k / NL, il = k - bb * NL;
-    if (!((used >> bb) & 1u)) continue;
-    const double lt = D.lt_x[k];
+    __syncthreads();
+    for (int iM = tid; iM < nm_t; iM += kSampleThreads) {
+      const double w = D.lnm_w[m0 + iM];
+      const double nm = w * n_s[iM], n0 = w * n_s[NT + iM], np = w * n_s[2 * NT + iM];
+      const double bm = b_s[iM], b0 = b_s[NT + iM], bp = b_s[2 * NT + iM];
+      double* v = wt + kMoments * iM;
+      v[0] = n0;
+      v[1] = np;
+      v[2] = nm;
+      v[3] = n0 * b0;
+      v[4] = n0 * bp + np * b0;
+      v[5] = np * bp;
+      v[6] = nm * b0 + n0 * bm;
+      v[7] = nm * bm;
+    }
+    __syncthreads();
+  };
+  if (NM <= kMassTile) factors(0, NM);
+  for (int k0 = 0; k0 < 4 * NL; k0 += kSampleThreads) {
+    const int k = k0 + tid, bb = k / NL, il = k - bb * NL;
+    const bool on = k < 4 * NL && ((used >> bb) & 1u);
+    const double lt = on ? D.lt_x[k] : 0.0;
     double acc[kMoments];
 #pragma unroll
     for (int m = 0; m < kMoments; ++m) acc[m] = 0.0;
+    for (int m0 = 0; m0 < NM; m0 += kMassTile) {
+      const int nm_t = min(kMassTile, NM - m0);
+      if (NM > kMassTile) {
+        __syncthreads();  // the last tile has been read
+        factors(m0, nm_t);
+      }
+      if (!on) continue;
 #pragma unroll 2
-    for (int iM = 0; iM < NM; ++iM) {
-      const double p = shifted_poisson(lt + mi_s[iM], lam_s[iM]);
+      for (int iM = 0; iM < nm_t; ++iM) {
+        const double p = shifted_poisson(lt + mi_s[iM], lam_s[iM]);
 #pragma unroll
-      for (int m = 0; m < kMoments; ++m) acc[m] = fma(wt[kMoments * iM + m], p, acc[m]);
+        for (int m = 0; m < kMoments; ++m) acc[m] = fma(wt[kMoments * iM + m], p, acc[m]);
+      }
     }
+    if (!on) continue;
     double* dst = mom + (size_t)s * D.mom + bb * D.mom_bin + (size_t)iz * kMoments * NL + il;
 #pragma unroll
     for (int m = 0; m < kMoments; ++m) dst[(size_t)m * NL] = acc[m];
@@ -914,7 +930,8 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
       count_launch();
       Y3B_CUDA(cudaGetLastError());
       bsel_sample_kernel<<<dim3(D.n_zr, nk), kSampleThreads,
-                           (8 + kMoments) * sizeof(double) * c.n_lnm, st>>>(D, blocks, need, mom);
+                           (8 + kMoments) * sizeof(double) * std::min(c.n_lnm, kMassTile), st>>>(
+        D, blocks, need, mom);
       count_launch();
       Y3B_CUDA(cudaGetLastError());
       // Few (grid point, sample) pairs: several blocks each, by theta.
