@@ -334,3 +334,10 @@ def test_engines_of_different_bin_counts_side_by_side(gpu):
 def test_selection_bias_many_masses(gpu, n_lnm, n_lt):
     _compare(dict(kind="bsel", n=2, n_lt=n_lt, n_zring=4, n_zouter=3, n_lnm=n_lnm, n_theta=3,
                   n_zt_ref=12), 1e-10)
+
+
+# lambda_true tables that do not fit in shared memory beside the mass sums.
+@pytest.mark.parametrize("n_lt,n_zring,n_zouter", [(4500, 1, 1), (2600, 3, 1)])
+def test_selection_bias_many_richness_nodes(gpu, n_lt, n_zring, n_zouter):
+    _compare(dict(kind="bsel", n=1, n_lt=n_lt, n_zring=n_zring, n_zouter=n_zouter, n_lnm=5,
+                  n_theta=2, n_zt_ref=12), 1e-10)

@@ -91,9 +91,9 @@ struct BselDims {
   int need_words;
   long g_z, g_th, grid;
   // constants (device): lnM nodes / weights, lambda_true nodes / weights /
-  // R_lambda per bin [4][n_lt], reference z grid, photo-z width table,
+  // R_lambda / 1 / (pi R_lambda^2) per bin [4][n_lt], reference z grid, photo-z width table,
   // grid points
-  const double *lnm_x, *lnm_w, *lt_x, *lt_w, *rl, *zr, *zk_z, *zk_s;
+  const double *lnm_x, *lnm_w, *lt_x, *lt_w, *rl, *ia, *zr, *zk_z, *zk_s;
   const double *gl_out, *gl_ring, *gl_th, *gl_th1, *gl_th2;  // nodes | weights on [-1, 1]
   const double *gp_zob, *gp_zfg, *gp_zbg;
   const int* gp_bin;
@@ -359,14 +359,14 @@ bsel_sample_kernel(BselDims D, const double* __restrict__ blocks,
   }
 }
 
-// Shared-memory doubles of bsel_point_kernel for the shapes in D (all theta
-// nodes in one block).
-__host__ __device__ inline long
-point_smem_doubles(const BselDims& D)
+// Shared-memory doubles of bsel_point_kernel<LT> for the shapes in D (all
+// theta nodes in one block).
+inline long
+point_smem_doubles(const BselDims& D, bool lt)
 {
   const long NZ = D.nz_max, NT = D.n_th;
-  return 2L * D.n_lt * NZ + 2L * D.n_lt + 3 * NZ + (NZ & 1) + NT * NZ + (NT * NZ + 7) / 8 +
-         2 * (NT + kPointWarps);
+  return 2L * D.n_lt * NZ + (lt ? 2L * D.n_lt : 0L) + 3 * NZ + (NZ & 1) + NT * NZ +
+         (NT * NZ + 7) / 8 + 2 * (NT + kPointWarps);
 }
 
 // One block per (grid point, sample, group of theta nodes): the mass sums
@@ -377,6 +377,9 @@ point_smem_doubles(const BselDims& D)
 // fastest, so that a warp's lanes share the overlap's branch; a run's sums are
 // written per theta and added in the order of the warps.  Bound by the FP64
 // units (the overlap's two angles and square root).
+// LT: the lambda_true tables in shared memory too; where they do not fit
+// beside the mass sums (hundreds of nodes) they are read from global memory.
+template <bool LT>
 __global__ void __launch_bounds__(kPointThreads, 2)
 bsel_point_kernel(BselDims D, const double* __restrict__ blocks,
                   const double* __restrict__ grids, const double* __restrict__ mom,
@@ -400,18 +403,18 @@ bsel_point_kernel(BselDims D, const double* __restrict__ blocks,
   const int Nz = (int)G[2], n_pair = Nz * NL;
   double* WP = sm;                    // [NL][Nz]
   double* WI = WP + (size_t)NL * NZ;
-  double* rl = WI + (size_t)NL * NZ;  // [NL] R_lambda(lambda_true)
-  double* ia = rl + NL;               // [NL] 1 / (pi R_lambda^2)
-  double* thx = ia + NL;              // [Nz]
+  double* lt_s = WI + (size_t)NL * NZ;
+  const double* rl = LT ? lt_s : D.rl + bin * NL;       // [NL] R_lambda(lambda_true)
+  const double* ia = LT ? lt_s + NL : D.ia + bin * NL;  // [NL] 1 / (pi R_lambda^2)
+  double* thx = lt_s + (LT ? 2 * NL : 0);               // [Nz]
   double* ic1 = thx + NZ;             // [Nz] (1 + z) / chi
   double* c2 = ic1 + NZ;              // [Nz] its inverse square
   double2* red = reinterpret_cast<double2*>(c2 + NZ + (NZ & 1));
   double* xi = reinterpret_cast<double*>(red + nt + kPointWarps);  // [nt][Nz]
   uint8_t* on = reinterpret_cast<uint8_t*>(xi + (size_t)nt * NZ);  // [nt][Nz]
-  for (int il = tid; il < NL; il += kPointThreads) {
-    const double r = D.rl[bin * NL + il];
-    rl[il] = r;
-    ia[il] = 1.0 / (kPi * r * r);
+  for (int il = tid; LT && il < NL; il += kPointThreads) {
+    lt_s[il] = D.rl[bin * NL + il];
+    lt_s[NL + il] = D.ia[bin * NL + il];
   }
   for (int iz = tid; iz < Nz; iz += kPointThreads) {
     const double c = Z[5 * NZ + iz];
@@ -562,7 +565,7 @@ struct y3b_bsel {
   y3b_bsel_config cfg;
   std::vector<double> gp_zlo, gp_zhi, gp_zob, gp_zfg, gp_zbg;
   std::vector<int> gp_bin;
-  std::vector<double> lnm_x, lnm_w, lt_x, lt_w, rl, zr;  // lt_x, lt_w, rl: [4][n_lt]
+  std::vector<double> lnm_x, lnm_w, lt_x, lt_w, rl, ia, zr;  // lt_x, lt_w, rl, ia: [4][n_lt]
   int n_sm = 1;
   int max_samples = 64;
   y3b::DevBuf<double> d_const, d_blocks, d_work, d_out;
@@ -731,7 +734,9 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
     for (int il = 0; il < cfg->n_lt; ++il) {
       h->lt_x.push_back(x[il]);
       h->lt_w.push_back(w[il]);
-      h->rl.push_back(std::pow(x[il] / 100.0, 0.2));
+      const double r = std::pow(x[il] / 100.0, 0.2);
+      h->rl.push_back(r);
+      h->ia.push_back(1.0 / (kPi * r * r));
     }
   }
   const double dz_ref = (cfg->zt_ref_high - cfg->zt_ref_low) / (cfg->n_zt_ref - 1);
@@ -744,6 +749,7 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
   put(h->lt_x.data(), h->lt_x.size());
   put(h->lt_w.data(), h->lt_w.size());
   put(h->rl.data(), h->rl.size());
+  put(h->ia.data(), h->ia.size());
   put(h->zr.data(), h->zr.size());
   put(kZKernelZ, kZKernelNodes);
   put(kZKernelSigma, kZKernelNodes);
@@ -760,7 +766,8 @@ y3b_bsel_create(const y3b_bsel_config* cfg, y3b_bsel** out)
   cudaGetDevice(&dev);
   int rc = cuda_status(cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, dev),
                        "cudaDeviceGetAttribute");
-  if (!rc) rc = allow_max_smem(bsel_point_kernel);
+  if (!rc) rc = allow_max_smem(bsel_point_kernel<true>);
+  if (!rc) rc = allow_max_smem(bsel_point_kernel<false>);
   if (!rc) rc = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking),
                        "cudaStreamCreate");
   const std::vector<int>& ints = h->gp_bin;
@@ -830,7 +837,9 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
   }
   BselDims D;
   layout(h, s0, D);
-  const size_t smem = (size_t)point_smem_doubles(D) * sizeof(double);
+  size_t smem = (size_t)point_smem_doubles(D, true) * sizeof(double);
+  const bool lt_smem = smem <= 227 * 1024;
+  if (!lt_smem) smem = (size_t)point_smem_doubles(D, false) * sizeof(double);
   if (smem > 227 * 1024) {
     set_error("y3b_bsel_eval: node counts need %zu bytes of shared memory per grid point "
               "(at most 227 KB)", smem);
@@ -843,7 +852,8 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
   D.lt_x = D.lnm_w + c.n_lnm;
   D.lt_w = D.lt_x + 4 * NL;
   D.rl = D.lt_w + 4 * NL;
-  D.zr = D.rl + 4 * NL;
+  D.ia = D.rl + 4 * NL;
+  D.zr = D.ia + 4 * NL;
   D.zk_z = D.zr + c.n_zt_ref;
   D.zk_s = D.zk_z + kZKernelNodes;
   D.gp_zob = D.zk_s + kZKernelNodes;
@@ -936,8 +946,8 @@ y3b_bsel_eval(y3b_bsel* h, int n_samples, const y3b_bsel_sample* S, double* out)
       Y3B_CUDA(cudaGetLastError());
       // Few (grid point, sample) pairs: several blocks each, by theta.
       const int split = std::max(1, std::min(c.n_theta, 2 * h->n_sm / std::max(1, ngp * nk)));
-      bsel_point_kernel<<<dim3(ngp, nk, split), kPointThreads, smem, st>>>(D, blocks, grids, mom,
-                                                                          part);
+      auto point = lt_smem ? bsel_point_kernel<true> : bsel_point_kernel<false>;
+      point<<<dim3(ngp, nk, split), kPointThreads, smem, st>>>(D, blocks, grids, mom, part);
       count_launch();
       Y3B_CUDA(cudaGetLastError());
       bsel_sum_kernel<<<(ngp * nk + 127) / 128, 128, 0, st>>>(D, grids, part, ngp * nk, o);
