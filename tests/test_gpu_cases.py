@@ -341,3 +341,25 @@ def test_selection_bias_many_masses(gpu, n_lnm, n_lt):
 def test_selection_bias_many_richness_nodes(gpu, n_lt, n_zring, n_zouter):
     _compare(dict(kind="bsel", n=1, n_lt=n_lt, n_zring=n_zring, n_zouter=n_zouter, n_lnm=5,
                   n_theta=2, n_zt_ref=12), 1e-10)
+
+
+def test_selection_bias_pieces_of_a_batch(gpu):
+    """A batch is evaluated in pieces of a chunk: two unequal pieces, chunks of
+    several pieces with a short last chunk, then smaller and larger batches on
+    the same handles (reused work blocks).  With one theta node a grid point's
+    terms are dealt to the warps alike in every batch: bit for bit the samples
+    one at a time."""
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+
+    nodes = dict(n_lt=5, n_zring=4, n_zouter=3, n_lnm=6, n_theta=1, n_zt_ref=12)
+    state = cases.prepare(dict(kind="bsel", n=130, **nodes), 7)
+    samples, whole = state["samples"], state["h"]
+    want = np.concatenate([whole.eval([s]) for s in samples])
+    grid = dict(zo_low=np.repeat(cases.ZOB_EDGES[:3], 4), zo_high=np.repeat(cases.ZOB_EDGES[1:], 4),
+                lambda_bin=np.tile(np.arange(4), 3))
+    chunked = E.BselMarg(grid, *cases.LNM, max_samples=60, **nodes)
+    for h in (whole, chunked):
+        for a, b in ((0, 53), (0, 130), (53, 60), (3, 128), (129, 130)):
+            np.testing.assert_array_equal(h.eval(samples[a:b]), want[a:b])
+    chunked.close()
