@@ -39,6 +39,15 @@ def _address(a):
         return a.ctypes.data
 
 
+def _pack_format(t):
+    """struct format characters of a ctypes type, structures flattened."""
+    if issubclass(t, C.Structure):
+        return "".join(_pack_format(f) for _, f in t._fields_)
+    if issubclass(t, C.Array):
+        return t._length_ * _pack_format(t._type_)
+    return "P" if issubclass(t, C._Pointer) else t._type_
+
+
 def _plob(z, coef, keep):
     z, coef = f64(z), f64(coef)
     keep += [z, coef]
@@ -285,8 +294,8 @@ class BselMarg:
 
     __del__ = close
 
-    # y3b_bsel_sample after its cosmology, as _RECORD packs it.
-    _RECORD = struct.Struct("@iPiPPiPPiPPP2i3P2i3P6d")
+    # y3b_bsel_sample after its cosmology.
+    _RECORD = struct.Struct("@" + "".join(_pack_format(f) for _, f in A.BselSample._fields_[1:]))
 
     def eval(self, samples):
         n = len(samples)
