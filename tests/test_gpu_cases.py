@@ -363,3 +363,53 @@ def test_selection_bias_pieces_of_a_batch(gpu):
         for a, b in ((0, 53), (0, 130), (53, 60), (3, 128), (129, 130)):
             np.testing.assert_array_equal(h.eval(samples[a:b]), want[a:b])
     chunked.close()
+
+
+@pytest.mark.parametrize("c_slope,R_lo,R_hi,rtol", [(-0.1, 0.1, 30.0, 1e-14),
+                                                    (-0.1, 0.1, 1e6, 2e-14),
+                                                    (-1.5, 10.0, 1e8, 2e-13)])
+def test_fp64_shear_profile_interpolation(gpu, c_slope, R_lo, R_hi, rtol):
+    """The centred profile (f_mis = 0) of the FP64 form over the radii's usual
+    range, over one that makes the table three times as coarse as that, and
+    past the spacing that is interpolated, against 40-digit values summed with
+    the engine's own mass weights (Sigma_crit^-1 = 1).  The closed form (at x
+    above 0.1, where it keeps its digits) and the sum of 33 positive terms leave
+    about 5e-15; the last case's concentrations near 0.03 cost its normalisation
+    two digits more."""
+    import mpmath as mp
+
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+    from y3_cluster_cpp_b200 import synthetic
+
+    p = synthetic.fiducial(1)
+    p.tables["sci_val"] = np.ones_like(p.tables["sci_val"])
+    g = synthetic.grid(1, n_m=33, n_z=16, n_t=40, n_o=16, n_zo=8)
+    so = synthetic.shear_opts(n_theta=16, n_s=32, n_R=7)
+    so.update(R=np.geomspace(R_lo, R_hi, 7), c_slope=c_slope, f_mis=0.0)
+    t = p.tables
+    eng = E.Engine([g], len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]),
+                   synthetic.plob_baseline(), max_points=1, n_sci=len(t["sci_z"]), shear=so)
+    out = eng.eval([p], E.FP64, grid_of=lambda _: 0, weights=True)
+    eng.close()
+    lnM, wm = (v.cpu().numpy() for v in cases._gl(g["lnm_lo"], g["lnm_hi"], 33))
+
+    def profile(R, x):
+        M = mp.exp(mp.mpf(x))
+        c = so["c0"] * (M / so["c_pivot"]) ** mp.mpf(c_slope)
+        rho = mp.mpf(cases.RHO_CRIT) * mp.mpf(p.om)
+        rs = mp.cbrt(3 * M / (800 * mp.pi * rho)) / c
+        delta = mp.mpf(200) / 3 * c ** 3 / (mp.log(1 + c) - c / (1 + c))
+        q = mp.mpf(R) / rs
+        v = 1 - q * q
+        y = mp.sqrt(abs(v))
+        gq = mp.atan(y) / y if q > 1 else mp.log((1 + y) / q) / y
+        return 2 * rs * delta * rho * mp.mpf("1e-12") * (2 * (gq + mp.log(q / 2)) / q ** 2
+                                                         - (gq - 1) / v)
+
+    with mp.workdps(40):
+        prof = [[profile(R, x) for x in lnM] for R in so["R"]]
+        want = np.array([[float(sum(mp.mpf(w) * mp.mpf(k) * f for w, k, f in
+                                    zip(out["W"][0, b], wm, row))) for row in prof]
+                         for b in range(12)])
+    np.testing.assert_allclose(out["shear"][0], want, rtol=rtol)

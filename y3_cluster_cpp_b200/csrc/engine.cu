@@ -1291,7 +1291,8 @@ direct_wreduce_kernel(const GridDev* grids, const PointDev* pts, const double* s
 // + f DSigma_mis(R / r_s, tau R_lambda(lam_i) / r_s)], c(M) = c0 (M/Mp)^s,
 // rho = Omega_m rho_crit, by direct quadrature: the FP64 form's points whose
 // x = R / r_s leaves the engine's profile table (Omega_m outside 0.01 to 1),
-// listed by shear_tab64_kernel.  One warp per (point, i, R, k).
+// or whose table is too coarse, listed by shear_tab64_kernel.  One warp per
+// (point, i, R, k).
 __global__ void __launch_bounds__(128)
 shear_phi_kernel(const GridDev* grids, const PointDev* pts, const int* list, const int* n_list,
                  int w_stride, ShearDev sh, MisQuad quad, double* Phi, int nI_max)
@@ -1330,11 +1331,16 @@ shear_phi_kernel(const GridDev* grids, const PointDev* pts, const int* list, con
 // alone: tabulated once per engine in FP64 at kMisNx nodes per (i, R) pair
 // (the direct quadrature).  The mixed form reads it with 4-point Lagrange
 // interpolation in u (relative error ~1e-8 at this spacing), the FP64 form
-// with 6 points: DeltaSigma is analytic for |Im u| < pi, so at the spacing
-// du ~ 0.006 their error is about (5/2 3/2 1/2)^2 (du / pi)^6 ~ 1e-16.  One
-// more row after the (i, R) pairs holds the centred DeltaSigma_NFW(x) on the
-// same nodes, so both profiles are read with the same weights.
+// with 8 points: DeltaSigma is analytic for |Im u| < pi, and against 40-digit
+// values at x from e^-8 to e^8 eight points err by at most 7e-17 of it at a
+// spacing du of 0.0125, 3e-15 at 0.02 (six points: 3e-15 at 0.005, 7e-13 at
+// 0.0125).  du is 0.005 for radii from 0.1 to 30; beyond kMaxDu64 (radii and
+// masses over more than 25 e-folds of x) the FP64 form takes the direct
+// quadrature.  One more row after the (i, R) pairs holds the centred
+// DeltaSigma_NFW(x) on the same nodes, so both profiles are read with the same
+// weights.
 constexpr int kMisNx = 2048;
+constexpr double kMaxDu64 = 0.0125;
 
 // The miscentred rows come from launch_mis_pairs, the centred one from here.
 __global__ void __launch_bounds__(128)
@@ -1512,12 +1518,12 @@ shear_tab64_kernel(const GridDev* grids, const PointDev* pts, int n_points, int 
   const double rho = kRhoCrit * pt.om;
   auto conc = [&](double lnM) { return sh.c0 * pow(exp(lnM) / sh.c_pivot, sh.c_slope); };
   if (k == 0 && iR == 0) {
-    bool in = true;
+    bool in = inv_du >= 1.0 / kMaxDu64;
     for (int e = 0; e < 2; ++e) {
       const double lnM = G.xm[e ? G.n_m - 1 : 0], l = log(nfw_rs(lnM, conc(lnM), rho));
       for (int r = 0; r < sh.n_R; ++r) {
         const double tt = (sh.lnR[r] - l - u0) * inv_du;
-        in &= tt >= 3.0 && tt <= kMisNx - 5.0;
+        in &= tt >= 4.0 && tt <= kMisNx - 6.0;
       }
     }
     if (!in) list[atomicAdd(n_list, 1)] = p;
@@ -1525,18 +1531,28 @@ shear_tab64_kernel(const GridDev* grids, const PointDev* pts, int n_points, int 
   const double lnM = G.xm[k], c = conc(lnM);
   const double norm = nfw_norm(lnM, c, rho);
   const double tt = (sh.lnR[iR] - log(nfw_rs(lnM, c, rho)) - u0) * inv_du;
-  const int j = (int)fmin(fmax(floor(tt), 2.0), kMisNx - 4.0);
-  // Lagrange weights of the nodes j - 2 .. j + 3 at f = tt - j.
+  const int j = (int)fmin(fmax(floor(tt), 3.0), kMisNx - 5.0);
+  // Lagrange weights of the nodes j - 3 .. j + 4 at f = tt - j: the products
+  // of the other nodes' distances over prod_{m != k} (k - m).
+  constexpr int kN = 8;
+  constexpr double kDen[kN] = {-5040.0, 720.0, -240.0, 144.0, -144.0, 240.0, -720.0, 5040.0};
   const double f = tt - j;
-  const double a = f + 2.0, b = f + 1.0, d = f - 1.0, e = f - 2.0, g = f - 3.0;
-  const double l[6] = {-b * f * d * e * g / 120.0, a * f * d * e * g / 24.0,
-                       -a * b * d * e * g / 12.0,  a * b * f * e * g / 12.0,
-                       -a * b * f * d * g / 24.0,  a * b * f * d * e / 120.0};
+  double l[kN], left = 1.0, right = 1.0;
+#pragma unroll
+  for (int m = 0; m < kN; ++m) {
+    l[m] = left / kDen[m];
+    left *= f - (m - 3);
+  }
+#pragma unroll
+  for (int m = kN - 1; m >= 0; --m) {
+    l[m] *= right;
+    right *= f - (m - 3);
+  }
   auto read = [&](const double* row) {
-    const double* y = row + j - 2;
+    const double* y = row + j - 3;
     double v = 0.0;
 #pragma unroll
-    for (int m = 0; m < 6; ++m) v += l[m] * __ldg(y + m);
+    for (int m = 0; m < kN; ++m) v += l[m] * __ldg(y + m);
     return v;
   };
   const double cen = (1.0 - sh.f_mis) * read(tab + (size_t)nI_max * sh.n_R * kMisNx);
