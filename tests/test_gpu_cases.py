@@ -413,3 +413,62 @@ def test_fp64_shear_profile_interpolation(gpu, c_slope, R_lo, R_hi, rtol):
                                     zip(out["W"][0, b], wm, row))) for row in prof]
                          for b in range(12)])
     np.testing.assert_allclose(out["shear"][0], want, rtol=rtol)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_fp64_product_against_direct_sum(gpu, seed):
+    """The FP64 form's matrix product, where its bounds admit a point, against
+    the direct sum (an engine whose memory budget leaves the product no
+    workspace), over node counts, bin layouts, scatters from 0.03 to 0.6 and
+    mass-richness relations that leave bins out of reach: the direct sum's
+    rounding of mu leaves 1e-14 of a cell, 2e-14 of a count."""
+    import re
+
+    from y3_cluster_cpp_b200 import _capi, prj_params, synthetic
+    from y3_cluster_cpp_b200 import engine as E
+
+    r = np.random.default_rng(seed)
+    g = synthetic.grid(1, n_m=int(r.integers(2, 200)), n_z=16 * int(r.integers(1, 5)),
+                       n_t=int(r.integers(20, 260)), n_o=16, n_zo=8,
+                       lam_edges=np.geomspace(10, 200, int(r.integers(2, 7))),
+                       zob_edges=np.linspace(0.2, 0.65, int(r.integers(2, 6))))
+    plob = synthetic.plob_baseline() if seed % 2 else prj_params.default_table()
+    pts = [synthetic.fiducial(1) for _ in range(10)]
+    for p in pts:
+        p.sigma = float(np.exp(r.uniform(np.log(0.03), np.log(0.6))))
+        p.A, p.B, p.C = r.uniform(-1, 5), r.uniform(0.3, 1.5), r.uniform(-1, 1.5)
+    t = pts[0].tables
+
+    def engine(budget):
+        return E.Engine([g], len(t["hmf_m_h"]), len(t["hmf_z"]), len(t["dist_z"]), plob,
+                        max_points=10, n_sci=len(t["sci_z"]), hbm_budget=budget)
+
+    with pytest.raises(_capi.Y3BError) as err:
+        engine(1)
+    direct = engine(int(re.search(r"(\d+) bytes for", str(err.value)).group(1)))
+    product = engine(0)
+    want = direct.eval(pts, E.FP64, grid_of=lambda _: 0)["counts"]
+    got = product.eval(pts, E.FP64, grid_of=lambda _: 0)["counts"]
+    assert np.all(want > 0)
+    np.testing.assert_allclose(got, want, rtol=2e-14)
+    direct.close()
+    product.close()
+
+
+@pytest.mark.parametrize("edges", [(20, 30, 45, 60, 200), (5, 10, 15, 20, 25, 30, 40, 60, 100),
+                                   (5, 10, 15, 20, 25, 30, 40, 60, 100, 200)])
+def test_selection_bins_in_and_out_of_order(gpu, edges):
+    """Bins that follow one another (at most nine edges) take their CDF
+    differences from registers, others from arrays: the same table, by a few
+    roundings of its largest value, from the bins in reverse."""
+    from perf import cases
+    from y3_cluster_cpp_b200 import engine as E
+
+    s = cases._module_inputs(dict(mor="hod", tab_m=20, tab_z=9, n_q=17, radii=2), 3)
+    e = np.array(edges, dtype=float)
+    bins = dict(lam_min=e[:-1], lam_max=e[1:], zob_min=np.full(len(e) - 1, 0.2),
+                zob_max=np.full(len(e) - 1, 0.35), sigma_z=np.full(len(e) - 1, 0.01))
+    a = E.sel_function(dict(s["cfg"], **bins), s["kind"], s["mor"], *s["plob"])[2]
+    b = E.sel_function(dict(s["cfg"], **{k: v[::-1].copy() for k, v in bins.items()}), s["kind"],
+                       s["mor"], *s["plob"])[2]
+    np.testing.assert_allclose(a[::-1], b, rtol=0, atol=1e-15 * a.max())
