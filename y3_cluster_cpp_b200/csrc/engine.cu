@@ -314,7 +314,8 @@ prep_kernel(PrepArgs a)
     // point's lnM tiles): start bringing it into L2 now.
     if (tid == 7 && a.mixed) {
       const size_t n_dn = (size_t)n_hz * n_hm;
-      const uint32_t hb = (uint32_t)(L.hmf_f32 ? ((n_dn + 1) / 2 + 1) / 2 * 16 : (n_dn * 8 + 15) & ~size_t(15));
+      const uint32_t hb =
+        (uint32_t)(L.hmf_f32 ? ((n_dn + 1) / 2 + 1) / 2 * 16 : (n_dn * 8 + 15) & ~size_t(15));
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + L.off[2]), "r"(hb)
                    : "memory");
     }
@@ -452,7 +453,8 @@ prep_kernel(PrepArgs a)
       const int warp = tid >> 5, lane = tid & 31, nw = kPrepThreads / 32;
       const int x0 = k_x[0], x1 = k_x[n_m - 1] + 1, y0 = q_y[0], y1 = q_y[n_z - 1] + 1;
       for (int y = warp; y < n_hz; y += 2 * nw) {  // two rows, 128 columns at a time
-        const bool two = y + nw < n_hz, in0 = y >= y0 && y <= y1, in1 = y + nw >= y0 && y + nw <= y1;
+        const bool two = y + nw < n_hz;
+        const bool in0 = y >= y0 && y <= y1, in1 = y + nw >= y0 && y + nw <= y1;
         const double* r0 = dn + (size_t)y * n_hm;
         const double* r1 = r0 + (two ? (size_t)nw * n_hm : 0);
         for (int xb = lane; xb < n_hm; xb += 128) {
@@ -1118,7 +1120,8 @@ yf_kernel(PrepArgs a)
               for (int j = 0; j < J; ++j) R0[j] = R1[j];
             } else {
 #pragma unroll
-              for (int j = 0; j < J; ++j) R0[j] = hmf_row(h1 - n_hm, rx_s, rt_s, rn_s, lane + 32 * j);
+              for (int j = 0; j < J; ++j)
+                R0[j] = hmf_row(h1 - n_hm, rx_s, rt_s, rn_s, lane + 32 * j);
             }
 #pragma unroll
             for (int j = 0; j < J; ++j) {
@@ -1379,9 +1382,9 @@ shear_mass_kernel(const GridDev* grids, const PointDev* pts, int n_points, int w
 // writing [point][bin][R][k] and one summing it, 2048 points at 64 masses and
 // 15 radii took 53 + 75 us; here 51 us, about half of it the shared-memory
 // wavefronts of the table reads.  Two blocks of 256 threads an SM: with more
-// warps the sixteen sums spill (384 threads 61 us, 512 threads 75 us).  A point whose x = R / r_s falls outside the table
-// reports a domain error (it covers Omega_m from 0.01 to 1 over the engine's
-// masses and radii).
+// warps the sixteen sums spill (384 threads 61 us, 512 threads 75 us).  A point
+// whose x = R / r_s falls outside the table reports a domain error (it covers
+// Omega_m from 0.01 to 1 over the engine's masses and radii).
 // FULL: whole passes of kShI x kShJ bins (the wall grids of the configs), so
 // no bin is tested.
 constexpr int kShThreads = 256;
@@ -2295,8 +2298,10 @@ y3b_engine_create(const y3b_grid* grids, int n_grids, const y3b_engine_config* c
   if (!rc) rc = cuda_status(cudaStreamSynchronize(e->stream), "sync");
   if (rc) return fail(rc);
   if ((rc = allow_max_smem(prep_kernel)) || (rc = allow_max_smem(yf_kernel)) ||
-      (rc = allow_max_smem(direct_main_kernel)) || (rc = allow_max_smem(shear_sum_kernel<true>)) ||
-      (rc = allow_max_smem(shear_sum_kernel<false>)))
+      (rc = allow_max_smem(direct_main_kernel)))
+    return fail(rc);
+  if (cfg->with_shear && ((rc = allow_max_smem(shear_sum_kernel<true>)) ||
+                          (rc = allow_max_smem(shear_sum_kernel<false>))))
     return fail(rc);
   // Several 256-thread CTAs per SM (three for yf_kernel, the register limit,
   // at ~37 KB each at 256 lnM x 128 z nodes): ask for the largest carveout.
@@ -2479,7 +2484,8 @@ enqueue(y3b_engine* e, int prec, int n, const PointDev* d_pts, const double* d_t
                                                                        : shear_sum_kernel<false>;
       kernel<<<dim3(groups, e->shear.n_R), kShThreads, e->shear_smem, s>>>(
         e->d_grids.get(), (int)e->grids.size(), e->nI_max, e->grids[0].nJ, d_pts, n, e->w_stride,
-        e->shear, e->mis_tab.get(), e->mis_u0, 1.0 / e->mis_du, Phi, Wg, e->nB_max, d_shear, grid_mask, e->status.get());
+        e->shear, e->mis_tab.get(), e->mis_u0, 1.0 / e->mis_du, Phi, Wg, e->nB_max, d_shear,
+        grid_mask, e->status.get());
     }
     count_launch();
     Y3B_CUDA(cudaGetLastError());
@@ -2712,8 +2718,6 @@ y3b_engine_eval(y3b_engine* e, int precision, int n, const y3b_point* pts,
   // compute stream, so they share the per-point scratch; their weights and
   // outputs land at their own offsets.
   cudaStream_t s = e->stream, xs = e->xstream;
-  // About 256 points a chunk: the copies are the long pole, and only the
-  // last chunk's kernels run after them.
   // Chunks of about 12.5 MB of host tables (at least 256 points, at most
   // eight): the copy of the next chunk then outlasts the evaluation of the
   // current one, whose fixed cost grows relative to its work as chunks

@@ -193,9 +193,8 @@ f64_gemm_kernel(F64Launch L)
 #pragma unroll
       for (int u = 0; u < kF64Chunk * kCols / 128; ++u) {
         const int e = tid + 128 * u, t = t0 + e / kCols, q = e % kCols;
-        bv[u] = t < n_t && q < nc
-                  ? __ldg(ws + w.g + (size_t)t * n_z + q0 + q) * __ldg(UK + (size_t)t * n_z + q0 + q)
-                  : 0.0;
+        const size_t at = (size_t)t * n_z + q0 + q;
+        bv[u] = t < n_t && q < nc ? __ldg(ws + w.g + at) * __ldg(UK + at) : 0.0;
       }
     };
     auto store_B = [&](int buf) {

@@ -443,8 +443,8 @@ tile_plan_kernel(const GridDev* __restrict__ grids, int n_grids, int grid_mask,
 // j+1.  Roles: warp 0 issues the MMAs; warps 1-16 generate A into an
 // n_stages-deep shared-memory ring (full/empty mbarriers, empty signalled by
 // tcgen05.commit) from the factor vectors that warp 25 stages; warp 26 streams
-// the F blocks of yf_kernel into their own ring; warps 17-24 read TMEM, apply Y(k,q) and the z-bin weights and write
-// W_ij(k) in FP64.  The tile's block of Y (n_z rows of 128 lnM values,
+// the F blocks of yf_kernel into their own ring; warps 17-24 read TMEM, apply
+// Y(k,q) and the z-bin weights and write W_ij(k) in FP64.  The tile's block of Y (n_z rows of 128 lnM values,
 // contiguous in the tile-blocked layout) is brought into shared memory by one
 // bulk async copy issued while the tile's MMAs run.
 template <int NJ, bool SHEAR>

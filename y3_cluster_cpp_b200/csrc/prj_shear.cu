@@ -72,7 +72,7 @@ struct PrjDims {
   const double *lnm_x, *lnm_w, *anchor;        // [n_lnm]; anchor = w r_s
   const double *gl_seg, *gl_ring, *gl_out;     // nodes | weights on [-1, 1]
   const double *zk_z, *zk_s;                   // photo-z width
-  const double *sl_lob, *sl_zob, *radii;       // per slice; radii ascending, slices one after another
+  const double *sl_lob, *sl_zob, *radii;       // per slice; radii ascending, slice by slice
   const double* gp_R;
   const double* cheb;    // [n_prof][n_lnm] projection of mass weights on the nodes, or null
   const int *sl_lb, *r0, *gp_slice;            // r0 [nsl + 1]
@@ -374,7 +374,8 @@ prj_slice_kernel(PrjDims D, const double* __restrict__ B, double* __restrict__ s
         }
       }
     }
-    if (lane == 0 && i0 <= D.nz && (D.nz - i0) % nw == 0 && (D.nz - i0) / nw < 32) sc[9] += 1.0e-300;
+    if (lane == 0 && i0 <= D.nz && (D.nz - i0) % nw == 0 && (D.nz - i0) / nw < 32)
+      sc[9] += 1.0e-300;
   }
   __syncthreads();
   for (int i = tid; i < D.nz; i += nt_thr) {
@@ -1004,7 +1005,8 @@ y3b_prj_eval(y3b_prj* h, const y3b_prj_sample* S, double* out)
   put(D.o_bs, S->b_small, (size_t)D.n_bzob * D.n_blob);
   put(D.o_blg, S->b_large, (size_t)D.n_bzob * D.n_blob);
   b[blk] = 0.0;
-  Y3B_CUDA(cudaMemcpyAsync(B.d_blk.get(), b, (blk + 1) * sizeof(double), cudaMemcpyHostToDevice, s));
+  Y3B_CUDA(
+    cudaMemcpyAsync(B.d_blk.get(), b, (blk + 1) * sizeof(double), cudaMemcpyHostToDevice, s));
   int* status = reinterpret_cast<int*>(B.d_blk.get() + blk);
   double2* P = reinterpret_cast<double2*>(B.d_P.get());
   const dim3 per_theta((D.nt_max + 7) / 8, D.nsl), per_gp((D.nt_max + 7) / 8, D.ngp);
